@@ -354,7 +354,7 @@ void init_dense(py::module& m) {
     TORCH_CHECK(rc == 0, "ragged_attention_fwd failed (code ", rc, ")");
     return std::make_tuple(out, lse);
   });
-  // Backward of the above: returns dqkv fp32 [T, 3 * H * 64].
+  // Backward of the above: returns dqkv bf16 [T, 3 * H * 64].
   m.def("ragged_attention_bwd", [](const Tensor& qkv, const Tensor& out, const Tensor& d_out, const Tensor& lse, const Tensor& offsets,
                                    int64_t H, int64_t max_len, double scale) {
     TORCH_CHECK(qkv.is_cuda() && qkv.scalar_type() == torch::kBFloat16 && qkv.is_contiguous() && qkv.size(1) == 3 * H * 64);
@@ -363,12 +363,16 @@ void init_dense(py::module& m) {
     TORCH_CHECK(lse.scalar_type() == torch::kFloat32 && lse.is_contiguous() && lse.numel() == qkv.size(0) * H);
     c10::cuda::CUDAGuard g(qkv.device());
     const int64_t T = qkv.size(0), B = offsets.numel() - 1;
-    auto dqkv = torch::zeros({T, 3 * H * 64}, qkv.options().dtype(torch::kFloat32));
-    auto delta = torch::empty({T, H}, dqkv.options());
-    const int rc = rb_ragged_attention_bwd(qkv.data_ptr(), out.data_ptr(), d_out.data_ptr(), lse.data_ptr<float>(), delta.data_ptr<float>(),
+    if (T == 0 || B <= 0 || H <= 0 || max_len <= 0) return torch::zeros({T, 3 * H * 64}, qkv.options());
+    auto f32 = qkv.options().dtype(torch::kFloat32);
+    auto dqkv = torch::empty({T, 3 * H * 64}, qkv.options());
+    auto scratch = torch::empty({T * H + 1}, f32);
+    Tensor dq_acc;
+    if (max_len > 128) dq_acc = torch::zeros({T, H * 64}, f32);
+    const int rc = rb_ragged_attention_bwd(qkv.data_ptr(), out.data_ptr(), d_out.data_ptr(), lse.data_ptr<float>(), scratch.data_ptr<float>(),
                                            offsets.data_ptr<int32_t>(), T, (int)B, (int)H, (int)max_len, (float)scale,
-                                           dqkv.data_ptr<float>(), status_word(qkv.device()).data_ptr<int64_t>(),
-                                           at::cuda::getCurrentCUDAStream());
+                                           dq_acc.defined() ? dq_acc.data_ptr<float>() : nullptr, dqkv.data_ptr(),
+                                           status_word(qkv.device()).data_ptr<int64_t>(), at::cuda::getCurrentCUDAStream());
     TORCH_CHECK(rc == 0, "ragged_attention_bwd failed (code ", rc, ")");
     return dqkv;
   });
