@@ -107,6 +107,46 @@ Tensor fm_bwd(const Tensor& cube, const Tensor& gout) {
   return dcube;
 }
 
+// (deep bf16 [B, ldp], lin fp32 [B, 1], sums fp32 [B, D]): see rb_fm_head_fwd
+std::tuple<Tensor, Tensor, Tensor> fm_head_fwd(const Tensor& dense, const Tensor& table, const Tensor& table_bias, const Tensor& emb, const Tensor& bias) {
+  for (const Tensor* t : {&dense, &table, &table_bias, &emb, &bias})
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == torch::kFloat32 && t->is_contiguous() && t->device() == dense.device(),
+                "fm_head: contiguous fp32 tensors on one CUDA device");
+  TORCH_CHECK(dense.dim() == 2 && table.dim() == 2 && table_bias.dim() == 1 && emb.dim() == 3 && bias.dim() == 3);
+  const int64_t B = dense.size(0), Nd = dense.size(1), F = emb.size(1), D = emb.size(2);
+  TORCH_CHECK(table.size(0) == Nd && table.size(1) == D && table_bias.size(0) == Nd && emb.size(0) == B && bias.size(0) == B && bias.size(1) == F &&
+              bias.size(2) >= 1, "fm_head: shapes do not match");
+  c10::cuda::CUDAGuard g(dense.device());
+  const int64_t ldp = ((Nd + F) * D + 7) / 8 * 8;
+  auto deep = torch::empty({B, ldp}, dense.options().dtype(torch::kBFloat16));
+  auto lin = torch::empty({B, 1}, dense.options());
+  auto sums = torch::empty({B, D}, dense.options());
+  const int rc = rb_fm_head_fwd(dense.data_ptr<float>(), table.data_ptr<float>(), table_bias.data_ptr<float>(), emb.data_ptr<float>(),
+                                bias.data_ptr<float>(), (int)B, (int)Nd, (int)F, (int)D, (int)bias.size(2), (int)ldp, deep.data_ptr(),
+                                lin.data_ptr<float>(), sums.data_ptr<float>(), at::cuda::getCurrentCUDAStream());
+  TORCH_CHECK(rc == 0, "fm_head_fwd failed (code ", rc, ")");
+  return {deep, lin, sums};
+}
+
+// (d_emb, d_bias, d_table, d_table_bias)
+std::tuple<Tensor, Tensor, Tensor, Tensor> fm_head_bwd(const Tensor& dense, const Tensor& table, const Tensor& emb, const Tensor& sums, int64_t bias_w,
+                                                       const Tensor& g_deep, const Tensor& g_lin) {
+  const int64_t B = dense.size(0), Nd = dense.size(1), F = emb.size(1), D = emb.size(2);
+  TORCH_CHECK(g_deep.is_cuda() && g_deep.scalar_type() == torch::kBFloat16 && g_deep.is_contiguous() && g_deep.dim() == 2 && g_deep.size(0) == B &&
+              g_deep.size(1) >= (Nd + F) * D && g_lin.scalar_type() == torch::kFloat32 && g_lin.is_contiguous() && g_lin.numel() == B,
+              "fm_head_bwd: contiguous bf16 [B, ldp] and fp32 [B, 1] gradients expected");
+  c10::cuda::CUDAGuard g(dense.device());
+  auto d_emb = torch::empty_like(emb);
+  auto d_bias = torch::empty({B, F, bias_w}, emb.options());
+  auto d_num = B > 0 ? torch::empty({Nd * (D + 1)}, emb.options()) : torch::zeros({Nd * (D + 1)}, emb.options());
+  auto partial = torch::empty({rb_fm_head_blocks((int)B) * Nd * (D + 1)}, emb.options());
+  const int rc = rb_fm_head_bwd(dense.data_ptr<float>(), table.data_ptr<float>(), emb.data_ptr<float>(), sums.data_ptr<float>(), g_deep.data_ptr(),
+                                g_lin.data_ptr<float>(), (int)B, (int)Nd, (int)F, (int)D, (int)bias_w, (int)g_deep.size(1), d_emb.data_ptr<float>(),
+                                d_bias.data_ptr<float>(), partial.data_ptr<float>(), d_num.data_ptr<float>(), at::cuda::getCurrentCUDAStream());
+  TORCH_CHECK(rc == 0, "fm_head_bwd failed (code ", rc, ")");
+  return {d_emb, d_bias, d_num.narrow(0, 0, Nd * D).view({Nd, D}), d_num.narrow(0, Nd * D, Nd)};
+}
+
 // returns (dy bf16 [M, N], db fp32 [N])
 std::tuple<Tensor, Tensor> relu_bwd_bias(const Tensor& y, const Tensor& dout, bool relu, OptT db_out = c10::nullopt) {
   TORCH_CHECK(dout.is_cuda() && dout.scalar_type() == torch::kBFloat16 && dout.is_contiguous() && dout.dim() == 2);
@@ -337,6 +377,8 @@ void init_dense(py::module& m) {
   m.def("dot_interaction_bwd", &dot_interaction_bwd);
   m.def("fm_fwd", &fm_fwd);
   m.def("fm_bwd", &fm_bwd);
+  m.def("fm_head_fwd", &fm_head_fwd);
+  m.def("fm_head_bwd", &fm_head_bwd);
   m.def("relu_bwd_bias", &relu_bwd_bias, py::arg("y"), py::arg("dout"), py::arg("relu"), py::arg("db_out") = c10::nullopt);
   m.def("cast_pad_bf16", &cast_pad_bf16);
   // Ragged self-attention forward on the tensor cores (head width 64): returns (out bf16 [T, H * 64], lse2 fp32 [T, H]).

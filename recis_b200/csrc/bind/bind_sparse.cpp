@@ -95,14 +95,16 @@ struct DescRing {
   int head = 0;
 };
 
-std::vector<std::tuple<Tensor, Tensor>> coalesce_lanes(const std::vector<std::vector<Tensor>>& ids, const std::vector<std::vector<Tensor>>& offsets,
-                                                       const std::vector<std::vector<int64_t>>& children) {
+// A feature without offsets has n_seg segments of one width (its ids divided evenly); the kernel computes theirs.
+std::vector<std::tuple<Tensor, Tensor>> coalesce_lanes(const std::vector<std::vector<Tensor>>& ids, const std::vector<std::vector<OptT>>& offsets,
+                                                       const std::vector<std::vector<int64_t>>& n_seg, const std::vector<std::vector<int64_t>>& children) {
   const size_t L = ids.size();
-  TORCH_CHECK(L > 0 && offsets.size() == L && children.size() == L, "coalesce_lanes: one list of ids / offsets / children per lane");
+  TORCH_CHECK(L > 0 && offsets.size() == L && n_seg.size() == L && children.size() == L, "coalesce_lanes: one list of ids / offsets / n_seg / children per lane");
   const auto dev = ids[0][0].device();
   int64_t words = 0;
   for (size_t l = 0; l < L; ++l) {
-    TORCH_CHECK(!ids[l].empty() && offsets[l].size() == ids[l].size() && children[l].size() == ids[l].size(), "coalesce_lanes: ragged lists");
+    TORCH_CHECK(!ids[l].empty() && offsets[l].size() == ids[l].size() && n_seg[l].size() == ids[l].size() && children[l].size() == ids[l].size(),
+                "coalesce_lanes: ragged lists");
     words += 5 * ((int64_t)ids[l].size() + 1);
   }
   int64_t* host = nullptr;
@@ -131,15 +133,24 @@ std::vector<std::tuple<Tensor, Tensor>> coalesce_lanes(const std::vector<std::ve
     int64_t* d = host + pos;                                   // [5][F + 1]: id pointers, nnz prefix, offset pointers, segment prefix, child
     int64_t nnz = 0, segs = 0;
     for (int64_t f = 0; f < F; ++f) {
-      const Tensor& v = ids[l][f]; const Tensor& o = offsets[l][f];
-      TORCH_CHECK(v.scalar_type() == torch::kInt64 && v.is_contiguous() && o.scalar_type() == torch::kInt32 && o.is_contiguous() &&
-                  v.device() == dev && o.device() == dev, "coalesce_lanes: ids int64, offsets int32, contiguous, on one device");
+      const Tensor& v = ids[l][f];
+      TORCH_CHECK(v.scalar_type() == torch::kInt64 && v.is_contiguous() && v.device() == dev, "coalesce_lanes: ids int64, contiguous, on one device");
+      int64_t segs_f = n_seg[l][f], off = 0;
+      if (offsets[l][f].has_value() && offsets[l][f]->defined()) {
+        const Tensor& o = *offsets[l][f];
+        TORCH_CHECK(o.scalar_type() == torch::kInt32 && o.is_contiguous() && o.device() == dev, "coalesce_lanes: offsets int32, contiguous, on one device");
+        segs_f = o.numel() - 1;
+        off = reinterpret_cast<int64_t>(o.data_ptr());
+      } else {
+        TORCH_CHECK(segs_f >= 0 && (segs_f == 0 ? v.numel() == 0 : v.numel() % segs_f == 0), "coalesce_lanes: ", v.numel(), " ids in ", segs_f, " equal segments");
+        off = segs_f > 0 ? -(v.numel() / segs_f) : 0;             // no pointer: minus the width
+      }
       d[f] = reinterpret_cast<int64_t>(v.data_ptr());
       d[(F + 1) + f] = nnz;
-      d[2 * (F + 1) + f] = reinterpret_cast<int64_t>(o.data_ptr());
+      d[2 * (F + 1) + f] = off;
       d[3 * (F + 1) + f] = segs;
       d[4 * (F + 1) + f] = children[l][f];
-      nnz += v.numel(); segs += o.numel() - 1;
+      nnz += v.numel(); segs += segs_f;
     }
     d[F] = 0; d[(F + 1) + F] = nnz; d[2 * (F + 1) + F] = 0; d[3 * (F + 1) + F] = segs; d[4 * (F + 1) + F] = 0;
     meta[l] = {F, nnz, segs, pos};

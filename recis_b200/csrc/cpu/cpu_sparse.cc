@@ -239,9 +239,10 @@ void rbc_encode_merge(const int64_t* desc, const int64_t* table_idx, int F, int6
     for (int64_t i = 0; i < n; ++i)
       ids_out[nnz_prefix[f] + i] = (int64_t)(((uint64_t)src[i] & 0x000FFFFFFFFFFFFFull) | ((uint64_t)table_idx[f] << 52));
     if (offsets_out) {
-      const int32_t* so = reinterpret_cast<const int32_t*>(off_ptr[f]);
+      const int64_t off = off_ptr[f];                              // a pointer, or minus the width of equal segments
+      const int32_t* so = off > 0 ? reinterpret_cast<const int32_t*>(off) : nullptr;
       const int64_t ns = seg_prefix[f + 1] - seg_prefix[f];
-      for (int64_t j = 0; j < ns; ++j) offsets_out[seg_prefix[f] + j] = so[j] + (int32_t)nnz_prefix[f];
+      for (int64_t j = 0; j < ns; ++j) offsets_out[seg_prefix[f] + j] = (so ? so[j] : (int32_t)(-off * j)) + (int32_t)nnz_prefix[f];
     }
   }
   if (offsets_out) offsets_out[total_seg] = (int32_t)total_nnz;

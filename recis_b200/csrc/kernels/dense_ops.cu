@@ -173,6 +173,121 @@ fm_bwd_kernel(const float* __restrict__ cube, const float* __restrict__ gout, in
   }
 }
 
+// ---------------------------------------------------------------------------------- DeepFM input head
+// Everything a DeepFM step computes between the embedding lookup and the deep tower, one warp per sample: the field vectors
+// v_f (numeric fields f < Nd: dense[b, f] * table[f]; the others from the embedding cube) go to the tower's input as bf16, and the
+// linear part is the first-order terms plus the second-order interaction of all fields. A lane owns one float4 column group (Q = D/4
+// of them) of every (32/Q)-th field; the partial sums meet in shuffles. Written with tensor ops this is a stack over the fields, an
+// outer product, a concatenation, a cast, three reductions and their backward (one zero-fill, copy and addition per field): at 1024
+// samples x (13 + 26) fields x 16 that was 270 of the 364 launches of a training step, each shorter than its own launch (step: 3.9 ms
+// before, 1.5 ms with this head and the offsets of single-hot fields written by the coalescing kernel).
+template <int Q>
+__global__ void __launch_bounds__(256)
+fm_head_fwd_kernel(const float* __restrict__ dense, const float* __restrict__ table, const float* __restrict__ table_bias,
+                   const float* __restrict__ emb, const float* __restrict__ bias, int B, int Nd, int F, int bias_w, int ldp,
+                   __nv_bfloat16* __restrict__ deep, float* __restrict__ lin, float* __restrict__ sums) {
+  constexpr int D = Q * 4, FS = 32 / Q;
+  const int lane = threadIdx.x & 31, q = lane % Q, fs = lane / Q;
+  const int n_all = Nd + F;
+  for (int64_t b = blockIdx.x * 8 + (threadIdx.x >> 5); b < B; b += (int64_t)gridDim.x * 8) {
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    float s2 = 0.f, first = 0.f;
+    __nv_bfloat16* row = deep + b * ldp;
+#pragma unroll 4
+    for (int f = fs; f < n_all; f += FS) {
+      float4 v;
+      if (f < Nd) {
+        const float x = dense[b * Nd + f];
+        v = *reinterpret_cast<const float4*>(table + (int64_t)f * D + q * 4);
+        v.x *= x; v.y *= x; v.z *= x; v.w *= x;
+        if (q == 0) first = fmaf(x, table_bias[f], first);
+      } else {
+        v = *reinterpret_cast<const float4*>(emb + (b * F + (f - Nd)) * D + q * 4);
+        if (q == 0) first += bias[(b * F + (f - Nd)) * bias_w];
+      }
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+      s2 = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, s2))));
+      __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+      uint2 u; u.x = *reinterpret_cast<uint32_t*>(&lo); u.y = *reinterpret_cast<uint32_t*>(&hi);
+      *reinterpret_cast<uint2*>(row + f * D + q * 4) = u;
+    }
+    for (int c = n_all * D + lane; c < ldp; c += 32) row[c] = __float2bfloat16(0.f);
+#pragma unroll
+    for (int o = 16; o >= Q; o >>= 1) {
+      s.x += __shfl_xor_sync(0xffffffffu, s.x, o); s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+      s.z += __shfl_xor_sync(0xffffffffu, s.z, o); s.w += __shfl_xor_sync(0xffffffffu, s.w, o);
+    }
+    if (fs == 0) *reinterpret_cast<float4*>(sums + b * D + q * 4) = s;
+    float part = fs == 0 ? 0.5f * (s.x * s.x + s.y * s.y + s.z * s.z + s.w * s.w) : 0.f;
+    part += first - 0.5f * s2;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+    if (lane == 0) lin[b] = part;
+  }
+}
+
+// d v_f = g_deep_f + g_lin (sum - v_f): gradients of the embedding cube and of the first-order cube (column 0 of its width), and per
+// block the sums over its samples of dense * d v_f and dense * g_lin (the numeric fields' parameters); fm_head_reduce_kernel adds the
+// blocks in a fixed order. A warp's lanes own disjoint elements of its partial sums in shared memory, so nothing is atomic.
+template <int Q>
+__global__ void __launch_bounds__(256)
+fm_head_bwd_kernel(const float* __restrict__ dense, const float* __restrict__ table, const float* __restrict__ emb, const float* __restrict__ sums,
+                   const __nv_bfloat16* __restrict__ g_deep, const float* __restrict__ g_lin, int B, int Nd, int F, int bias_w, int ldp,
+                   float* __restrict__ d_emb, float* __restrict__ d_bias, float* __restrict__ partial) {
+  constexpr int D = Q * 4, FS = 32 / Q;
+  extern __shared__ __align__(16) float acc_all[];          // [8 warps][Nd * (D + 1)]
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, q = lane % Q, fs = lane / Q;
+  const int n_all = Nd + F, per = Nd * (D + 1);
+  float* acc = acc_all + w * per;
+  for (int j = lane; j < per; j += 32) acc[j] = 0.f;
+  __syncwarp();
+  for (int64_t b = blockIdx.x * 8 + w; b < B; b += (int64_t)gridDim.x * 8) {
+    const float4 s = *reinterpret_cast<const float4*>(sums + b * D + q * 4);
+    const float gl = g_lin[b];
+    const __nv_bfloat16* row = g_deep + b * ldp;
+#pragma unroll 4
+    for (int f = fs; f < n_all; f += FS) {
+      const uint2 u = *reinterpret_cast<const uint2*>(row + f * D + q * 4);
+      const float2 g01 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x)), g23 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+      if (f < Nd) {
+        const float x = dense[b * Nd + f];
+        const float4 t = *reinterpret_cast<const float4*>(table + (int64_t)f * D + q * 4);
+        float* a = acc + f * D + q * 4;
+        a[0] = fmaf(x, g01.x + gl * (s.x - x * t.x), a[0]); a[1] = fmaf(x, g01.y + gl * (s.y - x * t.y), a[1]);
+        a[2] = fmaf(x, g23.x + gl * (s.z - x * t.z), a[2]); a[3] = fmaf(x, g23.y + gl * (s.w - x * t.w), a[3]);
+        if (q == 0) acc[Nd * D + f] = fmaf(x, gl, acc[Nd * D + f]);
+      } else {
+        const int64_t at = b * F + (f - Nd);
+        const float4 v = *reinterpret_cast<const float4*>(emb + at * D + q * 4);
+        *reinterpret_cast<float4*>(d_emb + at * D + q * 4) =
+            make_float4(g01.x + gl * (s.x - v.x), g01.y + gl * (s.y - v.y), g23.x + gl * (s.z - v.z), g23.y + gl * (s.w - v.w));
+        if (q == 0) {
+          d_bias[at * bias_w] = gl;
+          for (int c = 1; c < bias_w; ++c) d_bias[at * bias_w + c] = 0.f;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < per; j += 256) {
+    float t = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) t += acc_all[k * per + j];
+    partial[(int64_t)blockIdx.x * per + j] = t;
+  }
+}
+
+__global__ void __launch_bounds__(256)
+fm_head_reduce_kernel(const float* __restrict__ partial, int blocks, int n, float* __restrict__ out) {
+  const int j = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;       // a warp per element
+  if (j >= n) return;
+  float t = 0.f;
+  for (int k = lane; k < blocks; k += 32) t += partial[(int64_t)k * n + j];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (lane == 0) out[j] = t;
+}
+
 template <typename Fn>
 inline bool fm_dispatch_q(int D, const void* p0, const void* p1, Fn&& fn) {
   if (D % 4 != 0 || (reinterpret_cast<uintptr_t>(p0) & 15) || (reinterpret_cast<uintptr_t>(p1) & 15)) return false;
@@ -275,6 +390,43 @@ void rb_fm_bwd(const float* cube, const float* gout, int B, int F, int D, float*
   });
   if (!vec) fm_bwd_kernel<<<B, 128, 0, st>>>(cube, gout, B, F, D, dcube);
   rb::note_launch();
+}
+
+int rb_fm_head_blocks(int B) { return std::min(std::max((B + 7) / 8, 1), 148 * 2); }
+
+int rb_fm_head_fwd(const float* dense, const float* table, const float* table_bias, const float* emb, const float* bias, int B, int Nd, int F,
+                   int D, int bias_w, int ldp, void* deep, float* lin, float* sums, cudaStream_t st) {
+  if (B <= 0) return 0;
+  if ((reinterpret_cast<uintptr_t>(deep) & 15) || (reinterpret_cast<uintptr_t>(sums) & 15) || ldp % 8 || ldp < (Nd + F) * D) return 1;
+  const bool ok = fm_dispatch_q(D, table, emb, [&](auto q) {
+    constexpr int Q = decltype(q)::value;
+    fm_head_fwd_kernel<Q><<<std::min((B + 7) / 8, 148 * 8), 256, 0, st>>>(dense, table, table_bias, emb, bias, B, Nd, F, bias_w, ldp,
+                                                                       reinterpret_cast<__nv_bfloat16*>(deep), lin, sums);
+  });
+  if (!ok) return 1;
+  rb::note_launch();
+  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+
+// partial: rb_fm_head_blocks(B) * Nd * (D + 1) floats of scratch; d_num: Nd * (D + 1) floats (the table's gradient, then its bias's)
+int rb_fm_head_bwd(const float* dense, const float* table, const float* emb, const float* sums, const void* g_deep, const float* g_lin, int B,
+                   int Nd, int F, int D, int bias_w, int ldp, float* d_emb, float* d_bias, float* partial, float* d_num, cudaStream_t st) {
+  if (B <= 0) return 0;
+  const int per = Nd * (D + 1);
+  const size_t smem = (size_t)8 * per * sizeof(float);
+  if ((reinterpret_cast<uintptr_t>(g_deep) & 15) || (reinterpret_cast<uintptr_t>(d_emb) & 15) || (reinterpret_cast<uintptr_t>(sums) & 15) ||
+      ldp % 8 || smem > 48 * 1024)
+    return 1;
+  const int blocks = rb_fm_head_blocks(B);
+  const bool ok = fm_dispatch_q(D, table, emb, [&](auto q) {
+    constexpr int Q = decltype(q)::value;
+    fm_head_bwd_kernel<Q><<<blocks, 256, smem, st>>>(dense, table, emb, sums, reinterpret_cast<const __nv_bfloat16*>(g_deep), g_lin, B, Nd, F,
+                                                    bias_w, ldp, d_emb, d_bias, partial);
+  });
+  if (!ok) return 1;
+  if (per > 0) fm_head_reduce_kernel<<<(per + 7) / 8, 256, 0, st>>>(partial, blocks, per, d_num);
+  rb::note_launch(per > 0 ? 2 : 1);
+  return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
 void rb_relu_bwd_bias(const void* y, const void* dout, int M, int N, int relu, void* dy, float* db, cudaStream_t st) {

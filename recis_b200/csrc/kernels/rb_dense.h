@@ -65,6 +65,14 @@ int rb_ragged_attention_bwd(const void* qkv, const void* out, const void* d_out,
                             int64_t T, int B, int H, int max_len, float scale, float* dq_acc, void* dqkv, int64_t* status, cudaStream_t st);
 void rb_fm_fwd(const float* cube, int B, int F, int D, float* out, cudaStream_t st);
 void rb_fm_bwd(const float* cube, const float* gout, int B, int F, int D, float* dcube, cudaStream_t st);
+// DeepFM input head (dense_ops.cu): dense fp32 [B, Nd], table [Nd, D], table_bias [Nd], emb [B, F, D], bias [B, F, bias_w] (column 0 counts)
+// -> deep bf16 [B, ldp] (field vectors, zero padded), lin fp32 [B] (first-order + FM terms), sums fp32 [B, D]. 0 = ran, 1 = shape or
+// alignment outside the kernels' range (D / 4 must be a power of two up to 32).
+int rb_fm_head_blocks(int B);
+int rb_fm_head_fwd(const float* dense, const float* table, const float* table_bias, const float* emb, const float* bias, int B, int Nd, int F,
+                   int D, int bias_w, int ldp, void* deep, float* lin, float* sums, cudaStream_t st);
+int rb_fm_head_bwd(const float* dense, const float* table, const float* emb, const float* sums, const void* g_deep, const float* g_lin, int B,
+                   int Nd, int F, int D, int bias_w, int ldp, float* d_emb, float* d_bias, float* partial, float* d_num, cudaStream_t st);
 // dy = relu ? dout * (y > 0) : dout (bf16, may be null to skip the store); db[n] += column sums of dy (fp32, may be null)
 void rb_relu_bwd_bias(const void* y, const void* dout, int M, int N, int relu, void* dy, float* db, cudaStream_t st);
 void rb_cast_pad_bf16(const float* src, int rows, int cols, int src_ld, void* dst, int rows_p, int cols_p, cudaStream_t st);

@@ -127,7 +127,8 @@ encode_merge_kernel(const int64_t* __restrict__ desc, const int64_t* __restrict_
       const int64_t j = w - total_nnz;
       if (j == total_seg) { offsets_out[j] = (int32_t)total_nnz; continue; }
       const int f = find_tensor(seg_prefix, F, j);
-      offsets_out[j] = reinterpret_cast<const int32_t*>(off_ptr[f])[j - seg_prefix[f]] + (int32_t)nnz_prefix[f];
+      const int64_t off = off_ptr[f], k = j - seg_prefix[f];          // a pointer, or minus the width of equal segments
+      offsets_out[j] = (off > 0 ? reinterpret_cast<const int32_t*>(off)[k] : (int32_t)(-off * k)) + (int32_t)nnz_prefix[f];
     }
   }
 }

@@ -9,7 +9,7 @@ from torch import nn
 
 from ..nn import EmbeddingEngine, EmbeddingOption
 from ..nn.initializers import NormalInitializer
-from ..ops.dense import MLP, fm_interaction
+from ..ops.dense import MLP, fm_head, fm_interaction
 
 
 class DeepFM(nn.Module):
@@ -37,10 +37,20 @@ class DeepFM(nn.Module):
         for f in self.fields:
             feats[f"{f}_emb"] = batch[f]
             feats[f"{f}_bias"] = batch[f]
-        out = self.embedding_engine(feats)
+        out = self.embedding_engine(feats, views=False)
         B = dense.shape[0]
-        emb = torch.stack([out[f"{f}_emb"] for f in self.fields], dim=1)                 # [B, F, D]
-        bias = torch.stack([out[f"{f}_bias"][:, 0] for f in self.fields], dim=1)         # [B, F]
+        packed = {tuple(names): cube for cube, names in self.embedding_engine.packed.values()}        # [B, F, width], no stacking copy
+        emb, bias = packed.get(tuple(f"{f}_emb" for f in self.fields)), packed.get(tuple(f"{f}_bias" for f in self.fields))
+        if emb is None:
+            emb = torch.stack([out[f"{f}_emb"] for f in self.fields], dim=1)             # [B, F, D]
+        if bias is None:
+            bias = torch.stack([out[f"{f}_bias"] for f in self.fields], dim=1)           # [B, F, 4]
+        head = fm_head(dense, self.numeric_embs, self.numeric_bias, emb, bias) if self.dnn.dtype == torch.bfloat16 else None
+        if head is not None:
+            deep_in, linear = head
+            logit = linear + self.dnn(deep_in)[:, :1].float()
+            return self.loss_fn(logit, label), logit
+        bias = bias[:, :, 0]                                                             # [B, F]
         num_emb = dense.unsqueeze(-1) * self.numeric_embs.unsqueeze(0)                   # [B, dense, D]
         cube = torch.cat([num_emb, emb], dim=1).contiguous()
         first = (dense * self.numeric_bias).sum(1, keepdim=True) + bias.sum(1, keepdim=True)

@@ -36,7 +36,7 @@ class DLRM(nn.Module):
     def forward(self, batch: dict):
         dense = batch["dense"]
         label = batch["label"]
-        self.embedding_engine({f: batch[f] for f in self.fields})
+        self.embedding_engine({f: batch[f] for f in self.fields}, views=False)
         (cube, names), = self.embedding_engine.packed.values()      # [B, F, D] fp32, no stacking copy
         assert names == self.fields
         x = self.bottom(dense)                                        # [B, D] compute dtype

@@ -106,7 +106,8 @@ class EmbeddingEngine(nn.Module):
 
     @staticmethod
     def _format(fea, opt: EmbeddingOption, device):
-        """feature tensor -> (ids int64 [n], offsets int32 [S+1], weights or None, n_segments, out shape)."""
+        """feature tensor -> (ids int64 [n], offsets int32 [S+1] or None for segments of equal width, weights or None, n_segments,
+        out shape)."""
         dim = opt.embedding_dim
         if isinstance(fea, RaggedTensor):
             ids = fea.values()
@@ -129,10 +130,12 @@ class EmbeddingEngine(nn.Module):
             if fea.dim() == 1:
                 fea = fea.unsqueeze(-1)
             width = fea.shape[-1]
-            n_seg = fea.numel() // max(width, 1)
+            if width == 0:
+                raise RuntimeError("EmbeddingEngine: a dense feature needs at least one id per segment")
+            n_seg = fea.numel() // width
             ids = fea.reshape(-1)
             weight = None
-            offsets = torch.arange(0, (n_seg + 1) * width, width, dtype=torch.int32, device=fea.device)
+            offsets = None                  # segments of one width: the coalescing kernel writes their offsets
             if opt.combiner == "tile":
                 shape = (fea.shape[0], dim * opt.combiner_kwargs["tile_len"])
             else:
@@ -140,13 +143,15 @@ class EmbeddingEngine(nn.Module):
         else:
             raise TypeError(f"EmbeddingEngine only support tensor but get {type(fea)}")
         if _debug.enabled():
-            _debug.check_ragged("embedding input", ids, offsets, weight)
+            _debug.check_ragged("embedding input", ids, offsets if offsets is not None else
+                                torch.arange(0, ids.numel() + 1, width, dtype=torch.int32), weight)
         if ids.dtype != torch.int64:
             ids = ids.to(torch.int64)
-        if offsets.dtype != torch.int32:
-            offsets = offsets.to(torch.int32)
         ids = ids.to(device).contiguous()
-        offsets = offsets.to(device).contiguous()
+        if offsets is not None:
+            if offsets.dtype != torch.int32:
+                offsets = offsets.to(torch.int32)
+            offsets = offsets.to(device).contiguous()
         if not opt.use_weight:
             weight = None
         elif weight is not None:
@@ -162,7 +167,7 @@ class EmbeddingEngine(nn.Module):
         tables of all of them travel to the device in ONE asynchronous copy, then one kernel per list prefixes ids and rebases
         offsets."""
         merged = native().coalesce_lanes([[f["ids"] for f in feats] for feats in parts], [[f["offsets"] for f in feats] for feats in parts],
-                                         [[int(f["child"]) for f in feats] for feats in parts])
+                                         [[f["n_seg"] for f in feats] for feats in parts], [[f["child"] for f in feats] for feats in parts])
         out = []
         for feats, (ids, offsets) in zip(parts, merged):
             weights = None
@@ -234,7 +239,10 @@ class EmbeddingEngine(nn.Module):
         return ht.lookup_pool_group(parts, opt.combiner, 0, 0, seg_off, opt.admit_hook)
 
     # ------------------------------------------------------------------ forward
-    def forward(self, input_features: dict):
+    def forward(self, input_features: dict, views: bool = True):
+        """Returns feature name -> embeddings. With ``views=False`` the features of interleaved groups are only in ``packed`` (one tensor
+        per group) and not in the result: a model that takes them from there saves a view, and in backward a gradient buffer, per
+        feature."""
         grouped = defaultdict(lambda: defaultdict(list))
         outs = {}
         direct = {}
@@ -292,7 +300,7 @@ class EmbeddingEngine(nn.Module):
             if perm is not None:
                 cube = pooled.view(segs[0], len(feats), D)
                 self.packed[(ht_name, run_key)] = (cube, [f["name"] for f in feats])
-                for j, f in enumerate(feats):
+                for j, f in enumerate(feats if views else ()):
                     outs[f["name"]] = cube[:, j, :].reshape(f["shape"]) if len(f["shape"]) != 2 else cube[:, j, :]
             else:
                 rows_per = segs

@@ -256,3 +256,36 @@ def fm_interaction(cube: torch.Tensor) -> torch.Tensor:
         return _FMFn.apply(cube.contiguous())
     s = cube.sum(dim=1)
     return 0.5 * (s * s - (cube * cube).sum(dim=1)).sum(dim=1, keepdim=True)
+
+
+class _FMHeadFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, dense, table, table_bias, emb, bias):
+        deep, lin, sums = native().fm_head_fwd(dense, table, table_bias, emb, bias)
+        ctx.save_for_backward(dense, table, emb, sums)
+        ctx.bias_w = bias.shape[2]
+        return deep, lin
+
+    @staticmethod
+    def backward(ctx, g_deep, g_lin):
+        dense, table, emb, sums = ctx.saved_tensors
+        d_emb, d_bias, d_table, d_table_bias = native().fm_head_bwd(dense, table, emb, sums, ctx.bias_w, g_deep.contiguous(),
+                                                                    g_lin.contiguous())
+        return None, d_table, d_table_bias, d_emb, d_bias
+
+
+def fm_head(dense: torch.Tensor, table: torch.Tensor, table_bias: torch.Tensor, emb: torch.Tensor, bias: torch.Tensor):
+    """The DeepFM step between lookup and tower in one kernel per direction: ``dense`` [B, Nd] numeric values with their field vectors
+    ``table`` [Nd, D] and weights ``table_bias`` [Nd], ``emb`` [B, F, D] and ``bias`` [B, F, w] (column 0 counts) of the sparse fields
+    -> (tower input bf16 [B, (Nd + F) D padded to 8], first-order + second-order terms fp32 [B, 1]). ``None`` when the inputs are outside
+    the kernels' range; the caller then computes the same with tensor ops."""
+    Nd, D = table.shape
+    tensors = (dense, table, table_bias, emb, bias)
+    if (not all(t.is_cuda and t.dtype == torch.float32 for t in tensors) or dense.dim() != 2 or dense.requires_grad
+            or D not in (4, 8, 16, 32, 64, 128) or Nd * (D + 1) * 32 > 48 * 1024 or dense.shape[1] != Nd
+            or emb.dim() != 3 or bias.dim() != 3 or dense.shape[0] == 0):
+        return None
+    tensors = [t.contiguous() for t in tensors]
+    if tensors[1].data_ptr() % 16 or tensors[3].data_ptr() % 16:
+        return None
+    return _FMHeadFn.apply(*tensors)

@@ -237,3 +237,32 @@ def test_bf16_weight_copies_follow_the_optimizer_and_any_other_change():
     ref = torch.relu(torch.relu(x.to(torch.bfloat16).float() @ mlp.layers[0].weight.detach().to(torch.bfloat16).float().t() + mlp.layers[0].bias))
     out = mlp.layers[0](x.to(torch.bfloat16)).float()
     assert float((out - ref).norm() / ref.norm()) < 1e-2
+
+
+@pytest.mark.parametrize("B,Nd,F,D,w", [(1, 1, 2, 8, 4), (5, 13, 26, 16, 4), (37, 3, 7, 32, 1), (1024, 13, 39, 16, 4), (9, 0, 3, 4, 2), (2500, 5, 2, 64, 4),
+                                        (17, 2, 3, 128, 4)])
+def test_fm_head_matches_tensor_ops(B, Nd, F, D, w):
+    """The fused DeepFM head against the same computation with tensor ops in 64 bits, forward and backward. The tower input is bf16
+    (2^-9 relative); everything else is fp32 over at most (Nd + F) * D products resp. B samples: 1e-5 of the sum of magnitudes."""
+    from recis_b200.ops.dense import fm_head
+    g = torch.Generator().manual_seed(B + D)
+    dense = torch.randn(B, Nd, generator=g)
+    leaves = [torch.randn(Nd, D, generator=g), torch.randn(Nd, generator=g), torch.randn(B, F, D, generator=g), torch.randn(B, F, w, generator=g)]
+    g_lin = torch.randn(B, 1, generator=g)
+    g_deep = torch.randn(B, (Nd + F) * D, generator=g).to(torch.bfloat16)
+    gpu = [t.to("cuda").requires_grad_() for t in leaves]
+    deep, lin = fm_head(dense.to("cuda"), *gpu)
+    pad = deep.shape[1] - (Nd + F) * D
+    assert deep.dtype == torch.bfloat16 and deep.shape[1] % 8 == 0 and torch.count_nonzero(deep[:, deep.shape[1] - pad:]) == 0
+    torch.autograd.backward([deep, lin], [torch.nn.functional.pad(g_deep, (0, pad)).to("cuda"), g_lin.to("cuda")])
+    ref = [t.double().requires_grad_() for t in leaves]
+    cube = torch.cat([dense.double().unsqueeze(-1) * ref[0].unsqueeze(0), ref[2]], dim=1)
+    s = cube.sum(1)
+    lin_r = (dense.double() * ref[1]).sum(1, keepdim=True) + ref[3][:, :, 0].sum(1, keepdim=True) + 0.5 * (s * s - (cube * cube).sum(1)).sum(1, keepdim=True)
+    torch.autograd.backward([cube.reshape(B, -1), lin_r], [g_deep.double(), g_lin.double()])
+    assert torch.allclose(deep[:, :(Nd + F) * D].double().cpu(), cube.reshape(B, -1), rtol=2 ** -8, atol=1e-6)
+    mag = float((cube.abs().sum(1) ** 2).sum(1).max()) + 1
+    assert (lin.double().cpu() - lin_r).abs().max() < 1e-5 * mag
+    for a, b in zip(gpu, ref):
+        if a.numel():
+            assert (a.grad.double().cpu() - b.grad).abs().max() < 1e-5 * (float(b.grad.abs().max()) * max(B, Nd + F) ** 0.5 + mag ** 0.5), b.shape
