@@ -345,7 +345,8 @@ Tensor grad_reduce(const Tensor& grad_out, const Tensor& gsrc, const Tensor& gsc
   if (n == 0) return gu;
   if (grad_out.is_cuda()) {
     c10::cuda::CUDAGuard g(grad_out.device());
-    const int64_t n_chunks = (n + rb_grad_reduce_chunk() - 1) / rb_grad_reduce_chunk();
+    const int chunk = rb_grad_reduce_chunk_for(n, (int)D);
+    const int64_t n_chunks = (n + chunk - 1) / chunk;
     auto span = torch::zeros({n_chunks, D}, grad_out.options());
     rb_grad_reduce(grad_out.data_ptr<float>(), gsrc.data_ptr<int32_t>(), gscale.data_ptr<float>(), csr_u.data_ptr<int32_t>(),
                    csr_elem.data_ptr<int32_t>(), start.data_ptr<int32_t>(), n, (int)D, span.data_ptr<float>(), opt_i32(rows), gup,

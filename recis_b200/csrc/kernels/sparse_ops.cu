@@ -33,6 +33,7 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kChunk = 32;  // CSR positions per work item of the gradient reduction
+constexpr int kChunkSmall = 8;  // ... where chunks of 32 leave too few groups to fill the GPU (rb_grad_reduce_chunk_for below)
 
 inline int grid_stride_blocks(int64_t work_items, int threads = kThreads) {
   int64_t b = (work_items + threads - 1) / threads;
@@ -314,7 +315,7 @@ __global__ void __launch_bounds__(kThreads) csr_heads_kernel(const int32_t* __re
 }
 
 // ------------------------------------------------------------------ chunked segmented gradient reduction
-// VEC = 4: float4 columns, G lanes x NACC slots per group. Work item = kChunk consecutive CSR positions.
+// VEC = 4: float4 columns, G lanes x NACC slots per group. Work item = CH consecutive CSR positions.
 // Shared-memory copy of a push descriptor: row_ptr(u) is where the gradient of unique index u is stored (nullptr = dropped).
 struct PushTable {
   int32_t off[17];
@@ -333,7 +334,7 @@ struct PushTable {
   }
 };
 
-template <int G, int NACC, bool PUSH, typename T>
+template <int G, int NACC, int CH, bool PUSH, typename T>
 __global__ void __launch_bounds__(kThreads)
 grad_reduce_kernel(const float* __restrict__ grad_out, const int32_t* __restrict__ gsrc, const float* __restrict__ gscale,
                    const int32_t* __restrict__ csr_u, const int32_t* __restrict__ csr_elem, const int32_t* __restrict__ start,
@@ -345,17 +346,17 @@ grad_reduce_kernel(const float* __restrict__ grad_out, const int32_t* __restrict
   // dependent chain for the whole chunk instead of one per position) and park it in shared memory.
   // Phase 2: walk the segments of the chunk; the optimizer state of a row is requested when its segment starts, so
   // those loads are in flight together with the gradient gathers of the segment.
-  __shared__ int32_t meta[(kThreads / G) * kChunk * 5];
+  __shared__ int32_t meta[(kThreads / G) * CH * 5];
   auto tile = cg::tiled_partition<G>(cg::this_thread_block());
   const int lane = threadIdx.x % G;
   const int gid = threadIdx.x / G;
-  int32_t* m_u = meta + gid * kChunk * 5;
-  int32_t* m_gs = m_u + kChunk;
-  int32_t* m_row = m_u + 2 * kChunk;      // >= 0 row to update / unique index to store, -1 skip, -2 segment crosses the chunk
-  int32_t* m_dst = m_u + 3 * kChunk;      // chunk that owns a crossing segment
-  float* m_sc = reinterpret_cast<float*>(m_u + 4 * kChunk);
+  int32_t* m_u = meta + gid * CH * 5;
+  int32_t* m_gs = m_u + CH;
+  int32_t* m_row = m_u + 2 * CH;      // >= 0 row to update / unique index to store, -1 skip, -2 segment crosses the chunk
+  int32_t* m_dst = m_u + 3 * CH;      // chunk that owns a crossing segment
+  float* m_sc = reinterpret_cast<float*>(m_u + 4 * CH);
   const int cols = D >> 2;
-  const int64_t n_chunks = (n + kChunk - 1) / kChunk;
+  const int64_t n_chunks = (n + CH - 1) / CH;
   const int64_t n_groups = (int64_t)gridDim.x * (kThreads / G);
   // The sorted positions are bucketed by owner rank, so chunks in their natural order would make every rank write to owner 0
   // first, then to owner 1, ...: all ranks' stores would converge on one GPU's links at a time (measured on 4 GPUs: 0.38 TB/s
@@ -368,7 +369,7 @@ grad_reduce_kernel(const float* __restrict__ grad_out, const int32_t* __restrict
   for (int64_t v = blockIdx.x * (int64_t)(kThreads / G) + gid; v < n_virtual; v += n_groups) {
     const int64_t c = PUSH ? (v % kSpread) * spread_cols + v / kSpread : v;
     if (c >= n_chunks) continue;              // uniform for the group (c depends on v and the group id only)
-    const int64_t p0 = c * kChunk, p1 = min(p0 + (int64_t)kChunk, n);
+    const int64_t p0 = c * CH, p1 = min(p0 + (int64_t)CH, n);
     const int cnt = (int)(p1 - p0);
     for (int j = lane; j < cnt; j += G) {
       const int32_t u = csr_u[p0 + j];
@@ -379,7 +380,7 @@ grad_reduce_kernel(const float* __restrict__ grad_out, const int32_t* __restrict
       m_gs[j] = gsrc[e];
       m_sc[j] = gscale[e];
       m_row[j] = complete ? (apply ? (rows ? rows[u] : u) : u) : -2;
-      m_dst[j] = s0 / kChunk;
+      m_dst[j] = s0 / CH;
     }
     tile.sync();
     int j = 0;
@@ -446,7 +447,7 @@ grad_reduce_kernel(const float* __restrict__ grad_out, const int32_t* __restrict
 
 // Rows whose occurrences cross a chunk boundary were accumulated in span_acc[chunk of their first
 // occurrence]; finish them here and leave span_acc zeroed for the next step.
-template <int G, int NACC, bool PUSH, typename T>
+template <int G, int NACC, int CH, bool PUSH, typename T>
 __global__ void __launch_bounds__(kThreads)
 grad_span_finish_kernel(const int32_t* __restrict__ csr_u, const int32_t* __restrict__ start, int64_t n, int D,
                         float* __restrict__ span_acc, const int32_t* __restrict__ rows, float* __restrict__ gu, int apply, RbOpt opt,
@@ -455,10 +456,10 @@ grad_span_finish_kernel(const int32_t* __restrict__ csr_u, const int32_t* __rest
   if (PUSH) ptab.load(push);
   const int lane = threadIdx.x % G;
   const int cols = D >> 2;
-  const int64_t n_chunks = (n + kChunk - 1) / kChunk;
+  const int64_t n_chunks = (n + CH - 1) / CH;
   const int64_t n_groups = (int64_t)gridDim.x * (kThreads / G);
   for (int64_t c = blockIdx.x * (int64_t)(kThreads / G) + threadIdx.x / G; c < n_chunks; c += n_groups) {
-    const int64_t p0 = c * kChunk, p1 = min(p0 + (int64_t)kChunk, n);
+    const int64_t p0 = c * CH, p1 = min(p0 + (int64_t)CH, n);
     const int32_t u = csr_u[p1 - 1];
     const int32_t s0 = start[u], s1 = start[u + 1];
     if (!(s0 >= p0 && s1 > p1)) continue;
@@ -648,22 +649,38 @@ void rb_iota_i32(int32_t* out, int64_t n, cudaStream_t st) {
 
 int rb_grad_reduce_chunk() { return kChunk; }
 
+// Positions per chunk for a reduction of n elements of D columns. A group of lanes walks its chunk's rows one after the other, each
+// with the latency of fetching and updating a row, so the number of groups is what hides latency: chunks of 8 as long as chunks of
+// 32 would give less than one full load of the GPU (148 SMs x 2048 threads). Longer chunks cost less metadata and fewer rows that
+// cross a boundary (those are summed with reductions into span_acc). Measured, D = 16, 27k elements: 71 -> 18 us; D = 8, 180k: 83 ->
+// 24 us; D = 128, 293k: 96 -> 94 us with the finish kernel, the line; 4.3M elements stay at 32.
+int rb_grad_reduce_chunk_for(int64_t n, int D) {
+  const int cols = D >> 2;
+  const int lanes = cols <= 4 ? 4 : cols <= 8 ? 8 : cols <= 16 ? 16 : 32;
+  return n / kChunk * lanes < (int64_t)148 * 2048 ? kChunkSmall : kChunk;
+}
+
 void rb_grad_reduce(const float* grad_out, const int32_t* gsrc, const float* gscale, const int32_t* csr_u, const int32_t* csr_elem,
                     const int32_t* start, int64_t n, int D, float* span_acc, const int32_t* rows, float* gu, int apply, RbOpt opt,
                     cudaStream_t st) {
   if (n <= 0) return;
-  const int64_t n_chunks = (n + kChunk - 1) / kChunk;
+  const int chunk = rb_grad_reduce_chunk_for(n, D);
+  const int64_t n_chunks = (n + chunk - 1) / chunk;
   const int dtype = apply ? opt.w_dtype : (int)rb::kRowF32;      // without an update no row is touched: one instantiation serves
   RB_DISPATCH_ROW(dtype, false, {
     const bool ok = dispatch_cols(D, [&](auto g, auto nacc) {
       constexpr int G = decltype(g)::value, NACC = decltype(nacc)::value;
       const int64_t blocks = (n_chunks + (kThreads / G) - 1) / (kThreads / G);
       const int grid = (int)std::min<int64_t>(blocks, 148 * 64);
-      grad_reduce_kernel<G, NACC, false, T><<<grid, kThreads, 0, st>>>(grad_out, gsrc, gscale, csr_u, csr_elem, start, n, D, span_acc, rows,
-                                                                       gu, apply, opt, RbGuPush{});
-      rb::note_launch();
-      grad_span_finish_kernel<G, NACC, false, T><<<grid, kThreads, 0, st>>>(csr_u, start, n, D, span_acc, rows, gu, apply, opt, RbGuPush{});
-      rb::note_launch();
+      auto run = [&](auto ch) {
+        constexpr int CH = decltype(ch)::value;
+        grad_reduce_kernel<G, NACC, CH, false, T><<<grid, kThreads, 0, st>>>(grad_out, gsrc, gscale, csr_u, csr_elem, start, n, D, span_acc, rows,
+                                                                             gu, apply, opt, RbGuPush{});
+        grad_span_finish_kernel<G, NACC, CH, false, T><<<grid, kThreads, 0, st>>>(csr_u, start, n, D, span_acc, rows, gu, apply, opt, RbGuPush{});
+      };
+      if (chunk == kChunk) run(std::integral_constant<int, kChunk>{});
+      else run(std::integral_constant<int, kChunkSmall>{});
+      rb::note_launch(2);
     });
     if (!ok) {
       grad_reduce_scalar_kernel<T><<<grid_stride_blocks(n * D), kThreads, 0, st>>>(grad_out, gsrc, gscale, csr_u, csr_elem, start, n, D, rows,
@@ -683,10 +700,10 @@ void rb_grad_reduce_push(const float* grad_out, const int32_t* gsrc, const float
     const int64_t blocks = (n_chunks + (kThreads / G) - 1) / (kThreads / G);
     // max_blocks > 0 caps the grid (NVLink-bound kernel: a small grid leaves SMs to kernels of other streams)
     const int grid = (int)std::min<int64_t>(blocks, max_blocks > 0 ? max_blocks : 148 * 64);
-    grad_reduce_kernel<G, NACC, true, float><<<grid, kThreads, 0, st>>>(grad_out, gsrc, gscale, csr_u, csr_elem, start, n, D, span_acc, nullptr,
+    grad_reduce_kernel<G, NACC, kChunk, true, float><<<grid, kThreads, 0, st>>>(grad_out, gsrc, gscale, csr_u, csr_elem, start, n, D, span_acc, nullptr,
                                                                         nullptr, 0, opt, push);
     rb::note_launch();
-    grad_span_finish_kernel<G, NACC, true, float><<<grid, kThreads, 0, st>>>(csr_u, start, n, D, span_acc, nullptr, nullptr, 0, opt, push);
+    grad_span_finish_kernel<G, NACC, kChunk, true, float><<<grid, kThreads, 0, st>>>(csr_u, start, n, D, span_acc, nullptr, nullptr, 0, opt, push);
     rb::note_launch();
   });
 }

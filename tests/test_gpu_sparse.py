@@ -298,3 +298,29 @@ def test_table_grows_in_place_without_copying():
     t_full, t_empty = min(grow_time(900_000) for _ in range(2)), min(grow_time(0) for _ in range(2))
     # the pointer checks above are the proof that nothing moved; the clock only has to rule out a copy of the filled rows
     assert t_full < 5 * t_empty + 0.05, (t_full, t_empty)
+
+
+@pytest.mark.parametrize("n,D", [(1, 8), (7, 4), (8, 16), (9, 16), (31, 32), (33, 64), (2400, 128), (2048 * 148 * 8 // 32 * 32 // 128, 512),
+                                 (2048 * 148 // 32 * 32 - 32, 128), (2048 * 148 // 32 * 32, 128), (2048 * 148 // 4 * 32 // 8 - 1, 8)])
+def test_gradient_reduction_chunk_sizes(n, D):
+    """Both chunk lengths of the segmented gradient reduction and the line between them (fewer groups of lanes than the GPU holds threads
+    for), with ids that cross many chunks and ids that occur once, against an index_add in 64 bits. fp32 sums of c terms in any order
+    differ by at most c * 2^-24 of the sum of magnitudes."""
+    C = recis_b200.native()
+    g = torch.Generator().manual_seed(n + D)
+    rev = torch.randint(0, max(n // 3, 1), (n,), generator=g)
+    rev[torch.rand(n, generator=g) < 0.3] = 0
+    rev = torch.unique(rev, return_inverse=True)[1].to(torch.int32)
+    segs = max(n // 4, 1)
+    grad = torch.randn(segs, D, generator=g)
+    gsrc = torch.randint(0, segs, (n,), generator=g).to(torch.int32)
+    gscale = torch.rand(n, generator=g)
+    n_u = int(rev.max()) + 1
+    dev = [t.cuda() for t in (grad, gsrc, gscale, rev)]
+    csr_u, csr_elem, start = C.build_csr(dev[3])
+    gu = C.grad_reduce(dev[0], dev[1], dev[2], csr_u, csr_elem, start, D, None, False, 2, 0.0, 0.0, 0.0, 0.0, 1.0, 0.0, 1.0, None, None, None, n_u)
+    terms = grad[gsrc.long()].double() * gscale.double().unsqueeze(1)
+    ref = torch.zeros(n_u, D, dtype=torch.float64).index_add_(0, rev.long(), terms)
+    mag = torch.zeros(n_u, D, dtype=torch.float64).index_add_(0, rev.long(), terms.abs())
+    count = torch.bincount(rev.long(), minlength=n_u).double().unsqueeze(1)
+    assert ((gu.double().cpu() - ref).abs() <= (count + 2) * 2.0 ** -24 * mag + 1e-30).all()
