@@ -34,9 +34,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> dedup_partition(const Tensor& ids, in
   const int64_t n = ids.numel();
   auto o = ids.options();
   const int64_t cap = pow2_at_least(2 * std::max<int64_t>(n, 1));
-  auto set_keys = torch::empty({cap}, o);
-  auto set_pos = torch::empty({cap + 1}, o.dtype(torch::kInt32));
-  auto slot = torch::empty({std::max<int64_t>(n, 1)}, o.dtype(torch::kInt32));
+  TORCH_CHECK(n <= (int64_t)1 << 30, "dedup_partition: too many ids in one call");
   Tensor counts = counts_out.has_value() && counts_out->defined() ? *counts_out : torch::empty({world}, o.dtype(torch::kInt32));
   TORCH_CHECK(counts.numel() >= world && counts.scalar_type() == torch::kInt32, "dedup_partition: counts_out: int32 [world]");
   Tensor offsets = offsets_out.has_value() && offsets_out->defined() ? *offsets_out : torch::empty({world + 1}, o.dtype(torch::kInt32));
@@ -47,11 +45,15 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> dedup_partition(const Tensor& ids, in
   auto reverse = torch::empty({n}, o.dtype(torch::kInt32));
   if (ids.is_cuda()) {
     c10::cuda::CUDAGuard g(ids.device());
-    rb_dedup_partition(ids.data_ptr<int64_t>(), n, (int)world, reinterpret_cast<uint64_t*>(set_keys.data_ptr<int64_t>()),
-                       set_pos.data_ptr<int32_t>(), cap, slot.data_ptr<int32_t>(), counts.data_ptr<int32_t>(),
+    auto scratch = torch::empty({cap + 2 * std::max<int64_t>(n, 1)}, o.dtype(torch::kInt32));       // the set, then two words per id
+    int32_t* set = scratch.data_ptr<int32_t>();
+    rb_dedup_partition(ids.data_ptr<int64_t>(), n, (int)world, set, cap, set + cap, set + cap + std::max<int64_t>(n, 1), counts.data_ptr<int32_t>(),
                        offsets.data_ptr<int32_t>(), unique_ids.data_ptr<int64_t>(), reverse.data_ptr<int32_t>(), unique_ids.numel(),
                        guarded ? status->data_ptr<int64_t>() : nullptr, cur_stream());
   } else {
+    auto set_keys = torch::empty({cap}, o);
+    auto set_pos = torch::empty({cap + 1}, o.dtype(torch::kInt32));
+    auto slot = torch::empty({std::max<int64_t>(n, 1)}, o.dtype(torch::kInt32));
     rbc_dedup_partition(ids.data_ptr<int64_t>(), n, (int)world, reinterpret_cast<uint64_t*>(set_keys.data_ptr<int64_t>()),
                         set_pos.data_ptr<int32_t>(), cap, slot.data_ptr<int32_t>(), counts.data_ptr<int32_t>(),
                         offsets.data_ptr<int32_t>(), unique_ids.data_ptr<int64_t>(), reverse.data_ptr<int32_t>(), unique_ids.numel(),

@@ -324,3 +324,25 @@ def test_gradient_reduction_chunk_sizes(n, D):
     mag = torch.zeros(n_u, D, dtype=torch.float64).index_add_(0, rev.long(), terms.abs())
     count = torch.bincount(rev.long(), minlength=n_u).double().unsqueeze(1)
     assert ((gu.double().cpu() - ref).abs() <= (count + 2) * 2.0 ** -24 * mag + 1e-30).all()
+
+
+@pytest.mark.parametrize("n,world", [(1, 1), (257, 3), (1023, 1), (4 * 148 * 2048 - 1, 1), (4 * 148 * 2048 + 5, 1), (4 * 148 * 2048 + 1030, 8)])
+def test_dedup_sizes_around_the_batched_probing(n, world):
+    """Both probing variants and remainders of their blocks, with ids of every kind (0, -1, -2, the extremes): every unique id once, the
+    reverse index leads back to it, owners in order, counts and offsets consistent."""
+    C = recis_b200.native()
+    g = torch.Generator().manual_seed(n)
+    ids = torch.randint(-n // 3 - 2, n // 3 + 2, (n,), generator=g)
+    for k, v in enumerate((-1, -2, 0, -(1 << 63), (1 << 63) - 1)):
+        ids[k::97] = v
+    ids = ids.cuda()
+    uniq, rev, counts, offs = C.dedup_partition(ids, world)
+    n_u = int(offs[-1])
+    assert torch.equal(uniq[rev.long()], ids) and n_u == int(counts.sum())
+    assert torch.equal(torch.sort(uniq[:n_u]).values, torch.unique(ids))
+    assert torch.equal(offs.cpu()[1:], counts.cpu().cumsum(0).to(torch.int32))
+    ref = C.dedup_partition(ids.cpu(), world)
+    assert torch.equal(ref[2], counts.cpu())
+    for w in range(world):
+        a, b = int(offs[w]), int(offs[w + 1])
+        assert torch.equal(torch.sort(uniq[a:b]).values.cpu(), torch.sort(ref[0][a:b]).values)
