@@ -97,6 +97,36 @@ struct DescRing {
   int head = 0;
 };
 
+// The number of segments of every feature when all of them are ready for coalesce_lanes as they are (int64 ids, int32 offsets, optional
+// fp32 weights, flat, contiguous, on `dev`), or nothing when some feature needs converting first.
+c10::optional<std::vector<int64_t>> plain_segments(const std::vector<Tensor>& ids, const std::vector<Tensor>& offsets, const std::vector<OptT>& weights,
+                                                   const torch::Device& dev) {
+  TORCH_CHECK(ids.size() == offsets.size() && ids.size() == weights.size(), "plain_segments: ragged lists");
+  std::vector<int64_t> segs(ids.size());
+  auto flat = [&](const Tensor& t, torch::ScalarType dt) { return t.scalar_type() == dt && t.dim() == 1 && t.is_contiguous() && t.device() == dev; };
+  for (size_t i = 0; i < ids.size(); ++i) {
+    if (!flat(ids[i], torch::kInt64) || !flat(offsets[i], torch::kInt32) || offsets[i].numel() < 1) return c10::nullopt;
+    if (weights[i].has_value() && weights[i]->defined() && !flat(*weights[i], torch::kFloat32)) return c10::nullopt;
+    segs[i] = offsets[i].numel() - 1;
+  }
+  return segs;
+}
+
+// The same for dense features ([n] or [n, width] int64): their flat ids and numbers of segments.
+c10::optional<std::tuple<std::vector<Tensor>, std::vector<int64_t>>> plain_dense(const std::vector<Tensor>& feats, const torch::Device& dev) {
+  std::vector<Tensor> ids(feats.size());
+  std::vector<int64_t> segs(feats.size());
+  for (size_t i = 0; i < feats.size(); ++i) {
+    const Tensor& t = feats[i];
+    if (t.layout() != torch::kStrided || t.scalar_type() != torch::kInt64 || t.dim() < 1 || t.dim() > 2 || !t.is_contiguous() || t.device() != dev ||
+        t.size(-1) == 0)
+      return c10::nullopt;
+    segs[i] = t.size(0);
+    ids[i] = t.dim() == 1 ? t : t.view({-1});
+  }
+  return std::make_tuple(std::move(ids), std::move(segs));
+}
+
 // A feature without offsets has n_seg segments of one width (its ids divided evenly); the kernel computes theirs.
 std::vector<std::tuple<Tensor, Tensor>> coalesce_lanes(const std::vector<std::vector<Tensor>>& ids, const std::vector<std::vector<OptT>>& offsets,
                                                        const std::vector<std::vector<int64_t>>& n_seg, const std::vector<std::vector<int64_t>>& children) {
@@ -418,6 +448,8 @@ void init_sparse(py::module& m) {
         py::arg("offsets_out") = py::none(), py::arg("status") = py::none(), py::arg("counts_out") = py::none());
   m.def("encode_merge", &encode_merge);
   m.def("coalesce_lanes", &coalesce_lanes);
+  m.def("plain_segments", &plain_segments);
+  m.def("plain_dense", &plain_dense);
   m.def("gather_rows", &gather_rows, py::arg("src"), py::arg("rows"), py::arg("n_dev") = py::none());
   m.def("scatter_rows", &scatter_rows);
   m.def("fill_rows_i64", &fill_rows_i64);

@@ -61,7 +61,35 @@ class _Group:
         )
 
 
+class _RunGroup:
+    """Features of one call that are looked up together: one physical table, one runtime configuration."""
+
+    __slots__ = ("ht_name", "run_key", "names", "children")
+
+    def __init__(self, ht_name, run_key):
+        self.ht_name, self.run_key = ht_name, run_key
+        self.names, self.children = [], []
+
+
+class _Feats:
+    """The formatted inputs of a ``_RunGroup``, as parallel lists."""
+
+    __slots__ = ("names", "children", "ids", "offsets", "weights", "n_seg", "shapes")
+
+    def __init__(self, names, children, ids, offsets, weights, n_seg, shapes):
+        self.names, self.children, self.ids, self.offsets, self.weights, self.n_seg, self.shapes = (
+            names, children, ids, offsets, weights, n_seg, shapes)
+
+    def __len__(self):
+        return len(self.names)
+
+    def part(self, a, b):
+        return _Feats(*(getattr(self, k)[a:b] for k in self.__slots__))
+
+
 class EmbeddingEngine(nn.Module):
+    _MAX_PLANS = 64
+
     def __init__(self, emb_options: dict, interleave: bool = False, exchange_lanes: int = 0):
         super().__init__()
         # exchange_lanes > 1 (or RECIS_EXCHANGE_LANES): the features of one (table, runtime group) are split into that many
@@ -75,7 +103,7 @@ class EmbeddingEngine(nn.Module):
         self._emb_opts = emb_options
         self._interleave = interleave
         self.packed = {}
-        self._desc_ring = {}
+        self._plans = {}                 # names of a call's features -> (run groups, names passed through)
         shared_to_ht = {}
         capacity = defaultdict(int)
         for fea_name, opt in emb_options.items():
@@ -158,6 +186,52 @@ class EmbeddingEngine(nn.Module):
             weight = weight.to(device=device, dtype=torch.float32).contiguous()
         return ids, offsets, weight, n_seg, shape
 
+    def _plan(self, names):
+        """How the features of a call group: depends on their names and order alone, so it is kept per name tuple."""
+        plan = self._plans.get(names)
+        if plan is None:
+            grouped, direct = {}, []
+            for name in names:
+                ht_name = self._fea_to_ht.get(name)
+                if ht_name is None:
+                    direct.append(name)
+                    continue
+                group = self._groups[ht_name]
+                run_key = group.fea_runtime[name]
+                runtimes = grouped.setdefault(ht_name, {})
+                if run_key not in runtimes:
+                    runtimes[run_key] = _RunGroup(ht_name, run_key)
+                runtimes[run_key].names.append(name)
+                runtimes[run_key].children.append(group.fea_child[name])
+            if len(self._plans) >= self._MAX_PLANS:
+                self._plans.clear()
+            plan = self._plans[names] = ([g for runtimes in grouped.values() for g in runtimes.values()], direct)
+        return plan
+
+    def _format_group(self, group, input_features, device) -> _Feats:
+        """The inputs of a run group. Plain ragged or dense features that need no conversion (what a data pipeline delivers) are checked by
+        one native call for all of them; anything else goes through ``_format`` one by one."""
+        names, opts = group.names, self._emb_opts
+        feats = [input_features[n] for n in names]
+        first = opts[names[0]]
+        if first.combiner != "tile" and not _debug.enabled() and all(type(f) is RaggedTensor and len(f._offsets) == 1 for f in feats):
+            ids, offsets = [f._values for f in feats], [f._offsets[0] for f in feats]
+            weights = [f._weight for f in feats] if first.use_weight else [None] * len(feats)
+            segs = native().plain_segments(ids, offsets, weights, device)
+            if segs is not None:
+                dim = first.embedding_dim
+                return _Feats(names, group.children, ids, offsets, weights, segs, [(s, dim) for s in segs])
+        elif first.combiner != "tile" and not _debug.enabled() and all(type(f) is torch.Tensor for f in feats):
+            flat = native().plain_dense(feats, device)
+            if flat is not None:
+                ids, segs = flat
+                dim = first.embedding_dim
+                none = [None] * len(feats)
+                return _Feats(names, group.children, ids, none, none, segs, [(s, dim) for s in segs])
+        rows = [self._format(f, opts[n], device) for n, f in zip(names, feats)]
+        ids, offsets, weights, segs, shapes = (list(c) for c in zip(*rows))
+        return _Feats(names, group.children, ids, offsets, weights, segs, shapes)
+
     def _coalesce(self, feats, device):
         """Concatenate formatted features: one kernel prefixes ids and rebases offsets for all of them."""
         return self._coalesce_many([feats], device)[0]
@@ -166,13 +240,12 @@ class EmbeddingEngine(nn.Module):
         """``_coalesce`` for several feature lists at once (the lanes of one runtime group), in one native call: the descriptor
         tables of all of them travel to the device in ONE asynchronous copy, then one kernel per list prefixes ids and rebases
         offsets."""
-        merged = native().coalesce_lanes([[f["ids"] for f in feats] for feats in parts], [[f["offsets"] for f in feats] for feats in parts],
-                                         [[f["n_seg"] for f in feats] for feats in parts], [[f["child"] for f in feats] for feats in parts])
+        merged = native().coalesce_lanes([f.ids for f in parts], [f.offsets for f in parts], [f.n_seg for f in parts], [f.children for f in parts])
         out = []
         for feats, (ids, offsets) in zip(parts, merged):
             weights = None
-            if any(f["weight"] is not None for f in feats):
-                ws = [f["weight"] if f["weight"] is not None else torch.ones(f["ids"].numel(), device=device) for f in feats]
+            if any(w is not None for w in feats.weights):
+                ws = [w if w is not None else torch.ones(i.numel(), device=device) for i, w in zip(feats.ids, feats.weights)]
                 weights = torch.cat(ws) if len(ws) > 1 else ws[0]
             out.append((ids, offsets, weights))
         return out
@@ -221,16 +294,17 @@ class EmbeddingEngine(nn.Module):
         """One runtime group as a pipeline of exchange lanes (``FusedExchange.forward_group``). Returns the pooled rows of the
         whole group: ``[segments_per_feature * n_features, D]`` in the interleaved layout when ``perm`` is set, else the features'
         segments one after the other."""
-        bounds = self._lane_ranges([f["child"] for f in feats], self._lanes)
+        bounds = self._lane_ranges(feats.children, self._lanes)
         L = len(bounds) - 1
         parts, seg_off = [], 0
-        merged = self._coalesce_many([feats[bounds[i]:bounds[i + 1]] for i in range(L)], dev)
+        split = [feats.part(bounds[i], bounds[i + 1]) for i in range(L)]
+        merged = self._coalesce_many(split, dev)
         for i in range(L):
-            part = feats[bounds[i]:bounds[i + 1]]
+            part = split[i]
             ids, offsets, weights = merged[i]
             key = f"{run_key}#lane{i}of{L}"
-            ht.fused.lane_children[key] = frozenset(f["child"] for f in part)
-            n_seg = sum(f["n_seg"] for f in part)
+            ht.fused.lane_children[key] = frozenset(part.children)
+            n_seg = sum(part.n_seg)
             parts.append(dict(key=key, ids=ids, offsets=offsets, weights=weights, perm_f=len(part), n_seg=n_seg,
                               perm_off=bounds[i] if perm is not None else seg_off))
             seg_off += n_seg
@@ -243,45 +317,34 @@ class EmbeddingEngine(nn.Module):
         """Returns feature name -> embeddings. With ``views=False`` the features of interleaved groups are only in ``packed`` (one tensor
         per group) and not in the result: a model that takes them from there saves a view, and in backward a gradient buffer, per
         feature."""
-        grouped = defaultdict(lambda: defaultdict(list))
+        groups, direct = self._plan(tuple(input_features))
+        # every input is formatted (and refused, if it has to be) before anything runs
+        formatted = [self._format_group(g, input_features, self._ht[g.ht_name].impl.device) for g in groups]
         outs = {}
-        direct = {}
-        for fea_name, fea in input_features.items():
-            if fea_name not in self._fea_to_ht:
-                direct[fea_name] = fea
-                continue
-            ht_name = self._fea_to_ht[fea_name]
-            group = self._groups[ht_name]
-            opt = self._emb_opts[fea_name]
-            dev = self._ht[ht_name].impl.device
-            ids, offsets, weight, n_seg, shape = self._format(fea, opt, dev)
-            grouped[ht_name][group.fea_runtime[fea_name]].append(dict(
-                name=fea_name, ids=ids, offsets=offsets, weight=weight, n_seg=n_seg, shape=shape, child=group.fea_child[fea_name],
-                opt=opt))
         self.packed = {}
         # pass 1: coalesce every (table, runtime group) and, when there are several, start the id phase of all of them before
         # anything waits (the reference issues all its id all-to-alls up front, embedding_engine.py:739-801)
-        n_groups = sum(len(r) for r in grouped.values())
+        n_groups = len(groups)
         plan = []
-        for ht_name, runtimes in grouped.items():
+        for group, feats in zip(groups, formatted):
+            ht_name, run_key = group.ht_name, group.run_key
             ht: DynamicEmbedding = self._ht[ht_name]
             dev = ht.impl.device
-            for run_key, feats in runtimes.items():
-                opt = feats[0]["opt"]
-                tile_len = opt.combiner_kwargs["tile_len"] if opt.combiner == "tile" else 0
-                segs = [f["n_seg"] for f in feats]
-                perm = None
-                if self._interleave and opt.combiner != "tile" and len(set(segs)) == 1 and len(feats) > 1:
-                    perm = (segs[0], len(feats))
-                lanes = self._use_lanes(ht, feats, opt, n_groups)
-                ids = offsets = weights = prepared = None
-                if not lanes:
-                    ids, offsets, weights = self._coalesce(feats, dev)
-                    if getattr(ht, "fused", None) is not None:
-                        ht.fused.lane_children[run_key] = frozenset(f["child"] for f in feats)
-                    if n_groups > 1:
-                        prepared = ht.prepare_lookup(ids, lane=run_key)
-                plan.append((ht_name, ht, dev, run_key, feats, opt, tile_len, segs, perm, lanes, ids, offsets, weights, prepared))
+            opt = self._emb_opts[group.names[0]]
+            tile_len = opt.combiner_kwargs["tile_len"] if opt.combiner == "tile" else 0
+            segs = feats.n_seg
+            perm = None
+            if self._interleave and opt.combiner != "tile" and len(segs) > 1 and segs.count(segs[0]) == len(segs):
+                perm = (segs[0], len(feats))
+            lanes = self._use_lanes(ht, feats, opt, n_groups)
+            ids = offsets = weights = prepared = None
+            if not lanes:
+                ids, offsets, weights = self._coalesce(feats, dev)
+                if getattr(ht, "fused", None) is not None:
+                    ht.fused.lane_children[run_key] = frozenset(feats.children)
+                if n_groups > 1:
+                    prepared = ht.prepare_lookup(ids, lane=run_key)
+            plan.append((ht_name, ht, dev, run_key, feats, opt, tile_len, segs, perm, lanes, ids, offsets, weights, prepared))
         # pass 1b (fused exchange with staging): every group's owner-side work and EMB signal before the first EMB wait
         for entry in plan:
             if entry[-1] is not None:
@@ -299,17 +362,18 @@ class EmbeddingEngine(nn.Module):
             D = opt.embedding_dim
             if perm is not None:
                 cube = pooled.view(segs[0], len(feats), D)
-                self.packed[(ht_name, run_key)] = (cube, [f["name"] for f in feats])
-                for j, f in enumerate(feats if views else ()):
-                    outs[f["name"]] = cube[:, j, :].reshape(f["shape"]) if len(f["shape"]) != 2 else cube[:, j, :]
+                self.packed[(ht_name, run_key)] = (cube, list(feats.names))
+                if views:
+                    for j, (name, shape) in enumerate(zip(feats.names, feats.shapes)):
+                        outs[name] = cube[:, j, :].reshape(shape) if len(shape) != 2 else cube[:, j, :]
             else:
-                rows_per = segs
                 pooled = pooled.view(-1, (tile_len or 1) * D)
                 start = 0
-                for f, s in zip(feats, rows_per):
-                    outs[f["name"]] = pooled[start:start + s].reshape(f["shape"])
+                for name, s, shape in zip(feats.names, segs, feats.shapes):
+                    outs[name] = pooled[start:start + s].reshape(shape)
                     start += s
-        for k, v in direct.items():
+        for k in direct:
+            v = input_features[k]
             if isinstance(v, RaggedTensor):
                 outs[k] = v.to_dense()
             elif isinstance(v, torch.Tensor) and v.is_sparse:

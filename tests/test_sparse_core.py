@@ -6,6 +6,7 @@ import torch
 
 import recis_b200
 from recis_b200.nn import EmbeddingEngine, EmbeddingOption, HashTable, filter_out_sparse_param, gen_slice
+from recis_b200.nn.modules.hashtable import ChildrenInfo, HashtableRegister
 from recis_b200.nn.hashtable_hook import AdmitHook, FilterHook
 from recis_b200.nn.initializers import ConstantInitializer, NormalInitializer, TruncNormalInitializer, UniformInitializer
 from recis_b200.optim import SparseAdagrad, SparseAdam, SparseAdamW, SparseAdamWTF
@@ -390,3 +391,42 @@ print("ok")
     env = dict(os.environ, RECIS_DEBUG_BOUNDS="1")
     out = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, env=env, timeout=300)
     assert out.returncode == 0 and "ok" in out.stdout, out.stdout + out.stderr
+
+
+@pytest.mark.parametrize("kind", ["ragged", "ragged_weighted", "dense2d", "dense1d", "int32", "strided", "mixed"])
+def test_engine_checks_plain_inputs_together_and_converts_the_rest(kind):
+    """Inputs that need no conversion are checked by one native call; other types, strides, shapes and mixtures of ragged and dense
+    features are converted one by one. Both give what the tables hold, pooled by hand."""
+    g = torch.Generator().manual_seed(5)
+    B, names = 7, ["a", "b", "c"]
+    HashtableRegister().clear()
+    opts = {n: EmbeddingOption(embedding_dim=8, shared_name=f"pi_{kind}_{n}", combiner="sum", use_weight=True, device=torch.device("cpu"),
+                               initializer=NormalInitializer(0.0, 1.0)) for n in names}
+    engine = EmbeddingEngine(opts, interleave=True)
+    feats, bags = {}, {}
+    for j, n in enumerate(names):
+        if kind.startswith("ragged") or (kind == "mixed" and j == 1) or kind in ("int32", "strided"):
+            lens = torch.randint(0, 4, (B,), generator=g)
+            ids = torch.randint(0, 50, (int(lens.sum()),), generator=g)
+            off = torch.zeros(B + 1, dtype=torch.int32)
+            off[1:] = lens.cumsum(0)
+            w = torch.rand(ids.numel(), generator=g) if kind == "ragged_weighted" and j != 1 else None
+            raw = ids.to(torch.int32) if kind == "int32" else torch.stack([ids, ids], 1)[:, 0] if kind == "strided" else ids
+            feats[n] = RaggedTensor(raw, [off.to(torch.int64) if kind == "int32" else off], w, dense_shape=(B, -1))
+            bags[n] = [(ids[off[b]:off[b + 1]], None if w is None else w[off[b]:off[b + 1]]) for b in range(B)]
+        else:
+            ids = torch.randint(0, 50, (B,) if kind == "dense1d" else (B, 2), generator=g)
+            feats[n] = ids
+            bags[n] = [(ids[b].reshape(-1), None) for b in range(B)]
+    out = engine(feats)
+    (cube, packed_names), = engine.packed.values()
+    assert packed_names == names and engine(feats, views=False) == {}
+    for j, n in enumerate(names):
+        table = engine.table_of(n)
+        child = table.table.children_info().child_index(f"pi_{kind}_{n}")
+        ref = torch.zeros(B, 8)
+        for b, (ids, w) in enumerate(bags[n]):
+            if ids.numel():
+                rows = table.impl.embedding_lookup(ChildrenInfo.encode(ids, child), readonly=True)[1]
+                ref[b] = (rows * (1.0 if w is None else w.unsqueeze(1))).sum(0)
+        assert torch.allclose(out[n], ref, atol=1e-5) and torch.equal(out[n], cube[:, j, :])
