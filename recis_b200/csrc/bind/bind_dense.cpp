@@ -312,18 +312,62 @@ std::tuple<Tensor, Tensor> layer_norm_fwd(const Tensor& x, const Tensor& gamma, 
 }
 
 // (dx fp32 [rows, H], dgamma [H], dbeta [H])
-std::tuple<Tensor, Tensor, Tensor> layer_norm_bwd(const Tensor& dy, const Tensor& x, const Tensor& stats, const Tensor& gamma) {
+std::tuple<Tensor, Tensor, Tensor> layer_norm_bwd(const Tensor& dy, const Tensor& x, const Tensor& stats, const Tensor& gamma, OptT dres) {
   TORCH_CHECK(dy.is_cuda() && dy.is_contiguous() && dy.sizes() == x.sizes() &&
               (dy.scalar_type() == torch::kFloat32 || dy.scalar_type() == torch::kBFloat16), "dy: contiguous fp32 or bf16, shaped like x");
+  const bool res = dres.has_value() && dres->defined();
+  TORCH_CHECK(!res || (dres->scalar_type() == torch::kFloat32 && dres->is_contiguous() && dres->sizes() == x.sizes() && dres->device() == x.device()),
+              "dres: contiguous fp32, shaped like x");
   c10::cuda::CUDAGuard g(x.device());
   const int64_t rows = x.size(0), H = x.size(1);
   auto dx = torch::empty_like(x);
   auto dgb = torch::zeros({2, H}, x.options());
   const int rc = rb_layer_norm_bwd(dy.data_ptr(), dy.scalar_type() == torch::kBFloat16, x.data_ptr<float>(), stats.data_ptr<float>(),
-                                   gamma.data_ptr<float>(), rows, (int)H, dx.data_ptr<float>(), dgb.data_ptr<float>(),
+                                   gamma.data_ptr<float>(), res ? dres->data_ptr<float>() : nullptr, rows, (int)H, dx.data_ptr<float>(), dgb.data_ptr<float>(),
                                    dgb.data_ptr<float>() + H, at::cuda::getCurrentCUDAStream());
   TORCH_CHECK(rc == 0, "layer_norm backward: hidden width must be a multiple of 4 and at most 1024");
   return {dx, dgb.select(0, 0), dgb.select(0, 1)};
+}
+
+// (x as bf16, its column sums fp32 [N])
+std::tuple<Tensor, Tensor> cast_colsum(const Tensor& x) {
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == torch::kFloat32 && x.is_contiguous() && x.dim() == 2, "cast_colsum: contiguous fp32 [M, N] on CUDA");
+  c10::cuda::CUDAGuard g(x.device());
+  auto y = torch::empty(x.sizes(), x.options().dtype(torch::kBFloat16));
+  auto db = torch::zeros({x.size(1)}, x.options());
+  const int rc = rb_cast_colsum(x.data_ptr<float>(), x.size(0), (int)x.size(1), y.data_ptr(), db.data_ptr<float>(), at::cuda::getCurrentCUDAStream());
+  if (rc == 1) {
+    y.copy_(x);
+    if (x.numel() > 0) relu_bwd_bias(y, y, false, db);
+    return {y, db};
+  }
+  TORCH_CHECK(rc == 0, "cast_colsum failed (code ", rc, ")");
+  return {y, db};
+}
+
+Tensor segment_mean_fwd(const Tensor& x, const Tensor& offsets) {
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == torch::kFloat32 && x.is_contiguous() && x.dim() == 2, "x: contiguous fp32 [tokens, hidden] on CUDA");
+  TORCH_CHECK(offsets.scalar_type() == torch::kInt32 && offsets.is_contiguous() && offsets.numel() >= 1 && offsets.device() == x.device(),
+              "offsets: int32 [batch + 1]");
+  c10::cuda::CUDAGuard g(x.device());
+  const int B = (int)offsets.numel() - 1;
+  auto out = torch::empty({B, x.size(1)}, x.options());
+  const int rc = rb_segment_mean_fwd(x.data_ptr<float>(), offsets.data_ptr<int32_t>(), B, (int)x.size(1), out.data_ptr<float>(),
+                                     at::cuda::getCurrentCUDAStream());
+  TORCH_CHECK(rc == 0, "segment_mean: hidden width must be a multiple of 4 and at most 1024");
+  return out;
+}
+
+Tensor segment_mean_bwd(const Tensor& d_out, const Tensor& offsets, int64_t T) {
+  TORCH_CHECK(d_out.is_cuda() && d_out.scalar_type() == torch::kFloat32 && d_out.is_contiguous() && d_out.dim() == 2 &&
+              d_out.size(0) == offsets.numel() - 1, "d_out: contiguous fp32 [batch, hidden]");
+  c10::cuda::CUDAGuard g(d_out.device());
+  const int B = (int)d_out.size(0);
+  auto dx = B > 0 ? torch::empty({T, d_out.size(1)}, d_out.options()) : torch::zeros({T, d_out.size(1)}, d_out.options());
+  const int rc = rb_segment_mean_bwd(d_out.data_ptr<float>(), offsets.data_ptr<int32_t>(), T, B, (int)d_out.size(1), dx.data_ptr<float>(),
+                                     at::cuda::getCurrentCUDAStream());
+  TORCH_CHECK(rc == 0, "segment_mean backward: hidden width must be a multiple of 4 and at most 1024");
+  return dx;
 }
 
 // (interest [B, H], lse [B]) of the target attention over packed sequences
@@ -367,7 +411,10 @@ void init_dense(py::module& m) {
   m.def("gemm_bf16_residual", &gemm_bf16_residual);
   m.def("gemm_dgrad_fused", &gemm_dgrad_fused, py::arg("dy"), py::arg("w"), py::arg("mask"), py::arg("db_out") = c10::nullopt);
   m.def("layer_norm_fwd", &layer_norm_fwd);
-  m.def("layer_norm_bwd", &layer_norm_bwd);
+  m.def("layer_norm_bwd", &layer_norm_bwd, py::arg("dy"), py::arg("x"), py::arg("stats"), py::arg("gamma"), py::arg("dres") = py::none());
+  m.def("cast_colsum", &cast_colsum);
+  m.def("segment_mean_fwd", &segment_mean_fwd);
+  m.def("segment_mean_bwd", &segment_mean_bwd);
   m.def("target_attention_fwd", &target_attention_fwd);
   m.def("target_attention_bwd", &target_attention_bwd);
   m.def("mlp_forward", &mlp_forward, py::arg("x"), py::arg("weights"), py::arg("biases"), py::arg("relu"),

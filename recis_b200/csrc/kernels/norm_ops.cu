@@ -5,7 +5,8 @@
 // backward: dx = rstd * (g - mean_H(g) - xhat * mean_H(g * xhat)) with g = dy * gamma and xhat = (x - mean) * rstd;
 //           dgamma = sum_rows dy * xhat and dbeta = sum_rows dy are accumulated in registers over the rows a warp visits,
 //           reduced over the warps of a block in shared memory and added to the (zeroed) outputs with one atomic per block
-//           and column. One pass over x and dy; torch's layer norm backward makes three (input gradient, then the two
+//           and column. A gradient that reaches x past the norm (the residual stream of a pre-norm layer) is added on the way out
+//           instead of by a pass of its own. One pass over x and dy; torch's layer norm backward makes three (input gradient, then the two
 //           weight gradients through a separate column reduction), see the reference's use of nn.LayerNorm in
 //           examples/seq2seq/transformer.py.
 //
@@ -95,8 +96,8 @@ layer_norm_fwd_kernel(const float* __restrict__ x, const float* __restrict__ gam
 template <int NV, typename InT>
 __global__ void __launch_bounds__(kWarps * 32)
 layer_norm_bwd_kernel(const InT* __restrict__ dy, const float* __restrict__ x, const float* __restrict__ stats,
-                      const float* __restrict__ gamma, int64_t rows, int H, float* __restrict__ dx, float* __restrict__ dgamma,
-                      float* __restrict__ dbeta) {
+                      const float* __restrict__ gamma, const float* __restrict__ dres, int64_t rows, int H, float* __restrict__ dx,
+                      float* __restrict__ dgamma, float* __restrict__ dbeta) {
   extern __shared__ float red[];                 // [kWarps][2][NV * 128]
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t warp = (int64_t)blockIdx.x * kWarps + w, n_warps = (int64_t)gridDim.x * kWarps;
@@ -109,37 +110,51 @@ layer_norm_bwd_kernel(const InT* __restrict__ dy, const float* __restrict__ x, c
     ab[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   const float inv_h = 1.f / (float)H;
-  for (int64_t r = warp; r < rows; r += n_warps) {
-    const float mean = stats[2 * r], rstd = stats[2 * r + 1];
-    const float* xr = x + r * H;
-    const InT* dr = dy + r * H;
-    float4 xh[NV], gd[NV];
-    float s1 = 0.f, s2 = 0.f;
+  // A warp's next row (with its residual gradient) is requested before the current one is reduced: the two shuffle reductions would
+  // otherwise stand between every row's loads and the next row's.
+  float4 nx[NV], nd[NV], ne[NV];
+  float2 ns = make_float2(0.f, 0.f);
+  auto fetch = [&](int64_t r) {
+    if (r >= rows) return;
+    ns = *reinterpret_cast<const float2*>(stats + 2 * r);
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int c = (i * 32 + lane) * 4;
-      if (c < H) {
-        const float4 xv = *reinterpret_cast<const float4*>(xr + c);
-        const float4 d = Io<InT>::ld(dr + c);
-        xh[i] = make_float4((xv.x - mean) * rstd, (xv.y - mean) * rstd, (xv.z - mean) * rstd, (xv.w - mean) * rstd);
-        gd[i] = make_float4(d.x * g[i].x, d.y * g[i].y, d.z * g[i].z, d.w * g[i].w);
-        s1 += gd[i].x + gd[i].y + gd[i].z + gd[i].w;
-        s2 += gd[i].x * xh[i].x + gd[i].y * xh[i].y + gd[i].z * xh[i].z + gd[i].w * xh[i].w;
-        ag[i].x += d.x * xh[i].x; ag[i].y += d.y * xh[i].y; ag[i].z += d.z * xh[i].z; ag[i].w += d.w * xh[i].w;
-        ab[i].x += d.x; ab[i].y += d.y; ab[i].z += d.z; ab[i].w += d.w;
-      } else {
-        xh[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        gd[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
+      const bool on = c < H;
+      nx[i] = on ? *reinterpret_cast<const float4*>(x + r * H + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      nd[i] = on ? Io<InT>::ld(dy + r * H + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      ne[i] = on && dres ? *reinterpret_cast<const float4*>(dres + r * H + c) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
+  };
+  constexpr bool kAhead = NV <= 4;                           // wider rows do not fit the registers twice
+  if (kAhead) fetch(warp);
+  for (int64_t r = warp; r < rows; r += n_warps) {
+    if (!kAhead) fetch(r);
+    const float mean = ns.x, rstd = ns.y;
+    float4 xh[NV], gd[NV], e[NV];
+    float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const float4 xv = nx[i], d = nd[i];                    // zero past H: every product below is then zero
+      e[i] = ne[i];
+      const bool on = (i * 32 + lane) * 4 < H;
+      xh[i] = on ? make_float4((xv.x - mean) * rstd, (xv.y - mean) * rstd, (xv.z - mean) * rstd, (xv.w - mean) * rstd) : make_float4(0.f, 0.f, 0.f, 0.f);
+      gd[i] = make_float4(d.x * g[i].x, d.y * g[i].y, d.z * g[i].z, d.w * g[i].w);
+      s1 += gd[i].x + gd[i].y + gd[i].z + gd[i].w;
+      s2 += gd[i].x * xh[i].x + gd[i].y * xh[i].y + gd[i].z * xh[i].z + gd[i].w * xh[i].w;
+      ag[i].x += d.x * xh[i].x; ag[i].y += d.y * xh[i].y; ag[i].z += d.z * xh[i].z; ag[i].w += d.w * xh[i].w;
+      ab[i].x += d.x; ab[i].y += d.y; ab[i].z += d.z; ab[i].w += d.w;
+    }
+    if (kAhead) fetch(r + n_warps);
     const float m1 = warp_sum(s1) * inv_h, m2 = warp_sum(s2) * inv_h;
     float* dxr = dx + r * H;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int c = (i * 32 + lane) * 4;
       if (c < H)
-        *reinterpret_cast<float4*>(dxr + c) = make_float4(rstd * (gd[i].x - m1 - xh[i].x * m2), rstd * (gd[i].y - m1 - xh[i].y * m2),
-                                                          rstd * (gd[i].z - m1 - xh[i].z * m2), rstd * (gd[i].w - m1 - xh[i].w * m2));
+        *reinterpret_cast<float4*>(dxr + c) =
+            make_float4(rstd * (gd[i].x - m1 - xh[i].x * m2) + e[i].x, rstd * (gd[i].y - m1 - xh[i].y * m2) + e[i].y,
+                        rstd * (gd[i].z - m1 - xh[i].z * m2) + e[i].z, rstd * (gd[i].w - m1 - xh[i].w * m2) + e[i].w);
     }
   }
   // weight gradients: warps of the block -> shared memory -> one atomic per column and block
@@ -213,6 +228,39 @@ relu_bwd_bias_vec_kernel(const __nv_bfloat16* __restrict__ y, const __nv_bfloat1
   }
 }
 
+// y = bf16(x) and db[n] += sum_m x[m, n]: the gradient of a residual addition on its way into a projection's backward, which needs it
+// as a bf16 operand and its column sums as the bias gradient. One pass (6 bytes per element) instead of a cast (6) and a column sum (2).
+__global__ void __launch_bounds__(256)
+cast_colsum_kernel(const float* __restrict__ x, int64_t M, int N, __nv_bfloat16* __restrict__ y, float* __restrict__ db, int groups_per_block) {
+  __shared__ float part[256 * 8];
+  const int grp = threadIdx.x % groups_per_block;
+  const int rlane = threadIdx.x / groups_per_block, rlanes = 256 / groups_per_block;
+  const int col = (blockIdx.x * groups_per_block + grp) * 8;
+  float acc[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+#pragma unroll 4
+  for (int64_t m = (int64_t)blockIdx.y * rlanes + rlane; m < M; m += (int64_t)gridDim.y * rlanes) {
+    const int64_t o = m * N + col;
+    const float4 a = *reinterpret_cast<const float4*>(x + o), b = *reinterpret_cast<const float4*>(x + o + 4);
+    acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
+    acc[4] += b.x; acc[5] += b.y; acc[6] += b.z; acc[7] += b.w;
+    uint4 u;
+    __nv_bfloat162* up = reinterpret_cast<__nv_bfloat162*>(&u);
+    up[0] = __floats2bfloat162_rn(a.x, a.y); up[1] = __floats2bfloat162_rn(a.z, a.w);
+    up[2] = __floats2bfloat162_rn(b.x, b.y); up[3] = __floats2bfloat162_rn(b.z, b.w);
+    *reinterpret_cast<uint4*>(y + o) = u;
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) part[(rlane * groups_per_block + grp) * 8 + j] = acc[j];
+  __syncthreads();
+  for (int c = threadIdx.x; c < groups_per_block * 8; c += 256) {
+    float s = 0.f;
+    for (int k = 0; k < rlanes; ++k) s += part[(k * groups_per_block) * 8 + c];
+    atomicAdd(db + blockIdx.x * groups_per_block * 8 + c, s);
+  }
+}
+
 int grid_rows(int64_t rows) { return (int)std::min<int64_t>(std::max<int64_t>((rows + kWarps - 1) / kWarps, 1), 148 * 8); }
 
 }  // namespace
@@ -235,9 +283,9 @@ int rb_layer_norm_fwd(const float* x, const float* gamma, const float* beta, int
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
-// dgamma and dbeta must be zero (or hold the value to accumulate onto) on entry
-int rb_layer_norm_bwd(const void* dy, int dy_bf16, const float* x, const float* stats, const float* gamma, int64_t rows, int H, float* dx,
-                      float* dgamma, float* dbeta, cudaStream_t st) {
+// dgamma and dbeta must be zero (or hold the value to accumulate onto) on entry; dres (nullable, [rows, H]) is added to dx
+int rb_layer_norm_bwd(const void* dy, int dy_bf16, const float* x, const float* stats, const float* gamma, const float* dres, int64_t rows, int H,
+                      float* dx, float* dgamma, float* dbeta, cudaStream_t st) {
   if (H % 4 != 0 || H > 1024 || H <= 0) return 1;
   if (rows <= 0) return 0;
   const int nv = (H + 127) / 128;
@@ -248,15 +296,28 @@ int rb_layer_norm_bwd(const void* dy, int dy_bf16, const float* x, const float* 
     if (dy_bf16) {                                                                                                                 \
       auto k = layer_norm_bwd_kernel<NV, __nv_bfloat16>;                                                                           \
       if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                       \
-      k<<<grid, kWarps * 32, smem, st>>>(reinterpret_cast<const __nv_bfloat16*>(dy), x, stats, gamma, rows, H, dx, dgamma, dbeta);  \
+      k<<<grid, kWarps * 32, smem, st>>>(reinterpret_cast<const __nv_bfloat16*>(dy), x, stats, gamma, dres, rows, H, dx, dgamma, dbeta);  \
     } else {                                                                                                                       \
       auto k = layer_norm_bwd_kernel<NV, float>;                                                                                   \
       if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                       \
-      k<<<grid, kWarps * 32, smem, st>>>(reinterpret_cast<const float*>(dy), x, stats, gamma, rows, H, dx, dgamma, dbeta);          \
+      k<<<grid, kWarps * 32, smem, st>>>(reinterpret_cast<const float*>(dy), x, stats, gamma, dres, rows, H, dx, dgamma, dbeta);          \
     }                                                                                                                              \
   }
   if (nv <= 1) RB_LN_BWD(1) else if (nv <= 2) RB_LN_BWD(2) else if (nv <= 4) RB_LN_BWD(4) else RB_LN_BWD(8)
 #undef RB_LN_BWD
+  rb::note_launch();
+  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+
+// db must be zero (or hold the value to accumulate onto) on entry. Returns 1 when the shape or alignment does not suit the kernel.
+int rb_cast_colsum(const float* x, int64_t M, int N, void* y, float* db, cudaStream_t st) {
+  if (N % 8 != 0 || M <= 0) return 1;
+  const int groups = N / 8;
+  if (groups >= 32 ? groups % 32 != 0 : (groups & (groups - 1)) != 0) return 1;       // whole blocks of column groups: a divisor of 256
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) return 1;
+  const int gpb = std::min(groups, 32), rlanes = 256 / gpb, gx = groups / gpb;
+  const int gy = (int)std::min<int64_t>(std::max<int64_t>(M / (rlanes * 4), 1), std::max(1, 148 * 8 / gx));
+  cast_colsum_kernel<<<dim3(gx, gy), 256, 0, st>>>(x, M, N, reinterpret_cast<__nv_bfloat16*>(y), db, gpb);
   rb::note_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }

@@ -135,6 +135,47 @@ target_attention_bwd_kernel(const float* __restrict__ x, const float* __restrict
   }
 }
 
+// Mean over each sequence's tokens: one block per sequence, a thread owns four columns of every rl-th token (rl = threads / (H / 4)), the
+// partial sums meet in shared memory. One read of x; with tensor ops it was an atomic scatter-add over the tokens (467 us for 269k
+// tokens x 256) and a gather plus division backward (190 us). Bound by the memory traffic of x and dx.
+__global__ void __launch_bounds__(256)
+segment_mean_fwd_kernel(const float* __restrict__ x, const int32_t* __restrict__ offsets, int H, float* __restrict__ out) {
+  __shared__ float4 part[256];
+  const int q = H >> 2, rl = 256 / q;
+  const int c = threadIdx.x % q, r = threadIdx.x / q;
+  const int b = blockIdx.x, beg = offsets[b], end = offsets[b + 1];
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (r < rl) {
+#pragma unroll 8
+    for (int t = beg + r; t < end; t += rl) {
+      const float4 v = rb::ld_f4(x + (int64_t)t * H + c * 4);
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+  }
+  part[threadIdx.x] = s;
+  __syncthreads();
+  if (r == 0) {
+    for (int k = 1; k < rl; ++k) { const float4 v = part[k * q + c]; s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w; }
+    const float n = (float)max(end - beg, 1);
+    rb::st_f4(out + (int64_t)b * H + c * 4, make_float4(s.x / n, s.y / n, s.z / n, s.w / n));
+  }
+}
+
+__global__ void __launch_bounds__(256)
+segment_mean_bwd_kernel(const float* __restrict__ d_out, const int32_t* __restrict__ offsets, int64_t T, int B, int H, float* __restrict__ dx) {
+  const int q = H >> 2, rl = 256 / q;
+  const int c = threadIdx.x % q, r = threadIdx.x / q;
+  if (r >= rl) return;
+  const int b = blockIdx.x, beg = offsets[b], end = offsets[b + 1];
+  const float n = (float)max(end - beg, 1);
+  float4 g = rb::ld_f4(d_out + (int64_t)b * H + c * 4);
+  g = make_float4(g.x / n, g.y / n, g.z / n, g.w / n);
+  for (int t = beg + r; t < end; t += rl) rb::st_f4(dx + (int64_t)t * H + c * 4, g);
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);                       // tokens of no sequence
+  if (b == 0) for (int t = r; t < beg; t += rl) rb::st_f4(dx + (int64_t)t * H + c * 4, zero);
+  if (b == B - 1) for (int64_t t = end + r; t < T; t += rl) rb::st_f4(dx + t * H + c * 4, zero);
+}
+
 template <typename F>
 bool dispatch_quads(int H, F&& f) {
   if (H % 4 != 0 || H > kMaxQuads * 128) return false;
@@ -170,4 +211,20 @@ extern "C" int rb_target_attention_bwd(const float* x, const float* q, const int
   });
   if (ok) rb::note_launch();
   return ok ? 0 : 1;
+}
+
+extern "C" int rb_segment_mean_fwd(const float* x, const int32_t* offsets, int B, int H, float* out, cudaStream_t st) {
+  if (H % 4 != 0 || H <= 0 || H > 1024) return 1;
+  if (B <= 0) return 0;
+  segment_mean_fwd_kernel<<<B, 256, 0, st>>>(x, offsets, H, out);
+  rb::note_launch();
+  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+
+extern "C" int rb_segment_mean_bwd(const float* d_out, const int32_t* offsets, int64_t T, int B, int H, float* dx, cudaStream_t st) {
+  if (H % 4 != 0 || H <= 0 || H > 1024) return 1;
+  if (B <= 0) return 0;
+  segment_mean_bwd_kernel<<<B, 256, 0, st>>>(d_out, offsets, T, B, H, dx);
+  rb::note_launch();
+  return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }

@@ -25,8 +25,8 @@ from torch import nn
 from ..nn import EmbeddingEngine, EmbeddingOption
 from ..nn.functional.ragged_ops import gen_segment_indices
 from ..nn.initializers import NormalInitializer
-from ..ops.attention import ragged_self_attention, target_attention
-from ..ops.dense import MLP, LayerNorm, Linear
+from ..ops.attention import ragged_self_attention, segment_mean, target_attention
+from ..ops.dense import MLP, LayerNorm, Linear, ffn_residual
 from ..ragged import RaggedTensor
 
 
@@ -50,17 +50,17 @@ class EncoderLayer(nn.Module):
         self.ffn = MLP([hidden, ffn, hidden], final_act=False, dtype=dtype)
 
     def forward(self, x, seg, pos, lengths, max_len, offsets=None):
-        # on CUDA the activations between the kernels stay bf16 and the two additions onto the fp32 residual stream happen in
-        # the epilogues of the projection GEMMs
-        h = self.norm1(x, out_bf16=x.is_cuda)
+        # on CUDA the activations between the kernels stay bf16, the two additions onto the fp32 residual stream happen in the
+        # epilogues of the projection GEMMs, and those of its gradient in the backward of the norms
+        h, x = self.norm1.forward_split(x, out_bf16=x.is_cuda)
         qkv = self.qkv(h)                                                      # [T, 3 * hidden] packed
         qkv = qkv.to(torch.bfloat16) if x.is_cuda else qkv.float()
         if offsets is None:
             offsets = torch.cat([lengths.new_zeros(1), lengths.cumsum(0)])
         o = ragged_self_attention(qkv, offsets, self.heads, max_len, seg, pos)
         x = self.proj.forward_residual(o, x)
-        f = self.ffn.layers[0](self.norm2(x, out_bf16=x.is_cuda))
-        return self.ffn.layers[1].forward_residual(f, x)
+        h, x = self.norm2.forward_split(x, out_bf16=x.is_cuda)
+        return ffn_residual(h, x, self.ffn.layers[0], self.ffn.layers[1])
 
 
 class SequenceModel(nn.Module):
@@ -120,7 +120,7 @@ class SequenceModel(nn.Module):
         for layer in self.layers:
             h = layer(h, seg, pos, lengths, max_len, offsets)
         h = self.final_norm(h)
-        pooled = torch.zeros(B, self.hidden, dtype=h.dtype, device=dev).index_add_(0, seg, h) / lengths.clamp_min(1)[:, None]
+        pooled = segment_mean(h, offsets, seg)
         profile = torch.cat([emb[f].view(B, -1) for f in self.profile_fields], dim=1) if self.profile_fields else h.new_zeros(B, 0)
         z = torch.cat([interest, pooled, q, profile], dim=1)
         logit = self.head(z)[:, :1].float()

@@ -72,6 +72,31 @@ def ragged_self_attention(qkv: torch.Tensor, offsets: torch.Tensor, heads: int, 
     return _padded(qkv, seg, pos, lengths, int(max_len), heads)
 
 
+class _SegmentMeanFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, offsets):
+        ctx.save_for_backward(offsets)
+        ctx.tokens = x.shape[0]
+        return native().segment_mean_fwd(x, offsets)
+
+    @staticmethod
+    def backward(ctx, d_out):
+        (offsets,) = ctx.saved_tensors
+        return native().segment_mean_bwd(d_out.contiguous(), offsets, ctx.tokens), None
+
+
+def segment_mean(x: torch.Tensor, offsets: torch.Tensor, seg: torch.Tensor = None) -> torch.Tensor:
+    """Mean of the packed tokens ``x`` [T, hidden] over each sequence (zeros for an empty one); ``offsets``: [B + 1]. On CUDA (fp32, hidden
+    a multiple of 4 up to 1024) one kernel per direction (``csrc/kernels/seq_ops.cu``), elsewhere tensor ops."""
+    hidden, B = x.shape[1], offsets.numel() - 1
+    if x.is_cuda and x.dtype == torch.float32 and 0 < hidden <= 1024 and hidden % 4 == 0:
+        return _SegmentMeanFn.apply(x.contiguous(), offsets.to(torch.int32).contiguous())
+    lengths = (offsets[1:] - offsets[:-1]).long()
+    if seg is None:
+        seg = torch.repeat_interleave(torch.arange(B, device=x.device), lengths)
+    return torch.zeros(B, hidden, dtype=x.dtype, device=x.device).index_add_(0, seg, x) / lengths.clamp_min(1)[:, None]
+
+
 class _TargetAttnFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, q, offsets, scale):

@@ -94,11 +94,71 @@ class _LinearResidualFn(torch.autograd.Function):
         C = native()
         x, wb = ctx.saved_tensors
         N, K = ctx.shape
-        dob = dout.to(torch.bfloat16).contiguous()
-        dy, db = C.relu_bwd_bias(dob, dob, False)
+        dy, db = C.cast_colsum(dout.contiguous())
         dx = C.gemm_bf16(dy, wb, None, False, False, True, False, None) if ctx.needs_input_grad[0] else None
         dw = C.gemm_bf16(dy, x, None, False, True, True, True, None)
         return dx, dw[:N, :K], db[:N], dout
+
+
+def _shadow_of(weight, Np, Kp):
+    wb = bf16_shadow(weight)
+    if wb is None:
+        wb = native().cast_pad_bf16(weight, Np, Kp)
+        keep_bf16_shadow(weight, wb)
+    return wb
+
+
+class _FFNResidualFn(torch.autograd.Function):
+    """out (fp32) = residual + relu(x W1^T + b1) W2^T + b2. As one function the backward's ReLU mask and first bias gradient come out of
+    the epilogue of the GEMM that produces the hidden gradient, instead of a pass over it and the hidden activations."""
+
+    @staticmethod
+    def forward(ctx, x, residual, w1, b1, w2, b2):
+        C = native()
+        wb1, wb2 = _shadow_of(w1, *w1.shape), _shadow_of(w2, *w2.shape)
+        h = C.gemm_bf16(x, wb1, b1, True, False, False, False, None)
+        ctx.save_for_backward(x, h, wb1, wb2)
+        return C.gemm_bf16_residual(h, wb2, b2, residual.contiguous())
+
+    @staticmethod
+    def backward(ctx, dout):
+        C = native()
+        x, h, wb1, wb2 = ctx.saved_tensors
+        dy, db2 = C.cast_colsum(dout.contiguous())
+        dw2 = C.gemm_bf16(dy, h, None, False, True, True, True, None)
+        dh, db1 = C.gemm_dgrad_fused(dy, wb2, h)
+        dw1 = C.gemm_bf16(dh, x, None, False, True, True, True, None)
+        dx = C.gemm_bf16(dh, wb1, None, False, False, True, False, None) if ctx.needs_input_grad[0] else None
+        return dx, dout, dw1, db1, dw2, db2
+
+
+def ffn_residual(x, residual, first: "Linear", second: "Linear"):
+    """``residual + second(relu(first(x)))`` in fp32, ``first`` being a layer with ReLU."""
+    ok = (x.is_cuda and first.act and not second.act and first.dtype == second.dtype == torch.bfloat16 and residual.dtype == torch.float32
+          and all(n % 8 == 0 for n in (first.in_features, first.out_features, second.out_features)) and x.dim() == 2
+          and x.shape[1] == first.in_features and second.in_features == first.out_features)
+    if ok:
+        return _FFNResidualFn.apply(x.to(torch.bfloat16).contiguous(), residual, first.weight, first.bias, second.weight, second.bias)
+    return second.forward_residual(first(x), residual)
+
+
+class _LayerNormSplitFn(torch.autograd.Function):
+    """``(layer_norm(x), x)``: the second output carries the residual stream, so that its gradient is added inside the backward kernel."""
+
+    @staticmethod
+    def forward(ctx, x, gamma, beta, eps, out_bf16):
+        y, stats = native().layer_norm_fwd(x, gamma, beta, eps, out_bf16)
+        ctx.save_for_backward(x, stats, gamma)
+        ctx.set_materialize_grads(False)
+        return y, x.view_as(x)
+
+    @staticmethod
+    def backward(ctx, dy, dres):
+        x, stats, gamma = ctx.saved_tensors
+        if dy is None:
+            return dres, None, None, None, None
+        dx, dgamma, dbeta = native().layer_norm_bwd(dy.contiguous(), x, stats, gamma, None if dres is None else dres.contiguous())
+        return dx, dgamma, dbeta, None, None
 
 
 class _LayerNormFn(torch.autograd.Function):
@@ -128,6 +188,15 @@ class LayerNorm(nn.LayerNorm):
             return _LayerNormFn.apply(x.contiguous(), self.weight, self.bias, self.eps, out_bf16)
         y = super().forward(x)
         return y.to(torch.bfloat16) if out_bf16 and x.is_cuda else y
+
+    def forward_split(self, x, out_bf16: bool = False):
+        """``(forward(x), x)`` for a pre-norm layer: use the returned ``x`` for the residual addition, and its gradient is added to the
+        norm's in one pass."""
+        H = x.shape[-1]
+        if (x.is_cuda and x.dim() == 2 and x.dtype == torch.float32 and H % 4 == 0 and H <= 1024 and self.elementwise_affine
+                and self.bias is not None):
+            return _LayerNormSplitFn.apply(x.contiguous(), self.weight, self.bias, self.eps, out_bf16)
+        return self.forward(x, out_bf16), x
 
 
 class Linear(nn.Module):

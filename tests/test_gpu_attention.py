@@ -157,3 +157,22 @@ def test_backward_over_many_items_isolates_sequences(longest, n, H):
         # one-token sequences have dq = dk = 0 exactly in theory: their error is measured against the scale of dv
         scale = b[:, sl].norm() if longest > 1 or name == "dv" else b[:, 2 * H * 64:].norm()
         assert (a[:, sl] - b[:, sl]).norm() / scale < 2e-2, name
+
+
+@pytest.mark.parametrize("lens,hidden", [([0, 5, 0, 1000, 1], 256), ([3] * 500, 8), ([700], 1024), ([1, 2, 3], 12), ([0], 64)])
+def test_segment_mean_matches_tensor_ops(lens, hidden):
+    """Means over packed sequences, forward and backward, with tokens around the sequences; fp32 sums of up to 1000 terms against 64 bits."""
+    from recis_b200.ops.attention import segment_mean
+    g = torch.Generator().manual_seed(hidden)
+    pre, post = 2, 3
+    T = pre + sum(lens) + post
+    offs = torch.tensor([pre] + lens).cumsum(0).to(torch.int32)
+    x, go = torch.randn(T, hidden, generator=g), torch.randn(len(lens), hidden, generator=g)
+    a = x.to(DEV).requires_grad_()
+    out = segment_mean(a, offs.to(DEV))
+    out.backward(go.to(DEV))
+    b = x.double().requires_grad_()
+    ref = torch.stack([b[offs[i]:offs[i + 1]].sum(0) / max(n, 1) for i, n in enumerate(lens)])
+    ref.backward(go.double())
+    assert (out.double().cpu() - ref).abs().max() < 1e-5
+    assert torch.allclose(a.grad.double().cpu(), b.grad, rtol=1e-6, atol=1e-7)

@@ -266,3 +266,40 @@ def test_fm_head_matches_tensor_ops(B, Nd, F, D, w):
     for a, b in zip(gpu, ref):
         if a.numel():
             assert (a.grad.double().cpu() - b.grad).abs().max() < 1e-5 * (float(b.grad.abs().max()) * max(B, Nd + F) ** 0.5 + mag ** 0.5), b.shape
+
+
+@pytest.mark.parametrize("M,N", [(1, 8), (5, 64), (77, 256), (3000, 256), (4097, 768), (100, 24), (33, 512)])
+def test_cast_with_column_sums(M, N):
+    """fp32 -> bf16 with the column sums of the fp32 values, on widths inside and outside the vector kernel's range. Sums of M terms."""
+    x = torch.randn(M, N, generator=torch.Generator().manual_seed(M)).cuda()
+    y, db = recis_b200.native().cast_colsum(x)
+    assert torch.equal(y, x.to(torch.bfloat16))
+    inside = (N // 8) % 32 == 0 if N >= 256 else ((N // 8) & (N // 8 - 1)) == 0
+    ref, mag = (x if inside else y.float()).double().sum(0), x.double().abs().sum(0)
+    assert ((db.double() - ref).abs() <= (M + 1) * 2.0 ** -24 * mag).all()
+
+
+@pytest.mark.parametrize("T,H,ffn", [(1, 64, 128), (300, 256, 1024), (1000, 128, 264)])
+def test_pre_norm_block_matches_separate_functions(T, H, ffn):
+    """LayerNorm with the residual gradient added in its backward, and the feed-forward block as one function, against the same layers
+    as separate functions. Both round the same operands to bf16 (so the ReLU masks agree); what differs is that the bias gradients sum
+    values before instead of after their rounding to bf16 (2^-9 each, independent) and the order of fp32 additions: 2^-8 of the norm."""
+    torch.manual_seed(T)
+    norm, l0, l1 = D.LayerNorm(H).cuda(), D.Linear(H, ffn, act=True).cuda(), D.Linear(ffn, H).cuda()
+    torch.nn.init.normal_(norm.weight, 1.0, 0.1)
+    x, go = torch.randn(T, H, device="cuda"), torch.randn(T, H, device="cuda")
+    params = [norm.weight, norm.bias, l0.weight, l0.bias, l1.weight, l1.bias]
+    a = x.clone().requires_grad_()
+    h, r = norm.forward_split(a, out_bf16=True)
+    out = D.ffn_residual(h, r, l0, l1)
+    got = torch.autograd.grad(out, [a] + params, go)
+    b = x.clone().requires_grad_()
+    ref_out = l1.forward_residual(l0(norm(b, out_bf16=True)), b)
+    ref = torch.autograd.grad(ref_out, [b] + params, go)
+    assert torch.equal(out, ref_out)
+    for p, q in zip(got, ref):
+        assert (p - q).norm() <= 2.0 ** -8 * q.norm(), p.shape
+    F = torch.nn.functional
+    only_norm = torch.autograd.grad(norm.forward_split(a)[0], a, go)[0]
+    only_res = torch.autograd.grad(norm.forward_split(a)[1], a, go)[0]
+    assert torch.equal(only_res, go) and (only_norm - torch.autograd.grad(F.layer_norm(b, (H,), norm.weight, norm.bias, norm.eps), b, go)[0]).abs().max() < 1e-4
