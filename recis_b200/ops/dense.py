@@ -252,7 +252,8 @@ class _MLPFn(torch.autograd.Function):
         saved = ctx.saved_tensors
         n = ctx.n
         xp, ys, wbs = saved[0], list(saved[1:1 + n]), list(saved[1 + n:1 + 2 * n])
-        dx, dws, dbs = native().mlp_backward(dout.to(torch.bfloat16), xp, ys, wbs, ctx.relu, ctx.shapes, ctx.needs_input_grad[0])
+        dx, dws, dbs = native().mlp_backward(dout.to(torch.bfloat16), xp, ys, wbs, ctx.relu, ctx.shapes, ctx.needs_input_grad[0],
+                                              ctx.x_dtype == torch.float32)
         if dx is not None and ctx.needs_input_grad[0]:
             dx = dx[:, :ctx.x_shape[1]].to(ctx.x_dtype)
         else:

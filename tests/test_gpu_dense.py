@@ -303,3 +303,18 @@ def test_pre_norm_block_matches_separate_functions(T, H, ffn):
     only_norm = torch.autograd.grad(norm.forward_split(a)[0], a, go)[0]
     only_res = torch.autograd.grad(norm.forward_split(a)[1], a, go)[0]
     assert torch.equal(only_res, go) and (only_norm - torch.autograd.grad(F.layer_norm(b, (H,), norm.weight, norm.bias, norm.eps), b, go)[0]).abs().max() < 1e-4
+
+
+@pytest.mark.parametrize("M,dims", [(1, [8, 16, 8]), (37, [100, 64, 1]), (1000, [480, 512, 256, 1]), (300, [264, 200])])
+def test_mlp_input_gradient_of_an_fp32_input(M, dims):
+    """An fp32 input gets the GEMM's fp32 accumulator as its gradient, a bf16 input the same rounded to bf16 (2^-9 relative, zero padding
+    cut off in both)."""
+    torch.manual_seed(M)
+    mlp = D.MLP(dims).cuda()
+    x = torch.randn(M, dims[0], device="cuda").to(torch.bfloat16)
+    a, b = x.float().requires_grad_(), x.clone().requires_grad_()
+    go = torch.randn(M, dims[-1], device="cuda").to(torch.bfloat16)
+    mlp(a).backward(go)
+    mlp(b).backward(go)
+    assert a.grad.dtype == torch.float32 and a.grad.shape == b.grad.shape == x.shape
+    assert torch.equal(a.grad.to(torch.bfloat16), b.grad) and not torch.equal(a.grad, b.grad.float())
