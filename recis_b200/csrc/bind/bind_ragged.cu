@@ -472,6 +472,8 @@ std::vector<Tensor> fused_hash(const std::vector<Tensor>& bytes, const std::vect
   return res;
 }
 
+// Boundaries that live on the host travel behind the descriptor table, in the same asynchronous copy (a copy of their own for every
+// feature, from pageable memory, is a synchronisation each).
 std::vector<Tensor> fused_bucketize(const std::vector<Tensor>& values, const std::vector<Tensor>& boundaries) {
   const int T = (int)values.size();
   TORCH_CHECK(T > 0 && (int)boundaries.size() == T);
@@ -479,15 +481,30 @@ std::vector<Tensor> fused_bucketize(const std::vector<Tensor>& values, const std
   c10::OptionalDeviceGuard guard(dev);
   std::vector<Tensor> v(T), bd(T);
   std::vector<std::vector<int64_t>> rows(4, std::vector<int64_t>(T + 1, 0));
+  const int64_t table_words = 4 * (int64_t)(T + 1);
+  int64_t words = table_words;                                       // of the upload: the table, then the host boundaries
+  std::vector<int64_t> at(T, -1);
   for (int t = 0; t < T; ++t) {
-    v[t] = values[t].to(torch::kFloat32).contiguous(); bd[t] = boundaries[t].to(dev, torch::kFloat32).contiguous();
+    v[t] = values[t].to(torch::kFloat32).contiguous();
+    const bool upload = dev.is_cuda() && boundaries[t].is_cpu();
+    bd[t] = upload ? boundaries[t].to(torch::kFloat32).contiguous() : boundaries[t].to(dev, torch::kFloat32).contiguous();
     rows[0][t] = (int64_t)v[t].data_ptr(); rows[1][t + 1] = rows[1][t] + v[t].numel();
     rows[2][t] = (int64_t)bd[t].data_ptr(); rows[3][t] = bd[t].numel();
+    if (upload) { at[t] = words; words += (bd[t].numel() + 1) / 2; }
   }
   const int64_t total = rows[1][T];
   auto out = torch::empty({total}, torch::TensorOptions().dtype(torch::kInt64).device(dev));
   if (dev.is_cuda()) {
-    auto desc = to_device_desc(rows, dev);
+    auto host = torch::empty({words}, torch::TensorOptions().dtype(torch::kInt64).pinned_memory(true));
+    auto desc = torch::empty({words}, torch::TensorOptions().dtype(torch::kInt64).device(dev));
+    int64_t* h = host.data_ptr<int64_t>();
+    for (int t = 0; t < T; ++t)
+      if (at[t] >= 0) {
+        rows[2][t] = (int64_t)(desc.data_ptr<int64_t>() + at[t]);
+        std::memcpy(h + at[t], bd[t].data_ptr<float>(), sizeof(float) * bd[t].numel());
+      }
+    for (int r = 0; r < 4; ++r) std::memcpy(h + r * (int64_t)(T + 1), rows[r].data(), sizeof(int64_t) * (T + 1));
+    desc.copy_(host, /*non_blocking=*/true);
     rb_fused_bucketize(desc.data_ptr<int64_t>(), T, total, out.data_ptr<int64_t>(), at::cuda::getCurrentCUDAStream());
   } else {
     int64_t* op = out.data_ptr<int64_t>();

@@ -166,3 +166,16 @@ def test_feature_cross_sorted_unique_matches_cpu():
     for r in (1, 7, 100):
         ux = xv[xo[r]:xo[r + 1]].unique().numel(); uy = yv[yo[r]:yo[r + 1]].unique().numel()
         assert int(ref[1][r + 1] - ref[1][r]) == ux * uy
+
+
+@pytest.mark.parametrize("sizes", [[1], [0, 3, 1], [200, 7, 2049, 1, 64]])
+def test_bucketize_boundaries_on_host_and_device(sizes):
+    """Boundary lists that travel with the descriptors (host memory; odd and even lengths, none at all) mixed with device-resident ones."""
+    import recis_b200
+    g = torch.Generator().manual_seed(len(sizes))
+    C = recis_b200.native()
+    bounds = [torch.randn(n, generator=g).sort().values for n in sizes]
+    vals = [torch.randn(50 * (i + 1) + 1, generator=g) for i in range(len(sizes))]
+    got = C.fused_bucketize([v.cuda() for v in vals], [b.cuda() if i % 2 else b for i, b in enumerate(bounds)])
+    for v, b, o in zip(vals, bounds, got):
+        assert torch.equal(o.cpu(), torch.bucketize(v, b, right=True))
