@@ -443,8 +443,10 @@ void init_dense(py::module& m) {
     TORCH_CHECK(offsets.is_cuda() && offsets.scalar_type() == torch::kInt32 && offsets.is_contiguous() && offsets.numel() >= 2);
     c10::cuda::CUDAGuard g(qkv.device());
     const int64_t T = qkv.size(0), B = offsets.numel() - 1;
-    auto out = torch::zeros({T, H * 64}, qkv.options());
-    auto lse = torch::zeros({T, H}, qkv.options().dtype(torch::kFloat32));
+    if (T == 0 || B <= 0 || H <= 0 || max_len <= 0)
+      return std::make_tuple(torch::zeros({T, H * 64}, qkv.options()), torch::zeros({T, H}, qkv.options().dtype(torch::kFloat32)));
+    auto out = torch::empty({T, H * 64}, qkv.options());                         // the kernel writes every row
+    auto lse = torch::empty({T, H}, qkv.options().dtype(torch::kFloat32));
     const int rc = rb_ragged_attention_fwd(qkv.data_ptr(), offsets.data_ptr<int32_t>(), T, (int)B, (int)H, (int)max_len, (float)scale,
                                            out.data_ptr(), lse.data_ptr<float>(), status_word(qkv.device()).data_ptr<int64_t>(),
                                            at::cuda::getCurrentCUDAStream());

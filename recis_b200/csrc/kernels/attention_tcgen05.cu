@@ -112,7 +112,7 @@ __device__ __forceinline__ float softmax_row(uint32_t trow, int valid, float sca
 }
 
 __global__ void __launch_bounds__(128, 2)
-ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const int32_t* __restrict__ offsets, int H, float scale_log2,
+ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const int32_t* __restrict__ offsets, int64_t T, int H, float scale_log2,
                             __nv_bfloat16* __restrict__ out, float* __restrict__ lse2, int64_t* __restrict__ status) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bar_q, bar_k, bar_v, bar_s, bar_o;
@@ -120,6 +120,18 @@ ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const i
   __shared__ int abort_flag;
   const int b = blockIdx.y, h = blockIdx.z, qt = blockIdx.x;
   const int s0 = offsets[b], L = offsets[b + 1] - s0;
+  // (Written here instead of clearing the whole output first: 39 us of 923 for 3000 short sequences, 8 heads.) Rows that no tile computes
+  // read as zeros: tokens in front of and behind the sequences, and those of a sequence that is longer than the
+  // bound the grid was sized with.
+  auto zero_rows = [&](int64_t from, int64_t to) {
+    for (int64_t row = from + (threadIdx.x >> 3); row < to; row += 16) {
+      reinterpret_cast<uint4*>(out + (row * H + h) * kHead)[threadIdx.x & 7] = make_uint4(0u, 0u, 0u, 0u);
+      if (lse2 && (threadIdx.x & 7) == 0) lse2[row * H + h] = 0.f;
+    }
+  };
+  if (qt == 0 && b == 0 && s0 > 0) zero_rows(0, s0);
+  if (qt == 0 && b == (int)gridDim.y - 1 && s0 + L < T) zero_rows(s0 + L, T);
+  if (qt == (int)gridDim.x - 1 && L > (qt + 1) * kTile) zero_rows((int64_t)s0 + (qt + 1) * kTile, (int64_t)s0 + L);
   if (qt * kTile >= L) return;                                   // uniform for the CTA, before any barrier or allocation
 
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -182,14 +194,16 @@ ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const i
 
     // ---- online softmax on this thread's row of S; only the sequence's last key tile can hold keys that do not exist
     const int valid = min(kTile, L - j * kTile);                 // key columns of this tile that exist
-    float alpha;
-    if (valid == kTile) alpha = softmax_row<false>(tmem + lane_base, kTile, scale_log2, t, ptile, m, l);
+    const int steps = (valid + 15) >> 4;                         // 16-key steps of the product with V
+    float alpha = 1.f;
+    if (qt * kTile + warp * 32 >= L) { /* none of this warp's rows exist: what their P holds only reaches rows that are not stored */ }
+    else if (valid == kTile) alpha = softmax_row<false>(tmem + lane_base, kTile, scale_log2, t, ptile, m, l);
     else alpha = softmax_row<true>(tmem + lane_base, valid, scale_log2, t, ptile, m, l);
 
     if (valid < kTile) {
       // last, partial tile: the V rows past the end of the sequence become zeros (this thread's row, once V has landed)
       ok = mbar_wait(&bar_v, ph, &abort_flag);
-      if (ok && t >= valid) {
+      if (ok && t >= valid && t < steps * 16) {
 #pragma unroll
         for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(vtile + swizzle128_offset(t, c * 8)) = make_uint4(0u, 0u, 0u, 0u);
       }
@@ -203,8 +217,7 @@ ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const i
       if (mbar_wait(&bar_v, ph, &abort_flag)) {
         fence_after_sync();
         const uint32_t sp = smem_u32(ptile), sv = smem_u32(vtile);
-#pragma unroll
-        for (int k = 0; k < kTile / 16; ++k)
+        for (int k = 0; k < steps; ++k)
           umma_bf16(tmem + 128u, make_desc(sp + (k >> 2) * kBlk + (k & 3) * 32, 16, 1024), make_desc(sv + k * 2048, kBlk, 1024), idesc_o,
                     k > 0 ? 1u : 0u);
         umma_commit(&bar_o);
@@ -777,7 +790,7 @@ extern "C" int rb_ragged_attention_fwd(const void* qkv, const int32_t* offsets, 
     attr = true;
   }
   dim3 grid((max_len + kTile - 1) / kTile, B, H);
-  ragged_attention_fwd_kernel<<<grid, 128, smem, st>>>(map_qkv, offsets, H, scale * 1.4426950408889634f,
+  ragged_attention_fwd_kernel<<<grid, 128, smem, st>>>(map_qkv, offsets, T, H, scale * 1.4426950408889634f,
                                                        reinterpret_cast<__nv_bfloat16*>(out), lse2, status);
   rb::note_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
