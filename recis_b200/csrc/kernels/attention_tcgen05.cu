@@ -322,8 +322,7 @@ attention_dq_store_kernel(const float* __restrict__ dq_acc, int64_t T, int cols,
 //   dQ  = dS K                                       (the dS tile read as a K-major A operand, K as an MN-major B)
 //
 // One persistent CTA per SM with separate roles: warps 0..7 compute (two threads per query row, each with two of the four chunks of 32
-// key columns), warp 8 fetches work and issues the TMA loads, warp 9 issues the MMAs. Work items come from a counter, four at a
-// time, so that sequences of very different length balance; K / V and Q / dO are double buffered across items, so the loads of the
+// key columns), warp 8 fetches work and issues the TMA loads, warp 9 issues the MMAs. Work items come from a counter, so that sequences of very different length balance; K / V and Q / dO are double buffered across items, so the loads of the
 // next item run under this one. The S and dP of step g + 1 are multiplied as soon as step g has them in registers, and the three
 // products of step g - 1 run while step g computes its exponentials. What shared memory has to move per step bounds it: 208 KB of
 // operand reads for the MMAs, 64 KB of P and dS, 32 KB of arriving tiles, 64 KB for dQ on its way out.
@@ -336,13 +335,15 @@ attention_dq_store_kernel(const float* __restrict__ dq_acc, int64_t T, int cols,
 // theirs) and converted by attention_dq_store_kernel.
 //
 // Measured on a B200 (this kernel alone; before: one CTA of 128 threads per item, loads / MMAs / exponentials one after the other):
-//   256 sequences of 50..1000 tokens, 4 heads:  807 -> 584 us (231 GFLOP in existing elements: 395 TFLOP/s)
+//   256 sequences of 50..1000 tokens, 4 heads:  807 -> 523 us (231 GFLOP in existing elements: 440 TFLOP/s)
 //   3000 sequences of 1..90 tokens, 8 heads:   1288 -> 407 us (2.2 GFLOP, 0.84 GB read and written: 2.1 TB/s; fixed cost per item)
 // and no zeroed fp32 gradient of q, k and v (413 MB resp. 826 MB of it) nor its conversion to bf16 around it any more.
 constexpr uint32_t kColS = 0, kColDP = 128, kColDV = 256, kColDK = 320, kColDQ = 384;
 constexpr int kBwdCompute = 8;                       // compute warps
 constexpr int kBwdThreads = (kBwdCompute + 4) * 32;  // and one warpgroup of control warps, two of them idle (register split below)
-constexpr int kBwdChunk = 4;                         // work items fetched at a time
+// Work items fetched at a time: four where an item is one step and a fetch would not hide behind it, one where items are up to many steps
+// long and a group of four made some SMs finish a sixth later than the rest (256 sequences of 50..1000 tokens: 585 -> 523 us).
+constexpr int kBwdChunkShort = 4, kBwdChunkLong = 1;
 
 // N key columns of one query row: pk = bf16 pairs of P, dk = bf16 pairs of dS. kMask: columns >= valid give exact zeros (S and dP
 // of rows and keys that do not exist can be anything, so both results are selected, not multiplied to zero).
@@ -401,6 +402,7 @@ ragged_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const _
   uint8_t* outstage = smem + 12 * kBlk;    // 4 KB per compute warp: results on their way out
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int kProducer = kBwdCompute, kMma = kProducer + 1;
+  constexpr int kChunk = kSingle ? kBwdChunkShort : kBwdChunkLong;
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
@@ -428,16 +430,16 @@ ragged_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const _
       // ------------------------------------------------------------------ work fetch + TMA producer
       const unsigned total = (unsigned)tiles * (unsigned)B * (unsigned)H;
       unsigned next = 0;
-      if (lane == 0) next = atomicAdd(counter, (unsigned)kBwdChunk);
+      if (lane == 0) next = atomicAdd(counter, (unsigned)kChunk);
       int it = 0, g = 0;
       bool ok = true;
       while (ok) {
         const unsigned base = __shfl_sync(0xffffffffu, next, 0);
         if (base >= total) break;
-        if (lane == 0) next = atomicAdd(counter, (unsigned)kBwdChunk);       // needed only after these items: its latency is hidden
+        if (lane == 0) next = atomicAdd(counter, (unsigned)kChunk);       // needed only after these items: its latency is hidden
         AttnItem mine{0, 0, 0, 0};
         const unsigned idx = base + (unsigned)lane;
-        bool have = lane < kBwdChunk && idx < total;
+        bool have = lane < kChunk && idx < total;
         if (have) {
           const unsigned bh = idx / (unsigned)tiles;
           const int b = (int)(bh / (unsigned)H);
