@@ -31,6 +31,16 @@ class DeepFM(nn.Module):
         self.dnn = MLP([(dense_dim + len(self.fields)) * emb_dim] + list(hidden) + [1], final_act=False, dtype=compute_dtype)
         self.loss_fn = nn.BCEWithLogitsLoss()
 
+    def _stacked(self, out, suffix):
+        """``[B, F, width]`` of one kind of feature: the engine's packed cube where it holds exactly these. At ``emb_dim`` 4 both kinds
+        share one table and one cube, a single field is not packed at all, and a field may be named twice: then a stack."""
+        names = [f + suffix for f in self.fields]
+        for cube, packed in self.embedding_engine.packed.values():
+            if packed == names:
+                return cube
+            out = {**out, **{n: cube[:, packed.index(n)] for n in names if n in packed}}
+        return torch.stack([out[n] for n in names], dim=1)
+
     def forward(self, batch: dict):
         dense, label = batch["dense"], batch["label"]
         feats = {}
@@ -39,12 +49,7 @@ class DeepFM(nn.Module):
             feats[f"{f}_bias"] = batch[f]
         out = self.embedding_engine(feats, views=False)
         B = dense.shape[0]
-        packed = {tuple(names): cube for cube, names in self.embedding_engine.packed.values()}        # [B, F, width], no stacking copy
-        emb, bias = packed.get(tuple(f"{f}_emb" for f in self.fields)), packed.get(tuple(f"{f}_bias" for f in self.fields))
-        if emb is None:
-            emb = torch.stack([out[f"{f}_emb"] for f in self.fields], dim=1)             # [B, F, D]
-        if bias is None:
-            bias = torch.stack([out[f"{f}_bias"] for f in self.fields], dim=1)           # [B, F, 4]
+        emb, bias = self._stacked(out, "_emb"), self._stacked(out, "_bias")              # [B, F, D], [B, F, 4]
         head = fm_head(dense, self.numeric_embs, self.numeric_bias, emb, bias) if self.dnn.dtype == torch.bfloat16 else None
         if head is not None:
             deep_in, linear = head

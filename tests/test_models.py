@@ -8,6 +8,7 @@ import sys
 import pytest
 import torch
 
+from recis_b200.models import DeepFM
 from recis_b200.models.seq_model import EncoderLayer, SequenceModel, segment_softmax
 from recis_b200.nn import filter_out_sparse_param
 from recis_b200.nn.modules.hashtable import HashtableRegister
@@ -69,6 +70,38 @@ def test_sequence_model_trains_on_cpu():
         do.zero_grad(); so.zero_grad(); loss.backward(); so.step(); do.step()
         losses.append(float(loss.detach()))
     assert logit.shape == (B, 1) and losses[-1] < 0.5 * losses[0]
+
+
+@pytest.mark.parametrize("device", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+@pytest.mark.parametrize("emb_dim,fields", [(4, "abc"), (4, "a"), (8, "abc"), (16, "a"), (16, "aba")])
+def test_deepfm_at_every_width_and_field_list(device, emb_dim, fields):
+    """Width 4 shares one table and one packed cube between embeddings and first-order weights; a single field is not packed; a field may
+    be named twice. Logits and gradients against the model's formula over the engine's per-feature results, in fp32 (sums of at most
+    6 * 16 fp32 terms: 1e-5; on CUDA the tower's operands are bf16: at most 12 roundings of 2^-9 one after the other, 2^-5 of the norm)."""
+    torch.manual_seed(emb_dim)
+    fields, B, dev = list(fields), 9, torch.device(device)
+    bf16 = dev.type == "cuda"
+    m = DeepFM(fields, dense_dim=3, emb_dim=emb_dim, hidden=(8, 16), device=dev, init_std=0.5,
+               compute_dtype=torch.bfloat16 if bf16 else torch.float32).to(dev)
+    batch = {f: torch.randint(0, 5, (B, 2), device=dev) for f in set(fields)}
+    batch["dense"], batch["label"] = torch.randn(B, 3, device=dev), (torch.rand(B, 1, device=dev) < 0.5).float()
+    params = [m.numeric_embs, m.numeric_bias] + list(m.dnn.parameters())
+    loss, logit = m(batch)
+    got = [logit] + list(torch.autograd.grad(loss, params))
+    m.eval()
+    out = m.embedding_engine({f + k: batch[f] for f in set(fields) for k in ("_emb", "_bias")})
+    cube = torch.cat([batch["dense"].unsqueeze(-1) * m.numeric_embs, torch.stack([out[f + "_emb"] for f in fields], 1)], 1)
+    first = (batch["dense"] * m.numeric_bias).sum(1, keepdim=True) + sum(out[f + "_bias"][:, :1] for f in fields)
+    s, h = cube.sum(1), cube.reshape(B, -1)
+    for i, layer in enumerate(m.dnn.layers):
+        h = torch.nn.functional.linear(h, layer.weight, layer.bias)
+        h = h.relu() if i < len(m.dnn.layers) - 1 else h
+    ref_logit = first + 0.5 * (s * s - (cube * cube).sum(1)).sum(1, keepdim=True) + h
+    ref = [ref_logit] + list(torch.autograd.grad(torch.nn.functional.binary_cross_entropy_with_logits(ref_logit, batch["label"]), params))
+    ref = [r.detach() for r in ref]
+    scale = max(float(r.norm()) for r in ref[1:])
+    for a, b in zip(got, ref):
+        assert (a - b).detach().norm() <= (2.0 ** -5 if bf16 else 1e-5) * max(float(b.norm()), scale), tuple(b.shape)
 
 
 def _run(script, *args):
