@@ -9,7 +9,7 @@ from torch import nn
 
 from ..nn import EmbeddingEngine, EmbeddingOption
 from ..nn.initializers import NormalInitializer
-from ..ops.dense import MLP, fm_head, fm_interaction
+from ..ops.dense import MLP, fm_head, fm_interaction, runs_plain
 
 
 class DeepFM(nn.Module):
@@ -33,8 +33,11 @@ class DeepFM(nn.Module):
 
     def _stacked(self, out, suffix):
         """``[B, F, width]`` of one kind of feature: the engine's packed cube where it holds exactly these. At ``emb_dim`` 4 both kinds
-        share one table and one cube, a single field is not packed at all, and a field may be named twice: then a stack."""
+        share one table and one cube, a single field is not packed at all, a field may be named twice, and a hook of the engine may have
+        put something else into its results: then a stack."""
         names = [f + suffix for f in self.fields]
+        if all(n in out for n in names):
+            return torch.stack([out[n] for n in names], dim=1)
         for cube, packed in self.embedding_engine.packed.values():
             if packed == names:
                 return cube
@@ -47,10 +50,12 @@ class DeepFM(nn.Module):
         for f in self.fields:
             feats[f"{f}_emb"] = batch[f]
             feats[f"{f}_bias"] = batch[f]
-        out = self.embedding_engine(feats, views=False)
+        views = {"views": False} if runs_plain(self.embedding_engine, EmbeddingEngine) else {}
+        out = self.embedding_engine(feats, **views)
         B = dense.shape[0]
         emb, bias = self._stacked(out, "_emb"), self._stacked(out, "_bias")              # [B, F, D], [B, F, 4]
-        head = fm_head(dense, self.numeric_embs, self.numeric_bias, emb, bias) if self.dnn.dtype == torch.bfloat16 else None
+        fused = runs_plain(self.dnn, MLP) and self.dnn.dtype == torch.bfloat16
+        head = fm_head(dense, self.numeric_embs, self.numeric_bias, emb, bias) if fused else None
         if head is not None:
             deep_in, linear = head
             logit = linear + self.dnn(deep_in)[:, :1].float()

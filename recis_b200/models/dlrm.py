@@ -9,7 +9,7 @@ from torch import nn
 
 from ..nn import EmbeddingEngine, EmbeddingOption
 from ..nn.initializers import NormalInitializer
-from ..ops.dense import MLP, dot_interaction
+from ..ops.dense import MLP, dot_interaction, runs_plain
 
 
 class DLRM(nn.Module):
@@ -36,8 +36,10 @@ class DLRM(nn.Module):
     def forward(self, batch: dict):
         dense = batch["dense"]
         label = batch["label"]
-        self.embedding_engine({f: batch[f] for f in self.fields}, views=False)
-        (cube, names), = self.embedding_engine.packed.values()      # [B, F, D] fp32, no stacking copy
+        engine = self.embedding_engine
+        views = {"views": False} if runs_plain(engine, EmbeddingEngine) else {}       # a hook gets every feature's result
+        engine({f: batch[f] for f in self.fields}, **views)
+        (cube, names), = engine.packed.values()      # [B, F, D] fp32, no stacking copy
         assert names == self.fields
         x = self.bottom(dense)                                        # [B, D] compute dtype
         z = dot_interaction(x, cube)                                  # [B, D + pairs] compute dtype

@@ -26,7 +26,7 @@ from ..nn import EmbeddingEngine, EmbeddingOption
 from ..nn.functional.ragged_ops import gen_segment_indices
 from ..nn.initializers import NormalInitializer
 from ..ops.attention import ragged_self_attention, segment_mean, target_attention
-from ..ops.dense import MLP, LayerNorm, Linear, ffn_residual
+from ..ops.dense import MLP, LayerNorm, Linear, ffn_residual, norm_residual_split
 from ..ragged import RaggedTensor
 
 
@@ -52,14 +52,14 @@ class EncoderLayer(nn.Module):
     def forward(self, x, seg, pos, lengths, max_len, offsets=None):
         # on CUDA the activations between the kernels stay bf16, the two additions onto the fp32 residual stream happen in the
         # epilogues of the projection GEMMs, and those of its gradient in the backward of the norms
-        h, x = self.norm1.forward_split(x, out_bf16=x.is_cuda)
+        h, x = norm_residual_split(self.norm1, x, out_bf16=x.is_cuda)
         qkv = self.qkv(h)                                                      # [T, 3 * hidden] packed
         qkv = qkv.to(torch.bfloat16) if x.is_cuda else qkv.float()
         if offsets is None:
             offsets = torch.cat([lengths.new_zeros(1), lengths.cumsum(0)])
         o = ragged_self_attention(qkv, offsets, self.heads, max_len, seg, pos)
         x = self.proj.forward_residual(o, x)
-        h, x = self.norm2.forward_split(x, out_bf16=x.is_cuda)
+        h, x = norm_residual_split(self.norm2, x, out_bf16=x.is_cuda)
         return ffn_residual(h, x, self.ffn.layers[0], self.ffn.layers[1])
 
 

@@ -39,6 +39,15 @@ def keep_bf16_shadow(weight: torch.Tensor, wb: torch.Tensor):
     weight._rb_bf16 = (wb, weight._version, weight.data_ptr())
 
 
+def runs_plain(module: nn.Module, cls: type) -> bool:
+    """Whether calling ``module`` does what ``cls.forward`` does and nothing else: not another type or an overridden ``forward``, and no
+    forward or backward hook, of its own or of all modules, that a caller who fuses ``module`` with its neighbours would pass by."""
+    m = nn.modules.module
+    return (isinstance(module, cls) and type(module).forward is cls.forward and "forward" not in module.__dict__
+            and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks
+                     or m._global_forward_hooks or m._global_forward_pre_hooks or m._global_backward_hooks or m._global_backward_pre_hooks))
+
+
 class _LinearFn(torch.autograd.Function):
     """y[M, Np] = act(x[M, Kp] W^T + b) with W given as fp32 [N, K] (padded + cast to bf16 here)."""
 
@@ -133,13 +142,20 @@ class _FFNResidualFn(torch.autograd.Function):
 
 
 def ffn_residual(x, residual, first: "Linear", second: "Linear"):
-    """``residual + second(relu(first(x)))`` in fp32, ``first`` being a layer with ReLU."""
-    ok = (x.is_cuda and first.act and not second.act and first.dtype == second.dtype == torch.bfloat16 and residual.dtype == torch.float32
+    """``residual + second(relu(first(x)))`` in fp32, ``first`` being a layer with ReLU. A ``first`` that is hooked or not a plain
+    ``Linear`` is called as a module."""
+    ok = (runs_plain(first, Linear) and type(second).forward_residual is Linear.forward_residual and x.is_cuda and first.act and not second.act and first.dtype == second.dtype == torch.bfloat16 and residual.dtype == torch.float32
           and all(n % 8 == 0 for n in (first.in_features, first.out_features, second.out_features)) and x.dim() == 2
           and x.shape[1] == first.in_features and second.in_features == first.out_features)
     if ok:
         return _FFNResidualFn.apply(x.to(torch.bfloat16).contiguous(), residual, first.weight, first.bias, second.weight, second.bias)
     return second.forward_residual(first(x), residual)
+
+
+def norm_residual_split(norm, x, out_bf16: bool = False):
+    """``(norm(x), x)`` at the head of a pre-norm block: use the returned ``x`` for the residual addition, and its gradient is added to the
+    norm's in one pass. A ``norm`` that is hooked or not a plain ``LayerNorm`` is called as a module."""
+    return norm.forward_split(x, out_bf16) if runs_plain(norm, LayerNorm) else (norm(x, out_bf16=out_bf16), x)
 
 
 class _LayerNormSplitFn(torch.autograd.Function):
@@ -190,8 +206,7 @@ class LayerNorm(nn.LayerNorm):
         return y.to(torch.bfloat16) if out_bf16 and x.is_cuda else y
 
     def forward_split(self, x, out_bf16: bool = False):
-        """``(forward(x), x)`` for a pre-norm layer: use the returned ``x`` for the residual addition, and its gradient is added to the
-        norm's in one pass."""
+        """``(forward(x), x)`` as one function (``norm_residual_split``)."""
         H = x.shape[-1]
         if (x.is_cuda and x.dim() == 2 and x.dtype == torch.float32 and H % 4 == 0 and H <= 1024 and self.elementwise_affine
                 and self.bias is not None):

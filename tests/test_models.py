@@ -8,7 +8,7 @@ import sys
 import pytest
 import torch
 
-from recis_b200.models import DeepFM
+from recis_b200.models import DLRM, DeepFM
 from recis_b200.models.seq_model import EncoderLayer, SequenceModel, segment_softmax
 from recis_b200.nn import filter_out_sparse_param
 from recis_b200.nn.modules.hashtable import HashtableRegister
@@ -102,6 +102,45 @@ def test_deepfm_at_every_width_and_field_list(device, emb_dim, fields):
     scale = max(float(r.norm()) for r in ref[1:])
     for a, b in zip(got, ref):
         assert (a - b).detach().norm() <= (2.0 ** -5 if bf16 else 1e-5) * max(float(b.norm()), scale), tuple(b.shape)
+
+
+@pytest.mark.parametrize("device", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+def test_hooks_see_every_module_call(device):
+    """Hooks of a model's modules fire and their changes count where the model fuses a module with its neighbours: the encoder's norms and
+    first feed-forward layer, the click models' embedding engine, DeepFM's tower (whose input stays fp32 and unpadded)."""
+    torch.manual_seed(0)
+    dev, dt = torch.device(device), torch.bfloat16 if device == "cuda" else torch.float32
+    layer = EncoderLayer(hidden=64, heads=1, ffn=128, dtype=dt).to(dev)
+    lens, offs, T = _ragged_batch()
+    x, lens, offs = torch.randn(T, 64, device=dev), lens.to(dev), offs.to(dev)
+    seg = torch.repeat_interleave(torch.arange(lens.numel(), device=dev), lens)
+    args = (seg, torch.arange(T, device=dev) - offs[:-1].long()[seg], lens.long(), 20, offs)
+    before, calls = layer(x, *args), []
+    for name, mod in (("norm1", layer.norm1), ("qkv", layer.qkv), ("norm2", layer.norm2), ("first", layer.ffn.layers[0])):
+        mod.register_forward_hook(lambda m, i, o, name=name: calls.append(name))
+    assert torch.equal(layer(x, *args), before) and calls == ["norm1", "qkv", "norm2", "first"]
+    zero = layer.ffn.layers[0].register_forward_pre_hook(lambda m, i: (i[0] * 0,))
+    silent = layer(x, *args)
+    zero.remove()
+    layer.norm2.register_forward_hook(lambda m, i, o: o * 0)
+    assert torch.equal(layer(x, *args), silent) and not torch.equal(silent, before)
+
+    fields, B = ["a", "b"], 5
+    batch = {f: torch.randint(0, 9, (B, 2), device=dev) for f in fields}
+    batch["dense"], batch["label"] = torch.randn(B, 13, device=dev), torch.zeros(B, 1, device=dev)
+    seen = {}
+    for m in (DLRM(fields, emb_dim=64, bottom=(64,), top=(8, 1), device=dev, compute_dtype=dt).to(dev),
+              DeepFM(fields, emb_dim=8, hidden=(8,), device=dev, init_std=1.0, compute_dtype=dt).to(dev)):
+        before = m(batch)[1]
+        hook = m.embedding_engine.register_forward_hook(lambda mod, i, o: seen.update({k: v.shape for k, v in o.items()}))
+        assert torch.allclose(m(batch)[1], before, rtol=1e-2, atol=1e-2)
+        hook.remove()
+    assert seen == {"a": (B, 64), "b": (B, 64), "a_emb": (B, 8), "b_emb": (B, 8), "a_bias": (B, 4), "b_bias": (B, 4)}
+    m.embedding_engine.register_forward_hook(lambda mod, i, o: {k: v * 0 for k, v in o.items()})
+    assert (m(batch)[1] - before).abs().max() > 0.1
+    m.dnn.register_forward_pre_hook(lambda mod, i: seen.update(tower=(i[0].shape, i[0].dtype)))
+    m(batch)
+    assert seen["tower"] == ((B, 15 * 8), torch.float32)
 
 
 def _run(script, *args):
