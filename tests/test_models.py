@@ -93,8 +93,9 @@ def test_deepfm_at_every_width_and_field_list(device, emb_dim, fields):
     cube = torch.cat([batch["dense"].unsqueeze(-1) * m.numeric_embs, torch.stack([out[f + "_emb"] for f in fields], 1)], 1)
     first = (batch["dense"] * m.numeric_bias).sum(1, keepdim=True) + sum(out[f + "_bias"][:, :1] for f in fields)
     s, h = cube.sum(1), cube.reshape(B, -1)
+    q = (lambda t: t.to(torch.bfloat16).float()) if bf16 else (lambda t: t)        # the same roundings, so that the ReLU masks agree
     for i, layer in enumerate(m.dnn.layers):
-        h = torch.nn.functional.linear(h, layer.weight, layer.bias)
+        h = q(torch.nn.functional.linear(q(h), q(layer.weight), layer.bias))
         h = h.relu() if i < len(m.dnn.layers) - 1 else h
     ref_logit = first + 0.5 * (s * s - (cube * cube).sum(1)).sum(1, keepdim=True) + h
     ref = [ref_logit] + list(torch.autograd.grad(torch.nn.functional.binary_cross_entropy_with_logits(ref_logit, batch["label"]), params))
