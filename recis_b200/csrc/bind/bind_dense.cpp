@@ -3,10 +3,12 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include "../kernels/rb_dense.h"
+#include "bind_shared.h"
 
 namespace py = pybind11;
 using torch::Tensor;
 using OptT = c10::optional<Tensor>;
+using rbx::aligned16;
 
 namespace {
 
@@ -108,7 +110,9 @@ Tensor fm_bwd(const Tensor& cube, const Tensor& gout) {
 }
 
 // (deep bf16 [B, ldp], lin fp32 [B, 1], sums fp32 [B, D]): see rb_fm_head_fwd
-std::tuple<Tensor, Tensor, Tensor> fm_head_fwd(const Tensor& dense, const Tensor& table, const Tensor& table_bias, const Tensor& emb, const Tensor& bias) {
+std::tuple<Tensor, Tensor, Tensor> fm_head_fwd(const Tensor& dense, const Tensor& table_in, const Tensor& table_bias, const Tensor& emb_in,
+                                               const Tensor& bias) {
+  const Tensor table = aligned16(table_in), emb = aligned16(emb_in);
   for (const Tensor* t : {&dense, &table, &table_bias, &emb, &bias})
     TORCH_CHECK(t->is_cuda() && t->scalar_type() == torch::kFloat32 && t->is_contiguous() && t->device() == dense.device(),
                 "fm_head: contiguous fp32 tensors on one CUDA device");
@@ -129,8 +133,9 @@ std::tuple<Tensor, Tensor, Tensor> fm_head_fwd(const Tensor& dense, const Tensor
 }
 
 // (d_emb, d_bias, d_table, d_table_bias)
-std::tuple<Tensor, Tensor, Tensor, Tensor> fm_head_bwd(const Tensor& dense, const Tensor& table, const Tensor& emb, const Tensor& sums, int64_t bias_w,
-                                                       const Tensor& g_deep, const Tensor& g_lin) {
+std::tuple<Tensor, Tensor, Tensor, Tensor> fm_head_bwd(const Tensor& dense, const Tensor& table_in, const Tensor& emb_in, const Tensor& sums,
+                                                       int64_t bias_w, const Tensor& g_deep_in, const Tensor& g_lin) {
+  const Tensor table = aligned16(table_in), emb = aligned16(emb_in), g_deep = aligned16(g_deep_in);
   const int64_t B = dense.size(0), Nd = dense.size(1), F = emb.size(1), D = emb.size(2);
   TORCH_CHECK(g_deep.is_cuda() && g_deep.scalar_type() == torch::kBFloat16 && g_deep.is_contiguous() && g_deep.dim() == 2 && g_deep.size(0) == B &&
               g_deep.size(1) >= (Nd + F) * D && g_lin.scalar_type() == torch::kFloat32 && g_lin.is_contiguous() && g_lin.numel() == B,
@@ -304,7 +309,8 @@ Tensor gemm_bf16_residual(const Tensor& a, const Tensor& b, OptT bias, const Ten
 }
 
 // (y [rows, H] bf16 or fp32, stats [rows, 2] = mean and rstd)
-std::tuple<Tensor, Tensor> layer_norm_fwd(const Tensor& x, const Tensor& gamma, const Tensor& beta, double eps, bool out_bf16) {
+std::tuple<Tensor, Tensor> layer_norm_fwd(const Tensor& x_in, const Tensor& gamma_in, const Tensor& beta_in, double eps, bool out_bf16) {
+  const Tensor x = aligned16(x_in), gamma = aligned16(gamma_in), beta = aligned16(beta_in);
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == torch::kFloat32 && x.is_contiguous() && x.dim() == 2, "x: contiguous fp32 [rows, hidden] on CUDA");
   const int64_t rows = x.size(0), H = x.size(1);
   TORCH_CHECK(gamma.scalar_type() == torch::kFloat32 && beta.scalar_type() == torch::kFloat32 && gamma.is_contiguous() && beta.is_contiguous() &&
@@ -319,18 +325,20 @@ std::tuple<Tensor, Tensor> layer_norm_fwd(const Tensor& x, const Tensor& gamma, 
 }
 
 // (dx fp32 [rows, H], dgamma [H], dbeta [H])
-std::tuple<Tensor, Tensor, Tensor> layer_norm_bwd(const Tensor& dy, const Tensor& x, const Tensor& stats, const Tensor& gamma, OptT dres) {
+std::tuple<Tensor, Tensor, Tensor> layer_norm_bwd(const Tensor& dy_in, const Tensor& x_in, const Tensor& stats, const Tensor& gamma_in, OptT dres_in) {
+  const Tensor dy = aligned16(dy_in), x = aligned16(x_in), gamma = aligned16(gamma_in);
   TORCH_CHECK(dy.is_cuda() && dy.is_contiguous() && dy.sizes() == x.sizes() &&
               (dy.scalar_type() == torch::kFloat32 || dy.scalar_type() == torch::kBFloat16), "dy: contiguous fp32 or bf16, shaped like x");
-  const bool res = dres.has_value() && dres->defined();
-  TORCH_CHECK(!res || (dres->scalar_type() == torch::kFloat32 && dres->is_contiguous() && dres->sizes() == x.sizes() && dres->device() == x.device()),
+  const bool res = dres_in.has_value() && dres_in->defined();
+  const Tensor dres = res ? aligned16(*dres_in) : Tensor();
+  TORCH_CHECK(!res || (dres.scalar_type() == torch::kFloat32 && dres.is_contiguous() && dres.sizes() == x.sizes() && dres.device() == x.device()),
               "dres: contiguous fp32, shaped like x");
   c10::cuda::CUDAGuard g(x.device());
   const int64_t rows = x.size(0), H = x.size(1);
   auto dx = torch::empty_like(x);
   auto dgb = torch::zeros({2, H}, x.options());
   const int rc = rb_layer_norm_bwd(dy.data_ptr(), dy.scalar_type() == torch::kBFloat16, x.data_ptr<float>(), stats.data_ptr<float>(),
-                                   gamma.data_ptr<float>(), res ? dres->data_ptr<float>() : nullptr, rows, (int)H, dx.data_ptr<float>(), dgb.data_ptr<float>(),
+                                   gamma.data_ptr<float>(), res ? dres.data_ptr<float>() : nullptr, rows, (int)H, dx.data_ptr<float>(), dgb.data_ptr<float>(),
                                    dgb.data_ptr<float>() + H, at::cuda::getCurrentCUDAStream());
   TORCH_CHECK(rc == 0, "layer_norm backward: hidden width must be a multiple of 4 and at most 1024");
   return {dx, dgb.select(0, 0), dgb.select(0, 1)};
@@ -352,7 +360,8 @@ std::tuple<Tensor, Tensor> cast_colsum(const Tensor& x) {
   return {y, db};
 }
 
-Tensor segment_mean_fwd(const Tensor& x, const Tensor& offsets) {
+Tensor segment_mean_fwd(const Tensor& x_in, const Tensor& offsets) {
+  const Tensor x = aligned16(x_in);
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == torch::kFloat32 && x.is_contiguous() && x.dim() == 2, "x: contiguous fp32 [tokens, hidden] on CUDA");
   TORCH_CHECK(offsets.scalar_type() == torch::kInt32 && offsets.is_contiguous() && offsets.numel() >= 1 && offsets.device() == x.device(),
               "offsets: int32 [batch + 1]");
@@ -365,7 +374,8 @@ Tensor segment_mean_fwd(const Tensor& x, const Tensor& offsets) {
   return out;
 }
 
-Tensor segment_mean_bwd(const Tensor& d_out, const Tensor& offsets, int64_t T) {
+Tensor segment_mean_bwd(const Tensor& d_out_in, const Tensor& offsets, int64_t T) {
+  const Tensor d_out = aligned16(d_out_in);
   TORCH_CHECK(d_out.is_cuda() && d_out.scalar_type() == torch::kFloat32 && d_out.is_contiguous() && d_out.dim() == 2 &&
               d_out.size(0) == offsets.numel() - 1, "d_out: contiguous fp32 [batch, hidden]");
   c10::cuda::CUDAGuard g(d_out.device());
@@ -378,7 +388,8 @@ Tensor segment_mean_bwd(const Tensor& d_out, const Tensor& offsets, int64_t T) {
 }
 
 // (interest [B, H], lse [B]) of the target attention over packed sequences
-std::tuple<Tensor, Tensor> target_attention_fwd(const Tensor& x, const Tensor& q, const Tensor& offsets, double scale) {
+std::tuple<Tensor, Tensor> target_attention_fwd(const Tensor& x_in, const Tensor& q_in, const Tensor& offsets, double scale) {
+  const Tensor x = aligned16(x_in), q = aligned16(q_in);
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == torch::kFloat32 && x.is_contiguous() && x.dim() == 2, "x: contiguous fp32 [tokens, hidden] on CUDA");
   TORCH_CHECK(q.scalar_type() == torch::kFloat32 && q.is_contiguous() && q.dim() == 2 && q.size(1) == x.size(1), "q: contiguous fp32 [batch, hidden]");
   TORCH_CHECK(offsets.scalar_type() == torch::kInt32 && offsets.is_contiguous() && offsets.numel() == q.size(0) + 1, "offsets: int32 [batch + 1]");
@@ -393,8 +404,9 @@ std::tuple<Tensor, Tensor> target_attention_fwd(const Tensor& x, const Tensor& q
 }
 
 // (dx [T, H], dq [B, H])
-std::tuple<Tensor, Tensor> target_attention_bwd(const Tensor& x, const Tensor& q, const Tensor& offsets, const Tensor& interest, const Tensor& lse,
-                                                const Tensor& d_interest, double scale) {
+std::tuple<Tensor, Tensor> target_attention_bwd(const Tensor& x_in, const Tensor& q_in, const Tensor& offsets, const Tensor& interest, const Tensor& lse,
+                                                const Tensor& d_interest_in, double scale) {
+  const Tensor x = aligned16(x_in), q = aligned16(q_in), d_interest = aligned16(d_interest_in);
   TORCH_CHECK(d_interest.scalar_type() == torch::kFloat32 && d_interest.is_contiguous() && d_interest.sizes() == interest.sizes());
   c10::cuda::CUDAGuard g(x.device());
   const int B = (int)q.size(0), H = (int)q.size(1);

@@ -31,6 +31,12 @@ inline torch::Tensor debug_prefix(const torch::Tensor& idx, const c10::optional<
   return idx.reshape({-1}).narrow(0, 0, n);
 }
 
+// `t`, or a copy of it where it does not start on a 16-byte line. For kernels that read rows as vectors: a contiguous tensor may be a
+// view at any element, and autograd hands such views in (the gradient of one part of a concatenation, for instance).
+inline torch::Tensor aligned16(const torch::Tensor& t) {
+  return t.is_cuda() && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) != 0 ? t.clone(at::MemoryFormat::Contiguous) : t;
+}
+
 // storage type code (RbRowDType) of a tensor of embedding rows; raises for anything but fp32 / fp16 / bf16 / int8
 inline int row_dtype_of(const torch::Tensor& t) {
   switch (t.scalar_type()) {

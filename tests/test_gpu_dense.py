@@ -318,3 +318,54 @@ def test_mlp_input_gradient_of_an_fp32_input(M, dims):
     mlp(b).backward(go)
     assert a.grad.dtype == torch.float32 and a.grad.shape == b.grad.shape == x.shape
     assert torch.equal(a.grad.to(torch.bfloat16), b.grad) and not torch.equal(a.grad, b.grad.float())
+
+
+def _at(t, first):
+    """The values of ``t`` as a contiguous view that starts ``first`` elements into a buffer."""
+    buf = torch.empty(t.numel() + first, dtype=t.dtype, device=t.device)
+    return buf[first:].copy_(t.reshape(-1)).view(t.shape)
+
+
+@pytest.mark.parametrize("first", [1, 2, 3])
+def test_vector_readers_take_views_at_any_element(first):
+    """Contiguous inputs and gradients that do not start on a 16-byte line (autograd hands such views in, see the concatenation) give the
+    bits of aligned ones: norm with and without the residual gradient, means and target attention over sequences, the DeepFM head. Weight
+    gradients meet in atomics: fp32 sums of 37 terms in any order."""
+    from recis_b200.ops.attention import segment_mean, target_attention
+    torch.manual_seed(first)
+    H, T = 64, 37
+    offs = torch.tensor([0, 5, 5, T], dtype=torch.int32, device=DEV)
+    x, q, go = torch.randn(T, H, device=DEV), torch.randn(3, H, device=DEV), torch.randn(3, H, device=DEV)
+    gy, gr = torch.randn(T, H, device=DEV), torch.randn(T, H, device=DEV)
+    w, b = torch.randn(H, device=DEV), torch.randn(H, device=DEV)
+    cube, bias, num = torch.randn(T, 3, 8, device=DEV), torch.randn(T, 3, 4, device=DEV), torch.randn(T, 2, device=DEV)
+    table, table_bias = torch.randn(2, 8, device=DEV), torch.randn(2, device=DEV)
+    g_deep, g_lin = torch.randn(T, 40, device=DEV).to(torch.bfloat16), torch.randn(T, 1, device=DEV)
+
+    def grads(place):
+        p = lambda t: place(t).detach().requires_grad_()
+        res = []
+        for dtype in (torch.float32, torch.bfloat16):
+            leaves = [p(x), p(w), p(b)]
+            y, r = D._LayerNormSplitFn.apply(*leaves, 1e-5, dtype == torch.bfloat16)
+            res += [y] + list(torch.autograd.grad([y, r], leaves, [place(gy.to(dtype)), place(gr)]))
+        leaves = [p(x), p(w), p(b)]
+        y = D._LayerNormFn.apply(*leaves, 1e-5, False)
+        res += [y] + list(torch.autograd.grad(y, leaves, place(gy)))
+        for fn, leaves in ((lambda a: segment_mean(a, offs), [p(x)]), (lambda a, c: target_attention(a, c, offs), [p(x), p(q)])):
+            y = fn(*leaves)
+            res += [y] + list(torch.autograd.grad(y, leaves, place(go)))
+        leaves = [p(table), p(table_bias), p(cube), p(bias)]
+        y = D._FMHeadFn.apply(place(num), *leaves)
+        return res + list(y) + list(torch.autograd.grad(y, leaves, [place(g_deep), place(g_lin)]))
+
+    for a, b_ in zip(grads(lambda t: _at(t, first)), grads(lambda t: t)):
+        if a.dim() == 1 and a.numel() == H:
+            assert torch.allclose(a, b_, rtol=1e-4, atol=1e-4)
+        else:
+            assert torch.equal(a, b_), tuple(a.shape)
+    # the same through autograd: what stands in front of a concatenation is an odd number of elements
+    norm, a = D.LayerNorm(H).to(DEV), x.clone().requires_grad_()
+    y, r = norm.forward_split(a)
+    (torch.cat([a.new_ones(first), r.reshape(-1), y.reshape(-1)]) * torch.arange(1., 1 + first + 2 * T * H, device=DEV)).sum().backward()
+    assert torch.isfinite(a.grad).all()
