@@ -171,9 +171,10 @@ std::tuple<Tensor, Tensor> comm_owner_reduce(const Tensor& rows_in, Tensor head,
 // Requester side of the backward exchange: reduce the pooled gradient to one gradient per unique id and store each of
 // them straight into the window of the rank that owns the id (peer stores). offsets = this rank's bucket boundaries
 // [world+1]; meta = the tensor written by comm_pull_ids (the destination bases sit at meta[2*world+1 ..]).
-void comm_grad_reduce_push(const Tensor& grad_out, const Tensor& gsrc, const Tensor& gscale, const Tensor& csr_u, const Tensor& csr_elem,
+void comm_grad_reduce_push(const Tensor& grad_in, const Tensor& gsrc, const Tensor& gscale, const Tensor& csr_u, const Tensor& csr_elem,
                            const Tensor& start, int64_t D, const Tensor& offsets, const Tensor& meta,
                            const std::vector<int64_t>& peer_gin, int64_t cap_rows, int64_t max_blocks) {
+  const Tensor grad_out = rbx::aligned16(grad_in);
   if (!grad_out.is_cuda()) {
     // host twin: per-unique gradients first (the CPU reduction), then one row copy per unique id into its owner's window
     TORCH_CHECK(grad_out.is_contiguous() && grad_out.scalar_type() == torch::kFloat32, "grad_out must be contiguous fp32");

@@ -272,10 +272,11 @@ std::tuple<Tensor, std::vector<std::vector<Tensor>>, std::vector<int64_t>> excha
 // Backward of exchange_forward_group: per lane, the element sort on the main stream, the NVLink-bound reduce + push on the
 // link stream behind an event, then the GRAD signal. saved[i] = (rev, gsrc, gscale, rows_in, prefix).
 void exchange_backward_group(std::vector<LanePtr> lanes, std::vector<std::vector<Tensor>> saved, std::vector<int64_t> epochs,
-                             const Tensor& grad_out, Tensor status, int64_t link_stream, int64_t max_blocks) {
+                             const Tensor& grad_in, Tensor status, int64_t link_stream, int64_t max_blocks) {
   const size_t L = lanes.size();
   TORCH_CHECK(saved.size() == L && epochs.size() == L);
-  TORCH_CHECK(grad_out.is_contiguous() && grad_out.scalar_type() == torch::kFloat32, "grad_out must be contiguous fp32");
+  TORCH_CHECK(grad_in.is_contiguous() && grad_in.scalar_type() == torch::kFloat32, "grad_out must be contiguous fp32");
+  const Tensor grad_out = rbx::aligned16(grad_in);
   ExLane& l0 = *lanes[0];
   c10::cuda::OptionalCUDAGuard guard;
   if (l0.cuda) guard.set_device(l0.flags.device());

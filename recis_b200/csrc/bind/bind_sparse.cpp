@@ -265,10 +265,11 @@ void fill_rows_i64(Tensor dst, const Tensor& rows, int64_t value) {
 
 // Pooling forward. Returns (out, gsrc, gscale); gsrc/gscale are empty tensors unless need_grad. With `out` given (a
 // [batch * perm_total, D] tensor shared by several calls) the call fills features perm_off .. perm_off + perm_f - 1 of it.
-std::tuple<Tensor, Tensor, Tensor> pool_forward(const Tensor& base, OptT rows, const Tensor& rev, const Tensor& offsets, OptT weights,
+std::tuple<Tensor, Tensor, Tensor> pool_forward(const Tensor& base_in, OptT rows, const Tensor& rev, const Tensor& offsets, OptT weights,
                                                 int64_t mode, int64_t perm_b, int64_t perm_f, bool need_grad, OptT out_opt,
                                                 int64_t perm_off, int64_t perm_total) {
-  TORCH_CHECK(base.dim() == 2 && base.is_contiguous());
+  TORCH_CHECK(base_in.dim() == 2 && base_in.is_contiguous());
+  const Tensor base = rbx::aligned16(base_in);
   const int base_dtype = rbx::row_dtype_of(base);
   TORCH_CHECK(rev.scalar_type() == torch::kInt32 && offsets.scalar_type() == torch::kInt32);
   const int64_t n_seg = offsets.numel() - 1, n = rev.numel(); const int D = (int)base.size(1);
@@ -311,9 +312,10 @@ std::tuple<Tensor, Tensor, Tensor> pool_forward(const Tensor& base, OptT rows, c
   return {out, gsrc, gscale};
 }
 
-std::tuple<Tensor, Tensor, Tensor> tile_forward(const Tensor& base, OptT rows, const Tensor& rev, const Tensor& offsets, OptT weights,
+std::tuple<Tensor, Tensor, Tensor> tile_forward(const Tensor& base_in, OptT rows, const Tensor& rev, const Tensor& offsets, OptT weights,
                                                 int64_t tile_len, bool need_grad) {
-  TORCH_CHECK(base.dim() == 2 && base.is_contiguous());
+  TORCH_CHECK(base_in.dim() == 2 && base_in.is_contiguous());
+  const Tensor base = rbx::aligned16(base_in);
   const int base_dtype = rbx::row_dtype_of(base);
   const int64_t n_seg = offsets.numel() - 1, n = rev.numel(); const int D = (int)base.size(1);
   auto f32 = base.options().dtype(torch::kFloat32);
@@ -365,10 +367,11 @@ using rbx::make_opt;
 
 // Per-unique gradient reduction. apply=false: returns gu [n_unique_max, D] (rows beyond the unique count are undefined).
 // apply=true: runs the optimizer on row rows[u] of (w, s1, s2) in the same kernel and returns an empty tensor.
-Tensor grad_reduce(const Tensor& grad_out, const Tensor& gsrc, const Tensor& gscale, const Tensor& csr_u, const Tensor& csr_elem,
+Tensor grad_reduce(const Tensor& grad_in, const Tensor& gsrc, const Tensor& gscale, const Tensor& csr_u, const Tensor& csr_elem,
                    const Tensor& start, int64_t D, OptT rows, bool apply, int64_t kind, double lr, double beta1, double beta2, double eps,
                    double decay, double alpha, double grad_scale, OptT w, OptT s1, OptT s2, int64_t n_unique_max, OptT gu_out) {
-  TORCH_CHECK(grad_out.is_contiguous() && grad_out.scalar_type() == torch::kFloat32, "grad_out must be contiguous fp32");
+  TORCH_CHECK(grad_in.is_contiguous() && grad_in.scalar_type() == torch::kFloat32, "grad_out must be contiguous fp32");
+  const Tensor grad_out = rbx::aligned16(grad_in);
   const int64_t n = csr_u.numel();
   RbOpt opt = make_opt(kind, lr, beta1, beta2, eps, decay, alpha, grad_scale, w, s1, s2);
   if (apply) TORCH_CHECK(opt.w != nullptr, "apply needs the weight slab");
@@ -390,9 +393,10 @@ Tensor grad_reduce(const Tensor& grad_out, const Tensor& gsrc, const Tensor& gsc
   return gu;
 }
 
-void sparse_apply(const Tensor& rows, const Tensor& grads, OptT n_dev, int64_t kind, double lr, double beta1, double beta2, double eps,
+void sparse_apply(const Tensor& rows, const Tensor& grads_in, OptT n_dev, int64_t kind, double lr, double beta1, double beta2, double eps,
                   double decay, double alpha, double grad_scale, Tensor w, OptT s1, OptT s2) {
-  TORCH_CHECK(rows.scalar_type() == torch::kInt32 && grads.is_contiguous() && grads.scalar_type() == torch::kFloat32);
+  TORCH_CHECK(rows.scalar_type() == torch::kInt32 && grads_in.is_contiguous() && grads_in.scalar_type() == torch::kFloat32);
+  const Tensor grads = rbx::aligned16(grads_in);
   const int64_t n = rows.numel(); const int D = (int)w.size(1);
   if (n == 0) return;
   rbx::debug_check_range("sparse_apply: rows", rbx::debug_prefix(rows, n_dev), -1, w.size(0));

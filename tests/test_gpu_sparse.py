@@ -346,3 +346,42 @@ def test_dedup_sizes_around_the_batched_probing(n, world):
     for w in range(world):
         a, b = int(offs[w]), int(offs[w + 1])
         assert torch.equal(torch.sort(uniq[a:b]).values.cpu(), torch.sort(ref[0][a:b]).values)
+
+
+@pytest.mark.parametrize("first", [1, 2, 3])
+def test_lookup_kernels_take_views_at_any_element(first):
+    """Rows and gradients that are contiguous but do not start on a 16-byte line give the bits of aligned ones; the packed result of an
+    engine behind an odd number of elements of a concatenation hands such a gradient in."""
+    def at(t):
+        return torch.empty(t.numel() + first, dtype=t.dtype, device=DEV)[first:].copy_(t.reshape(-1)).view(t.shape)
+    g = torch.Generator().manual_seed(first)
+    D, n, U, S = 16, 500, 90, 60
+    emb, grad = torch.randn(U, D, generator=g).to(DEV), torch.randn(S, D, generator=g).to(DEV)
+    rev = torch.unique(torch.randint(0, U, (n,), generator=g), return_inverse=True)[1].to(torch.int32).to(DEV)
+    offs = torch.linspace(0, n, S + 1).to(torch.int32).to(DEV)
+    csr, n_u = C.build_csr(rev), int(rev.max()) + 1
+    rows = torch.arange(n_u, dtype=torch.int32, device=DEV)
+    got = []
+    for place in (at, lambda t: t):
+        pooled, gsrc, gscale = C.pool_forward(place(emb), None, rev, offs, None, 0, 0, 0, True)
+        gu = C.grad_reduce(place(grad), gsrc, gscale, *csr, D, None, False, 2, 0.0, 0.0, 0.0, 0.0, 1.0, 0.0, 1.0, None, None, None, n_u)
+        w, s1, s2 = emb.clone(), torch.zeros_like(emb), torch.zeros_like(emb)
+        C.sparse_apply(rows, place(gu), None, 0, 0.01, 0.9, 0.999, 1e-8, 0.99, -0.02, 0.5, w, s1, s2)
+        got.append([pooled, C.tile_forward(place(emb), None, rev, offs, None, 2, True)[0], w])
+        half = place(emb.to(torch.bfloat16))
+        got[-1].append(C.pool_forward(half, None, rev, offs, None, 1, 0, 0, False)[0])
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    opts = {k: EmbeddingOption(embedding_dim=8, shared_name=k, combiner="sum", use_weight=False, device=torch.device(DEV),
+                               initializer=NormalInitializer(0.0, 1.0)) for k in "ab"}
+    engine = EmbeddingEngine(opts, interleave=True)
+    batch = {k: torch.randint(0, 9, (1, 3), device=DEV) for k in "ab"}
+    opt = SparseAdagrad(filter_out_sparse_param(engine), lr=0.1)
+    engine(batch)
+    (cube, _), = engine.packed.values()
+    before = cube.detach().clone()
+    torch.cat([cube.new_ones(1, first), cube.view(1, -1)], 1).sum().backward()
+    opt.step()
+    engine(batch)
+    (cube, _), = engine.packed.values()
+    assert torch.isfinite(cube).all() and (cube < before).all()
