@@ -360,7 +360,7 @@ std::tuple<Tensor, Tensor> cast_colsum(const Tensor& x) {
   return {y, db};
 }
 
-Tensor segment_mean_fwd(const Tensor& x_in, const Tensor& offsets) {
+Tensor segment_mean_fwd(const Tensor& x_in, const Tensor& offsets, int64_t longest) {
   const Tensor x = aligned16(x_in);
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == torch::kFloat32 && x.is_contiguous() && x.dim() == 2, "x: contiguous fp32 [tokens, hidden] on CUDA");
   TORCH_CHECK(offsets.scalar_type() == torch::kInt32 && offsets.is_contiguous() && offsets.numel() >= 1 && offsets.device() == x.device(),
@@ -368,20 +368,21 @@ Tensor segment_mean_fwd(const Tensor& x_in, const Tensor& offsets) {
   c10::cuda::CUDAGuard g(x.device());
   const int B = (int)offsets.numel() - 1;
   auto out = torch::empty({B, x.size(1)}, x.options());
-  const int rc = rb_segment_mean_fwd(x.data_ptr<float>(), offsets.data_ptr<int32_t>(), B, (int)x.size(1), out.data_ptr<float>(),
-                                     at::cuda::getCurrentCUDAStream());
+  auto partial = torch::empty({rb_segment_mean_pieces(x.size(0), longest) * 2, x.size(1)}, x.options());
+  const int rc = rb_segment_mean_fwd(x.data_ptr<float>(), offsets.data_ptr<int32_t>(), x.size(0), B, (int)x.size(1), longest,
+                                     partial.data_ptr<float>(), out.data_ptr<float>(), at::cuda::getCurrentCUDAStream());
   TORCH_CHECK(rc == 0, "segment_mean: hidden width must be a multiple of 4 and at most 1024");
   return out;
 }
 
-Tensor segment_mean_bwd(const Tensor& d_out_in, const Tensor& offsets, int64_t T) {
+Tensor segment_mean_bwd(const Tensor& d_out_in, const Tensor& offsets, int64_t T, int64_t longest) {
   const Tensor d_out = aligned16(d_out_in);
   TORCH_CHECK(d_out.is_cuda() && d_out.scalar_type() == torch::kFloat32 && d_out.is_contiguous() && d_out.dim() == 2 &&
               d_out.size(0) == offsets.numel() - 1, "d_out: contiguous fp32 [batch, hidden]");
   c10::cuda::CUDAGuard g(d_out.device());
   const int B = (int)d_out.size(0);
   auto dx = B > 0 ? torch::empty({T, d_out.size(1)}, d_out.options()) : torch::zeros({T, d_out.size(1)}, d_out.options());
-  const int rc = rb_segment_mean_bwd(d_out.data_ptr<float>(), offsets.data_ptr<int32_t>(), T, B, (int)d_out.size(1), dx.data_ptr<float>(),
+  const int rc = rb_segment_mean_bwd(d_out.data_ptr<float>(), offsets.data_ptr<int32_t>(), T, B, (int)d_out.size(1), longest, dx.data_ptr<float>(),
                                      at::cuda::getCurrentCUDAStream());
   TORCH_CHECK(rc == 0, "segment_mean backward: hidden width must be a multiple of 4 and at most 1024");
   return dx;
@@ -432,8 +433,8 @@ void init_dense(py::module& m) {
   m.def("layer_norm_fwd", &layer_norm_fwd);
   m.def("layer_norm_bwd", &layer_norm_bwd, py::arg("dy"), py::arg("x"), py::arg("stats"), py::arg("gamma"), py::arg("dres") = py::none());
   m.def("cast_colsum", &cast_colsum);
-  m.def("segment_mean_fwd", &segment_mean_fwd);
-  m.def("segment_mean_bwd", &segment_mean_bwd);
+  m.def("segment_mean_fwd", &segment_mean_fwd, py::arg("x"), py::arg("offsets"), py::arg("longest"));
+  m.def("segment_mean_bwd", &segment_mean_bwd, py::arg("d_out"), py::arg("offsets"), py::arg("T"), py::arg("longest"));
   m.def("target_attention_fwd", &target_attention_fwd);
   m.def("target_attention_bwd", &target_attention_bwd);
   m.def("mlp_forward", &mlp_forward, py::arg("x"), py::arg("weights"), py::arg("biases"), py::arg("relu"),

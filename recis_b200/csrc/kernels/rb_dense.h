@@ -114,9 +114,11 @@ int rb_layer_norm_bwd(const void* dy, int dy_bf16, const float* x, const float* 
 // y = bf16(x), db[n] += column sums of x (fp32 [M, N], N % 8 == 0); 1 = shape outside the kernel's range
 int rb_cast_colsum(const float* x, int64_t M, int N, void* y, float* db, cudaStream_t st);
 // Means over packed sequences (seq_ops.cu): out[b] = mean of x[offsets[b] .. offsets[b + 1]) (zero when empty), and its backward, which
-// writes all T rows of dx. fp32, H % 4 == 0, H <= 1024; 1 = outside that range.
-int rb_segment_mean_fwd(const float* x, const int32_t* offsets, int B, int H, float* out, cudaStream_t st);
-int rb_segment_mean_bwd(const float* d_out, const int32_t* offsets, int64_t T, int B, int H, float* dx, cudaStream_t st);
+// writes all T rows of dx. fp32, H % 4 == 0, H <= 1024; 1 = outside that range. longest: a bound of the lengths (it decides how the work is
+// split; longer sequences are still right); partial: rb_segment_mean_pieces(T, longest) * 2 * H floats of scratch.
+int64_t rb_segment_mean_pieces(int64_t T, int64_t longest);
+int rb_segment_mean_fwd(const float* x, const int32_t* offsets, int64_t T, int B, int H, int64_t longest, float* partial, float* out, cudaStream_t st);
+int rb_segment_mean_bwd(const float* d_out, const int32_t* offsets, int64_t T, int B, int H, int64_t longest, float* dx, cudaStream_t st);
 // ReLU backward + bias gradient with 16-byte accesses; returns 1 when the width does not suit it (not a multiple of 8, or neither
 // a power of two below 256 nor a multiple of 256), and the caller falls back to rb_relu_bwd_bias.
 int rb_relu_bwd_bias_vec(const void* y, const void* dout, int64_t M, int N, int relu, void* dy, float* db, cudaStream_t st);

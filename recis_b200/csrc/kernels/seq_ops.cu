@@ -13,6 +13,7 @@
 #include "../common/rb_common.cuh"
 #include "../common/rb_launch.h"
 #include "rb_dense.h"
+#include <climits>
 
 namespace {
 
@@ -137,41 +138,116 @@ target_attention_bwd_kernel(const float* __restrict__ x, const float* __restrict
 
 // Mean over each sequence's tokens: one block per sequence, a thread owns four columns of every rl-th token (rl = threads / (H / 4)), the
 // partial sums meet in shared memory. One read of x; with tensor ops it was an atomic scatter-add over the tokens (467 us for 269k
-// tokens x 256) and a gather plus division backward (190 us), now 73 and 60 us. Bound
-// by the memory traffic of x and dx.
-__global__ void __launch_bounds__(256)
-segment_mean_fwd_kernel(const float* __restrict__ x, const int32_t* __restrict__ offsets, int H, float* __restrict__ out) {
-  __shared__ float4 part[256];
-  const int q = H >> 2, rl = 256 / q;
-  const int c = threadIdx.x % q, r = threadIdx.x / q;
-  const int b = blockIdx.x, beg = offsets[b], end = offsets[b + 1];
+// tokens x 256) and a gather plus division backward (190 us), now 73 and 60 us. Bound by the memory traffic of x and dx.
+// One block reads about 57 GB/s, so sequences of more than kLongTokens are taken in pieces of kPiece tokens (cut at multiples of kPiece of the
+// packed matrix) by blocks of their own, and in forward a second launch adds each one's pieces in order. At 256 columns, forward and both
+// directions: one sequence of 100000 tokens 3604 -> 46 and 6850 -> 84 us, four of 5000 89 -> 19 and 173 -> 73 us. 512 sequences of 50..1000
+// tokens pay 9 us for the second launch when the caller gives no bound, nothing when it does.
+constexpr int kLongTokens = 1024, kPiece = 512;
+
+// Sum of the rows x[from], x[from + 1], .. x[to - 1] (of H floats) into the threads with r == 0; all threads of the block call it.
+__device__ __forceinline__ float4 block_sum_rows(const float* __restrict__ x, int64_t from, int64_t to, int H, int q, int c, int r, int rl, float4* part) {
   float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
   if (r < rl) {
 #pragma unroll 8
-    for (int t = beg + r; t < end; t += rl) {
-      const float4 v = rb::ld_f4(x + (int64_t)t * H + c * 4);
+    for (int64_t t = from + r; t < to; t += rl) {
+      const float4 v = rb::ld_f4(x + t * H + c * 4);
       s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
     }
   }
   part[threadIdx.x] = s;
   __syncthreads();
-  if (r == 0) {
+  if (r == 0)
     for (int k = 1; k < rl; ++k) { const float4 v = part[k * q + c]; s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w; }
+  __syncthreads();
+  return s;
+}
+
+// The sequence that holds token t, or -1: the last one that starts at or before t (empty ones share their start with it).
+__device__ __forceinline__ int sequence_of(const int32_t* __restrict__ offsets, int B, int64_t t) {
+  if (t < offsets[0] || t >= offsets[B]) return -1;
+  int lo = 0, hi = B;                                   // offsets[lo] <= t < offsets[hi]
+  while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (offsets[mid] <= t) lo = mid; else hi = mid; }
+  return lo;
+}
+
+// The long sequences in piece p: slot 0 is the one that holds its first token, slot 1 the one that starts inside and runs past its end.
+// (Two are all there can be: a sequence inside a piece is not long.) Returns the sequence or -1.
+__device__ __forceinline__ int long_sequence(const int32_t* __restrict__ offsets, int B, int64_t T, int64_t p, int slot, int long_tokens) {
+  const int b = sequence_of(offsets, B, slot == 0 ? p * kPiece : min((p + 1) * (int64_t)kPiece, T) - 1);
+  if (b < 0 || offsets[b + 1] - offsets[b] <= long_tokens || (slot == 1 && offsets[b] <= p * kPiece)) return -1;
+  return b;
+}
+
+// Blocks 0 .. B - 1: a sequence each; further blocks: a piece each (partial [pieces][2][H]). long_tokens: kLongTokens, or INT_MAX without pieces.
+__global__ void __launch_bounds__(256)
+segment_mean_fwd_kernel(const float* __restrict__ x, const int32_t* __restrict__ offsets, int64_t T, int B, int H, int long_tokens,
+                        float* __restrict__ partial, float* __restrict__ out) {
+  __shared__ float4 part[256];
+  const int q = H >> 2, rl = 256 / q;
+  const int c = threadIdx.x % q, r = threadIdx.x / q;
+  if (blockIdx.x < (unsigned)B) {
+    const int b = blockIdx.x, beg = offsets[b], end = offsets[b + 1];
+    if (end - beg > long_tokens) return;
+    const float4 s = block_sum_rows(x, beg, end, H, q, c, r, rl, part);
     const float n = (float)max(end - beg, 1);
-    rb::st_f4(out + (int64_t)b * H + c * 4, make_float4(s.x / n, s.y / n, s.z / n, s.w / n));
+    if (r == 0) rb::st_f4(out + (int64_t)b * H + c * 4, make_float4(s.x / n, s.y / n, s.z / n, s.w / n));
+    return;
+  }
+  const int64_t p = blockIdx.x - B, p0 = p * kPiece, p1 = p0 + kPiece;
+  for (int slot = 0; slot < 2; ++slot) {
+    const int b = long_sequence(offsets, B, T, p, slot, long_tokens);
+    if (b < 0) continue;                                // uniform for the block
+    const float4 s = block_sum_rows(x, max((int64_t)offsets[b], p0), min((int64_t)offsets[b + 1], p1), H, q, c, r, rl, part);
+    if (r == 0) rb::st_f4(partial + (2 * p + slot) * H + c * 4, s);
+  }
+}
+
+// One block per piece: finishes the long sequence that starts in it. Its pieces are slot 0 of every later piece, and slot 0 or 1 of this one.
+__global__ void __launch_bounds__(256)
+segment_mean_finish_kernel(const float* __restrict__ partial, const int32_t* __restrict__ offsets, int64_t T, int B, int H, int long_tokens,
+                           float* __restrict__ out) {
+  __shared__ float4 part[256];
+  const int q = H >> 2, rl = 256 / q;
+  const int c = threadIdx.x % q, r = threadIdx.x / q;
+  const int64_t p = blockIdx.x;
+  int b = long_sequence(offsets, B, T, p, 1, long_tokens);
+  const int slot = b >= 0 ? 1 : 0;
+  if (b < 0) {
+    b = long_sequence(offsets, B, T, p, 0, long_tokens);
+    if (b < 0 || offsets[b] != p * kPiece) return;
+  }
+  const int64_t last = ((int64_t)offsets[b + 1] - 1) / kPiece;
+  float4 s = block_sum_rows(partial, p + 1, last + 1, 2 * H, q, c, r, rl, part);
+  if (r == 0) {
+    const float4 f = rb::ld_f4(partial + (2 * p + slot) * H + c * 4);
+    const float n = (float)(offsets[b + 1] - offsets[b]);
+    rb::st_f4(out + (int64_t)b * H + c * 4, make_float4((f.x + s.x) / n, (f.y + s.y) / n, (f.z + s.z) / n, (f.w + s.w) / n));
   }
 }
 
 __global__ void __launch_bounds__(256)
-segment_mean_bwd_kernel(const float* __restrict__ d_out, const int32_t* __restrict__ offsets, int64_t T, int B, int H, float* __restrict__ dx) {
+segment_mean_bwd_kernel(const float* __restrict__ d_out, const int32_t* __restrict__ offsets, int64_t T, int B, int H, int long_tokens,
+                        float* __restrict__ dx) {
   const int q = H >> 2, rl = 256 / q;
   const int c = threadIdx.x % q, r = threadIdx.x / q;
   if (r >= rl) return;
+  auto spread = [&](int b, int64_t from, int64_t to) {
+    const float n = (float)max(offsets[b + 1] - offsets[b], 1);
+    float4 g = rb::ld_f4(d_out + (int64_t)b * H + c * 4);
+    g = make_float4(g.x / n, g.y / n, g.z / n, g.w / n);
+    for (int64_t t = from + r; t < to; t += rl) rb::st_f4(dx + t * H + c * 4, g);
+  };
+  if (blockIdx.x >= (unsigned)B) {
+    const int64_t p = blockIdx.x - B, p0 = p * kPiece, p1 = p0 + kPiece;
+    for (int slot = 0; slot < 2; ++slot) {
+      const int b = long_sequence(offsets, B, T, p, slot, long_tokens);
+      if (b >= 0) spread(b, max((int64_t)offsets[b], p0), min((int64_t)offsets[b + 1], p1));
+    }
+    return;
+  }
   const int b = blockIdx.x, beg = offsets[b], end = offsets[b + 1];
-  const float n = (float)max(end - beg, 1);
-  float4 g = rb::ld_f4(d_out + (int64_t)b * H + c * 4);
-  g = make_float4(g.x / n, g.y / n, g.z / n, g.w / n);
-  for (int t = beg + r; t < end; t += rl) rb::st_f4(dx + (int64_t)t * H + c * 4, g);
+  if (end - beg <= long_tokens) spread(b, beg, end);
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);                       // tokens of no sequence
   if (b == 0) for (int t = r; t < beg; t += rl) rb::st_f4(dx + (int64_t)t * H + c * 4, zero);
   if (b == B - 1) for (int64_t t = end + r; t < T; t += rl) rb::st_f4(dx + t * H + c * 4, zero);
@@ -214,18 +290,27 @@ extern "C" int rb_target_attention_bwd(const float* x, const float* q, const int
   return ok ? 0 : 1;
 }
 
-extern "C" int rb_segment_mean_fwd(const float* x, const int32_t* offsets, int B, int H, float* out, cudaStream_t st) {
+extern "C" int64_t rb_segment_mean_pieces(int64_t T, int64_t longest) {
+  return T > kLongTokens && longest > kLongTokens ? (T + kPiece - 1) / kPiece : 0;
+}
+
+extern "C" int rb_segment_mean_fwd(const float* x, const int32_t* offsets, int64_t T, int B, int H, int64_t longest, float* partial, float* out,
+                                   cudaStream_t st) {
   if (H % 4 != 0 || H <= 0 || H > 1024) return 1;
   if (B <= 0) return 0;
-  segment_mean_fwd_kernel<<<B, 256, 0, st>>>(x, offsets, H, out);
-  rb::note_launch();
+  const int64_t pieces = rb_segment_mean_pieces(T, longest);
+  const int long_tokens = pieces ? kLongTokens : INT_MAX;
+  segment_mean_fwd_kernel<<<(unsigned)(B + pieces), 256, 0, st>>>(x, offsets, T, B, H, long_tokens, partial, out);
+  if (pieces) segment_mean_finish_kernel<<<(unsigned)pieces, 256, 0, st>>>(partial, offsets, T, B, H, long_tokens, out);
+  rb::note_launch(pieces ? 2 : 1);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
-extern "C" int rb_segment_mean_bwd(const float* d_out, const int32_t* offsets, int64_t T, int B, int H, float* dx, cudaStream_t st) {
+extern "C" int rb_segment_mean_bwd(const float* d_out, const int32_t* offsets, int64_t T, int B, int H, int64_t longest, float* dx, cudaStream_t st) {
   if (H % 4 != 0 || H <= 0 || H > 1024) return 1;
   if (B <= 0) return 0;
-  segment_mean_bwd_kernel<<<B, 256, 0, st>>>(d_out, offsets, T, B, H, dx);
+  const int64_t pieces = rb_segment_mean_pieces(T, longest);
+  segment_mean_bwd_kernel<<<(unsigned)(B + pieces), 256, 0, st>>>(d_out, offsets, T, B, H, pieces ? kLongTokens : INT_MAX, dx);
   rb::note_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }

@@ -120,7 +120,7 @@ class SequenceModel(nn.Module):
         for layer in self.layers:
             h = layer(h, seg, pos, lengths, max_len, offsets)
         h = self.final_norm(h)
-        pooled = segment_mean(h, offsets, seg)
+        pooled = segment_mean(h, offsets, seg, max_len)
         profile = torch.cat([emb[f].view(B, -1) for f in self.profile_fields], dim=1) if self.profile_fields else h.new_zeros(B, 0)
         z = torch.cat([interest, pooled, q, profile], dim=1)
         logit = self.head(z)[:, :1].float()

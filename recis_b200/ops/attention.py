@@ -74,23 +74,24 @@ def ragged_self_attention(qkv: torch.Tensor, offsets: torch.Tensor, heads: int, 
 
 class _SegmentMeanFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, offsets):
+    def forward(ctx, x, offsets, longest):
         ctx.save_for_backward(offsets)
-        ctx.tokens = x.shape[0]
-        return native().segment_mean_fwd(x, offsets)
+        ctx.tokens, ctx.longest = x.shape[0], longest
+        return native().segment_mean_fwd(x, offsets, longest)
 
     @staticmethod
     def backward(ctx, d_out):
         (offsets,) = ctx.saved_tensors
-        return native().segment_mean_bwd(d_out.contiguous(), offsets, ctx.tokens), None
+        return native().segment_mean_bwd(d_out.contiguous(), offsets, ctx.tokens, ctx.longest), None, None
 
 
-def segment_mean(x: torch.Tensor, offsets: torch.Tensor, seg: torch.Tensor = None) -> torch.Tensor:
+def segment_mean(x: torch.Tensor, offsets: torch.Tensor, seg: torch.Tensor = None, max_len: int = None) -> torch.Tensor:
     """Mean of the packed tokens ``x`` [T, hidden] over each sequence (zeros for an empty one); ``offsets``: [B + 1]. On CUDA (fp32, hidden
-    a multiple of 4 up to 1024) one kernel per direction (``csrc/kernels/seq_ops.cu``), elsewhere tensor ops."""
+    a multiple of 4 up to 1024) one kernel per direction (``csrc/kernels/seq_ops.cu``), elsewhere tensor ops. ``max_len``: a bound of the
+    lengths if one is known; it saves a launch where it is small and changes nothing else."""
     hidden, B = x.shape[1], offsets.numel() - 1
     if x.is_cuda and x.dtype == torch.float32 and 0 < hidden <= 1024 and hidden % 4 == 0:
-        return _SegmentMeanFn.apply(x.contiguous(), offsets.to(torch.int32).contiguous())
+        return _SegmentMeanFn.apply(x.contiguous(), offsets.to(torch.int32).contiguous(), x.shape[0] if max_len is None else int(max_len))
     lengths = (offsets[1:] - offsets[:-1]).long()
     if seg is None:
         seg = torch.repeat_interleave(torch.arange(B, device=x.device), lengths)

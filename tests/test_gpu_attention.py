@@ -200,3 +200,26 @@ def test_forward_writes_every_row(lens, bound):
     assert torch.count_nonzero(got[~computed]) == 0 and torch.count_nonzero(lse[~computed]) == 0
     a, b = got[computed], ref[computed[pre:T - post]]
     assert (a - b).norm() / b.norm() < 1e-2 and (a - b).abs().max() < 3e-2 and torch.isfinite(lse).all()
+
+
+@pytest.mark.parametrize("hinted", [False, True])
+@pytest.mark.parametrize("lens,hidden,pre", [([1024, 1025], 64, 0), ([513, 1025, 511], 256, 0), ([1536], 128, 512), ([0, 5000, 0, 3, 4096, 0], 256, 7), ([1025] * 5, 1024, 511),
+                                             ([2, 1030, 506, 2000], 4, 0), ([1], 8, 3000)])
+def test_segment_mean_of_long_sequences(lens, hidden, pre, hinted):
+    """Sequences on both sides of the length from which they are taken in pieces, starting and ending at and beside the pieces' edges, with
+    tokens around them and a bound that holds or is too small. fp32 sums of up to 5000 terms in pieces, against 64 bits."""
+    from recis_b200.ops.attention import segment_mean
+    g = torch.Generator().manual_seed(hidden)
+    T = pre + sum(lens) + 5
+    offs = torch.tensor([pre] + lens).cumsum(0).to(torch.int32)
+    x, go = torch.randn(T, hidden, generator=g), torch.randn(len(lens), hidden, generator=g)
+    a = x.to(DEV).requires_grad_()
+    out = segment_mean(a, offs.to(DEV), max_len=1000 if hinted else None)
+    out.backward(go.to(DEV))
+    b = x.double().requires_grad_()
+    ref = torch.stack([b[offs[i]:offs[i + 1]].sum(0) / max(n, 1) for i, n in enumerate(lens)])
+    ref.backward(go.double())
+    assert (out.double().cpu() - ref).abs().max() < 1e-5
+    assert torch.allclose(a.grad.double().cpu(), b.grad, rtol=1e-6, atol=1e-9)
+    again = segment_mean(a, offs.to(DEV))
+    assert torch.equal(again, segment_mean(a, offs.to(DEV)))
