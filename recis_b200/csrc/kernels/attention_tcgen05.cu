@@ -330,9 +330,14 @@ attention_dq_store_kernel(const float* __restrict__ dq_acc, int64_t T, int cols,
 // neither computed nor written, and the reductions stop at the last 16 rows that hold one. (Left-over values in unwritten parts only
 // reach rows of the results that are not stored.)
 //
-// kSingle: every sequence fits one tile (the caller's bound on the length is at most 128), so dQ is complete after its only step
-// and leaves as bf16 from the registers. Otherwise dQ is added to an fp32 buffer with TMA add-reductions (other key tiles add
-// theirs) and converted by attention_dq_store_kernel.
+// kSingle: the caller's bound on the length is at most 128, so every query that the forward computed is in one tile: dQ leaves as bf16
+// from the registers. Otherwise dQ is added to an fp32 buffer with TMA add-reductions (other key tiles add theirs) and converted by
+// attention_dq_store_kernel.
+//
+// A sequence may be longer than the bound. The forward then computes the queries in the `tiles` tiles of the bound, over all keys, and
+// leaves zeros for the others. The same queries are walked here, for all key tiles (those past the bound belong to the item of the key tile
+// `tiles` below); the others get a zero dQ. With kSingle that is query tile 0 with one key tile after the other, whose dQ add up in
+// tensor memory until the last of them.
 //
 // Measured on a B200 (this kernel alone; before: one CTA of 128 threads per item, loads / MMAs / exponentials one after the other):
 //   256 sequences of 50..1000 tokens, 4 heads:  807 -> 523 us (231 GFLOP in existing elements: 440 TFLOP/s)
@@ -342,7 +347,9 @@ constexpr uint32_t kColS = 0, kColDP = 128, kColDV = 256, kColDK = 320, kColDQ =
 constexpr int kBwdCompute = 8;                       // compute warps
 constexpr int kBwdThreads = (kBwdCompute + 4) * 32;  // and one warpgroup of control warps, two of them idle (register split below)
 // Work items fetched at a time: four where an item is one step and a fetch would not hide behind it, one where items are up to many steps
-// long and a group of four made some SMs finish a sixth later than the rest (256 sequences of 50..1000 tokens: 585 -> 523 us).
+// long and a group of four made some SMs finish a sixth later than the rest (256 sequences of 50..1000 tokens: 585 -> 523 us). Which of the
+// two is chosen by the caller's bound, the only thing the host knows. Under a loose bound most items are empty and a single fetch costs more
+// (3000 sequences of 1..90 tokens, 8 heads: 0.46 ms under a bound of 90, 1.39 ms under 1000).
 constexpr int kBwdChunkShort = 4, kBwdChunkLong = 1;
 
 // N key columns of one query row: pk = bf16 pairs of P, dk = bf16 pairs of dS. kMask: columns >= valid give exact zeros (S and dP
@@ -419,6 +426,7 @@ ragged_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const _
   __syncthreads();
   fence_after_sync();
   const uint32_t tmem = tmem_slot;
+  auto query_tiles = [&](int len) { return kSingle ? 1 : min((len + kTile - 1) / kTile, tiles); };        // as many as the forward computed
   auto wait_all = [&](uint64_t* bar, uint32_t parity) -> bool {               // one outcome for the whole warp
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, &abort_flag) ? 1 : 0) != 0;
   };
@@ -458,7 +466,7 @@ ragged_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const _
           item.head = __shfl_sync(0xffffffffu, mine.head, src); item.kt = __shfl_sync(0xffffffffu, mine.kt, src);
           if (lane == 0) {
             const int xq = item.head * kHead, xk = (H + item.head) * kHead, xv = (2 * H + item.head) * kHead;
-            // (a sequence longer than the caller's bound is still covered: this item also takes the key tiles past the grid)
+            // (this item also takes the key tiles past the caller's bound)
             for (; item.kt * kTile < item.len && ok; item.kt += tiles, ++it) {
               const int st = it & 1;
               ok = mbar_wait(&kv_empty[st], (uint32_t)((it >> 1) & 1) ^ 1u, &abort_flag);
@@ -467,12 +475,12 @@ ragged_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const _
               mbar_expect_tx(&kv_full[st], 2 * kBlk);
               tma_load_2d(kvtiles + st * 2 * kBlk, &map_qkv, xk, item.s0 + item.kt * kTile, &kv_full[st]);
               tma_load_2d(kvtiles + st * 2 * kBlk + kBlk, &map_qkv, xv, item.s0 + item.kt * kTile, &kv_full[st]);
-              const int n_q = kSingle ? 1 : (item.len + kTile - 1) / kTile;
+              const int n_q = query_tiles(item.len);
               for (int i = 0; i < n_q && ok; ++i, ++g) {
                 const int buf = g & 1;
                 ok = mbar_wait(&in_empty[buf], (uint32_t)((g >> 1) & 1) ^ 1u, &abort_flag);
                 if (!ok) break;
-                const int row0 = item.s0 + (kSingle ? item.kt : i) * kTile;
+                const int row0 = item.s0 + i * kTile;
                 mbar_expect_tx(&in_full[buf], 2 * kBlk);
                 tma_load_2d(qotiles + buf * 2 * kBlk, &map_qkv, xq, row0, &in_full[buf]);
                 tma_load_2d(qotiles + buf * 2 * kBlk + kBlk, &map_do, xq, row0, &in_full[buf]);
@@ -497,7 +505,7 @@ ragged_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const _
       const uint32_t sp = smem_u32(ptile), sds = smem_u32(dstile);
       int g = 0;
       int p_st = 0, p_kq = 0, p_kk = 0;                 // the previous step: K / V stage, 16-row reduction steps over queries and keys
-      bool p_first = false, p_last = false;
+      bool p_first = false, p_last = false, p_dq_acc = false;
       auto products = [&](int gs) -> bool {             // dV, dK, dQ of step gs
         if (!mbar_wait(&p_full, (uint32_t)(gs & 1), &abort_flag)) return false;
         if (gs > 0 && !mbar_wait(&post_empty, (uint32_t)((gs - 1) & 1), &abort_flag)) return false;
@@ -515,7 +523,7 @@ ragged_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const _
           d_p += 128; d_ds += 128; d_do += 128; d_q += 128; acc = 1u;
         }
         uint64_t d_k = make_desc(sk, kBlk, 1024);
-        acc = 0u;
+        acc = p_dq_acc ? 1u : 0u;
 #pragma unroll 1
         for (int k = 0; k < p_kk; ++k) {                // reduction over the keys of the tile: dS read K-major, K read MN-major
           umma_bf16(tmem + kColDQ, make_desc(sds, 16, 1024) + (uint64_t)((k >> 2) * (kBlk >> 4) + (k & 3) * 2), d_k, idesc_km, acc);
@@ -534,7 +542,7 @@ ragged_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const _
         const AttnItem item = slot[st];
         if (item.len < 0) break;
         const uint32_t sk = smem_u32(kvtiles + st * 2 * kBlk);
-        const int n_q = kSingle ? 1 : (item.len + kTile - 1) / kTile;
+        const int n_q = query_tiles(item.len);
         for (int i = 0; i < n_q; ++i, ++g) {
           ok = mbar_wait(&in_full[g & 1], (uint32_t)((g >> 1) & 1), &abort_flag) &&
                (g == 0 || mbar_wait(&s_empty, (uint32_t)((g - 1) & 1), &abort_flag));
@@ -550,8 +558,8 @@ ragged_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const _
           }
           umma_commit(&s_full);
           if (g > 0) { ok = products(g - 1); if (!ok) break; }
-          p_st = st; p_first = i == 0; p_last = i == n_q - 1;
-          p_kq = (min(kTile, item.len - (kSingle ? item.kt : i) * kTile) + 15) >> 4;
+          p_st = st; p_first = i == 0; p_last = i == n_q - 1; p_dq_acc = kSingle && item.kt > 0;
+          p_kq = (min(kTile, item.len - i * kTile) + 15) >> 4;
           p_kk = (min(kTile, item.len - item.kt * kTile) + 15) >> 4;
         }
       }
@@ -569,7 +577,7 @@ ragged_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const _
     // The step whose products are still running: where its dQ goes, and (after the last step of an item) its keys. Row counts are
     // those of this warp's 32 rows and may be <= 0. A warp takes 32 of the 64 columns of each result.
     int p_row0 = 0, p_vq = 0, p_head = 0, p_key0 = 0, p_vk = 0;
-    bool p_last = false;
+    bool p_last = false, p_zero_q = false;                // p_zero_q: the key rows are no query rows of this pass (kSingle past the first tile)
     // 32 bf16 columns of the warp's first `valid` rows to global memory through a 2 KB corner of its box, four lanes per row and
     // eight rows per store instruction (a thread per row would touch 32 lines with each).
     auto stage16 = [&](uint32_t at, const uint32_t (&r)[32]) {
@@ -614,6 +622,9 @@ ragged_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const _
         __nv_bfloat16* kdst = dqkv + (int64_t)p_key0 * ld + (H + p_head) * kHead + half * 32;
         copy_out(box, kdst, p_vk);
         copy_out(box + 2048u, kdst + H * kHead, p_vk);
+        if (kSingle && p_zero_q)
+          for (int row = lane >> 2; row < min(p_vk, 32); row += 8)
+            reinterpret_cast<uint4*>(kdst - H * kHead + (int64_t)row * ld)[lane & 3] = make_uint4(0u, 0u, 0u, 0u);
         __syncwarp();
       }
       if (p_vq <= 0) return;
@@ -655,17 +666,16 @@ ragged_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const _
         i = 0;
         more = item.len >= 0;
         if (more) {
-          n_q = kSingle ? 1 : (item.len + kTile - 1) / kTile;
+          n_q = query_tiles(item.len);
           valid_k = min(kTile, item.len - item.kt * kTile);
-          const int q = (kSingle ? item.kt : 0) * kTile + row;
-          if (q < item.len) {
-            const int64_t at = (int64_t)(item.s0 + q) * H + item.head;
+          if (row < item.len) {
+            const int64_t at = (int64_t)(item.s0 + row) * H + item.head;
             lse_next = lse2[at];
             delta_next = delta[at];
           }
         }
       }
-      const int q0 = (kSingle ? item.kt : i) * kTile;
+      const int q0 = i * kTile;
       const int valid_q = min(kTile, item.len - q0);
       if (more) {
         const int read_k = (valid_k + 15) & ~15;                              // keys that the reduction of dQ reads
@@ -759,6 +769,10 @@ ragged_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const _
       }
       if (g > 0) post();
       p_row0 = item.s0 + q0 + quarter * 32; p_vq = valid_q - quarter * 32; p_head = item.head; p_last = i == n_q - 1;
+      if (kSingle) {
+        p_zero_q = item.kt > 0;
+        if ((item.kt + 1) * kTile < item.len) p_vq = 0;                       // dQ goes on with the next key tile
+      }
       p_key0 = item.s0 + item.kt * kTile + quarter * 32; p_vk = valid_k - quarter * 32;
       ++i; ++g;
     }

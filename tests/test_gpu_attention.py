@@ -223,3 +223,28 @@ def test_segment_mean_of_long_sequences(lens, hidden, pre, hinted):
     assert torch.allclose(a.grad.double().cpu(), b.grad, rtol=1e-6, atol=1e-9)
     again = segment_mean(a, offs.to(DEV))
     assert torch.equal(again, segment_mean(a, offs.to(DEV)))
+
+
+@pytest.mark.parametrize("lens,bound,H", [([200, 128, 31], 100, 2), ([5, 300, 129, 0, 700], 64, 3), ([129], 1, 1), ([700, 90, 257, 300, 256], 200, 2),
+                                          ([1000, 3], 129, 1), ([130, 400] * 200, 128, 2)])
+def test_backward_of_sequences_longer_than_the_bound(lens, bound, H):
+    """The forward computes the queries in the bound's tiles of 128 over all keys and leaves zeros for the rest, so only those queries
+    contribute to the gradients, to every key, and the others' own gradient is zero; the outputs' gradients there do not count, however
+    large. Against the fp32 oracle with the same rows taken out; rounding as above."""
+    import recis_b200
+    C = recis_b200.native()
+    qkv, offs, d_out = _case(lens, H, seed=7)
+    T, hidden = qkv.shape[0], H * 64
+    computed = torch.zeros(T, dtype=torch.bool)
+    for i, n in enumerate(lens):
+        computed[int(offs[i]):int(offs[i]) + min(n, (bound + 127) // 128 * 128)] = True
+    _, ref = _oracle(qkv, lens, H, torch.where(computed[:, None], d_out, torch.zeros_like(d_out)))
+    q_dev, o_dev = qkv.to(DEV), offs.to(DEV)
+    out, lse = C.ragged_attention_fwd(q_dev, o_dev, H, bound, 0.125)
+    got = C.ragged_attention_bwd(q_dev, out, torch.where(computed[:, None], d_out, d_out * 1e4).to(DEV), lse, o_dev, H, bound, 0.125)
+    torch.cuda.synchronize()
+    assert C.dense_status("cuda:0") == 0
+    got = got.float().cpu()
+    assert torch.count_nonzero(got[~computed][:, :hidden]) == 0 and torch.isfinite(got).all()
+    for name, sl in (("dq", slice(0, hidden)), ("dk", slice(hidden, 2 * hidden)), ("dv", slice(2 * hidden, 3 * hidden))):
+        assert (got[:, sl] - ref[:, sl]).norm() / ref[:, sl].norm() < 2e-2, name
