@@ -120,7 +120,7 @@ void rb_grad_reduce(const float* grad_out, const int32_t* gsrc, const float* gsc
 void rb_grad_reduce_push(const float* grad_out, const int32_t* gsrc, const float* gscale, const int32_t* csr_u, const int32_t* csr_elem,
                          const int32_t* start, int64_t n, int D, float* span_acc, RbGuPush push, int max_blocks, cudaStream_t st);
 int rb_grad_reduce_chunk();                            // of rb_grad_reduce_push
-int rb_grad_reduce_chunk_for(int64_t n, int D);        // of rb_grad_reduce: span_acc holds ceil(n / chunk) rows of D, zero on entry and exit
+int rb_grad_reduce_chunk_for(int64_t n, int D);        // of rb_grad_reduce: span_acc holds ceil(n / chunk) rows of D, zero on entry
 void rb_sparse_apply(const int32_t* rows, const float* grads, int64_t n_max, const int32_t* n_dev, int D, RbOpt opt, cudaStream_t st);
 
 #ifdef __cplusplus

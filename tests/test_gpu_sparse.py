@@ -385,3 +385,20 @@ def test_lookup_kernels_take_views_at_any_element(first):
     engine(batch)
     (cube, _), = engine.packed.values()
     assert torch.isfinite(cube).all() and (cube < before).all()
+
+
+@pytest.mark.parametrize("n,D", [(3000, 16), (70_001, 16), (30_000, 64), (9_999, 128), (20_000, 200)])
+def test_gradient_sums_of_up_to_33_occurrences_repeat(n, D):
+    """Rows of up to 33 occurrences give the same bits in every run, on either side of the chunk edges (longer ones meet in reductions of
+    any order); chunks of 8 take the pieces of a row that crosses several of them in order."""
+    g = torch.Generator().manual_seed(n)
+    lens = torch.randint(1, 34, (n // 8,), generator=g)
+    rev = torch.repeat_interleave(torch.arange(lens.numel()), lens)[:n]
+    rev = rev[torch.randperm(rev.numel(), generator=g)].to(torch.int32).to(DEV)
+    grad = torch.randn(rev.numel(), D, generator=g).to(DEV)
+    gsrc = torch.randint(0, rev.numel(), (rev.numel(),), generator=g).to(torch.int32).to(DEV)
+    gscale = torch.rand(rev.numel(), generator=g).to(DEV)
+    csr = C.build_csr(rev)
+    n_u = int(rev.max()) + 1
+    sums = [C.grad_reduce(grad, gsrc, gscale, *csr, D, None, False, 2, 0.0, 0.0, 0.0, 0.0, 1.0, 0.0, 1.0, None, None, None, n_u) for _ in range(30)]
+    assert all(torch.equal(s, sums[0]) for s in sums[1:])
