@@ -402,3 +402,33 @@ def test_gradient_sums_of_up_to_33_occurrences_repeat(n, D):
     n_u = int(rev.max()) + 1
     sums = [C.grad_reduce(grad, gsrc, gscale, *csr, D, None, False, 2, 0.0, 0.0, 0.0, 0.0, 1.0, 0.0, 1.0, None, None, None, n_u) for _ in range(30)]
     assert all(torch.equal(s, sums[0]) for s in sums[1:])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("kind", [0, 1, 2])
+@pytest.mark.parametrize("n", [148 * 2048 - 32, 148 * 2048])
+def test_fused_update_on_both_sides_of_the_chunk_rule(n, kind, dtype):
+    """The reduction with the row update in it, in chunks of 8 and of 32 (128 columns: the line is 148 * 2048 elements): rows that occur
+    once, rows across several chunks, one of a thousand occurrences, rows that are not admitted. Against 64-bit sums and the CPU update;
+    sums of at most 1000 fp32 terms, and one rounding of the row type."""
+    D, g = 128, torch.Generator().manual_seed(kind)
+    rev = torch.randint(0, n // 3, (n,), generator=g)
+    rev[:1000] = 5
+    rev[1000:60_000] = torch.randint(0, 3000, (59_000,), generator=g)            # about 20 occurrences each
+    rev = torch.unique(rev[torch.randperm(n, generator=g)], return_inverse=True)[1].to(torch.int32)
+    n_u, segs = int(rev.max()) + 1, n // 4
+    rows = torch.randperm(n_u + 50, generator=g)[:n_u].to(torch.int32)
+    rows[::97] = -1
+    grad, gscale = torch.randn(segs, D, generator=g), torch.rand(n, generator=g)
+    gsrc = torch.randint(0, segs, (n,), generator=g).to(torch.int32)
+    w, s1, s2 = (torch.rand(n_u + 50, D, generator=g) for _ in range(3))
+    hyper = (kind, 0.01, 0.9, 0.999, 1e-8, 0.99, -0.02, 0.5)
+    dev = [t.to(DEV) for t in (w.to(dtype), s1, s2)]
+    C.grad_reduce(grad.to(DEV), gsrc.to(DEV), gscale.to(DEV), *C.build_csr(rev.to(DEV)), D, rows.to(DEV), True, *hyper, *dev, 0)
+    sums = torch.zeros(n_u, D, dtype=torch.float64).index_add_(0, rev.long(), grad[gsrc.long()].double() * gscale.double()[:, None])
+    ref = [w.to(dtype), s1.clone(), s2.clone()]
+    C.sparse_apply(rows, sums.float(), None, *hyper, *ref)
+    ulp = {torch.float32: 0.0, torch.bfloat16: 2.0 ** -7, torch.float16: 2.0 ** -10}[dtype]
+    for a, b, rel in zip(dev, ref, (1e-4 + ulp, 1e-4, 1e-4)):
+        assert torch.allclose(a.float().cpu(), b.float(), rtol=rel, atol=1e-4)
+    assert not torch.equal(dev[0].cpu(), w.to(dtype))
