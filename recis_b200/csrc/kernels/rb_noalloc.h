@@ -6,9 +6,9 @@
 //     serving loop with a no-allocation rule on its latency path),
 //   * plain C / C++ hosts that link the shared object directly and have no tensor framework (and therefore no caching
 //     allocator) to borrow scratch buffers from.
-// The regular entry point (rb_dedup_partition in rb_kernels.h) takes its scratch (hash-set keys, hash-set positions and one
-// slot index per id) from the caller. Here the scratch is a fixed array compiled into the library: every GPU that loads the
-// library carries it (about 7.3 MB) until the process exits.
+// The regular entry point (rb_dedup_partition in rb_kernels.h) takes its scratch (a hash set of int32 positions, and two int32 words
+// per id: its place among its owner's unique ids and the position that claimed it) from the caller. Here the scratch is a fixed
+// array compiled into the library: every GPU that loads the library carries it (4 MB) until the process exits.
 //
 // Contract
 //   * All pointers are device pointers owned by the caller: ids [n] in; counts [world], offsets [world + 1],
