@@ -8,16 +8,31 @@
 // traffic per clock at full tensor rate - operand reads plus the TMA fill of the next stage - against the 128 an SM has; the
 // pair needs half of that per SM for the same math, which is what lifts the ceiling of the one-CTA kernel.
 //
-// Protocol per reduction step s (ring of kStages, the barriers live at the same shared-memory offsets in both CTAs):
+// The grid is persistent, one pair per two SMs: the accumulator is double buffered in tensor memory, so a tile's epilogue and stores run
+// under the loads and MMAs of the next tile.
+//
+// Protocol per reduction step (ring of stages, counted over all tiles; the barriers live at the same shared-memory offsets in both CTAs):
 //   * both producers (warp 0) wait for their own empty[s]; the leader arms ITS full[s] with the bytes of both CTAs;
 //     both issue their loads with the leader's full[s] as the completion barrier (no load is multicast);
 //   * the leader's MMA thread (warp 1) waits for full[s], issues four 256 x 256 x 16 MMAs and commits them to empty[s] of
-//     both CTAs (tcgen05.commit with a two-CTA mask), and after the last step to accumulator_full of both CTAs;
-//   * the epilogue warps (2..9) of each CTA drain their own accumulator, two warps per lane quarter with 128 columns each:
-//     tcgen05.ld, bias / residual / ReLU, conversion, staging in the by then idle operand stages in the 128-byte-swizzled box
-//     layout, TMA stores (add-reductions for a split reduction) of 32-row slabs.
-// Operands may be K-major or MN-major as in the one-CTA kernel. Every wait is bounded: on a timeout the CTA records
-// kStatusWaitTimeout, gives outstanding copies time to land, joins the cluster barrier, frees its tensor memory and returns.
+//     both CTAs (tcgen05.commit with a two-CTA mask), and after a tile's last step to accumulator_full of both CTAs;
+//   * the epilogue warps (2..9) of each CTA drain their own accumulator, two warps per lane quarter with 128 columns each, box by box
+//     (32 rows x 128 bytes): tcgen05.ld, bias / residual / ReLU / mask, conversion, staging in the 128-byte swizzle, TMA store
+//     (add-reduction for a split reduction). A warp has its own small ring of staging slots; a residual or mask box travels into the slot
+//     two boxes ahead. Each warp reports to the leader's accumulator_empty when it has read its part.
+//
+// Every wait is bounded: on a timeout the CTA records kStatusWaitTimeout, gives outstanding copies time to land, joins the cluster
+// barrier, frees its tensor memory and returns.
+//
+// Operands may be K-major or MN-major as in the one-CTA kernel.
+//
+// Measured on a B200 (L2 cold; before: one tile per CTA, two CTAs to an SM, a row per lane and conditions per element in the epilogue):
+//   269000 x 1024 x 256, bias + ReLU, bf16 out:   321 -> 141 us (its 551 MB of output alone take 145 us to fill)
+//   the same with mask and column sums:           497 -> 249 us (1.24 GB: 5.0 TB/s)
+//   269000 x 256 x 1024, fp32 residual in / out:  332 -> 180 us (1.1 GB: 6.1 TB/s)
+//   16384 x 2048 x 3200, bias + ReLU:             172 -> 143 us (1.50 PFLOP/s)
+// What bounded the short reductions was the epilogue: first its instructions (finish_box), then the arrival on the leader's
+// accumulator_empty, which with release semantics at cluster scope waited for the warp's stores (206 -> 141 us in the first case).
 //
 // The reference has no GEMM kernel of its own: its dense layers are nn.Linear (cuBLAS), examples/deepfm/deepfm_model.py:49-52.
 #include "../common/rb_common.cuh"
@@ -39,11 +54,17 @@ constexpr int TM = 128;        // rows of D per CTA (the pair covers 256)
 constexpr int TN = 256;        // columns of D per pair; each CTA stages 128 rows of B
 constexpr int BK = 64;
 constexpr int UK = 16;
-constexpr int kStages = 3;     // 3 x 32 KB per CTA: two CTAs (of different pairs) share an SM
+constexpr int kPairs = 74;      // pairs of SMs
 constexpr int kThreads = 320;     // producer warp, MMA warp, 8 epilogue warps (two per tensor-memory lane quarter)
 constexpr uint32_t kHalfBytes = 128 * BK * 2;                   // 16 KB: one operand half of one stage
 constexpr uint32_t kStageBytes = 2 * kHalfBytes;                // this CTA's A half + B half
-constexpr uint32_t kSmemBytes = kStages * kStageBytes + 1024;
+constexpr int kGroup = 8;                                       // column tiles per group of the walk
+// Shared memory per CTA: a ring of operand stages and, for each of the eight epilogue warps, a ring of 4 KB staging slots. A second input
+// of the epilogue needs a third slot, so that its boxes can travel two boxes ahead; then a stage less fits.
+template <bool kSrc> struct Ring {
+  static constexpr int kStages = kSrc ? 4 : 5, kSlots = kSrc ? 3 : 2;
+  static constexpr uint32_t kBytes = kStages * kStageBytes + 8 * kSlots * 4096 + 1024;
+};
 constexpr uint32_t kPeerMask = 0xFEFFFFFFu;                     // clears the CTA-rank bit of a shared::cluster address: rank 0's copy
 
 __device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
@@ -70,45 +91,61 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
                ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
 }
 
-template <bool A_MN, bool B_MN, typename OutT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 2)
+// one arrival on the barrier at this offset in the leader CTA (it hands back tensor memory that was only read: nothing to make visible)
+__device__ __forceinline__ void arrive_leader(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(smem_u32(bar) & kPeerMask) : "memory");
+}
+
+// Tile t of the walk: this CTA's rows, the pair's columns, and its share of the reduction (may be empty when the reduction is split).
+// Tiles are walked in groups of kGroup column tiles, columns fastest: the pairs at work read the same rows of A at the same time and the
+// group's rows of B stay in L2. (Rows fastest, A came from DRAM once per column tile: 1055 instead of 690 MB at 269000 x 1024 x 256.)
+struct PairTile {
+  int m0, n0, kb_begin, num_kb;
+  bool first_split;
+  __device__ __forceinline__ PairTile(int t, int mt, int nt, int splits, int total_kb, uint32_t rank) {
+    const int z = t / (mt * nt), tile = t - z * mt * nt;
+    const int group = tile / (kGroup * mt), in_group = tile - group * kGroup * mt, width = min(kGroup, nt - group * kGroup);
+    const int kb_per = (total_kb + splits - 1) / splits;
+    m0 = in_group / width * 2 * TM + (int)rank * TM;
+    n0 = (group * kGroup + in_group % width) * TN;
+    kb_begin = z * kb_per;
+    num_kb = max(0, min(total_kb, kb_begin + kb_per) - kb_begin);
+    first_split = z == 0;
+  }
+};
+
+template <bool A_MN, bool B_MN, bool kSrc, typename OutT>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                              const __grid_constant__ CUtensorMap map_o, const float* __restrict__ bias,
-                              const float* __restrict__ beta_src, const RbGemmEpilogue epi, int MM, int NN, int KK, int ldo, int relu,
-                              int64_t* __restrict__ status) {
+                              const __grid_constant__ CUtensorMap map_o, const __grid_constant__ CUtensorMap map_src,
+                              const float* __restrict__ bias, float* __restrict__ colsum, int MM, int NN, int KK, int relu, int splits,
+                              int reduce_out, int64_t* __restrict__ status) {
+  constexpr int kStages = Ring<kSrc>::kStages, kSlots = Ring<kSrc>::kSlots;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[kStages];
   __shared__ __align__(8) uint64_t empty_bar[kStages];
-  __shared__ __align__(8) uint64_t tmem_full_bar;
+  __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2];
+  __shared__ __align__(8) uint64_t src_bar[8 * kSlots];
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
-  __shared__ __align__(16) float bias_s[TN];
 
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();                        // 0 = leader
-  const int m0 = (int)(blockIdx.x >> 1) * 2 * TM + (int)rank * TM;      // this CTA's rows of D (and of A)
-  const int n0 = (int)blockIdx.y * TN;                                   // the pair's columns of D
-  const int nb0 = n0 + (int)rank * 128;                                  // this CTA's rows of B
+  const int mt = (MM + 2 * TM - 1) / (2 * TM), nt = (NN + TN - 1) / TN;
   const int total_kb = (KK + BK - 1) / BK;
-  const int kb_per = (total_kb + (int)gridDim.z - 1) / (int)gridDim.z;
-  const int kb_begin = (int)blockIdx.z * kb_per;
-  const int num_kb = max(0, min(total_kb, kb_begin + kb_per) - kb_begin);
-  const bool split = gridDim.z > 1;
-  if (split && num_kb == 0) return;          // uniform for the whole cluster (same blockIdx.z), before any barrier or allocation
+  const int n_tiles = mt * nt * splits, first = (int)(blockIdx.x >> 1), stride = (int)(gridDim.x >> 1);
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
     for (int s = 0; s < kStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    mbar_init(&tmem_full_bar, 1);
+    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 16); }     // 8 epilogue warps of both CTAs
+    for (int s = 0; s < 8 * kSlots; ++s) mbar_init(&src_bar[s], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"((uint32_t)TN) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"((uint32_t)(2 * TN)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-  } else if (warp >= 2) {
-    const int c = (int)threadIdx.x - 64;                 // 256 epilogue threads, one column of the tile's bias each
-    bias_s[c] = (bias != nullptr && n0 + c < NN && (!split || blockIdx.z == 0)) ? bias[n0 + c] : 0.f;
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -122,20 +159,24 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const _
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
     bool ok = true;
-    for (int kb = 0; kb < num_kb && ok; ++kb) {
-      const int s = kb % kStages;
-      const uint32_t ph = (uint32_t)(kb / kStages) & 1u;
-      ok = mbar_wait(&empty_bar[s], ph ^ 1u, &abort_flag);
-      if (!ok) break;
-      uint8_t* sa = smem + s * kStageBytes;
-      uint8_t* sb = sa + kHalfBytes;
-      if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * kStageBytes);        // both CTAs' loads complete on the leader's barrier
-      const uint32_t bar = smem_u32(&full_bar[s]) & kPeerMask;
-      const int k0 = (kb_begin + kb) * BK;
-      if (!A_MN) tma_load_2d_pair(sa, &map_a, k0, m0, bar);                                   // box {BK, 128}
-      else { tma_load_2d_pair(sa, &map_a, m0, k0, bar); tma_load_2d_pair(sa + kHalfBytes / 2, &map_a, m0 + 64, k0, bar); }   // 2 x box {64, BK}
-      if (!B_MN) tma_load_2d_pair(sb, &map_b, k0, nb0, bar);
-      else { tma_load_2d_pair(sb, &map_b, nb0, k0, bar); tma_load_2d_pair(sb + kHalfBytes / 2, &map_b, nb0 + 64, k0, bar); }
+    uint32_t s = 0, ph = 1;                                    // stage and the parity of its next release
+    for (int t = first; t < n_tiles && ok; t += stride) {
+      const PairTile tile(t, mt, nt, splits, total_kb, rank);
+      const int m0 = tile.m0, nb0 = tile.n0 + (int)rank * 128;                 // this CTA's rows of A and of B
+      for (int kb = 0; kb < tile.num_kb; ++kb) {
+        ok = mbar_wait(&empty_bar[s], ph, &abort_flag);
+        if (!ok) break;
+        uint8_t* sa = smem + s * kStageBytes;
+        uint8_t* sb = sa + kHalfBytes;
+        if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * kStageBytes);        // both CTAs' loads complete on the leader's barrier
+        const uint32_t bar = smem_u32(&full_bar[s]) & kPeerMask;
+        const int k0 = (tile.kb_begin + kb) * BK;
+        if (!A_MN) tma_load_2d_pair(sa, &map_a, k0, m0, bar);                                   // box {BK, 128}
+        else { tma_load_2d_pair(sa, &map_a, m0, k0, bar); tma_load_2d_pair(sa + kHalfBytes / 2, &map_a, m0 + 64, k0, bar); }   // 2 x box {64, BK}
+        if (!B_MN) tma_load_2d_pair(sb, &map_b, k0, nb0, bar);
+        else { tma_load_2d_pair(sb, &map_b, nb0, k0, bar); tma_load_2d_pair(sb + kHalfBytes / 2, &map_b, nb0 + 64, k0, bar); }
+        if (++s == (uint32_t)kStages) { s = 0; ph ^= 1u; }
+      }
     }
   } else if (warp == 1 && lane == 0 && rank == 0) {
     // ------------------------------------------------------------------ MMA issuer (leader only)
@@ -143,103 +184,150 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const _
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((A_MN ? 1u : 0u) << 15) | ((B_MN ? 1u : 0u) << 16) |
                            ((uint32_t)(TN >> 3) << 17) | ((uint32_t)((2 * TM) >> 4) << 24);
     bool ok = true;
-    for (int kb = 0; kb < num_kb && ok; ++kb) {
-      const int s = kb % kStages;
-      const uint32_t ph = (uint32_t)(kb / kStages) & 1u;
-      ok = mbar_wait(&full_bar[s], ph, &abort_flag);
+    uint32_t s = 0, ph = 0;
+    int ti = 0;                                                // tiles since the start
+    for (int t = first; t < n_tiles && ok; t += stride) {
+      const PairTile tile(t, mt, nt, splits, total_kb, rank);
+      if (tile.num_kb == 0) continue;
+      const int buf = ti & 1;
+      ok = mbar_wait(&acc_empty[buf], (uint32_t)((ti >> 1) & 1) ^ 1u, &abort_flag);      // the epilogues of tile ti - 2 have read it
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t sa = smem_u32(smem + s * kStageBytes), sb = sa + kHalfBytes;
+      const uint32_t acc = tmem_base + (uint32_t)(buf * TN);
+      for (int kb = 0; kb < tile.num_kb; ++kb) {
+        ok = mbar_wait(&full_bar[s], ph, &abort_flag);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t sa = smem_u32(smem + s * kStageBytes), sb = sa + kHalfBytes;
 #pragma unroll
-      for (int k = 0; k < BK / UK; ++k) {
-        const uint64_t da = A_MN ? make_desc(sa + k * 2048, BK * 128, 1024) : make_desc(sa + k * 32, 16, 1024);
-        const uint64_t db = B_MN ? make_desc(sb + k * 2048, BK * 128, 1024) : make_desc(sb + k * 32, 16, 1024);
-        umma_bf16_pair(tmem_base, da, db, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+        for (int k = 0; k < BK / UK; ++k) {
+          const uint64_t da = A_MN ? make_desc(sa + k * 2048, BK * 128, 1024) : make_desc(sa + k * 32, 16, 1024);
+          const uint64_t db = B_MN ? make_desc(sb + k * 2048, BK * 128, 1024) : make_desc(sb + k * 32, 16, 1024);
+          umma_bf16_pair(acc, da, db, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+        }
+        umma_commit_pair(&empty_bar[s]);
+        if (++s == (uint32_t)kStages) { s = 0; ph ^= 1u; }
       }
-      umma_commit_pair(&empty_bar[s]);
+      if (ok) umma_commit_pair(&acc_full[buf]);
+      ++ti;
     }
-    if (ok) umma_commit_pair(&tmem_full_bar);
   } else if (warp >= 2) {
     // ------------------------------------------------------------------ epilogue (8 warps: lane quarter warp & 3, column half (warp - 2) / 4)
-    const bool ok = num_kb > 0 ? mbar_wait(&tmem_full_bar, 0, &abort_flag) : true;
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (ok) {
-      const int q = warp & 3, half = (warp - 2) >> 2;
-      const int row = m0 + q * 32 + lane;
-      const bool add_beta = beta_src != nullptr && (!split || blockIdx.z == 0);
-      // every MMA of the pair has completed, so neither CTA's operand stages are read any more: they become the staging area.
-      // A warp stages kPass columns at a time into its own 8 KB slab: boxes of 32 rows x 128 bytes.
-      constexpr int kPass = 256 / (int)sizeof(OutT);                   // 128 columns of bf16, 64 of fp32: 8 KB per 32 rows
-      constexpr int kBoxes = kPass / Store<OutT>::kBoxCols;            // 2
-      uint8_t* slab = smem + (half * 4 + q) * 8192;
+    constexpr int kCols = Store<OutT>::kBoxCols, kBoxes = 128 / kCols;
+    const int q = warp & 3, half = (warp - 2) >> 2;
+    uint8_t* slots = smem + kStages * kStageBytes + (warp - 2) * kSlots * 4096;
+    uint64_t* bars = src_bar + (warp - 2) * kSlots;
+    const rb::gemm::EpilogueWork work{&map_o, MM, relu != 0, reduce_out != 0, colsum != nullptr};
+    // Column sums stay in registers while the column tile stays the same (with the grid a multiple of the column tiles: always). Added to
+    // global memory box by box they cost more than the rest of the epilogue.
+    float sums[kBoxes][kCols / 32];
+#pragma unroll
+    for (int b = 0; b < kBoxes; ++b)
+#pragma unroll
+      for (int e = 0; e < kCols / 32; ++e) sums[b][e] = 0.f;
+    int sums_n0 = -1;
+    auto flush_sums = [&]() {
+      const int at = sums_n0 + half * 128 + rb::gemm::column_of<kCols>(lane);
+#pragma unroll
+      for (int b = 0; b < kBoxes; ++b)
+#pragma unroll
+        for (int e = 0; e < kCols / 32; ++e) {
+          if (at + b * kCols + e < NN) atomicAdd(colsum + at + b * kCols + e, sums[b][e]);
+          sums[b][e] = 0.f;
+        }
+    };
+    // Boxes are counted over all tiles: box g of this warp uses slot g % kSlots. `ahead` walks the boxes whose second input is fetched.
+    int g = 0, ti = 0;
+    int ahead_t = first, ahead_b = 0, ahead_g = 0;
+    auto fetch_next = [&]() {                                  // lane 0: the next box's second input into its slot
+      while (ahead_t < n_tiles) {
+        const PairTile tile(ahead_t, mt, nt, splits, total_kb, rank);
+        const int row0 = tile.m0 + q * 32, col = tile.n0 + half * 128 + ahead_b * kCols;
+        if (row0 >= MM || col >= NN) { ahead_t += stride; ahead_b = 0; continue; }
+        const int slot = ahead_g % kSlots;
+        mbar_expect_tx(&bars[slot], 4096);
+        tma_load_2d(slots + slot * 4096, &map_src, col, row0, &bars[slot]);
+        ++ahead_g;
+        if (++ahead_b == kBoxes) { ahead_t += stride; ahead_b = 0; }
+        return;
+      }
+    };
+    if (kSrc && lane == 0) { fetch_next(); fetch_next(); }
+    bool ok = true;
+    for (int t = first; t < n_tiles && ok; t += stride) {
+      const PairTile tile(t, mt, nt, splits, total_kb, rank);
+      if (tile.num_kb == 0) continue;
+      const int row0 = tile.m0 + q * 32, buf = ti & 1;
+      ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[buf], (uint32_t)((ti >> 1) & 1), &abort_flag) ? 1 : 0) != 0;
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t acc = tmem_base + (uint32_t)(buf * TN) + ((uint32_t)(q * 32) << 16);
+      if (colsum != nullptr && tile.n0 != sums_n0) {
+        if (sums_n0 >= 0) flush_sums();
+        sums_n0 = tile.n0;
+      }
+      bool released = false;
 #pragma unroll 1
-      for (int p0 = half * 128; p0 < half * 128 + 128; p0 += kPass) {
-        if (n0 + p0 >= NN) break;
-        if (p0 > half * 128) {
-          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the previous pass's boxes have been read
+      for (int b = 0; b < kBoxes; ++b, ++g) {
+        const int c0 = half * 128 + b * kCols, col = tile.n0 + c0;
+        if (row0 >= MM || col >= NN) break;
+        const int slot = g % kSlots;
+        float v[kCols];
+        rb::gemm::load_box<kCols>(acc + (uint32_t)c0, v);
+        if (b == kBoxes - 1) {                                 // the accumulator has been read: the tile after next may overwrite it
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) arrive_leader(&acc_empty[buf]);
+          released = true;
+        }
+        if (kSrc) {
+          ok = __all_sync(0xffffffffu, mbar_wait(&bars[slot], (uint32_t)(g / kSlots) & 1u, &abort_flag) ? 1 : 0) != 0;
+          if (!ok) break;
+          if (lane == 0) {
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");    // the box before this one has left its slot
+            fetch_next();
+          }
+        } else {
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");      // the box before the last has left this slot
           __syncwarp();
         }
-#pragma unroll 1
-        for (int c0 = p0; c0 < p0 + kPass; c0 += 32) {
-          if (n0 + c0 >= NN) break;
-          uint32_t r[32];
-          if (num_kb > 0) {
-            tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          } else {
+        const float* bias_at = bias != nullptr && tile.first_split ? bias + col : nullptr;
+        if (bias_at != nullptr && (col + kCols > NN || (reinterpret_cast<uintptr_t>(bias_at) & 7))) {      // edge or odd address: one by one
 #pragma unroll
-            for (int j = 0; j < 32; ++j) r[j] = 0u;
+          for (int j = 0; j < kCols; ++j) {
+            const int c = 8 * ((j & (kCols / 2 - 1)) >> 2) + 2 * (lane & 3) + (j & 1);
+            if (col + c < NN) v[j] += bias_at[c];
           }
-          float v[32];
-          const int valid = min(32, NN - (n0 + c0));
-          const float* brow = beta_src + (int64_t)row * ldo + n0 + c0;
-          const bool beta_here = add_beta && row < MM;
-          const bool beta_vec = beta_here && valid == 32 && (ldo % 4 == 0) && ((reinterpret_cast<uintptr_t>(beta_src) & 15) == 0);
-#pragma unroll
-          for (int j4 = 0; j4 < 32; j4 += 4) {
-            float4 bt = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (beta_vec) bt = *reinterpret_cast<const float4*>(brow + j4);
-            else if (beta_here) {
-              if (j4 + 0 < valid) bt.x = brow[j4 + 0];
-              if (j4 + 1 < valid) bt.y = brow[j4 + 1];
-              if (j4 + 2 < valid) bt.z = brow[j4 + 2];
-              if (j4 + 3 < valid) bt.w = brow[j4 + 3];
-            }
-            const float4 bs = *reinterpret_cast<const float4*>(&bias_s[c0 + j4]);
-            const float x0 = __uint_as_float(r[j4 + 0]) + bs.x + bt.x, x1 = __uint_as_float(r[j4 + 1]) + bs.y + bt.y;
-            const float x2 = __uint_as_float(r[j4 + 2]) + bs.z + bt.z, x3 = __uint_as_float(r[j4 + 3]) + bs.w + bt.w;
-            v[j4 + 0] = relu ? fmaxf(x0, 0.f) : x0; v[j4 + 1] = relu ? fmaxf(x1, 0.f) : x1;
-            v[j4 + 2] = relu ? fmaxf(x2, 0.f) : x2; v[j4 + 3] = relu ? fmaxf(x3, 0.f) : x3;
-          }
-          if (epi.mask_src != nullptr)
-            rb::gemm::apply_mask32(v, reinterpret_cast<const __nv_bfloat16*>(epi.mask_src) + (int64_t)row * epi.mask_ld + n0 + c0, valid, row < MM);
-          Store<OutT>::stage32(slab, lane, c0 - p0, v);
-          if (epi.colsum != nullptr) {
-            if (row >= MM) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] = 0.f;
-            }
-            rb::gemm::column_sums32(v, lane, valid, epi.colsum + n0 + c0);
-          }
+          bias_at = nullptr;
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        if (lane == 0 && m0 + q * 32 < MM) {
+        float sum[kCols / 32];
 #pragma unroll
-          for (int bx = 0; bx < kBoxes; ++bx) {
-            const int col = n0 + p0 + bx * Store<OutT>::kBoxCols;
-            if (col >= NN) break;
-            if (split)
-              asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.bulk_group [%0, {%2, %3}], [%1];"
-                           ::"l"(&map_o), "r"(smem_u32(slab + bx * 4096)), "r"(col), "r"(m0 + q * 32) : "memory");
-            else
-              asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
-                           ::"l"(&map_o), "r"(smem_u32(slab + bx * 4096)), "r"(col), "r"(m0 + q * 32) : "memory");
-          }
-          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        }
+        for (int e = 0; e < kCols / 32; ++e) sum[e] = 0.f;
+        rb::gemm::finish_box<OutT>(work, v, bias_at, kSrc, slots + slot * 4096, row0, col, lane, sum);
+#pragma unroll
+        for (int k = 0; k < kBoxes; ++k)
+#pragma unroll
+          for (int e = 0; e < kCols / 32; ++e) sums[k][e] += k == b ? sum[e] : 0.f;
       }
-      if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");       // the slab must stay until the copies have read it
+      if (ok && !released) {                                   // nothing, or not everything, of this part lies inside D
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) arrive_leader(&acc_empty[buf]);
+      }
+      ++ti;
+    }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");       // the slots must stay until the copies have read them
+    if (colsum != nullptr) {
+      // what is left, summed over the four row quarters first: a quarter of the additions to the same few addresses, whole lines of them
+      float* part = reinterpret_cast<float*>(smem + kStages * kStageBytes);
+      asm volatile("bar.sync 1, 256;" ::: "memory");             // every warp's boxes have left the slots
+#pragma unroll
+      for (int b = 0; b < kBoxes; ++b)
+#pragma unroll
+        for (int e = 0; e < kCols / 32; ++e) part[q * TN + half * 128 + b * kCols + rb::gemm::column_of<kCols>(lane) + e] = sums[b][e];
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      const int c = (int)threadIdx.x - 64;
+      if (sums_n0 >= 0 && sums_n0 + c < NN) atomicAdd(colsum + sums_n0 + c, (part[c] + part[TN + c]) + (part[2 * TN + c] + part[3 * TN + c]));
     }
   }
   if (abort_flag) {
@@ -252,51 +340,66 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const _
   cluster_sync();                            // both epilogues are done and nothing of the peer's is in flight towards this CTA
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)TN) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)(2 * TN)) : "memory");
   }
   if (threadIdx.x == 0 && abort_flag) rb::set_status(status, rb::kStatusWaitTimeout);
 }
 
-template <bool A_MN, bool B_MN, typename OutT>
-int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const float* bias, const float* beta_src,
-                const RbGemmEpilogue& epi, int MM, int NN, int KK, int ldo, int relu, int splits, int64_t* status, cudaStream_t st) {
-  auto kern = gemm_bf16_tcgen05_2cta_kernel<A_MN, B_MN, OutT>;
+template <bool A_MN, bool B_MN, bool kSrc, typename OutT>
+int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const CUtensorMap& ms, const float* bias, float* colsum,
+                int MM, int NN, int KK, int relu, int splits, int reduce_out, int64_t* status, cudaStream_t st) {
+  auto kern = gemm_bf16_tcgen05_2cta_kernel<A_MN, B_MN, kSrc, OutT>;
+  constexpr uint32_t smem = Ring<kSrc>::kBytes;
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes) != cudaSuccess) return 3;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 3;
     attr_set = true;
   }
-  dim3 grid(2 * ((MM + 2 * TM - 1) / (2 * TM)), (NN + TN - 1) / TN, splits);
-  kern<<<grid, kThreads, kSmemBytes, st>>>(ma, mb, mo, bias, beta_src, epi, MM, NN, KK, ldo, relu, status);
+  const int64_t tiles = (int64_t)((MM + 2 * TM - 1) / (2 * TM)) * ((NN + TN - 1) / TN) * splits;
+  if (tiles > (int64_t)1 << 30) return 7;
+  int pairs = (int)std::min<int64_t>(tiles, kPairs);
+  // with column sums a pair stays with one column tile where there are at most kGroup of them
+  const int width = std::min((NN + TN - 1) / TN, kGroup);
+  if (colsum != nullptr && pairs > width) pairs -= pairs % width;
+  kern<<<2 * pairs, kThreads, smem, st>>>(ma, mb, mo, ms, bias, colsum, MM, NN, KK, relu, splits, reduce_out, status);
   rb::note_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
 }  // namespace
 
-// Same contract as rb_gemm_bf16 (rb_dense.h), for outputs that can leave through TMA stores (base and row pitch 16-byte aligned).
+// Same contract as rb_gemm_bf16 (rb_dense.h), for outputs that can leave through TMA stores (base and row pitch 16-byte aligned); `reduce_out`:
+// the output is added to, by `splits` parts of the reduction.
 // Returns 7 when the problem does not suit the pair kernel (the caller then uses the one-CTA kernel).
 extern "C" int rb_gemm_bf16_pair(const void* a, int64_t lda, int a_mn, const void* b, int64_t ldb, int b_mn, void* out, int64_t ldo,
                                  int out_fp32, const float* bias, const float* beta_src, const RbGemmEpilogue* epi_in, int MM, int NN, int KK,
-                                 int relu, int splits, int64_t* status, cudaStream_t st) {
+                                 int relu, int splits, int reduce_out, int64_t* status, cudaStream_t st) {
   RbGemmEpilogue epi{nullptr, 0, nullptr};
   if (epi_in != nullptr) epi = *epi_in;
-  if ((epi.mask_src != nullptr || epi.colsum != nullptr) && splits > 1) return 6;
+  if ((epi.mask_src != nullptr || epi.colsum != nullptr) && reduce_out) return 6;
   if (MM < 192 || NN < 192 || KK <= 0) return 7;
   if ((reinterpret_cast<uintptr_t>(a) & 15) || (reinterpret_cast<uintptr_t>(b) & 15) || (lda % 8) || (ldb % 8)) return 1;
   const int es = out_fp32 ? 4 : 2;
   if ((reinterpret_cast<uintptr_t>(out) & 15) || (ldo * es) % 16) return 7;
-  if (splits > 1 && (!out_fp32 || relu)) return 6;
-  CUtensorMap ma, mb, mo;
+  if (reduce_out && (!out_fp32 || relu)) return 6;
+  // the second input of the epilogue comes as boxes in the layout of the output: a residual (fp32 output) or a mask (bf16 output)
+  const bool mask = epi.mask_src != nullptr;
+  if ((mask && (out_fp32 || beta_src != nullptr)) || (beta_src != nullptr && !out_fp32)) return 7;
+  const void* src = mask ? epi.mask_src : beta_src;
+  const int64_t src_ld = mask ? epi.mask_ld : ldo;
+  if (src != nullptr && (reduce_out || (reinterpret_cast<uintptr_t>(src) & 15) || (src_ld * es) % 16)) return 7;
+  CUtensorMap ma, mb, mo, ms;
   // boxes: K-major operands {BK, 128 rows}; MN-major operands {64, BK}; output {32 or 64 columns, 32 rows}
   const int ra = a_mn ? rb_tensor_map_2d(&ma, a, KK, MM, lda, 64, BK, 0) : rb_tensor_map_2d(&ma, a, MM, KK, lda, BK, 128, 0);
   const int rbm = b_mn ? rb_tensor_map_2d(&mb, b, KK, NN, ldb, 64, BK, 0) : rb_tensor_map_2d(&mb, b, NN, KK, ldb, BK, 128, 0);
   const int ro = rb_tensor_map_2d(&mo, out, MM, NN, ldo, out_fp32 ? 32 : 64, 32, out_fp32);
-  if (ra || rbm || ro) return 2;
+  const int rs = src != nullptr ? rb_tensor_map_2d(&ms, src, MM, NN, src_ld, out_fp32 ? 32 : 64, 32, out_fp32) : 0;
+  if (src == nullptr) ms = mo;
+  if (ra || rbm || ro || rs) return 2;
 #define RB_PAIR_CASE(AM, BMJ)                                                                                                    \
   if ((a_mn != 0) == AM && (b_mn != 0) == BMJ)                                                                                   \
-    return out_fp32 ? launch_pair<AM, BMJ, float>(ma, mb, mo, bias, beta_src, epi, MM, NN, KK, (int)ldo, relu, splits, status, st)    \
-                    : launch_pair<AM, BMJ, __nv_bfloat16>(ma, mb, mo, bias, beta_src, epi, MM, NN, KK, (int)ldo, relu, 1, status, st);
+    return out_fp32 ? (src != nullptr ? launch_pair<AM, BMJ, true, float> : launch_pair<AM, BMJ, false, float>)(ma, mb, mo, ms, bias, epi.colsum, MM, NN, KK, relu, splits, reduce_out, status, st)    \
+                    : (src != nullptr ? launch_pair<AM, BMJ, true, __nv_bfloat16> : launch_pair<AM, BMJ, false, __nv_bfloat16>)(ma, mb, mo, ms, bias, epi.colsum, MM, NN, KK, relu, 1, 0, status, st);
   RB_PAIR_CASE(false, false)
   RB_PAIR_CASE(false, true)
   RB_PAIR_CASE(true, false)

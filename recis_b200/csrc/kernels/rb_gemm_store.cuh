@@ -2,6 +2,7 @@
 // either straight to global memory (row32 / red32) or into a shared-memory slab laid out as boxes of 32 rows x 128 bytes in the
 // 128-byte swizzle, which is what a TMA store (or add-reduction) of such a box expects (stage32).
 #pragma once
+#include "../common/rb_tcgen05.cuh"
 #include <cuda_bf16.h>
 #include <stdint.h>
 
@@ -114,6 +115,176 @@ __device__ __forceinline__ void column_sums32(float (&v)[32], int lane, int vali
     }
   }
   if (lane < valid) atomicAdd(dst + lane, v[0]);
+}
+
+// a += b for two neighbouring floats in one instruction
+__device__ __forceinline__ void add_f32x2(float& a0, float& a1, float b0, float b1) {
+  asm("{\n\t.reg .b64 u, w;\n\tmov.b64 u, {%0, %1};\n\tmov.b64 w, {%2, %3};\n\tadd.rn.f32x2 u, u, w;\n\tmov.b64 {%0, %1}, u;\n\t}"
+      : "+f"(a0), "+f"(a1) : "f"(b0), "f"(b1));
+}
+
+// What the epilogue does to a finished accumulator. The second input has the layout of the output: the residual that is added (fp32
+// output) or the activations whose sign masks the result (bf16 output). Its boxes arrive by TMA in the slots that the output is then
+// staged in, in place.
+struct EpilogueWork {
+  const CUtensorMap* map_o;
+  int MM;
+  bool relu, reduce, colsum;       // reduce: the output is added to; colsum: column sums are wanted
+};
+
+// One box of the accumulator (32 rows of the warp's lane quarter x kCols columns) into registers, in the layout of an MMA accumulator: of every
+// 8 columns a lane holds columns 2 (lane & 3) and + 1 of the rows lane / 4 + 8 r, so that v[4 (h kCols / 8 + j) + 2 r + e] is row
+// 16 h + 8 r + lane / 4, column 8 j + 2 (lane & 3) + e. A lane then meets a quarter of the columns: the bias costs a quarter of the
+// shared-memory and L1 traffic it costs with a row per lane (25 us of 221 at 269000 x 1024 x 256), and a column sum 14 exchanges
+// per 64 columns instead of 62.
+template <int kCols> __device__ __forceinline__ void load_box(uint32_t taddr, float (&v)[kCols]) {
+  if constexpr (kCols == 64) {
+    tc::tmem_ld_16x64(taddr, reinterpret_cast<uint32_t(&)[32]>(v[0]));
+    tc::tmem_ld_16x64(taddr + (16u << 16), reinterpret_cast<uint32_t(&)[32]>(v[32]));
+  } else {
+    tc::tmem_ld_16x32(taddr, reinterpret_cast<uint32_t(&)[16]>(v[0]));
+    tc::tmem_ld_16x32(taddr + (16u << 16), reinterpret_cast<uint32_t(&)[16]>(v[16]));
+  }
+  tc::tmem_ld_wait();
+}
+
+// Column sums over the box's 32 rows: this lane's share, columns column_of(lane) .. + kCols / 32 - 1 of the box, is added to `sum`.
+template <int kCols> __device__ __forceinline__ void column_sums(const float (&v)[kCols], int lane, float (&sum)[kCols / 32]) {
+  constexpr int kBlocks = kCols / 8;
+  float s[2 * kBlocks];                          // s[2 j + e]: column 8 j + 2 (lane & 3) + e
+#pragma unroll
+  for (int j = 0; j < kBlocks; ++j)
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      s[2 * j + e] = (v[4 * j + e] + v[4 * j + 2 + e]) + (v[kCols / 2 + 4 * j + e] + v[kCols / 2 + 4 * j + 2 + e]);
+  // the eight lanes of a column: each step keeps half of the values and adds the other lane's copy of them
+#pragma unroll
+  for (int step = 0; step < 3; ++step) {
+    const int off = 16 >> step, half = kBlocks >> step;
+    const bool up = (lane & off) != 0;
+#pragma unroll
+    for (int k = 0; k < half; ++k) {
+      const float keep = up ? s[half + k] : s[k], give = up ? s[k] : s[half + k];
+      s[k] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < kCols / 32; ++e) sum[e] += s[e];
+}
+template <int kCols> __device__ __forceinline__ int column_of(int lane) {
+  constexpr int kBlocks = kCols / 8;
+  const int at = ((lane & 16) ? kBlocks : 0) + ((lane & 8) ? kBlocks / 2 : 0) + ((lane & 4) ? kBlocks / 4 : 0);
+  return 8 * (at >> 1) + 2 * (lane & 3) + (at & 1);
+}
+
+// One box of 32 rows x 128 bytes, already in registers (load_box): bias, second input (in `box`, which has landed), ReLU, mask, conversion,
+// staging in `box` and the copy out to rows row0 .. and columns col .. of D, as a bulk group of its own. `bias`: null, or the box's first
+// column, readable for the whole box and 8-byte aligned. Column sums of the final values are
+// added to `sum` (column_sums). Whole-warp call, destroys v.
+//
+// With two or four warps to a scheduler and a chain of dependent instructions per element the epilogue was bound by its own instruction
+// latency, not by memory: 13,000 warp instructions per 128 x 256 tile, 0.32 per cycle and scheduler, and 7 bytes of output per cycle and
+// SM whatever the order of the tiles. Hence no per-element conditions here (edges are clipped by the copies), packed additions, the ReLU
+// on packed pairs, and second inputs by TMA instead of a row per lane.
+template <typename OutT>
+__device__ __forceinline__ void finish_box(const EpilogueWork& w, float (&v)[Store<OutT>::kBoxCols], const float* bias, bool has_src, uint8_t* box, int row0,
+                                           int col, int lane, float (&sum)[Store<OutT>::kBoxCols / 32]) {
+  constexpr int kCols = Store<OutT>::kBoxCols, kBlocks = kCols / 8;
+  if (bias != nullptr) {
+#pragma unroll
+    for (int j = 0; j < kBlocks; ++j) {
+      const float2 b = *reinterpret_cast<const float2*>(bias + 8 * j + 2 * (lane & 3));
+#pragma unroll
+      for (int r = 0; r < 4; ++r) add_f32x2(v[(r >> 1) * (kCols / 2) + 4 * j + 2 * (r & 1)], v[(r >> 1) * (kCols / 2) + 4 * j + 2 * (r & 1) + 1], b.x, b.y);
+    }
+  }
+  if constexpr (sizeof(OutT) == 4) {
+    const uint32_t base = tc::smem_u32(box) + (uint32_t)((lane >> 2) * 128 + ((((lane >> 1) & 1) ^ (lane >> 2)) << 4) + (lane & 1) * 8);
+    if (has_src) {
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int j = 0; j < kBlocks; ++j) {
+          float x, y;
+          asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(x), "=f"(y) : "r"((base ^ (uint32_t)(j << 5)) + (uint32_t)(r * 1024)) : "memory");
+          const int at = (r >> 1) * (kCols / 2) + 4 * j + 2 * (r & 1);
+          add_f32x2(v[at], v[at + 1], x, y);
+        }
+    }
+    if (w.relu) {
+#pragma unroll
+      for (int j = 0; j < kCols; ++j) v[j] = fmaxf(v[j], 0.f);
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int j = 0; j < kBlocks; ++j) {
+        const int at = (r >> 1) * (kCols / 2) + 4 * j + 2 * (r & 1);
+        asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"((base ^ (uint32_t)(j << 5)) + (uint32_t)(r * 1024)), "f"(v[at]), "f"(v[at + 1]) : "memory");
+      }
+  } else {
+    // 8 x 8 matrices, four at a time: rows 0 .. 7 and 8 .. 15 of two neighbouring blocks of 8 columns
+    const uint32_t base = tc::smem_u32(box) + (uint32_t)((lane & 15) * 128 + (((lane >> 4) ^ (lane & 7)) << 4));
+    if (has_src) {
+      // 0xffff for every bf16 above zero (a NaN is not), spread to a 32-bit mask per value
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          uint32_t m[4];
+          asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(m[0]), "=r"(m[1]), "=r"(m[2]), "=r"(m[3])
+                       : "r"((base ^ (uint32_t)(i << 5)) + (uint32_t)(h * 2048)) : "memory");
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const uint32_t on = __hgt2_mask(*reinterpret_cast<const __nv_bfloat162*>(&m[e]), __float2bfloat162_rn(0.f));
+            float& x = v[h * 32 + 8 * i + 2 * e];
+            float& y = v[h * 32 + 8 * i + 2 * e + 1];
+            x = __uint_as_float(__float_as_uint(x) & __byte_perm(on, 0u, 0x1010));
+            y = __uint_as_float(__float_as_uint(y) & __byte_perm(on, 0u, 0x3232));
+          }
+        }
+    }
+    if (w.relu && w.colsum) {
+#pragma unroll
+      for (int j = 0; j < kCols; ++j) v[j] = fmaxf(v[j], 0.f);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        uint32_t u[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          __nv_bfloat162 p = __floats2bfloat162_rn(v[h * 32 + 8 * i + 2 * e], v[h * 32 + 8 * i + 2 * e + 1]);
+          if (w.relu) p = __hmax2(p, __float2bfloat162_rn(0.f));
+          u[e] = *reinterpret_cast<uint32_t*>(&p);
+        }
+        asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};"
+                     ::"r"((base ^ (uint32_t)(i << 5)) + (uint32_t)(h * 2048)), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]) : "memory");
+      }
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncwarp();
+  if (lane == 0) {
+    if (w.reduce)
+      asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.bulk_group [%0, {%2, %3}], [%1];"
+                   ::"l"(w.map_o), "r"(tc::smem_u32(box)), "r"(col), "r"(row0) : "memory");
+    else
+      asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
+                   ::"l"(w.map_o), "r"(tc::smem_u32(box)), "r"(col), "r"(row0) : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  }
+  if (w.colsum) {
+    if (row0 + 32 > w.MM) {
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        if (row0 + 8 * r + (lane >> 2) >= w.MM) {
+#pragma unroll
+          for (int j = 0; j < kBlocks; ++j) { v[(r >> 1) * (kCols / 2) + 4 * j + 2 * (r & 1)] = 0.f; v[(r >> 1) * (kCols / 2) + 4 * j + 2 * (r & 1) + 1] = 0.f; }
+        }
+    }
+    column_sums<kCols>(v, lane, sum);
+  }
 }
 
 }  // namespace gemm

@@ -70,3 +70,27 @@ def test_dgrad_with_relu_mask_and_bias_gradient_in_the_epilogue(M, N, K, masked)
         assert float(dx.float().cpu()[(y_below.float() <= 0)].abs().max()) == 0.0       # masked entries are exact zeros
     assert rel(db, ref.sum(0)) < 2e-3
     assert C.dense_status(DEV) == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(19001, 264, 72), (20480, 2312, 64), (9500, 520, 1000), (4700, 72, 264), (1100, 136, 200)])
+@pytest.mark.parametrize("odd", [False, True])
+def test_gemm_epilogues_over_several_rounds_of_tiles(M, N, K, odd):
+    """Bias + ReLU, residual and mask + column sums where a pair of SMs walks several tiles (ten column tiles included) and where one
+    CTA has one tile, with rows and columns that end inside a box. ``odd``: a bias off its 8-byte line, a residual and a mask that no TMA
+    map takes. Bounds: bf16 rounding 2^-9 per entry of bf16 outputs, accumulation order in fp32 ones (as above)."""
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    rn = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    x, w = rn(M, K).bfloat16(), (rn(N, K) * 0.1).bfloat16()
+    bias = rn(N + 1)[1:] if odd else rn(N)
+    res = rn(M * N + 1)[1:].view(M, N) if odd else rn(M, N)
+    mask = rn(M, N + 1).bfloat16()[:, :N] if odd else rn(M, N).bfloat16()
+    mask[0, 0], mask[M - 1, N - 1], mask[1, 0] = float("nan"), float("inf"), -0.0
+    ref = x.float() @ w.float().t()
+    rel = lambda a, b: float((a.float() - b).norm() / b.norm())
+    assert rel(C.gemm_bf16(x, w, bias, True, False, False, False, None), torch.relu(ref + bias)) < 4e-3
+    assert rel(C.gemm_bf16_residual(x, w, bias, res), ref + bias + res) < 1e-4
+    dx, db = C.gemm_dgrad_fused(x, w.t().contiguous(), mask)
+    keep = (mask > 0).float()
+    assert rel(dx, ref * keep) < 4e-3 and float(dx[keep == 0].float().abs().max()) == 0.0
+    assert rel(db, (ref * keep).sum(0)) < 1e-4
+    assert C.dense_status(DEV) == 0
