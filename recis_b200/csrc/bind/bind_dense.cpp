@@ -459,9 +459,11 @@ void init_dense(py::module& m) {
     if (T == 0 || B <= 0 || H <= 0 || max_len <= 0)
       return std::make_tuple(torch::zeros({T, H * 64}, qkv.options()), torch::zeros({T, H}, qkv.options().dtype(torch::kFloat32)));
     auto out = torch::empty({T, H * 64}, qkv.options());                         // the kernel writes every row
-    auto lse = torch::empty({T, H}, qkv.options().dtype(torch::kFloat32));
+    auto lse_buf = torch::empty({T * H + 1}, qkv.options().dtype(torch::kFloat32));     // and the kernel's work counter behind it
+    auto lse = lse_buf.narrow(0, 0, T * H).view({T, H});
     const int rc = rb_ragged_attention_fwd(qkv.data_ptr(), offsets.data_ptr<int32_t>(), T, (int)B, (int)H, (int)max_len, (float)scale,
-                                           out.data_ptr(), lse.data_ptr<float>(), status_word(qkv.device()).data_ptr<int64_t>(),
+                                           out.data_ptr(), lse.data_ptr<float>(), reinterpret_cast<unsigned*>(lse_buf.data_ptr<float>() + T * H),
+                                           status_word(qkv.device()).data_ptr<int64_t>(),
                                            at::cuda::getCurrentCUDAStream());
     TORCH_CHECK(rc == 0, "ragged_attention_fwd failed (code ", rc, ")");
     return std::make_tuple(out, lse);

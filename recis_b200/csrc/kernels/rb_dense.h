@@ -56,9 +56,9 @@ int rb_dot_interaction_tc_fwd(const void* x, const float* cube, int B, int F, in
 int rb_dot_interaction_tc_bwd(const void* x, const float* cube, const void* dout, int B, int F, int D, int out_ld, float* dx,
                               float* dcube, int64_t* status, cudaStream_t st);
 // Ragged multi-head self-attention forward, head width 64 (attention_tcgen05.cu). qkv: bf16 [T, 3 * H * 64] packed, offsets:
-// int32 [B + 1] (device), out: bf16 [T, H * 64], lse2: fp32 [T, H] or null. 0 = launched, 1 = unsuitable arguments, > 1 = error.
+// int32 [B + 1] (device), out: bf16 [T, H * 64], lse2: fp32 [T, H] or null, counter: a word of scratch. 0 = launched, 1 = unsuitable arguments, > 1 = error.
 int rb_ragged_attention_fwd(const void* qkv, const int32_t* offsets, int64_t T, int B, int H, int max_len, float scale, void* out,
-                            float* lse2, int64_t* status, cudaStream_t st);
+                            float* lse2, unsigned* counter, int64_t* status, cudaStream_t st);
 // Backward: out / d_out bf16 [T, H * 64], lse2 from the forward, scratch fp32 [T * H + 1], dq_acc fp32 [T, H * 64] zeroed (may be null
 // when max_len <= 128), dqkv bf16 [T, 3 * H * 64].
 int rb_ragged_attention_bwd(const void* qkv, const void* out, const void* d_out, const float* lse2, float* scratch, const int32_t* offsets,

@@ -248,3 +248,28 @@ def test_backward_of_sequences_longer_than_the_bound(lens, bound, H):
     assert torch.count_nonzero(got[~computed][:, :hidden]) == 0 and torch.isfinite(got).all()
     for name, sl in (("dq", slice(0, hidden)), ("dk", slice(hidden, 2 * hidden)), ("dv", slice(2 * hidden, 3 * hidden))):
         assert (got[:, sl] - ref[:, sl]).norm() / ref[:, sl].norm() < 2e-2, name
+
+
+@pytest.mark.parametrize("lens,H", [([1] * 900 + [64, 65, 33, 128, 129, 191, 193], 3), ([700, 31, 1000, 257, 96, 97], 2), ([64, 65, 127, 192, 16, 17] * 70, 5),
+                                    ([90] * 200, 4)])
+@pytest.mark.parametrize("spread", [1.0, 40.0])
+def test_forward_on_every_work_split_and_with_growing_scores(lens, H, spread):
+    """Items dealt out, fetched with long and with short steps, and key counts on both sides of a step and of a 32-column chunk. With ``spread``
+    the scores of a row reach hundreds and grow along the sequence, so that the reference exponent is raised in the middle of a step. The
+    last key of every sequence is non-finite in the tensor's tail and must not be read. Bounds as above."""
+    import recis_b200
+    C = recis_b200.native()
+    qkv, offs, _ = _case(lens, H, seed=len(lens))
+    if spread > 1:
+        pos = torch.cat([torch.arange(L) / max(L, 2) for L in lens])
+        k = slice(H * 64, 2 * H * 64)
+        qkv[:, k] = (qkv[:, k].float() * (1 + spread * pos[:, None])).to(torch.bfloat16)
+    tail = torch.full((7, 3 * H * 64), float("nan")).to(torch.bfloat16)
+    for bound in (max(lens), 4 * max(lens)):
+        out, lse = C.ragged_attention_fwd(torch.cat([qkv, tail]).to(DEV), offs.to(DEV), H, bound, 0.125)
+        assert C.dense_status("cuda:0") == 0
+        ref, _ = _oracle(qkv, lens, H)
+        got = out.float().cpu()
+        assert float(got[len(qkv):].abs().max()) == 0.0 and float(lse[len(qkv):].abs().max()) == 0.0
+        err = (got[:len(qkv)] - ref).norm() / ref.norm()
+        assert err < 1e-2, (bound, float(err))
