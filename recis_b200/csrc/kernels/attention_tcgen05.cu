@@ -695,70 +695,85 @@ ragged_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const _
           mbar_arrive(&kv_full[st]);
         }
       }
-    } else if (warp == kMma && lane == 0) {
-      // ------------------------------------------------------------------ MMA issuer
+    } else if (warp == kMma) {
+      // ------------------------------------------------------------------ MMA issuer (the whole warp; one lane issues)
       const uint32_t idesc_kk = make_idesc_bf16(kTile, kTile, false, false);    // S, dP: both operands K-major
       const uint32_t idesc_mm = make_idesc_bf16(kTile, kHead, true, true);      // dV, dK: both operands MN-major
       const uint32_t idesc_km = make_idesc_bf16(kTile, kHead, false, true);     // dQ: A K-major, B MN-major
-      const uint32_t sp = smem_u32(ptile), sds = smem_u32(dstile);
+      // Descriptors advance by adding to the 16-byte address field: they stay in a few registers.
+      // A = P^T / dS^T: [q][key] tiles read MN-major (M = key: two 64-wide blocks kBlk apart, 16 q rows = 2048 bytes per step)
+      // B = dO / Q:     [q][d] tiles read MN-major (N = d, one 64-wide block)
+      const uint64_t d_qk = make_desc(smem_u32(qotiles), 16, 1024), d_kk = make_desc(smem_u32(kvtiles), 16, 1024);      // read K-major
+      const uint64_t d_qm = make_desc(smem_u32(qotiles), kBlk, 1024), d_km = make_desc(smem_u32(kvtiles), kBlk, 1024);  // read MN-major
+      const uint64_t d_p = make_desc(smem_u32(ptile), kBlk, 1024), d_ds = make_desc(smem_u32(dstile), kBlk, 1024), d_dsk = make_desc(smem_u32(dstile), 16, 1024);
+      const bool leader = elect_one();
       int g = 0;
       int p_st = 0, p_kq = 0, p_kk = 0;                 // the previous step: K / V stage, 16-row reduction steps over queries and keys
       bool p_first = false, p_last = false, p_dq_acc = false;
       auto products = [&](int gs) -> bool {             // dV, dK, dQ of step gs
-        if (!mbar_wait(&p_full, (uint32_t)(gs & 1), &abort_flag)) return false;
-        if (gs > 0 && !mbar_wait(&post_empty, (uint32_t)((gs - 1) & 1), &abort_flag)) return false;
+        if (gs > 0 && !wait_all(&post_empty, (uint32_t)((gs - 1) & 1))) return false;
+        if (!wait_all(&p_full, (uint32_t)(gs & 1))) return false;
         fence_after_sync();
-        const uint32_t sq = smem_u32(qotiles + (gs & 1) * 2 * kBlk), sdo = sq + kBlk, sk = smem_u32(kvtiles + p_st * 2 * kBlk);
-        // Descriptors advance by adding to the 16-byte address field: they stay in a few registers.
-        // A = P^T / dS^T: [q][key] tiles read MN-major (M = key: two 64-wide blocks kBlk apart, 16 q rows = 2048 bytes per step)
-        // B = dO / Q:     [q][d] tiles read MN-major (N = d, one 64-wide block)
-        uint64_t d_p = make_desc(sp, kBlk, 1024), d_ds = make_desc(sds, kBlk, 1024), d_do = make_desc(sdo, kBlk, 1024), d_q = make_desc(sq, kBlk, 1024);
-        uint32_t acc = p_first ? 0u : 1u;
+        const uint64_t q = d_qm + (uint64_t)((gs & 1) * (2 * kBlk >> 4)), d_o = q + (uint64_t)(kBlk >> 4), kt = d_km + (uint64_t)(p_st * (2 * kBlk >> 4));
+        const uint32_t acc = p_first ? 0u : 1u, acc_q = p_dq_acc ? 1u : 0u;
+        if (leader) {
+          if (p_kq == kTile / 16) {                     // (a whole tile is spelt out: built in a loop, the 24 MMAs took 2400 cycles to issue)
+#pragma unroll
+            for (int k = 0; k < kTile / 16; ++k) {      // reduction over the queries of the tile, 16 rows per step
+              umma_bf16(tmem + kColDV, d_p + (uint64_t)(k * 128), d_o + (uint64_t)(k * 128), idesc_mm, k > 0 ? 1u : acc);
+              umma_bf16(tmem + kColDK, d_ds + (uint64_t)(k * 128), q + (uint64_t)(k * 128), idesc_mm, k > 0 ? 1u : acc);
+            }
+          } else {
 #pragma unroll 1
-        for (int k = 0; k < p_kq; ++k) {                // reduction over the queries of the tile, 16 rows per step
-          umma_bf16(tmem + kColDV, d_p, d_do, idesc_mm, acc);
-          umma_bf16(tmem + kColDK, d_ds, d_q, idesc_mm, acc);
-          d_p += 128; d_ds += 128; d_do += 128; d_q += 128; acc = 1u;
-        }
-        uint64_t d_k = make_desc(sk, kBlk, 1024);
-        acc = p_dq_acc ? 1u : 0u;
+            for (int k = 0; k < p_kq; ++k) {
+              umma_bf16(tmem + kColDV, d_p + (uint64_t)(k * 128), d_o + (uint64_t)(k * 128), idesc_mm, k > 0 ? 1u : acc);
+              umma_bf16(tmem + kColDK, d_ds + (uint64_t)(k * 128), q + (uint64_t)(k * 128), idesc_mm, k > 0 ? 1u : acc);
+            }
+          }
+          if (p_kk == kTile / 16) {
+#pragma unroll
+            for (int k = 0; k < kTile / 16; ++k)        // reduction over the keys of the tile: dS read K-major, K read MN-major
+              umma_bf16(tmem + kColDQ, d_dsk + (uint64_t)((k >> 2) * (kBlk >> 4) + (k & 3) * 2), kt + (uint64_t)(k * 128), idesc_km, k > 0 ? 1u : acc_q);
+          } else {
 #pragma unroll 1
-        for (int k = 0; k < p_kk; ++k) {                // reduction over the keys of the tile: dS read K-major, K read MN-major
-          umma_bf16(tmem + kColDQ, make_desc(sds, 16, 1024) + (uint64_t)((k >> 2) * (kBlk >> 4) + (k & 3) * 2), d_k, idesc_km, acc);
-          d_k += 128; acc = 1u;
+            for (int k = 0; k < p_kk; ++k)
+              umma_bf16(tmem + kColDQ, d_dsk + (uint64_t)((k >> 2) * (kBlk >> 4) + (k & 3) * 2), kt + (uint64_t)(k * 128), idesc_km, k > 0 ? 1u : acc_q);
+          }
+          umma_commit(&m2_full);
+          umma_commit(&in_empty[gs & 1]);
+          if (p_last) umma_commit(&kv_empty[p_st]);
         }
-        umma_commit(&m2_full);
-        umma_commit(&in_empty[gs & 1]);
-        if (p_last) umma_commit(&kv_empty[p_st]);
+        __syncwarp();
         return true;
       };
       bool ok = true;
       for (int it = 0; ok; ++it) {
         const int st = it & 1;
-        ok = mbar_wait(&kv_full[st], (uint32_t)((it >> 1) & 1), &abort_flag);
+        ok = wait_all(&kv_full[st], (uint32_t)((it >> 1) & 1));
         if (!ok) break;
-        const AttnItem item = slot[st];
-        if (item.len < 0) break;
-        const uint32_t sk = smem_u32(kvtiles + st * 2 * kBlk);
-        const int n_q = query_tiles(item.len);
+        const int len = __shfl_sync(0xffffffffu, slot[st].len, 0), kt0 = __shfl_sync(0xffffffffu, slot[st].kt, 0);
+        if (len < 0) break;
+        const uint64_t d_k = d_kk + (uint64_t)(st * (2 * kBlk >> 4));
+        const int n_q = query_tiles(len);
         for (int i = 0; i < n_q; ++i, ++g) {
-          ok = mbar_wait(&in_full[g & 1], (uint32_t)((g >> 1) & 1), &abort_flag) &&
-               (g == 0 || mbar_wait(&s_empty, (uint32_t)((g - 1) & 1), &abort_flag));
+          ok = wait_all(&in_full[g & 1], (uint32_t)((g >> 1) & 1)) && (g == 0 || wait_all(&s_empty, (uint32_t)((g - 1) & 1)));
           if (!ok) break;
           fence_after_sync();
-          uint64_t d_a = make_desc(smem_u32(qotiles + (g & 1) * 2 * kBlk), 16, 1024), d_b = make_desc(sk, 16, 1024);
-#pragma unroll 1
-          for (int half = 0; half < 2; ++half) {         // S = Q K^T, then dP = dO V^T: dO and V lie one block behind Q and K
+          const uint64_t d_q = d_qk + (uint64_t)((g & 1) * (2 * kBlk >> 4));
+          if (leader) {
 #pragma unroll
             for (int k = 0; k < kHead / 16; ++k)
-              umma_bf16(tmem + kColS + (uint32_t)(half * (kColDP - kColS)), d_a + (uint64_t)(k * 2), d_b + (uint64_t)(k * 2), idesc_kk, k > 0 ? 1u : 0u);
-            d_a += kBlk >> 4; d_b += kBlk >> 4;
+              umma_bf16(tmem + kColS, d_q + (uint64_t)(k * 2), d_k + (uint64_t)(k * 2), idesc_kk, k > 0 ? 1u : 0u);
+#pragma unroll
+            for (int k = 0; k < kHead / 16; ++k)         // dP = dO V^T: dO and V lie one block behind Q and K
+              umma_bf16(tmem + kColDP, d_q + (uint64_t)((kBlk >> 4) + k * 2), d_k + (uint64_t)((kBlk >> 4) + k * 2), idesc_kk, k > 0 ? 1u : 0u);
+            umma_commit(&s_full);
           }
-          umma_commit(&s_full);
+          __syncwarp();
           if (g > 0) { ok = products(g - 1); if (!ok) break; }
-          p_st = st; p_first = i == 0; p_last = i == n_q - 1; p_dq_acc = kSingle && item.kt > 0;
-          p_kq = (min(kTile, item.len - i * kTile) + 15) >> 4;
-          p_kk = (min(kTile, item.len - item.kt * kTile) + 15) >> 4;
+          p_st = st; p_first = i == 0; p_last = i == n_q - 1; p_dq_acc = kSingle && kt0 > 0;
+          p_kq = (min(kTile, len - i * kTile) + 15) >> 4;
+          p_kk = (min(kTile, len - kt0 * kTile) + 15) >> 4;
         }
       }
       if (ok && g > 0) products(g - 1);
