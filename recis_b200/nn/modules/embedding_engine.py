@@ -368,10 +368,12 @@ class EmbeddingEngine(nn.Module):
                         outs[name] = cube[:, j, :].reshape(shape) if len(shape) != 2 else cube[:, j, :]
             else:
                 pooled = pooled.view(-1, (tile_len or 1) * D)
-                start = 0
-                for name, s, shape in zip(feats.names, segs, feats.shapes):
-                    outs[name] = pooled[start:start + s].reshape(shape)
-                    start += s
+                # One node for all features: their gradients come back as one concatenation. (A slice each returned a gradient of the whole
+                # tensor per feature, cleared, copied into and added up: 0.4 ms and 60 launches of the sequence model's step.) The pieces may
+                # be changed in place like any tensor, hence not `split`, whose outputs may not.
+                pieces = (pooled,) if len(segs) == 1 else torch.unsafe_split_with_sizes(pooled, list(segs))
+                for name, piece, shape in zip(feats.names, pieces, feats.shapes):
+                    outs[name] = piece.reshape(shape)
         for k in direct:
             v = input_features[k]
             if isinstance(v, RaggedTensor):

@@ -195,3 +195,28 @@ def test_three_stage_lookup_interface_matches_forward():
     got = emb.emb_reduce(r2, None, "mean", {})
     assert torch.allclose(got.view_as(want), want)
     assert emb.emb_reduce(emb.lookup_exchange_emb(emb.exchange_ids(ids, offsets)), None, "sum", fp16_enable=True).dtype == torch.float16
+
+
+@pytest.mark.parametrize("combiner,width", [("sum", 3), ("tile", 6)])
+def test_gradients_of_features_taken_apart(combiner, width):
+    """The features of one lookup come back as pieces of it: one that takes no part in the loss contributes nothing, one that is changed in
+    place passes its gradient through the change, and the row updates are those of the features looked up one by one."""
+    kw = {"combiner_kwargs": {"tile_len": 2}} if combiner == "tile" else {}
+    def run(names):
+        HashtableRegister().clear()
+        opts = {n: EmbeddingOption(embedding_dim=3, shared_name="t", combiner=combiner, device="cpu", initializer=ConstantInitializer(0.5), **kw) for n in "abc"}
+        engine = EmbeddingEngine(opts)
+        opt = SparseSGD(filter_out_sparse_param(engine), lr=1.0)
+        feats = {n: RaggedTensor(torch.tensor([7 + i, 3, 3 + i]), [torch.tensor([0, 2, 3], dtype=torch.int32)], dense_shape=(2, -1)) for i, n in enumerate("abc")}
+        for group in names:
+            out = engine({n: feats[n] for n in group})
+            assert all(out[n].numel() == 2 * width for n in group)
+            loss = 0.0
+            for n in group:
+                if n != "b":
+                    loss = loss + (out[n].mul_(3.0) if n == "c" else out[n]).sum()
+            if not isinstance(loss, float):
+                loss.backward()
+        opt.step()
+        return engine.table_of("a").table.impl.embedding_lookup(torch.tensor([3, 4, 5, 7, 8, 9]), readonly=True)[1]
+    assert torch.equal(run(["abc"]), run(["a", "b", "c"]))
