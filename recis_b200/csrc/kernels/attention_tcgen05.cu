@@ -8,21 +8,22 @@
 //                     in the 128-byte swizzle; fp32 result in tensor memory
 //   P  = exp2(S * scale * log2 e - m)   each thread owns one query row: it reads its row of S with tcgen05.ld, keeps the maximum m and the
 //                     sum l in registers and writes P (bf16) into shared memory
-//   O += P V          tcgen05.mma, A = P, B = the V tile read as an MN-major operand (N = head column, K = key row); O stays in tensor
-//                     memory and is rescaled there when a maximum of the warp's rows has grown. (Rescaling only from some growth on saves
-//                     a tenth of the time, but then the largest P of a row is not exactly one: up to 12 % more error.)
+//   O += P V          tcgen05.mma, A = P, B = the V tile read as an MN-major operand (N = head column, K = key row); with steps of 64
+//                     keys O stays in tensor memory and is rescaled there when a maximum of the warp's rows has grown, with 128 each step's
+//                     product is added to O in registers. (Rescaling only from some growth on saves a tenth of the time, but then the
+//                     largest P of a row is not exactly one: up to 12 % more error.)
 //
 // and finally writes O / l (bf16) and the log-sum-exp (base 2) of the row. Persistent CTAs with separate roles: four softmax warps, one
 // that fetches work and issues the TMA loads, one that issues the MMAs. S of the next step is multiplied as soon as this one's has been read,
 // under P V. Keys past the end of a sequence are masked in the softmax; query rows past the end are computed on whatever is there and not
 // stored; of a partial tile only the 32-row boxes that hold a row are loaded.
 //
-// What bounds it is the latency of a step - score, exponentials, product, in sequence for a query tile - with four query tiles to an SM
-// (tensor memory holds no more); the exponentials take two fifths of the special-function units' cycles. Measured on a B200
+// What bounds it is the latency of a step - score, exponentials, product, in sequence for a query tile - with two or four query
+// tiles to an SM (tensor memory holds no more); the exponentials take two fifths of the special-function units' cycles. Measured on a B200
 // (before: one CTA of 128 threads per item, loads, MMAs and exponentials one after the other, P through shared memory, O in registers):
-//   256 sequences of 50..1000 tokens, 4 heads:  290 -> 207 us (83 GFLOP in existing elements: 400 TFLOP/s)
-//   3000 sequences of 1..90 tokens, 8 heads:    418 -> 170 us; under a bound of 1000 instead of 90: 1210 -> 180 us
-//   37 sequences of 1..1000 tokens, 4 heads:     55 -> 53 us;  one sequence of 1000 tokens, 8 heads: 27 -> 24.6 us
+//   256 sequences of 50..1000 tokens, 4 heads:  290 -> 225 us (83 GFLOP in existing elements: 367 TFLOP/s)
+//   3000 sequences of 1..90 tokens, 8 heads:    418 -> 166 us; under a bound of 1000 instead of 90: 1210 -> 235 us
+//   37 sequences of 1..1000 tokens, 4 heads:     55 -> 51 us;  one sequence of 1000 tokens, 8 heads: 27 -> 24.6 us
 //
 // The reference has no attention kernel; its sequence example pads to the longest sequence and calls the library SDPA
 // (examples/seq2seq/transformer.py:36-38). Waits are bounded; a timeout sets the status word and the CTA frees its tensor
@@ -61,9 +62,11 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 // ---------------------------------------------------------------------------------------------- forward
 struct AttnItem { int s0, len, head, kt; };          // len < 0: no more work; kt: the item's tile (of queries here, of keys in the backward)
 
-// Keys per step and CTAs per SM: 64 keys and four CTAs where the GPU is full, so that sixteen softmax warps hide one another's waits
-// (tensor memory: S 64 + O 64 columns each); 128 keys and two CTAs where every CTA has one item at most, since half as many steps of a
-// sequence then follow one another.
+// Keys per step and CTAs per SM: 64 keys and four CTAs where a sequence has one query tile (tensor memory: S 64 + O 64 columns each), so that
+// sixteen softmax warps hide one another's waits (3000 sequences of 1..90 tokens, 8 heads: 170 us, with 128 keys 206); 128 keys and two CTAs
+// elsewhere, with the rows of O in registers. (There 64 keys and O in tensor memory would be a little faster, 207 us at 256 sequences of
+// 50..1000 tokens, 4 heads, but P is then rounded against the maxima of half as many keys and O summed in another order; as it is, every
+// output is the same to the bit as with one CTA per tile, and a training run takes the same course.)
 template <int kKeys_> struct FwdCfg {
   static constexpr int kKeys = kKeys_, kCtas = kKeys == 64 ? 4 : 2;
   static constexpr int kKvBlk = kKeys * 128;                     // bytes of one [keys x 64 bf16] swizzled block
@@ -291,7 +294,7 @@ ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           if (left > kKeys) issue_s(min(kKeys, left - kKeys));                         // (S of this step has been read)
           else fence_after_sync();
           if (leader) {
-            umma_bf16(tmem + kFwdO, d_p, d_v, idesc_o, j > 0 ? 1u : 0u);
+            umma_bf16(tmem + kFwdO, d_p, d_v, idesc_o, kKeys == 64 && j > 0 ? 1u : 0u);
             if (steps == kKeys / 16) {
 #pragma unroll
               for (int k = 1; k < kKeys / 16; ++k) umma_bf16(tmem + kFwdO, d_p + (uint64_t)((k >> 2) * (kBlk >> 4) + (k & 3) * 2), d_v + (uint64_t)(k * 128), idesc_o, 1u);
@@ -318,7 +321,20 @@ ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       const AttnItem item = slot[it & 1];
       if (item.len < 0) break;
       const int rows = item.len - item.kt * kTile - warp * 32;                // rows of this warp that exist (may be <= 0, or more than 32)
-      float m = -INFINITY, l = 0.f;                                           // maximum so far (in powers of two), sum of P
+      float m = -INFINITY, l = 0.f, alpha = 0.f;                              // maximum so far (in powers of two), sum of P, the last step's rescale
+      float o[kKeys == 64 ? 1 : kHead];                                       // with 128 keys the rows of O are here, each step's P V is added to them
+#pragma unroll
+      for (int d = 0; d < (kKeys == 64 ? 1 : kHead); ++d) o[d] = 0.f;
+      auto add_pv = [&]() {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          uint32_t r[32];
+          tmem_ld32(trow + kFwdO + (uint32_t)(e * 32), r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int d = 0; d < 32; ++d) o[(e * 32 + d) & (kKeys == 64 ? 0 : kHead - 1)] = fmaf(o[(e * 32 + d) & (kKeys == 64 ? 0 : kHead - 1)], alpha, __uint_as_float(r[d]));
+        }
+      };
       for (int j = 0; j * kKeys < item.len; ++j, ++g) {
         const int valid = min(kKeys, item.len - j * kKeys);                   // key columns of this step that exist
         ok = wait_all(&s_full, (uint32_t)(g & 1));
@@ -356,9 +372,14 @@ ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             ok = wait_all(&o_full, (uint32_t)((g - 1) & 1));
             if (!ok) break;
           }
-          if (j > 0) {
-            const float alpha = fast_exp2(m - m_new);
-            l *= alpha;
+          if constexpr (kKeys == 128) {
+            if (j > 0) {
+              fence_after_sync();
+              add_pv();
+              alpha = fast_exp2(m - m_new);
+            }
+          } else if (j > 0) {
+            alpha = fast_exp2(m - m_new);
             if (__any_sync(0xffffffffu, m_new > m && lane < rows)) {
               fence_after_sync();
 #pragma unroll 1
@@ -375,14 +396,13 @@ ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           }
           m = m_new;
           const float neg_m = -m;
+          float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
           for (int c = 0; c < whole; c += 32) {
             uint32_t s[32], pk[16];
-            float sum[4] = {0.f, 0.f, 0.f, 0.f};
             tmem_ld32(trow + kFwdS + (uint32_t)c, s);
             tmem_ld_wait();
             exp_chunk<32>(s, scale_log2, neg_m, sum, pk);
-            l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
 #pragma unroll
             for (int e = 0; e < 4; ++e)
               st_shared16((prow ^ (uint32_t)((((c >> 3) & 4) + e) << 4)) + (uint32_t)((c >> 6) * kBlk), pk[4 * e], pk[4 * e + 1], pk[4 * e + 2], pk[4 * e + 3]);
@@ -390,15 +410,14 @@ ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 #pragma unroll 1
           for (int c = whole; c < end; c += 8) {
             uint32_t s[8], pk[4];
-            float sum[4] = {0.f, 0.f, 0.f, 0.f};
             tmem_ld8(trow + kFwdS + (uint32_t)c, s);
             tmem_ld_wait();
 #pragma unroll
             for (int i = 0; i < 8; ++i) s[i] = c + i < valid ? s[i] : 0xff800000u;
             exp_chunk<8>(s, scale_log2, neg_m, sum, pk);
-            l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
             st_shared16((prow ^ (uint32_t)(((c >> 3) & 7) << 4)) + (uint32_t)((c >> 6) * kBlk), pk[0], pk[1], pk[2], pk[3]);
           }
+          l = fmaf(l, alpha, (sum[0] + sum[2]) + (sum[1] + sum[3]));
         }
         if (valid & 15) {
           // V rows between the last key and the end of the last 16-key step become zeros, so that the zeros of P never meet a non-finite value
@@ -422,15 +441,26 @@ ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       // through this warp's rows of the P tile, which the item no longer needs: eight lanes store a row, so that every store is whole lines
       const float inv = l > 0.f ? 1.f / l : 0.f;
       if (rows > 0) {
+        if constexpr (kKeys == 128) {
+          add_pv();
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            uint32_t u[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) u[e] = pack_bf16x2(o[c * 8 + 2 * e] * inv, o[c * 8 + 2 * e + 1] * inv);
+            st_shared16(prow ^ (uint32_t)(c << 4), u[0], u[1], u[2], u[3]);
+          }
+        } else {
 #pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-          uint32_t r[16], u[8];
-          tmem_ld16(trow + kFwdO + (uint32_t)(c * 16), r);
-          tmem_ld_wait();
+          for (int c = 0; c < 4; ++c) {
+            uint32_t r[16], u[8];
+            tmem_ld16(trow + kFwdO + (uint32_t)(c * 16), r);
+            tmem_ld_wait();
 #pragma unroll
-          for (int e = 0; e < 8; ++e) u[e] = pack_bf16x2(__uint_as_float(r[2 * e]) * inv, __uint_as_float(r[2 * e + 1]) * inv);
+            for (int e = 0; e < 8; ++e) u[e] = pack_bf16x2(__uint_as_float(r[2 * e]) * inv, __uint_as_float(r[2 * e + 1]) * inv);
 #pragma unroll
-          for (int e = 0; e < 2; ++e) st_shared16(prow ^ (uint32_t)((2 * c + e) << 4), u[4 * e], u[4 * e + 1], u[4 * e + 2], u[4 * e + 3]);
+            for (int e = 0; e < 2; ++e) st_shared16(prow ^ (uint32_t)((2 * c + e) << 4), u[4 * e], u[4 * e + 1], u[4 * e + 2], u[4 * e + 3]);
+          }
         }
       }
       fence_before_sync();
@@ -1013,26 +1043,26 @@ extern "C" int rb_ragged_attention_fwd(const void* qkv, const int32_t* offsets, 
   const int tiles = (int)(((int64_t)max_len + kTile - 1) / kTile);
   const int64_t items = (int64_t)tiles * B * H;
   if (items > (int64_t)1 << 31) return 1;
-  // Few items: long steps, and up to three rounds of them dealt out one per CTA, which saves the counter (15 sequences of 1..1000 tokens, 4
-  // heads: 28.7 us, fetched 38.9, before 30.8; 37 sequences, 1184 items: 57 dealt out, 53 fetched, before 55).
-  const bool few = items <= 8 * FwdCfg<128>::kCtas * 148, dealt = tiles > 2 && items <= 3 * FwdCfg<128>::kCtas * 148;
-  const int keys = few ? 128 : 64;
+  // Up to three rounds of items of long sequences are dealt out one per CTA, which saves the counter (15 sequences of 1..1000 tokens, 4 heads:
+  // 28.7 us, fetched 38.9, before 30.8; 37 sequences, 1184 items: 57 dealt out, 51 fetched, before 55).
+  const bool long_steps = tiles > 1 || items <= 8 * FwdCfg<128>::kCtas * 148, dealt = tiles > 2 && items <= 3 * FwdCfg<128>::kCtas * 148;
+  const int keys = long_steps ? 128 : 64;
   CUtensorMap map_q, map_kv, map_rows;
   if (rb_tensor_map_2d(&map_q, qkv, T, (int64_t)3 * H * kHead, (int64_t)3 * H * kHead, kHead, kTile, 0) != 0 ||
       rb_tensor_map_2d(&map_kv, qkv, T, (int64_t)3 * H * kHead, (int64_t)3 * H * kHead, kHead, keys, 0) != 0 ||
       rb_tensor_map_2d(&map_rows, qkv, T, (int64_t)3 * H * kHead, (int64_t)3 * H * kHead, kHead, 32, 0) != 0)
     return 1;
-  auto kern = few ? ragged_attention_fwd_kernel<128> : ragged_attention_fwd_kernel<64>;
-  const size_t smem = few ? FwdCfg<128>::kSmem : FwdCfg<64>::kSmem;
+  auto kern = long_steps ? ragged_attention_fwd_kernel<128> : ragged_attention_fwd_kernel<64>;
+  const size_t smem = long_steps ? FwdCfg<128>::kSmem : FwdCfg<64>::kSmem;
   static bool attr[2] = {false, false};
-  if (!attr[few]) {
+  if (!attr[long_steps]) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 3;
-    attr[few] = true;
+    attr[long_steps] = true;
   }
   if (dealt) counter = nullptr;
   else if (cudaMemsetAsync(counter, 0, sizeof(unsigned), st) != cudaSuccess) return 4;
   // Items fetched at a time: one where that is about 32 fetches per CTA, more under a loose bound, where most items are empty.
-  const int slots = 148 * (few ? FwdCfg<128>::kCtas : FwdCfg<64>::kCtas), grid = (int)(dealt ? items : std::min<int64_t>(items, slots));
+  const int slots = 148 * (long_steps ? FwdCfg<128>::kCtas : FwdCfg<64>::kCtas), grid = (int)(dealt ? items : std::min<int64_t>(items, slots));
   const int chunk = (int)std::min<int64_t>(32, std::max<int64_t>(1, items / (32 * slots)));
   kern<<<grid, kFwdThreads, smem, st>>>(map_q, map_kv, map_rows, offsets, T, B, H, tiles, chunk, scale * 1.4426950408889634f,
                                         reinterpret_cast<__nv_bfloat16*>(out), lse2, counter, status);
