@@ -168,6 +168,45 @@ std::tuple<Tensor, Tensor> relu_bwd_bias(const Tensor& y, const Tensor& dout, bo
   return {dy, db};
 }
 
+// (loss fp32 [], logit fp32 [B, 1]) of y bf16 [B, ld] (column 0 counts), extra fp32 [B, 1] or none, label fp32 [B, 1]
+std::tuple<Tensor, Tensor> click_loss_fwd(const Tensor& y, OptT extra, const Tensor& label) {
+  TORCH_CHECK(y.is_cuda() && y.scalar_type() == torch::kBFloat16 && y.dim() == 2 && y.stride(1) == 1 && y.size(0) > 0, "y: bf16 [B, ld] on CUDA");
+  const int64_t B = y.size(0);
+  TORCH_CHECK(B < (int64_t)1 << 31, "click_loss: batch too large");
+  auto column = [&](const Tensor& t) {
+    return t.device() == y.device() && t.scalar_type() == torch::kFloat32 && t.is_contiguous() && t.dim() == 2 && t.size(0) == B && t.size(1) == 1;
+  };
+  const bool has_extra = extra.has_value() && extra->defined();
+  TORCH_CHECK(column(label) && (!has_extra || column(*extra)), "extra, label: contiguous fp32 [B, 1]");
+  c10::cuda::CUDAGuard g(y.device());
+  auto f32 = y.options().dtype(torch::kFloat32);
+  auto logit = torch::empty({B, 1}, f32), loss = torch::empty({}, f32);
+  const int blocks = rb_click_loss_blocks((int)B);
+  Tensor partial = blocks > 1 ? torch::empty({blocks}, f32) : Tensor();
+  const int rc = rb_click_loss_fwd(y.data_ptr(), (int)y.stride(0), has_extra ? extra->data_ptr<float>() : nullptr, label.data_ptr<float>(), (int)B,
+                                   logit.data_ptr<float>(), loss.data_ptr<float>(), partial.defined() ? partial.data_ptr<float>() : nullptr,
+                                   at::cuda::getCurrentCUDAStream());
+  TORCH_CHECK(rc == 0, "click_loss_fwd failed (code ", rc, ")");
+  return {loss, logit};
+}
+
+// (d_y bf16 [B, ld], d_extra fp32 [B, 1] or undefined)
+std::tuple<Tensor, Tensor> click_loss_bwd(const Tensor& logit, const Tensor& label, OptT g_loss, OptT g_logit, int64_t ld, bool need_extra) {
+  const int64_t B = logit.size(0);
+  auto ok = [&](const OptT& t, int64_t n) {
+    return !(t.has_value() && t->defined()) || (t->device() == logit.device() && t->scalar_type() == torch::kFloat32 && t->is_contiguous() && t->numel() == n);
+  };
+  TORCH_CHECK(ok(g_loss, 1) && ok(g_logit, B), "click_loss gradients: contiguous fp32");
+  c10::cuda::CUDAGuard g(logit.device());
+  auto d_y = torch::empty({B, ld}, logit.options().dtype(torch::kBFloat16));
+  Tensor d_extra = need_extra ? torch::empty({B, 1}, logit.options()) : Tensor();
+  auto ptr = [](const OptT& t) { return t.has_value() && t->defined() ? t->data_ptr<float>() : nullptr; };
+  const int rc = rb_click_loss_bwd(logit.data_ptr<float>(), label.data_ptr<float>(), ptr(g_loss), ptr(g_logit), (int)B, (int)ld, d_y.data_ptr(),
+                                   need_extra ? d_extra.data_ptr<float>() : nullptr, at::cuda::getCurrentCUDAStream());
+  TORCH_CHECK(rc == 0, "click_loss_bwd failed (code ", rc, ")");
+  return {d_y, d_extra};
+}
+
 Tensor cast_pad_bf16(const Tensor& src, int64_t rows_p, int64_t cols_p) {
   TORCH_CHECK(src.is_cuda() && src.scalar_type() == torch::kFloat32 && src.dim() == 2 && src.stride(1) == 1);
   c10::cuda::CUDAGuard g(src.device());
@@ -190,8 +229,15 @@ std::tuple<Tensor, std::vector<Tensor>, std::vector<Tensor>> mlp_forward(const T
   TORCH_CHECK(wb_cached.empty() || wb_cached.size() == weights.size(), "wb_cached must be empty or hold one entry per layer");
   c10::cuda::CUDAGuard g(x_in.device());
   const int64_t K0p = pad8(weights[0].size(1));
-  Tensor x = x_in.scalar_type() == torch::kBFloat16 ? x_in : x_in.to(torch::kBFloat16);
-  if (x.size(1) != K0p) x = torch::constant_pad_nd(x, {0, K0p - x.size(1)});
+  // (an fp32 input that needs columns is cast and padded in one pass, instead of a cast, a fill and a copy)
+  Tensor x;
+  if (x_in.scalar_type() == torch::kFloat32 && x_in.size(1) != K0p && x_in.size(0) > 0 && x_in.size(1) > 0 && x_in.stride(1) == 1 &&
+      x_in.size(0) < ((int64_t)1 << 31) && x_in.stride(0) < ((int64_t)1 << 31)) {
+    x = cast_pad_bf16(x_in, x_in.size(0), K0p);
+  } else {
+    x = x_in.scalar_type() == torch::kBFloat16 ? x_in : x_in.to(torch::kBFloat16);
+    if (x.size(1) != K0p) x = torch::constant_pad_nd(x, {0, K0p - x.size(1)});
+  }
   x = x.contiguous();
   std::vector<Tensor> ys, wbs;
   Tensor h = x;
@@ -206,8 +252,19 @@ std::tuple<Tensor, std::vector<Tensor>, std::vector<Tensor>> mlp_forward(const T
     } else {
       wb = cast_pad_bf16(weights[l], Np, Kp);
     }
-    Tensor bp = Np == N ? biases[l] : torch::constant_pad_nd(biases[l], {0, Np - N});
-    h = gemm_bf16(h, wb, bp, relu[l], false, false, false, c10::nullopt);
+    const Tensor& b = biases[l];
+    if (Np != N && Np < 192 && b.scalar_type() == torch::kFloat32 && b.is_contiguous() && b.numel() == N && b.device() == x.device()) {
+      // the padding columns have no bias: no padded copy of it (a fill and a copy for the last layer of every click model)
+      RbGemmEpilogue epi{nullptr, 0, nullptr, (int)N};
+      Tensor out = torch::empty({h.size(0), Np}, h.options());
+      const int rc = rb_gemm_bf16_ex(h.data_ptr(), h.stride(0), 0, wb.data_ptr(), wb.stride(0), 0, out.data_ptr(), out.stride(0), 0, b.data_ptr<float>(),
+                                     nullptr, &epi, (int)h.size(0), (int)Np, (int)Kp, relu[l], 1, status_word(x.device()).data_ptr<int64_t>(),
+                                     at::cuda::getCurrentCUDAStream());
+      TORCH_CHECK(rc == 0, "rb_gemm_bf16_ex failed with code ", rc);
+      h = out;
+    } else {
+      h = gemm_bf16(h, wb, Np == N ? b : torch::constant_pad_nd(b, {0, Np - N}), relu[l], false, false, false, c10::nullopt);
+    }
     ys.push_back(h); wbs.push_back(wb);
   }
   return {x, ys, wbs};
@@ -223,7 +280,7 @@ std::tuple<Tensor, Tensor> gemm_dgrad_fused(const Tensor& dy, const Tensor& w, O
   auto out = torch::empty({MM, NN}, dy.options());
   auto db = db_out.has_value() && db_out->defined() ? *db_out : torch::zeros({NN}, dy.options().dtype(torch::kFloat32));
   TORCH_CHECK(db.scalar_type() == torch::kFloat32 && db.is_contiguous() && db.numel() == NN, "db_out: contiguous fp32 [K]");
-  RbGemmEpilogue epi{nullptr, 0, db.data_ptr<float>()};
+  RbGemmEpilogue epi{nullptr, 0, db.data_ptr<float>(), 0};
   if (mask.has_value() && mask->defined()) {
     TORCH_CHECK(mask->scalar_type() == torch::kBFloat16 && mask->dim() == 2 && mask->stride(1) == 1 && mask->size(0) == MM && mask->size(1) == NN,
                 "mask: bf16 [M, K]");
@@ -449,6 +506,8 @@ void init_dense(py::module& m) {
   m.def("fm_head_bwd", &fm_head_bwd);
   m.def("relu_bwd_bias", &relu_bwd_bias, py::arg("y"), py::arg("dout"), py::arg("relu"), py::arg("db_out") = c10::nullopt);
   m.def("cast_pad_bf16", &cast_pad_bf16);
+  m.def("click_loss_fwd", &click_loss_fwd);
+  m.def("click_loss_bwd", &click_loss_bwd);
   // Ragged self-attention forward on the tensor cores (head width 64): returns (out bf16 [T, H * 64], lse2 fp32 [T, H]).
   m.def("ragged_attention_fwd", [](const Tensor& qkv, const Tensor& offsets, int64_t H, int64_t max_len, double scale) {
     TORCH_CHECK(qkv.is_cuda() && qkv.scalar_type() == torch::kBFloat16 && qkv.is_contiguous() && qkv.dim() == 2 &&

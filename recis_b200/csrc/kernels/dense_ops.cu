@@ -340,6 +340,61 @@ cast_pad_bf16_kernel(const float* __restrict__ src, int rows, int cols, int src_
   }
 }
 
+// ------------------------------------------------------------------ click loss
+// The last step of a click model in one kernel per direction: logit = column 0 of the tower's padded output (+ an fp32 term), and the mean
+// binary cross entropy of it. Launches bound it, not work: as tensor ops it was eight of them forward and eight backward, each a few
+// microseconds of host time for a few kilobytes.
+constexpr int kClickRows = 4096;                 // rows per block
+
+__global__ void __launch_bounds__(1024)
+click_loss_fwd_kernel(const __nv_bfloat16* __restrict__ y, int ld, const float* __restrict__ extra, const float* __restrict__ label, int B,
+                      float* __restrict__ logit, float* __restrict__ partial, float scale) {
+  __shared__ float warp_sum[32];
+  const int first = blockIdx.x * kClickRows, last = min(B, first + kClickRows);
+  float sum = 0.f;
+  for (int i = first + (int)threadIdx.x; i < last; i += 1024) {
+    float x = __bfloat162float(y[(int64_t)i * ld]);
+    if (extra != nullptr) x = extra[i] + x;
+    logit[i] = x;
+    // (1 - label) x - log sigmoid(x), the form of the tensor library: NaN and infinities come out as there
+    sum += (1.f - label[i]) * x - (fminf(x, 0.f) - log1pf(expf(-fabsf(x))));
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+  if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    sum = warp_sum[threadIdx.x];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    if (threadIdx.x == 0) partial[blockIdx.x] = sum * scale;
+  }
+}
+
+__global__ void __launch_bounds__(32) click_loss_sum_kernel(const float* __restrict__ partial, int n, float scale, float* __restrict__ loss) {
+  float sum = 0.f;
+  for (int i = threadIdx.x; i < n; i += 32) sum += partial[i];
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+  if (threadIdx.x == 0) *loss = sum * scale;
+}
+
+// d_y (bf16 [B, ld], zeros beyond column 0) and d_extra (fp32 [B], may be null) of g_loss (scalar) and g_logit (fp32 [B]), either may be null
+__global__ void __launch_bounds__(256)
+click_loss_bwd_kernel(const float* __restrict__ logit, const float* __restrict__ label, const float* __restrict__ g_loss,
+                      const float* __restrict__ g_logit, int B, int ld, __nv_bfloat16* __restrict__ d_y, float* __restrict__ d_extra) {
+  const float g = g_loss != nullptr ? *g_loss / (float)B : 0.f;
+  for (int i = blockIdx.x * 256 + (int)threadIdx.x; i < B; i += (int)gridDim.x * 256) {
+    float d = g_loss != nullptr ? (1.f / (1.f + expf(-logit[i])) - label[i]) * g : 0.f;
+    if (g_logit != nullptr) d += g_logit[i];
+    if (d_extra != nullptr) d_extra[i] = d;
+    uint4* row = reinterpret_cast<uint4*>(d_y + (int64_t)i * ld);
+    const uint32_t first = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(d));
+    row[0] = make_uint4(first, 0u, 0u, 0u);
+    for (int c = 1; c < ld / 8; ++c) row[c] = make_uint4(0u, 0u, 0u, 0u);
+  }
+}
+
 inline int blocks_for(int64_t n) { int64_t b = (n + 255) / 256; return (int)std::min<int64_t>(std::max<int64_t>(b, 1), 148 * 16); }
 
 }  // namespace
@@ -435,6 +490,29 @@ void rb_relu_bwd_bias(const void* y, const void* dout, int M, int N, int relu, v
   relu_bwd_bias_kernel<<<grid, 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(y), reinterpret_cast<const __nv_bfloat16*>(dout), M, N,
                                              relu, reinterpret_cast<__nv_bfloat16*>(dy), db);
   rb::note_launch();
+}
+
+int rb_click_loss_blocks(int B) { return (B + kClickRows - 1) / kClickRows; }
+
+int rb_click_loss_fwd(const void* y, int ld, const float* extra, const float* label, int B, float* logit, float* loss, float* partial, cudaStream_t st) {
+  if (B <= 0 || ld <= 0) return 1;
+  const int blocks = rb_click_loss_blocks(B);
+  click_loss_fwd_kernel<<<blocks, 1024, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(y), ld, extra, label, B, logit, blocks == 1 ? loss : partial,
+                                                 blocks == 1 ? 1.f / (float)B : 1.f);
+  rb::note_launch();
+  if (blocks > 1) {
+    click_loss_sum_kernel<<<1, 32, 0, st>>>(partial, blocks, 1.f / (float)B, loss);
+    rb::note_launch();
+  }
+  return cudaGetLastError() == cudaSuccess ? 0 : 4;
+}
+
+int rb_click_loss_bwd(const float* logit, const float* label, const float* g_loss, const float* g_logit, int B, int ld, void* d_y, float* d_extra,
+                      cudaStream_t st) {
+  if (B <= 0 || ld <= 0 || ld % 8 || (reinterpret_cast<uintptr_t>(d_y) & 15)) return 1;
+  click_loss_bwd_kernel<<<blocks_for(B), 256, 0, st>>>(logit, label, g_loss, g_logit, B, ld, reinterpret_cast<__nv_bfloat16*>(d_y), d_extra);
+  rb::note_launch();
+  return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
 void rb_cast_pad_bf16(const float* src, int rows, int cols, int src_ld, void* dst, int rows_p, int cols_p, cudaStream_t st) {

@@ -87,7 +87,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   } else if (warp >= 2) {
     // the tile's bias, fetched while the main loop has not even started (of a split reduction only the first part adds it)
     const int t = (int)threadIdx.x - 64;
-    if (t < BN) bias_s[t] = (bias != nullptr && n0 + t < NN && (!split || blockIdx.z == 0)) ? bias[n0 + t] : 0.f;
+    if (t < BN) bias_s[t] = (bias != nullptr && n0 + t < epi.bias_n && (!split || blockIdx.z == 0)) ? bias[n0 + t] : 0.f;
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -615,9 +615,10 @@ extern "C" int rb_gemm_bf16(const void* a, int64_t lda, int a_mn, const void* b,
 extern "C" int rb_gemm_bf16_ex(const void* a, int64_t lda, int a_mn, const void* b, int64_t ldb, int b_mn, void* out, int64_t ldo,
                                int out_fp32, const float* bias, const float* beta_src, const RbGemmEpilogue* epi_in, int MM, int NN, int KK,
                                int relu, int splits, int64_t* status, cudaStream_t st) {
-  RbGemmEpilogue epi{nullptr, 0, nullptr};
+  RbGemmEpilogue epi{nullptr, 0, nullptr, 0};
   if (epi_in != nullptr) epi = *epi_in;
-  const bool extra = epi.mask_src != nullptr || epi.colsum != nullptr;
+  const bool extra = epi.mask_src != nullptr || epi.colsum != nullptr, short_bias = epi.bias_n > 0 && epi.bias_n < NN;
+  if (!short_bias) epi.bias_n = NN;
   if (extra && splits > 1) return 6;                 // a mask or column sums need the whole reduction in one CTA
   if (MM <= 0 || NN <= 0) return 0;
   // TMA constraints: 16-byte aligned base, row pitch a multiple of 16 bytes
@@ -628,7 +629,7 @@ extern "C" int rb_gemm_bf16_ex(const void* a, int64_t lda, int a_mn, const void*
   // (two rounds), pairs take it when there is work for 96 of them (dW 512 x 1024 of 8192 rows: 23.6 against 18.4 us; dW 256 x 512 of 8192
   // rows, 64 parts: 13.3 against 15.3).
   const int pmode = pair_mode();
-  if (pmode != 0 && MM >= 192 && NN >= 192) {
+  if (pmode != 0 && MM >= 192 && NN >= 192 && !short_bias) {
     const int64_t pairs = (int64_t)((MM + 255) / 256) * ((NN + 255) / 256), total_kb = (KK + BK - 1) / BK;
     const int64_t psplits = splits > 1 ? std::max<int64_t>(1, std::min((128 + pairs - 1) / pairs, total_kb / 4)) : 1;
     if (pmode == 1 || (splits > 1 ? pairs * psplits >= 96 : pairs > (epi.colsum != nullptr ? 37 : 74))) {
@@ -649,14 +650,14 @@ extern "C" int rb_gemm_bf16_ex(const void* a, int64_t lda, int a_mn, const void*
                                          get_map(&ms, src, MM, NN, src_ld, out_fp32 ? 32 : 64, 32, out_fp32 != 0));
   const int tma_out = src_ok && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && (ldo * es) % 16 == 0 &&
                       get_map(&mo, out, MM, NN, ldo, out_fp32 ? 32 : 64, 32, out_fp32 != 0);
-  const int BN = tma_out && !persistent_enabled() ? tile_width(MM, NN, splits) : 128;
+  const int BN = tma_out && (!persistent_enabled() || short_bias) ? tile_width(MM, NN, splits) : 128;
   const bool oka = a_mn ? get_map(&ma, a, KK, MM, lda, 64, BK, false) : get_map(&ma, a, MM, KK, lda, BK, BM, false);
   const bool okb = b_mn ? get_map(&mb, b, KK, NN, ldb, 64, BK, false) : get_map(&mb, b, NN, KK, ldb, BK, BN, false);
   if (!oka || !okb) return 2;
   if (!tma_out) mo = ma;
   if (src == nullptr || !src_ok) ms = mo;
   if (splits > 1 && (!out_fp32 || relu)) return 6;   // partial tiles are accumulated with fp32 reductions into a zeroed output
-  if (persistent_enabled() && tma_out && splits <= 1 && KK > 0 && !extra) {
+  if (persistent_enabled() && tma_out && splits <= 1 && KK > 0 && !extra && !short_bias) {
 #define RB_GEMM_PCASE(AM, BMJ)                                                                                                  \
   if ((a_mn != 0) == AM && (b_mn != 0) == BMJ)                                                                                  \
     return out_fp32 ? launch_persistent<AM, BMJ, float>(ma, mb, mo, bias, beta_src, MM, NN, KK, (int)ldo, relu, status, st)             \

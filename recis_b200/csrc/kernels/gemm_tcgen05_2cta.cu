@@ -374,7 +374,7 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap&
 extern "C" int rb_gemm_bf16_pair(const void* a, int64_t lda, int a_mn, const void* b, int64_t ldb, int b_mn, void* out, int64_t ldo,
                                  int out_fp32, const float* bias, const float* beta_src, const RbGemmEpilogue* epi_in, int MM, int NN, int KK,
                                  int relu, int splits, int reduce_out, int64_t* status, cudaStream_t st) {
-  RbGemmEpilogue epi{nullptr, 0, nullptr};
+  RbGemmEpilogue epi{nullptr, 0, nullptr, 0};
   if (epi_in != nullptr) epi = *epi_in;
   if ((epi.mask_src != nullptr || epi.colsum != nullptr) && reduce_out) return 6;
   if (MM < 192 || NN < 192 || KK <= 0) return 7;

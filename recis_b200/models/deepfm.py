@@ -9,7 +9,7 @@ from torch import nn
 
 from ..nn import EmbeddingEngine, EmbeddingOption
 from ..nn.initializers import NormalInitializer
-from ..ops.dense import MLP, fm_head, fm_interaction, runs_plain
+from ..ops.dense import MLP, click_loss, fm_head, fm_interaction, runs_plain
 
 
 class DeepFM(nn.Module):
@@ -58,8 +58,7 @@ class DeepFM(nn.Module):
         head = fm_head(dense, self.numeric_embs, self.numeric_bias, emb, bias) if fused else None
         if head is not None:
             deep_in, linear = head
-            logit = linear + self.dnn(deep_in)[:, :1].float()
-            return self.loss_fn(logit, label), logit
+            return click_loss(self.dnn, deep_in, label, self.loss_fn, linear)
         bias = bias[:, :, 0]                                                             # [B, F]
         num_emb = dense.unsqueeze(-1) * self.numeric_embs.unsqueeze(0)                   # [B, dense, D]
         cube = torch.cat([num_emb, emb], dim=1).contiguous()

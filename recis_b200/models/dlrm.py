@@ -9,7 +9,7 @@ from torch import nn
 
 from ..nn import EmbeddingEngine, EmbeddingOption
 from ..nn.initializers import NormalInitializer
-from ..ops.dense import MLP, dot_interaction, runs_plain
+from ..ops.dense import MLP, click_loss, dot_interaction, runs_plain
 
 
 class DLRM(nn.Module):
@@ -43,5 +43,4 @@ class DLRM(nn.Module):
         assert names == self.fields
         x = self.bottom(dense)                                        # [B, D] compute dtype
         z = dot_interaction(x, cube)                                  # [B, D + pairs] compute dtype
-        logit = self.top(z)[:, :1].float()
-        return self.loss_fn(logit, label), logit
+        return click_loss(self.top, z, label, self.loss_fn)

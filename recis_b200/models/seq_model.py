@@ -26,7 +26,7 @@ from ..nn import EmbeddingEngine, EmbeddingOption
 from ..nn.functional.ragged_ops import gen_segment_indices
 from ..nn.initializers import NormalInitializer
 from ..ops.attention import ragged_self_attention, segment_mean, target_attention
-from ..ops.dense import MLP, LayerNorm, Linear, ffn_residual, norm_residual_split
+from ..ops.dense import MLP, LayerNorm, Linear, click_loss, ffn_residual, norm_residual_split
 from ..ragged import RaggedTensor
 
 
@@ -123,5 +123,4 @@ class SequenceModel(nn.Module):
         pooled = segment_mean(h, offsets, seg, max_len)
         profile = torch.cat([emb[f].view(B, -1) for f in self.profile_fields], dim=1) if self.profile_fields else h.new_zeros(B, 0)
         z = torch.cat([interest, pooled, q, profile], dim=1)
-        logit = self.head(z)[:, :1].float()
-        return self.loss_fn(logit, batch["label"]), logit
+        return click_loss(self.head, z, batch["label"], self.loss_fn)

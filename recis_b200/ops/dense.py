@@ -283,16 +283,54 @@ class MLP(nn.Module):
         self.layers = nn.ModuleList(
             [Linear(dims[i], dims[i + 1], act=(i < len(dims) - 2) or final_act, dtype=dtype) for i in range(len(dims) - 1)])
 
+    def forward_padded(self, x):
+        """The output with its width padded to a multiple of 8, as the kernels leave it (CUDA, bf16)."""
+        relu = tuple(bool(l.act) for l in self.layers)
+        return _MLPFn.apply(x, relu, *[l.weight for l in self.layers], *[l.bias for l in self.layers])
+
     def forward(self, x):
         n = len(self.layers)
         if x.is_cuda and self.dtype == torch.bfloat16:
-            relu = tuple(bool(l.act) for l in self.layers)
-            y = _MLPFn.apply(x, relu, *[l.weight for l in self.layers], *[l.bias for l in self.layers])
+            y = self.forward_padded(x)
             out = self.layers[-1].out_features
             return y if y.shape[1] == out else y[:, :out]
         for i, layer in enumerate(self.layers):
             x = layer(x, keep_pad=i < n - 1)
         return x
+
+
+class _ClickLossFn(torch.autograd.Function):
+    """``(loss, logit)`` of a tower's padded output, an optional term of the logit and the label, one kernel per direction."""
+
+    @staticmethod
+    def forward(ctx, y, extra, label):
+        loss, logit = native().click_loss_fwd(y, extra, label)
+        ctx.save_for_backward(logit, label)
+        ctx.ld = y.shape[1]
+        ctx.set_materialize_grads(False)
+        return loss, logit
+
+    @staticmethod
+    def backward(ctx, g_loss, g_logit):
+        if g_loss is None and g_logit is None:
+            return None, None, None
+        logit, label = ctx.saved_tensors
+        d_y, d_extra = native().click_loss_bwd(logit, label, g_loss, None if g_logit is None else g_logit.contiguous(), ctx.ld, ctx.needs_input_grad[1])
+        return d_y, d_extra, None
+
+
+def click_loss(mlp: "MLP", x: torch.Tensor, label: torch.Tensor, loss_fn: nn.Module, extra: torch.Tensor = None):
+    """``(loss_fn(logit, label), logit)`` with ``logit = extra + mlp(x)[:, :1]`` in fp32. For the plain mean binary cross entropy of a bf16 tower
+    on CUDA the step behind the tower is one kernel per direction; a hooked or replaced ``mlp`` or ``loss_fn`` is called as a module."""
+    if (runs_plain(mlp, MLP) and mlp.dtype == torch.bfloat16 and x.is_cuda and x.shape[0] > 0 and runs_plain(loss_fn, nn.BCEWithLogitsLoss)
+            and loss_fn.reduction == "mean" and loss_fn.weight is None and loss_fn.pos_weight is None
+            and all(t.dtype == torch.float32 and t.device == x.device and t.shape == (x.shape[0], 1) for t in ((label,) if extra is None else (label, extra)))
+            and not label.requires_grad):
+        return _ClickLossFn.apply(mlp.forward_padded(x), None if extra is None else extra.contiguous(), label.contiguous())
+    logit = mlp(x)[:, :1].float()
+    if extra is not None:
+        logit = extra + logit
+    return loss_fn(logit, label), logit
 
 
 class _DotInteractionFn(torch.autograd.Function):

@@ -369,3 +369,53 @@ def test_vector_readers_take_views_at_any_element(first):
     y, r = norm.forward_split(a)
     (torch.cat([a.new_ones(first), r.reshape(-1), y.reshape(-1)]) * torch.arange(1., 1 + first + 2 * T * H, device=DEV)).sum().backward()
     assert torch.isfinite(a.grad).all()
+
+
+@pytest.mark.parametrize("B", [1, 37, 1000, 4096, 4097, 20000])
+@pytest.mark.parametrize("with_extra", [False, True])
+def test_click_loss_matches_the_tensor_library(B, with_extra):
+    """Loss, logit and gradients of the fused last step against slice + cast + BCEWithLogitsLoss on the same tower output, with a gradient
+    of the logit too; fp32 sums of B terms in another order: 1e-5."""
+    from recis_b200.ops.dense import MLP, click_loss
+    torch.manual_seed(B)
+    mlp = MLP([24, 16, 1], final_act=False).to(DEV)
+    torch.nn.init.normal_(mlp.layers[-1].bias)
+    loss_fn = torch.nn.BCEWithLogitsLoss()
+    x = torch.randn(B, 24, device=DEV) * 4
+    label = (torch.rand(B, 1, device=DEV) < 0.3).float()
+    res = []
+    for fused in (True, False):
+        xi = x.clone().requires_grad_()
+        extra = torch.linspace(-60, 60, B, device=DEV).view(B, 1).requires_grad_() if with_extra else None
+        mlp.zero_grad()
+        if fused:
+            loss, logit = click_loss(mlp, xi, label, loss_fn, extra)
+            assert logit.grad_fn is loss.grad_fn
+        else:
+            y = mlp(xi)
+            assert y.shape == (B, 1)
+            logit = y.float() if extra is None else extra + y.float()
+            loss = loss_fn(logit, label)
+        (3 * loss + 1e-3 * logit.sin().sum()).backward()
+        res.append([loss.detach(), logit.detach(), xi.grad, *[p.grad for p in mlp.parameters()]] + ([extra.grad] if with_extra else []))
+    assert res[0][0].shape == res[1][0].shape and torch.equal(res[0][1], res[1][1])
+    assert abs(float(res[0][0] - res[1][0])) <= 1e-5 * abs(float(res[1][0]))
+    for a, b in zip(res[0][2:], res[1][2:]):
+        # the gradient of the tower's output is rounded to bf16 in both: a last-bit difference in front of it moves single entries by 2^-8
+        assert float((a - b).norm()) <= 2e-3 * float(b.norm()) + 1e-9
+
+
+def test_click_loss_leaves_other_losses_and_hooks_alone():
+    from recis_b200.ops.dense import MLP, click_loss
+    mlp = MLP([8, 1], final_act=False).to(DEV)
+    x, label = torch.randn(5, 8, device=DEV), torch.ones(5, 1, device=DEV)
+    calls = []
+    handle = mlp.register_forward_hook(lambda m, i, o: calls.append(o.shape))
+    loss, _ = click_loss(mlp, x, label, torch.nn.BCEWithLogitsLoss())
+    assert calls == [(5, 1)]
+    handle.remove()
+    for fn in (torch.nn.BCEWithLogitsLoss(reduction="sum"), torch.nn.BCEWithLogitsLoss(pos_weight=torch.tensor([2.0], device=DEV)), torch.nn.MSELoss()):
+        got, logit = click_loss(mlp, x, label, fn)
+        assert torch.equal(got, fn(logit, label))
+    with pytest.raises(ValueError):
+        click_loss(mlp, x, torch.ones(5, device=DEV), torch.nn.BCEWithLogitsLoss())
