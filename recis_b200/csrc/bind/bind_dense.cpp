@@ -190,21 +190,28 @@ std::tuple<Tensor, Tensor> click_loss_fwd(const Tensor& y, OptT extra, const Ten
   return {loss, logit};
 }
 
-// (d_y bf16 [B, ld], d_extra fp32 [B, 1] or undefined)
-std::tuple<Tensor, Tensor> click_loss_bwd(const Tensor& logit, const Tensor& label, OptT g_loss, OptT g_logit, int64_t ld, bool need_extra) {
+// d_logit fp32 [B, 1] of the mean loss
+Tensor click_loss_bwd(const Tensor& logit, const Tensor& label, const Tensor& g_loss) {
   const int64_t B = logit.size(0);
-  auto ok = [&](const OptT& t, int64_t n) {
-    return !(t.has_value() && t->defined()) || (t->device() == logit.device() && t->scalar_type() == torch::kFloat32 && t->is_contiguous() && t->numel() == n);
-  };
-  TORCH_CHECK(ok(g_loss, 1) && ok(g_logit, B), "click_loss gradients: contiguous fp32");
+  auto ok = [&](const Tensor& t, int64_t n) { return t.device() == logit.device() && t.scalar_type() == torch::kFloat32 && t.is_contiguous() && t.numel() == n; };
+  TORCH_CHECK(logit.is_cuda() && ok(logit, B) && ok(label, B) && ok(g_loss, 1), "click_loss_bwd: contiguous fp32 on CUDA");
   c10::cuda::CUDAGuard g(logit.device());
-  auto d_y = torch::empty({B, ld}, logit.options().dtype(torch::kBFloat16));
-  Tensor d_extra = need_extra ? torch::empty({B, 1}, logit.options()) : Tensor();
-  auto ptr = [](const OptT& t) { return t.has_value() && t->defined() ? t->data_ptr<float>() : nullptr; };
-  const int rc = rb_click_loss_bwd(logit.data_ptr<float>(), label.data_ptr<float>(), ptr(g_loss), ptr(g_logit), (int)B, (int)ld, d_y.data_ptr(),
-                                   need_extra ? d_extra.data_ptr<float>() : nullptr, at::cuda::getCurrentCUDAStream());
+  auto d_logit = torch::empty_like(logit);
+  const int rc = rb_click_loss_bwd(logit.data_ptr<float>(), label.data_ptr<float>(), g_loss.data_ptr<float>(), (int)B, d_logit.data_ptr<float>(),
+                                   at::cuda::getCurrentCUDAStream());
   TORCH_CHECK(rc == 0, "click_loss_bwd failed (code ", rc, ")");
-  return {d_y, d_extra};
+  return d_logit;
+}
+
+// d_y bf16 [B, ld] of the logit's gradient
+Tensor click_logit_bwd(const Tensor& g_logit, int64_t ld) {
+  const int64_t B = g_logit.size(0);
+  TORCH_CHECK(g_logit.is_cuda() && g_logit.scalar_type() == torch::kFloat32 && g_logit.is_contiguous() && g_logit.numel() == B, "g_logit: contiguous fp32 [B, 1] on CUDA");
+  c10::cuda::CUDAGuard g(g_logit.device());
+  auto d_y = torch::empty({B, ld}, g_logit.options().dtype(torch::kBFloat16));
+  const int rc = rb_click_logit_bwd(g_logit.data_ptr<float>(), (int)B, (int)ld, d_y.data_ptr(), at::cuda::getCurrentCUDAStream());
+  TORCH_CHECK(rc == 0, "click_logit_bwd failed (code ", rc, ")");
+  return d_y;
 }
 
 Tensor cast_pad_bf16(const Tensor& src, int64_t rows_p, int64_t cols_p) {
@@ -508,6 +515,7 @@ void init_dense(py::module& m) {
   m.def("cast_pad_bf16", &cast_pad_bf16);
   m.def("click_loss_fwd", &click_loss_fwd);
   m.def("click_loss_bwd", &click_loss_bwd);
+  m.def("click_logit_bwd", &click_logit_bwd);
   // Ragged self-attention forward on the tensor cores (head width 64): returns (out bf16 [T, H * 64], lse2 fp32 [T, H]).
   m.def("ragged_attention_fwd", [](const Tensor& qkv, const Tensor& offsets, int64_t H, int64_t max_len, double scale) {
     TORCH_CHECK(qkv.is_cuda() && qkv.scalar_type() == torch::kBFloat16 && qkv.is_contiguous() && qkv.dim() == 2 &&

@@ -341,7 +341,7 @@ cast_pad_bf16_kernel(const float* __restrict__ src, int rows, int cols, int src_
 }
 
 // ------------------------------------------------------------------ click loss
-// The last step of a click model in one kernel per direction: logit = column 0 of the tower's padded output (+ an fp32 term), and the mean
+// The last step of a click model in one kernel forward and two backward: logit = column 0 of the tower's padded output (+ an fp32 term), and the mean
 // binary cross entropy of it. Launches bound it, not work: as tensor ops it was eight of them forward and eight backward, each a few
 // microseconds of host time for a few kilobytes.
 constexpr int kClickRows = 4096;                 // rows per block
@@ -350,10 +350,10 @@ __global__ void __launch_bounds__(1024)
 click_loss_fwd_kernel(const __nv_bfloat16* __restrict__ y, int ld, const float* __restrict__ extra, const float* __restrict__ label, int B,
                       float* __restrict__ logit, float* __restrict__ partial, float scale) {
   __shared__ float warp_sum[32];
-  const int first = blockIdx.x * kClickRows, last = min(B, first + kClickRows);
+  const int64_t first = (int64_t)blockIdx.x * kClickRows, last = min((int64_t)B, first + kClickRows);
   float sum = 0.f;
-  for (int i = first + (int)threadIdx.x; i < last; i += 1024) {
-    float x = __bfloat162float(y[(int64_t)i * ld]);
+  for (int64_t i = first + threadIdx.x; i < last; i += 1024) {
+    float x = __bfloat162float(y[i * ld]);
     if (extra != nullptr) x = extra[i] + x;
     logit[i] = x;
     // (1 - label) x - log sigmoid(x), the form of the tensor library: NaN and infinities come out as there
@@ -379,18 +379,21 @@ __global__ void __launch_bounds__(32) click_loss_sum_kernel(const float* __restr
   if (threadIdx.x == 0) *loss = sum * scale;
 }
 
-// d_y (bf16 [B, ld], zeros beyond column 0) and d_extra (fp32 [B], may be null) of g_loss (scalar) and g_logit (fp32 [B]), either may be null
+// gradient of the loss to the logit, and of the logit to the tower's padded output (zeros beyond column 0). Two kernels, because loss and
+// logit are two steps to autograd: hooks on the logit and gradients with respect to it are between them.
 __global__ void __launch_bounds__(256)
-click_loss_bwd_kernel(const float* __restrict__ logit, const float* __restrict__ label, const float* __restrict__ g_loss,
-                      const float* __restrict__ g_logit, int B, int ld, __nv_bfloat16* __restrict__ d_y, float* __restrict__ d_extra) {
-  const float g = g_loss != nullptr ? *g_loss / (float)B : 0.f;
-  for (int i = blockIdx.x * 256 + (int)threadIdx.x; i < B; i += (int)gridDim.x * 256) {
-    float d = g_loss != nullptr ? (1.f / (1.f + expf(-logit[i])) - label[i]) * g : 0.f;
-    if (g_logit != nullptr) d += g_logit[i];
-    if (d_extra != nullptr) d_extra[i] = d;
-    uint4* row = reinterpret_cast<uint4*>(d_y + (int64_t)i * ld);
-    const uint32_t first = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(d));
-    row[0] = make_uint4(first, 0u, 0u, 0u);
+click_loss_bwd_kernel(const float* __restrict__ logit, const float* __restrict__ label, const float* __restrict__ g_loss, int B,
+                      float* __restrict__ d_logit) {
+  const float g = *g_loss / (float)B;
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < B; i += (int64_t)gridDim.x * 256)
+    d_logit[i] = (1.f / (1.f + expf(-logit[i])) - label[i]) * g;
+}
+
+__global__ void __launch_bounds__(256)
+click_logit_bwd_kernel(const float* __restrict__ g_logit, int B, int ld, __nv_bfloat16* __restrict__ d_y) {
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < B; i += (int64_t)gridDim.x * 256) {
+    uint4* row = reinterpret_cast<uint4*>(d_y + i * ld);
+    row[0] = make_uint4((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(g_logit[i])), 0u, 0u, 0u);
     for (int c = 1; c < ld / 8; ++c) row[c] = make_uint4(0u, 0u, 0u, 0u);
   }
 }
@@ -492,7 +495,7 @@ void rb_relu_bwd_bias(const void* y, const void* dout, int M, int N, int relu, v
   rb::note_launch();
 }
 
-int rb_click_loss_blocks(int B) { return (B + kClickRows - 1) / kClickRows; }
+int rb_click_loss_blocks(int B) { return (int)(((int64_t)B + kClickRows - 1) / kClickRows); }
 
 int rb_click_loss_fwd(const void* y, int ld, const float* extra, const float* label, int B, float* logit, float* loss, float* partial, cudaStream_t st) {
   if (B <= 0 || ld <= 0) return 1;
@@ -507,10 +510,16 @@ int rb_click_loss_fwd(const void* y, int ld, const float* extra, const float* la
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
-int rb_click_loss_bwd(const float* logit, const float* label, const float* g_loss, const float* g_logit, int B, int ld, void* d_y, float* d_extra,
-                      cudaStream_t st) {
+int rb_click_loss_bwd(const float* logit, const float* label, const float* g_loss, int B, float* d_logit, cudaStream_t st) {
+  if (B <= 0) return 1;
+  click_loss_bwd_kernel<<<blocks_for(B), 256, 0, st>>>(logit, label, g_loss, B, d_logit);
+  rb::note_launch();
+  return cudaGetLastError() == cudaSuccess ? 0 : 4;
+}
+
+int rb_click_logit_bwd(const float* g_logit, int B, int ld, void* d_y, cudaStream_t st) {
   if (B <= 0 || ld <= 0 || ld % 8 || (reinterpret_cast<uintptr_t>(d_y) & 15)) return 1;
-  click_loss_bwd_kernel<<<blocks_for(B), 256, 0, st>>>(logit, label, g_loss, g_logit, B, ld, reinterpret_cast<__nv_bfloat16*>(d_y), d_extra);
+  click_logit_bwd_kernel<<<blocks_for(B), 256, 0, st>>>(g_logit, B, ld, reinterpret_cast<__nv_bfloat16*>(d_y));
   rb::note_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }

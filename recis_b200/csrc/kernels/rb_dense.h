@@ -77,11 +77,12 @@ int rb_fm_head_bwd(const float* dense, const float* table, const float* emb, con
 // dy = relu ? dout * (y > 0) : dout (bf16, may be null to skip the store); db[n] += column sums of dy (fp32, may be null)
 void rb_relu_bwd_bias(const void* y, const void* dout, int M, int N, int relu, void* dy, float* db, cudaStream_t st);
 // logit [B] = column 0 of y (bf16 [B, ld]) + extra (fp32 [B] or null), loss = mean binary cross entropy of it against label (fp32 [B]); partial:
-// rb_click_loss_blocks(B) floats of scratch. Backward: d_y bf16 [B, ld] (ld % 8 == 0, zeros beyond column 0), d_extra fp32 [B] or null.
+// rb_click_loss_blocks(B) floats of scratch. Backward: d_logit fp32 [B] of the loss; d_y bf16 [B, ld]
+// (ld % 8 == 0, zeros beyond column 0) of the logit.
 int rb_click_loss_blocks(int B);
 int rb_click_loss_fwd(const void* y, int ld, const float* extra, const float* label, int B, float* logit, float* loss, float* partial, cudaStream_t st);
-int rb_click_loss_bwd(const float* logit, const float* label, const float* g_loss, const float* g_logit, int B, int ld, void* d_y, float* d_extra,
-                      cudaStream_t st);
+int rb_click_loss_bwd(const float* logit, const float* label, const float* g_loss, int B, float* d_logit, cudaStream_t st);
+int rb_click_logit_bwd(const float* g_logit, int B, int ld, void* d_y, cudaStream_t st);
 void rb_cast_pad_bf16(const float* src, int rows, int cols, int src_ld, void* dst, int rows_p, int cols_p, cudaStream_t st);
 
 // Multi-tensor dense Adam: one launch updates up to RB_DENSE_ADAM_MAX fp32 tensors (gridDim.y = tensor).

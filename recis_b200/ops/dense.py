@@ -299,34 +299,48 @@ class MLP(nn.Module):
         return x
 
 
-class _ClickLossFn(torch.autograd.Function):
-    """``(loss, logit)`` of a tower's padded output, an optional term of the logit and the label, one kernel per direction."""
+class _ClickLogitFn(torch.autograd.Function):
+    """The logit of a tower's padded output and an optional term. The same kernel has the mean loss, which goes to ``box``."""
 
     @staticmethod
-    def forward(ctx, y, extra, label):
+    def forward(ctx, y, extra, label, box):
         loss, logit = native().click_loss_fwd(y, extra, label)
-        ctx.save_for_backward(logit, label)
+        box.append(loss)
         ctx.ld = y.shape[1]
-        ctx.set_materialize_grads(False)
-        return loss, logit
+        return logit
 
     @staticmethod
-    def backward(ctx, g_loss, g_logit):
-        if g_loss is None and g_logit is None:
-            return None, None, None
+    def backward(ctx, g):
+        d_y = native().click_logit_bwd(g.contiguous(), ctx.ld) if ctx.needs_input_grad[0] else None
+        return d_y, g if ctx.needs_input_grad[1] else None, None, None
+
+
+class _ClickLossFn(torch.autograd.Function):
+    """The loss in ``box`` as a function of the logit: a step of its own, so that the logit's hooks and gradients stay between the two."""
+
+    @staticmethod
+    def forward(ctx, logit, label, box):
+        ctx.save_for_backward(logit, label)
+        return box.pop()
+
+    @staticmethod
+    def backward(ctx, g):
         logit, label = ctx.saved_tensors
-        d_y, d_extra = native().click_loss_bwd(logit, label, g_loss, None if g_logit is None else g_logit.contiguous(), ctx.ld, ctx.needs_input_grad[1])
-        return d_y, d_extra, None
+        if torch.is_grad_enabled():                        # a second derivative was asked for
+            return (torch.sigmoid(logit) - label) * (g / label.shape[0]), None, None
+        return native().click_loss_bwd(logit, label, g), None, None
 
 
 def click_loss(mlp: "MLP", x: torch.Tensor, label: torch.Tensor, loss_fn: nn.Module, extra: torch.Tensor = None):
     """``(loss_fn(logit, label), logit)`` with ``logit = extra + mlp(x)[:, :1]`` in fp32. For the plain mean binary cross entropy of a bf16 tower
-    on CUDA the step behind the tower is one kernel per direction; a hooked or replaced ``mlp`` or ``loss_fn`` is called as a module."""
+    on CUDA the step behind the tower is one kernel forward and two backward; a hooked or replaced ``mlp`` or ``loss_fn`` is called as a module."""
     if (runs_plain(mlp, MLP) and mlp.dtype == torch.bfloat16 and x.is_cuda and x.shape[0] > 0 and runs_plain(loss_fn, nn.BCEWithLogitsLoss)
             and loss_fn.reduction == "mean" and loss_fn.weight is None and loss_fn.pos_weight is None
             and all(t.dtype == torch.float32 and t.device == x.device and t.shape == (x.shape[0], 1) for t in ((label,) if extra is None else (label, extra)))
             and not label.requires_grad):
-        return _ClickLossFn.apply(mlp.forward_padded(x), None if extra is None else extra.contiguous(), label.contiguous())
+        box, label = [], label.contiguous()
+        logit = _ClickLogitFn.apply(mlp.forward_padded(x), None if extra is None else extra.contiguous(), label, box)
+        return _ClickLossFn.apply(logit, label, box), logit
     logit = mlp(x)[:, :1].float()
     if extra is not None:
         logit = extra + logit

@@ -390,7 +390,7 @@ def test_click_loss_matches_the_tensor_library(B, with_extra):
         mlp.zero_grad()
         if fused:
             loss, logit = click_loss(mlp, xi, label, loss_fn, extra)
-            assert logit.grad_fn is loss.grad_fn
+            assert "ClickLoss" in loss.grad_fn.name() and "ClickLogit" in logit.grad_fn.name()
         else:
             y = mlp(xi)
             assert y.shape == (B, 1)
@@ -403,6 +403,24 @@ def test_click_loss_matches_the_tensor_library(B, with_extra):
     for a, b in zip(res[0][2:], res[1][2:]):
         # the gradient of the tower's output is rounded to bf16 in both: a last-bit difference in front of it moves single entries by 2^-8
         assert float((a - b).norm()) <= 2e-3 * float(b.norm()) + 1e-9
+
+
+def test_click_loss_has_the_logit_in_its_graph():
+    from recis_b200.ops.dense import MLP, click_loss
+    torch.manual_seed(3)
+    mlp, loss_fn = MLP([8, 1], final_act=False).to(DEV), torch.nn.BCEWithLogitsLoss()
+    x, label = torch.randn(37, 8, device=DEV), (torch.rand(37, 1, device=DEV) < 0.5).float()
+    loss, logit = click_loss(mlp, x, label, loss_fn)
+    ref = logit.detach().clone().requires_grad_()
+    want, = torch.autograd.grad(loss_fn(ref, label), ref, create_graph=True)
+    got, = torch.autograd.grad(loss, logit, retain_graph=True)
+    torch.testing.assert_close(got, want.detach(), rtol=1e-5, atol=1e-8)
+    twice, = torch.autograd.grad(torch.autograd.grad(loss, logit, create_graph=True)[0].sum(), logit, retain_graph=True)
+    torch.testing.assert_close(twice, torch.autograd.grad(want.sum(), ref)[0], rtol=1e-5, atol=1e-8)
+    logit.register_hook(lambda g: g * 0)
+    loss /= 2                                                     # as when gradients of several steps are summed
+    loss.backward()
+    assert float(mlp.layers[0].weight.grad.abs().sum()) == 0
 
 
 def test_click_loss_leaves_other_losses_and_hooks_alone():
