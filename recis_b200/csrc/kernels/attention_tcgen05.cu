@@ -2,27 +2,26 @@
 //
 // Input is the packed projection output qkv [T, 3 * H * 64] (bf16) of all sequences of a batch back to back, plus the
 // sequence boundaries offsets [B + 1]; no padding exists anywhere. A work item of the forward is one (sequence, head, 128-query tile); it
-// walks the sequence's keys in steps of 64 or 128 with an online softmax:
+// walks the sequence's keys in steps of 128 with an online softmax:
 //
 //   S  = Q K^T        tcgen05.mma, A = Q tile, B = K tile, both K-major; the tiles arrive by TMA straight from the packed matrix
 //                     in the 128-byte swizzle; fp32 result in tensor memory
 //   P  = exp2(S * scale * log2 e - m)   each thread owns one query row: it reads its row of S with tcgen05.ld, keeps the maximum m and the
 //                     sum l in registers and writes P (bf16) into shared memory
-//   O += P V          tcgen05.mma, A = P, B = the V tile read as an MN-major operand (N = head column, K = key row); with steps of 64
-//                     keys O stays in tensor memory and is rescaled there when a maximum of the warp's rows has grown, with 128 each step's
-//                     product is added to O in registers. (Rescaling only from some growth on saves a tenth of the time, but then the
-//                     largest P of a row is not exactly one: up to 12 % more error.)
+//   O += P V          tcgen05.mma, A = P, B = the V tile read as an MN-major operand (N = head column, K = key row); each step's product is
+//                     added to O in registers. (Rescaling only from some growth on saves a tenth of the time, but then the largest P
+//                     of a row is not exactly one: up to 12 % more error.)
 //
 // and finally writes O / l (bf16) and the log-sum-exp (base 2) of the row. Persistent CTAs with separate roles: four softmax warps, one
 // that fetches work and issues the TMA loads, one that issues the MMAs. S of the next step is multiplied as soon as this one's has been read,
 // under P V. Keys past the end of a sequence are masked in the softmax; query rows past the end are computed on whatever is there and not
 // stored; of a partial tile only the 32-row boxes that hold a row are loaded.
 //
-// What bounds it is the latency of a step - score, exponentials, product, in sequence for a query tile - with two or four query
+// What bounds it is the latency of a step - score, exponentials, product, in sequence for a query tile - with two query
 // tiles to an SM (tensor memory holds no more); the exponentials take two fifths of the special-function units' cycles. Measured on a B200
 // (before: one CTA of 128 threads per item, loads, MMAs and exponentials one after the other, P through shared memory, O in registers):
 //   256 sequences of 50..1000 tokens, 4 heads:  290 -> 225 us (83 GFLOP in existing elements: 367 TFLOP/s)
-//   3000 sequences of 1..90 tokens, 8 heads:    418 -> 166 us; under a bound of 1000 instead of 90: 1210 -> 235 us
+//   3000 sequences of 1..90 tokens, 8 heads:    423 -> 235 us; under a bound of 360 instead of 90: 623 -> 240 us
 //   37 sequences of 1..1000 tokens, 4 heads:     55 -> 51 us;  one sequence of 1000 tokens, 8 heads: 27 -> 24.6 us
 //
 // The reference has no attention kernel; its sequence example pads to the longest sequence and calls the library SDPA
@@ -42,7 +41,7 @@ namespace {
 
 using namespace rb::tc;
 
-constexpr int kTile = 128;                 // queries per CTA = keys per step = tensor-memory lanes
+constexpr int kTile = 128;                 // queries of a work item = keys per step = tensor-memory lanes
 constexpr int kHead = 64;                  // head width (one 128-byte swizzle row)
 constexpr int kBlk = kTile * 128;          // bytes of one [128 rows x 64 bf16] swizzled block
 
@@ -62,33 +61,21 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 // ---------------------------------------------------------------------------------------------- forward
 struct AttnItem { int s0, len, head, kt; };          // len < 0: no more work; kt: the item's tile (of queries here, of keys in the backward)
 
-// Keys per step and CTAs per SM: 64 keys and four CTAs where a sequence has one query tile (tensor memory: S 64 + O 64 columns each), so that
-// sixteen softmax warps hide one another's waits (3000 sequences of 1..90 tokens, 8 heads: 170 us, with 128 keys 206); 128 keys and two CTAs
-// elsewhere, with the rows of O in registers. (There 64 keys and O in tensor memory would be a little faster, 207 us at 256 sequences of
-// 50..1000 tokens, 4 heads, but P is then rounded against the maxima of half as many keys and O summed in another order; as it is, every
-// output is the same to the bit as with one CTA per tile, and a training run takes the same course.)
-template <int kKeys_> struct FwdCfg {
-  static constexpr int kKeys = kKeys_, kCtas = kKeys == 64 ? 4 : 2;
-  static constexpr int kKvBlk = kKeys * 128;                     // bytes of one [keys x 64 bf16] swizzled block
-  static constexpr uint32_t kS = 0, kO = kKeys;                  // tensor-memory columns: S and O, fp32
-  static constexpr uint32_t kTmemCols = kKeys == 64 ? 128 : 256;
-  static constexpr int kPBlk = kKeys / 64;                       // blocks of [128 q x 64 keys] of P
-  static constexpr size_t kSmem = 1024 + (1 + kPBlk) * (size_t)kBlk + 2 * (size_t)kKvBlk;
-};
+// 128 keys a step and the rows of O in registers, whatever the batch: an output depends on its sequence alone, to the bit. (64 keys a step and
+// O in tensor memory let four CTAs share an SM, 166 against 235 us at 3000 sequences of 1..90 tokens, 8 heads, and 207 against 225 at
+// 256 sequences of 50..1000 tokens, 4 heads. But P is then rounded against the maxima of half as many keys and O rescaled and summed in
+// another order: 6e-4 of the first case's outputs by norm, and a sequence's outputs would depend on how many others are in its batch.)
+constexpr int kFwdCtas = 2;                                      // per SM
+constexpr uint32_t kFwdS = 0, kFwdO = kTile;                     // tensor-memory columns: S and O, fp32
+constexpr uint32_t kFwdTmemCols = 256;
+constexpr size_t kFwdSmem = 1024 + 5 * (size_t)kBlk;             // Q, two blocks of [128 q x 64 keys] of P, K, V
 constexpr int kFwdThreads = 192;                                 // four softmax warps, producer, MMA
 
-// 8 columns of tensor memory, one row per lane, and 16 columns into it
+// 8 columns of tensor memory, one row per lane
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
 }
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
-      "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void fma_f32x2(float& x0, float& x1, float a0, float a1, float b, float c) {      // x = a * b + c
   asm("{\n\t.reg .b64 u, w, z;\n\tmov.b64 u, {%2, %3};\n\tmov.b64 w, {%4, %4};\n\tmov.b64 z, {%5, %5};\n\tfma.rn.f32x2 u, u, w, z;\n\tmov.b64 {%0, %1}, u;\n\t}"
       : "=f"(x0), "=f"(x1) : "f"(a0), "f"(a1), "f"(b), "f"(c));
@@ -126,14 +113,11 @@ __device__ __forceinline__ void clear_rows(int64_t from, int64_t to, int H, __nv
   }
 }
 
-template <int kKeys>
-__global__ void __launch_bounds__(kFwdThreads, FwdCfg<kKeys>::kCtas)
-ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv, const __grid_constant__ CUtensorMap map_rows,
+__global__ void __launch_bounds__(kFwdThreads, kFwdCtas)
+ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const __grid_constant__ CUtensorMap map_rows,
                             const int32_t* __restrict__ offsets, int64_t T, int B, int H, int tiles, int chunk, float scale_log2,
                             __nv_bfloat16* __restrict__ out, float* __restrict__ lse2, unsigned* __restrict__ counter,
                             int64_t* __restrict__ status) {
-  constexpr int kKvBlk = FwdCfg<kKeys>::kKvBlk;
-  constexpr uint32_t kFwdS = FwdCfg<kKeys>::kS, kFwdO = FwdCfg<kKeys>::kO, kFwdTmemCols = FwdCfg<kKeys>::kTmemCols;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t q_full[2], k_full, v_full;
   __shared__ __align__(8) uint64_t s_full, p_full, o_full, o_empty;
@@ -142,9 +126,9 @@ ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   __shared__ int abort_flag;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* qtile = smem;                             // [128 q][64 d]   K-major A of S = Q K^T
-  uint8_t* ptile = smem + kBlk;                      // 64 keys wide blocks of [128 q][64 keys]   K-major A of O += P V; then the rows of O on their way out
-  uint8_t* ktile = ptile + FwdCfg<kKeys>::kPBlk * kBlk;      // [keys][64 d]     K-major B of S
-  uint8_t* vtile = ktile + kKvBlk;                           // [keys][64 d]     MN-major B of O += P V (N = d, K = key)
+  uint8_t* ptile = smem + kBlk;                      // 2 x [128 q][64 keys]   K-major A of P V; then the rows of O on their way out
+  uint8_t* ktile = smem + 3 * kBlk;                  // [128 keys][64 d]       K-major B of S
+  uint8_t* vtile = smem + 4 * kBlk;                  // [128 keys][64 d]       MN-major B of P V (N = d, K = key)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int kProducer = 4, kMma = 5;
 
@@ -200,8 +184,8 @@ ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       bool ok = true;
       // `rows` rows of 64 columns from row `row`: whole tiles as one box, shorter ones in boxes of 32 rows (what lies behind is not read, or
       // only by rows and columns that are masked or not stored)
-      auto load = [&](uint8_t* dst, const CUtensorMap* map, int box, int x, int row, int rows, uint64_t* bar) {
-        if (rows > box - 32) tma_load_2d(dst, map, x, row, bar);
+      auto load = [&](uint8_t* dst, int x, int row, int rows, uint64_t* bar) {
+        if (rows > kTile - 32) tma_load_2d(dst, &map_qkv, x, row, bar);
         else for (int i = 0; i * 32 < rows; ++i) tma_load_2d(dst + i * 4096, &map_rows, x, row + i * 32, bar);
       };
       while (ok) {
@@ -231,23 +215,23 @@ ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           if (lane == 0) {
             const int xq = item.head * kHead, xk = (H + item.head) * kHead, xv = (2 * H + item.head) * kHead;
             // A buffer is free when the MMAs that read it are complete: Q and K with S, V with P V of the step before.
-            for (int j = 0; j * kKeys < item.len; ++j, ++g) {
-              const int rows = min(kKeys, item.len - j * kKeys);
+            for (int j = 0; j * kTile < item.len; ++j, ++g) {
+              const int rows = min(kTile, item.len - j * kTile);
               ok = g == 0 || mbar_wait(&s_full, (uint32_t)((g - 1) & 1), &abort_flag);
               if (!ok) break;
               if (j == 0) {
                 const int q_rows = min(kTile, item.len - item.kt * kTile);
                 slot[it & 1] = item;
                 mbar_expect_tx(&q_full[it & 1], (uint32_t)((q_rows + 31) & ~31) * 128u);
-                load(qtile, &map_q, kTile, xq, item.s0 + item.kt * kTile, q_rows, &q_full[it & 1]);
+                load(qtile, xq, item.s0 + item.kt * kTile, q_rows, &q_full[it & 1]);
                 ++it;
               }
               mbar_expect_tx(&k_full, (uint32_t)((rows + 31) & ~31) * 128u);
-              load(ktile, &map_kv, kKeys, xk, item.s0 + j * kKeys, rows, &k_full);
+              load(ktile, xk, item.s0 + j * kTile, rows, &k_full);
               ok = g == 0 || mbar_wait(&o_full, (uint32_t)((g - 1) & 1), &abort_flag);
               if (!ok) break;
               mbar_expect_tx(&v_full, (uint32_t)((rows + 31) & ~31) * 128u);
-              load(vtile, &map_kv, kKeys, xv, item.s0 + j * kKeys, rows, &v_full);
+              load(vtile, xv, item.s0 + j * kTile, rows, &v_full);
             }
           }
           ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
@@ -262,7 +246,7 @@ ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       // ------------------------------------------------------------------ MMA issuer (the whole warp; one lane issues)
       // Descriptors advance by adding to the 16-byte address field.
       const uint64_t d_q = make_desc(smem_u32(qtile), 16, 1024), d_k = make_desc(smem_u32(ktile), 16, 1024);
-      const uint64_t d_p = make_desc(smem_u32(ptile), 16, 1024), d_v = make_desc(smem_u32(vtile), kKvBlk, 1024);
+      const uint64_t d_p = make_desc(smem_u32(ptile), 16, 1024), d_v = make_desc(smem_u32(vtile), kBlk, 1024);
       const uint32_t idesc_o = make_idesc_bf16(kTile, kHead, false, true);
       const bool leader = elect_one();
       int g = 0;
@@ -284,20 +268,20 @@ ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         if (len < 0) break;
         ok = wait_all(&k_full, (uint32_t)(g & 1));
         if (!ok) break;
-        issue_s(min(kKeys, len));
-        for (int j = 0; j * kKeys < len; ++j, ++g) {
-          const int left = len - j * kKeys, steps = (min(kKeys, left) + 15) >> 4;      // of 16 keys
+        issue_s(min(kTile, len));
+        for (int j = 0; j * kTile < len; ++j, ++g) {
+          const int left = len - j * kTile, steps = (min(kTile, left) + 15) >> 4;      // of 16 keys
           // everything else is waited for before P, which comes last: between P and the next S lies only their issue
           ok = wait_all(&v_full, (uint32_t)(g & 1)) && (j > 0 || it == 0 || wait_all(&o_empty, (uint32_t)((it - 1) & 1))) &&
-               (left <= kKeys || wait_all(&k_full, (uint32_t)((g + 1) & 1))) && wait_all(&p_full, (uint32_t)(g & 1));
+               (left <= kTile || wait_all(&k_full, (uint32_t)((g + 1) & 1))) && wait_all(&p_full, (uint32_t)(g & 1));
           if (!ok) break;
-          if (left > kKeys) issue_s(min(kKeys, left - kKeys));                         // (S of this step has been read)
+          if (left > kTile) issue_s(min(kTile, left - kTile));                         // (S of this step has been read)
           else fence_after_sync();
           if (leader) {
-            umma_bf16(tmem + kFwdO, d_p, d_v, idesc_o, kKeys == 64 && j > 0 ? 1u : 0u);
-            if (steps == kKeys / 16) {
+            umma_bf16(tmem + kFwdO, d_p, d_v, idesc_o, 0u);
+            if (steps == kTile / 16) {
 #pragma unroll
-              for (int k = 1; k < kKeys / 16; ++k) umma_bf16(tmem + kFwdO, d_p + (uint64_t)((k >> 2) * (kBlk >> 4) + (k & 3) * 2), d_v + (uint64_t)(k * 128), idesc_o, 1u);
+              for (int k = 1; k < kTile / 16; ++k) umma_bf16(tmem + kFwdO, d_p + (uint64_t)((k >> 2) * (kBlk >> 4) + (k & 3) * 2), d_v + (uint64_t)(k * 128), idesc_o, 1u);
             } else {
 #pragma unroll 1
               for (int k = 1; k < steps; ++k) umma_bf16(tmem + kFwdO, d_p + (uint64_t)((k >> 2) * (kBlk >> 4) + (k & 3) * 2), d_v + (uint64_t)(k * 128), idesc_o, 1u);
@@ -322,9 +306,9 @@ ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       if (item.len < 0) break;
       const int rows = item.len - item.kt * kTile - warp * 32;                // rows of this warp that exist (may be <= 0, or more than 32)
       float m = -INFINITY, l = 0.f, alpha = 0.f;                              // maximum so far (in powers of two), sum of P, the last step's rescale
-      float o[kKeys == 64 ? 1 : kHead];                                       // with 128 keys the rows of O are here, each step's P V is added to them
+      float o[kHead];                                                         // the row of O: each step's P V is added to it
 #pragma unroll
-      for (int d = 0; d < (kKeys == 64 ? 1 : kHead); ++d) o[d] = 0.f;
+      for (int d = 0; d < kHead; ++d) o[d] = 0.f;
       auto add_pv = [&]() {
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
@@ -332,11 +316,11 @@ ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           tmem_ld32(trow + kFwdO + (uint32_t)(e * 32), r);
           tmem_ld_wait();
 #pragma unroll
-          for (int d = 0; d < 32; ++d) o[(e * 32 + d) & (kKeys == 64 ? 0 : kHead - 1)] = fmaf(o[(e * 32 + d) & (kKeys == 64 ? 0 : kHead - 1)], alpha, __uint_as_float(r[d]));
+          for (int d = 0; d < 32; ++d) o[e * 32 + d] = fmaf(o[e * 32 + d], alpha, __uint_as_float(r[d]));
         }
       };
-      for (int j = 0; j * kKeys < item.len; ++j, ++g) {
-        const int valid = min(kKeys, item.len - j * kKeys);                   // key columns of this step that exist
+      for (int j = 0; j * kTile < item.len; ++j, ++g) {
+        const int valid = min(kTile, item.len - j * kTile);                   // key columns of this step that exist
         ok = wait_all(&s_full, (uint32_t)(g & 1));
         if (!ok) break;
         fence_after_sync();
@@ -372,27 +356,10 @@ ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             ok = wait_all(&o_full, (uint32_t)((g - 1) & 1));
             if (!ok) break;
           }
-          if constexpr (kKeys == 128) {
-            if (j > 0) {
-              fence_after_sync();
-              add_pv();
-              alpha = fast_exp2(m - m_new);
-            }
-          } else if (j > 0) {
+          if (j > 0) {
+            fence_after_sync();
+            add_pv();
             alpha = fast_exp2(m - m_new);
-            if (__any_sync(0xffffffffu, m_new > m && lane < rows)) {
-              fence_after_sync();
-#pragma unroll 1
-              for (int e = 0; e < 4; ++e) {
-                uint32_t r[16];
-                tmem_ld16(trow + kFwdO + (uint32_t)(e * 16), r);
-                tmem_ld_wait();
-#pragma unroll
-                for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
-                tmem_st16(trow + kFwdO + (uint32_t)(e * 16), r);
-              }
-              tmem_st_wait();
-            }
           }
           m = m_new;
           const float neg_m = -m;
@@ -441,26 +408,13 @@ ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       // through this warp's rows of the P tile, which the item no longer needs: eight lanes store a row, so that every store is whole lines
       const float inv = l > 0.f ? 1.f / l : 0.f;
       if (rows > 0) {
-        if constexpr (kKeys == 128) {
-          add_pv();
+        add_pv();
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            uint32_t u[4];
+        for (int c = 0; c < 8; ++c) {
+          uint32_t u[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) u[e] = pack_bf16x2(o[c * 8 + 2 * e] * inv, o[c * 8 + 2 * e + 1] * inv);
-            st_shared16(prow ^ (uint32_t)(c << 4), u[0], u[1], u[2], u[3]);
-          }
-        } else {
-#pragma unroll 1
-          for (int c = 0; c < 4; ++c) {
-            uint32_t r[16], u[8];
-            tmem_ld16(trow + kFwdO + (uint32_t)(c * 16), r);
-            tmem_ld_wait();
-#pragma unroll
-            for (int e = 0; e < 8; ++e) u[e] = pack_bf16x2(__uint_as_float(r[2 * e]) * inv, __uint_as_float(r[2 * e + 1]) * inv);
-#pragma unroll
-            for (int e = 0; e < 2; ++e) st_shared16(prow ^ (uint32_t)((2 * c + e) << 4), u[4 * e], u[4 * e + 1], u[4 * e + 2], u[4 * e + 3]);
-          }
+          for (int e = 0; e < 4; ++e) u[e] = pack_bf16x2(o[c * 8 + 2 * e] * inv, o[c * 8 + 2 * e + 1] * inv);
+          st_shared16(prow ^ (uint32_t)(c << 4), u[0], u[1], u[2], u[3]);
         }
       }
       fence_before_sync();
@@ -1045,26 +999,23 @@ extern "C" int rb_ragged_attention_fwd(const void* qkv, const int32_t* offsets, 
   if (items > (int64_t)1 << 31) return 1;
   // Up to three rounds of items of long sequences are dealt out one per CTA, which saves the counter (15 sequences of 1..1000 tokens, 4 heads:
   // 28.7 us, fetched 38.9, before 30.8; 37 sequences, 1184 items: 57 dealt out, 51 fetched, before 55).
-  const bool long_steps = tiles > 1 || items <= 8 * FwdCfg<128>::kCtas * 148, dealt = tiles > 2 && items <= 3 * FwdCfg<128>::kCtas * 148;
-  const int keys = long_steps ? 128 : 64;
-  CUtensorMap map_q, map_kv, map_rows;
-  if (rb_tensor_map_2d(&map_q, qkv, T, (int64_t)3 * H * kHead, (int64_t)3 * H * kHead, kHead, kTile, 0) != 0 ||
-      rb_tensor_map_2d(&map_kv, qkv, T, (int64_t)3 * H * kHead, (int64_t)3 * H * kHead, kHead, keys, 0) != 0 ||
+  const int slots = kFwdCtas * 148;
+  const bool dealt = tiles > 2 && items <= 3 * slots;
+  CUtensorMap map_qkv, map_rows;
+  if (rb_tensor_map_2d(&map_qkv, qkv, T, (int64_t)3 * H * kHead, (int64_t)3 * H * kHead, kHead, kTile, 0) != 0 ||
       rb_tensor_map_2d(&map_rows, qkv, T, (int64_t)3 * H * kHead, (int64_t)3 * H * kHead, kHead, 32, 0) != 0)
     return 1;
-  auto kern = long_steps ? ragged_attention_fwd_kernel<128> : ragged_attention_fwd_kernel<64>;
-  const size_t smem = long_steps ? FwdCfg<128>::kSmem : FwdCfg<64>::kSmem;
-  static bool attr[2] = {false, false};
-  if (!attr[long_steps]) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 3;
-    attr[long_steps] = true;
+  static bool attr = false;
+  if (!attr) {
+    if (cudaFuncSetAttribute(ragged_attention_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem) != cudaSuccess) return 3;
+    attr = true;
   }
   if (dealt) counter = nullptr;
   else if (cudaMemsetAsync(counter, 0, sizeof(unsigned), st) != cudaSuccess) return 4;
   // Items fetched at a time: one where that is about 32 fetches per CTA, more under a loose bound, where most items are empty.
-  const int slots = 148 * (long_steps ? FwdCfg<128>::kCtas : FwdCfg<64>::kCtas), grid = (int)(dealt ? items : std::min<int64_t>(items, slots));
+  const int grid = (int)(dealt ? items : std::min<int64_t>(items, slots));
   const int chunk = (int)std::min<int64_t>(32, std::max<int64_t>(1, items / (32 * slots)));
-  kern<<<grid, kFwdThreads, smem, st>>>(map_q, map_kv, map_rows, offsets, T, B, H, tiles, chunk, scale * 1.4426950408889634f,
+  ragged_attention_fwd_kernel<<<grid, kFwdThreads, kFwdSmem, st>>>(map_qkv, map_rows, offsets, T, B, H, tiles, chunk, scale * 1.4426950408889634f,
                                         reinterpret_cast<__nv_bfloat16*>(out), lse2, counter, status);
   rb::note_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : 4;

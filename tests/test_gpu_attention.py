@@ -254,9 +254,9 @@ def test_backward_of_sequences_longer_than_the_bound(lens, bound, H):
                                     ([90] * 200, 4)])
 @pytest.mark.parametrize("spread", [1.0, 40.0])
 def test_forward_on_every_work_split_and_with_growing_scores(lens, H, spread):
-    """Items dealt out, fetched with long and with short steps, and key counts on both sides of a step and of a 32-column chunk. With ``spread``
-    the scores of a row reach hundreds and grow along the sequence, so that the reference exponent is raised in the middle of a step. The
-    last key of every sequence is non-finite in the tensor's tail and must not be read. Bounds as above."""
+    """Items dealt out one per CTA and fetched from the counter, one and several at a time, and key counts on both sides of a step and of a
+    32-column chunk. With ``spread`` the scores of a row reach hundreds and grow along the sequence, so that every step raises the reference
+    exponent. The rows behind the last sequence are non-finite and must not reach anything. Bounds as above."""
     import recis_b200
     C = recis_b200.native()
     qkv, offs, _ = _case(lens, H, seed=len(lens))
@@ -273,3 +273,30 @@ def test_forward_on_every_work_split_and_with_growing_scores(lens, H, spread):
         assert float(got[len(qkv):].abs().max()) == 0.0 and float(lse[len(qkv):].abs().max()) == 0.0
         err = (got[:len(qkv)] - ref).norm() / ref.norm()
         assert err < 1e-2, (bound, float(err))
+
+
+@pytest.mark.parametrize("repeat,H,bound", [(40, 8, 128), (100, 8, 60), (470, 8, 128)])
+@pytest.mark.parametrize("spread", [1.0, 20.0])
+def test_outputs_of_a_sequence_do_not_depend_on_its_batch(repeat, H, bound, spread):
+    """Short sequences by the thousand (up to several items per fetch), with some longer than the bound among them: output and log-sum-exp are
+    those of the same sequences in a batch of their own, to the bit, and of every length within the bounds above."""
+    import recis_b200
+    C = recis_b200.native()
+    some = [1, 16, 17, 63, 64, 65, 96, 127, 128, 300]
+    qkv, offs, _ = _case(some, H, seed=repeat)
+    if spread > 1:
+        pos = torch.cat([torch.arange(L) / max(L, 2) for L in some])
+        k = slice(H * 64, 2 * H * 64)
+        qkv[:, k] = (qkv[:, k].float() * (1 + spread * pos[:, None])).to(torch.bfloat16)
+    T = sum(some)
+    out, lse = C.ragged_attention_fwd(qkv.to(DEV), offs.to(DEV), H, bound, 0.125)
+    all_offs = torch.cat([offs[:-1] + i * T for i in range(repeat)] + [torch.tensor([repeat * T], dtype=torch.int32)])
+    many, many_lse = C.ragged_attention_fwd(qkv.to(DEV).repeat(repeat, 1), all_offs.to(DEV), H, bound, 0.125)
+    assert C.dense_status("cuda:0") == 0
+    assert torch.equal(many.view(repeat, T, -1), out.expand(repeat, T, -1)) and torch.equal(many_lse.view(repeat, T, -1), lse.expand(repeat, T, -1))
+    ref, _ = _oracle(qkv, some, H)
+    got = out.float().cpu()
+    for s0, L in zip(offs.tolist(), some):
+        n = min(L, 128)                                               # queries in the bound's one tile
+        assert (got[s0:s0 + n] - ref[s0:s0 + n]).norm() / ref[s0:s0 + n].norm() < 1e-2, L
+        assert torch.count_nonzero(got[s0 + n:s0 + L]) == 0
