@@ -889,6 +889,7 @@ ragged_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const _
           zero_half_row(rowbase, (uint32_t)((4 + (g & 1) * 2) * kBlk), half);
           zero_half_row(rowbase, (uint32_t)((5 + (g & 1) * 2) * kBlk), half);
         }
+        __syncwarp();                                                         // the zeros above are some lanes' work, tcgen05.ld the warp's
         const bool rows_on = quarter * 32 < valid_q, rows_full = quarter * 32 + 32 <= valid_q;      // uniform for the warp
         const float lse_q = lse_next, nds = -delta_next * scale;              // (dP - delta) * scale = dP * scale + nds
         if constexpr (kSingle) {

@@ -88,7 +88,7 @@ dot_interaction_tc_fwd_kernel(const __nv_bfloat16* __restrict__ x, const float* 
     for (int d = lane; d < D; d += 32) mine[d] = x[(int64_t)b * D + d];
     for (int c = D + P + lane; c < out_ld; c += 32) mine[c] = __float2bfloat16_rn(0.f);
   }
-  const bool ok = mbar_wait(&done_bar, 0, &abort_flag);
+  const bool ok = __all_sync(0xffffffffu, mbar_wait(&done_bar, 0, &abort_flag) ? 1 : 0) != 0;      // (and the warp meets before tcgen05.ld)
   fence_after_sync();
   if (ok) {
     uint32_t r[32];
@@ -112,7 +112,7 @@ dot_interaction_tc_fwd_kernel(const __nv_bfloat16* __restrict__ x, const float* 
   }
   fence_before_sync();
   __syncthreads();
-  if (w == 0) { fence_after_sync(); tmem_dealloc(tmem, 128); }
+  if (w == 0) { __syncwarp(); fence_after_sync(); tmem_dealloc(tmem, 128); }
   if (threadIdx.x == 0 && abort_flag) rb::set_status(status, rb::kStatusWaitTimeout);
 }
 
@@ -187,7 +187,7 @@ dot_interaction_tc_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* 
     }
     umma_commit(&done_bar);
   }
-  const bool ok = mbar_wait(&done_bar, 0, &abort_flag);
+  const bool ok = __all_sync(0xffffffffu, mbar_wait(&done_bar, 0, &abort_flag) ? 1 : 0) != 0;      // (and the warp meets before tcgen05.ld)
   fence_after_sync();
   if (ok) {
     const int i = lane;
@@ -214,7 +214,7 @@ dot_interaction_tc_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* 
   }
   fence_before_sync();
   __syncthreads();
-  if (w == 0) { fence_after_sync(); tmem_dealloc(tmem, 128); }
+  if (w == 0) { __syncwarp(); fence_after_sync(); tmem_dealloc(tmem, 128); }
   if (threadIdx.x == 0 && abort_flag) rb::set_status(status, rb::kStatusWaitTimeout);
 }
 

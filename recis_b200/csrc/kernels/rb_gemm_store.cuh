@@ -136,8 +136,9 @@ struct EpilogueWork {
 // 8 columns a lane holds columns 2 (lane & 3) and + 1 of the rows lane / 4 + 8 r, so that v[4 (h kCols / 8 + j) + 2 r + e] is row
 // 16 h + 8 r + lane / 4, column 8 j + 2 (lane & 3) + e. A lane then meets a quarter of the columns: the bias costs a quarter of the
 // shared-memory and L1 traffic it costs with a row per lane (25 us of 221 at 269000 x 1024 x 256), and a column sum 14 exchanges
-// per 64 columns instead of 62.
+// per 64 columns instead of 62. Lanes may arrive one by one (the caller's stores and copies are some lanes' work): they meet here.
 template <int kCols> __device__ __forceinline__ void load_box(uint32_t taddr, float (&v)[kCols]) {
+  __syncwarp();
   if constexpr (kCols == 64) {
     tc::tmem_ld_16x64(taddr, reinterpret_cast<uint32_t(&)[32]>(v[0]));
     tc::tmem_ld_16x64(taddr + (16u << 16), reinterpret_cast<uint32_t(&)[32]>(v[32]));
@@ -190,6 +191,7 @@ template <typename OutT>
 __device__ __forceinline__ void finish_box(const EpilogueWork& w, float (&v)[Store<OutT>::kBoxCols], const float* bias, bool has_src, uint8_t* box, int row0,
                                            int col, int lane, float (&sum)[Store<OutT>::kBoxCols / 32]) {
   constexpr int kCols = Store<OutT>::kBoxCols, kBlocks = kCols / 8;
+  __syncwarp();                                  // ldmatrix and stmatrix below want the whole warp at once
   if (bias != nullptr) {
 #pragma unroll
     for (int j = 0; j < kBlocks; ++j) {
