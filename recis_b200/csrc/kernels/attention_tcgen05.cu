@@ -385,6 +385,9 @@ ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const _
             st_shared16((prow ^ (uint32_t)(((c >> 3) & 7) << 4)) + (uint32_t)((c >> 6) * kBlk), pk[0], pk[1], pk[2], pk[3]);
           }
           l = fmaf(l, alpha, (sum[0] + sum[2]) + (sum[1] + sum[3]));
+        } else if (g > 0) {                                                   // every warp follows every phase of o_full: the wait behind the last step
+          ok = wait_all(&o_full, (uint32_t)((g - 1) & 1));                    // is for that step's product, not for an older one of the same parity
+          if (!ok) break;
         }
         if (valid & 15) {
           // V rows between the last key and the end of the last 16-key step become zeros, so that the zeros of P never meet a non-finite value
