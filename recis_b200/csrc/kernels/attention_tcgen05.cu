@@ -1001,10 +1001,16 @@ extern "C" int rb_ragged_attention_fwd(const void* qkv, const int32_t* offsets, 
   const int tiles = (int)(((int64_t)max_len + kTile - 1) / kTile);
   const int64_t items = (int64_t)tiles * B * H;
   if (items > (int64_t)1 << 31) return 1;
-  // Up to three rounds of items of long sequences are dealt out one per CTA, which saves the counter (15 sequences of 1..1000 tokens, 4 heads:
-  // 28.7 us, fetched 38.9, before 30.8; 37 sequences, 1184 items: 57 dealt out, 51 fetched, before 55).
+  // Items are dealt out one per CTA, which saves the counter and its clearing, where that is one round of them (a sequence of 100 tokens, 4 heads:
+  // 10.3 us, fetched 12.3; 64 of 1..128 tokens: 14.3, fetched 15.7), and up to three rounds of items of sequences of several tiles (15
+  // sequences of 1..1000 tokens, 4 heads: 28.6 us, fetched 34.4) or of few tokens (64 of 1..128 tokens under a bound of 256: 16.4, fetched
+  // 18.4). 37 sequences of 1..1000 tokens, 1184 items: 59 dealt out, 56 fetched. Under a loose bound most items are empty and cost a fetched
+  // batch less; where the tokens make about one round of items and are long ones, dealing stays ahead up to eight rounds (15 sequences under
+  // four times their length, 1800 items: 36.9, fetched 43.2; under eight times, 3600 items: 47.1, fetched 45.0).
   const int slots = kFwdCtas * 148;
-  const bool dealt = tiles > 2 && items <= 3 * slots;
+  const int64_t most = (T / kTile + B) * H;          // items that hold a token, at most
+  const bool few = most <= slots * 4 / 3;
+  const bool dealt = items <= slots || (items <= 3 * slots && (tiles > 2 || few)) || (few && T >= (int64_t)2 * kTile * B && items <= 8 * slots);
   CUtensorMap map_qkv, map_rows;
   if (rb_tensor_map_2d(&map_qkv, qkv, T, (int64_t)3 * H * kHead, (int64_t)3 * H * kHead, kHead, kTile, 0) != 0 ||
       rb_tensor_map_2d(&map_rows, qkv, T, (int64_t)3 * H * kHead, (int64_t)3 * H * kHead, kHead, 32, 0) != 0)

@@ -300,3 +300,18 @@ def test_outputs_of_a_sequence_do_not_depend_on_its_batch(repeat, H, bound, spre
         n = min(L, 128)                                               # queries in the bound's one tile
         assert (got[s0:s0 + n] - ref[s0:s0 + n]).norm() / ref[s0:s0 + n].norm() < 1e-2, L
         assert torch.count_nonzero(got[s0 + n:s0 + L]) == 0
+
+
+@pytest.mark.parametrize("lens,H", [([5], 1), ([100], 4), ([64, 1, 128] * 20, 4), ([300, 17], 8), ([1000, 400, 30, 999], 4), ([129, 0, 256] * 40, 2)])
+def test_forward_does_not_depend_on_the_bound(lens, H):
+    """The bound decides how work items are dealt out or fetched, on both sides of one, three and eight rounds of them, and nothing else."""
+    import recis_b200
+    C = recis_b200.native()
+    qkv, offs, _ = _case(lens, H, seed=11)
+    a = C.ragged_attention_fwd(qkv.to(DEV), offs.to(DEV), H, max(lens), 0.125)
+    for factor in (2, 3, 5, 9, 16, 33, 150):
+        b = C.ragged_attention_fwd(qkv.to(DEV), offs.to(DEV), H, factor * max(lens), 0.125)
+        assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1]), factor
+    assert C.dense_status("cuda:0") == 0
+    ref, _ = _oracle(qkv, [n for n in lens if n], H)
+    assert (a[0].float().cpu() - ref).norm() / ref.norm() < 1e-2
