@@ -14,12 +14,12 @@
 // Protocol per reduction step (ring of stages, counted over all tiles; the barriers live at the same shared-memory offsets in both CTAs):
 //   * both producers (warp 0) wait for their own empty[s]; the leader arms ITS full[s] with the bytes of both CTAs;
 //     both issue their loads with the leader's full[s] as the completion barrier (no load is multicast);
-//   * the leader's MMA thread (warp 1) waits for full[s], issues four 256 x 256 x 16 MMAs and commits them to empty[s] of
+//   * the leader's MMA warp (warp 1) waits for full[s], issues four 256 x 256 x 16 MMAs and commits them to empty[s] of
 //     both CTAs (tcgen05.commit with a two-CTA mask), and after a tile's last step to accumulator_full of both CTAs;
 //   * the epilogue warps (2..9) of each CTA drain their own accumulator, two warps per lane quarter with 128 columns each, box by box
 //     (32 rows x 128 bytes): tcgen05.ld, bias / residual / ReLU / mask, conversion, staging in the 128-byte swizzle, TMA store
-//     (add-reduction for a split reduction). A warp has its own small ring of staging slots; a residual or mask box travels into the slot
-//     two boxes ahead. Each warp reports to the leader's accumulator_empty when it has read its part.
+//     (add-reduction for a split reduction). A warp has its own staging slot, or with a residual or mask a ring of three, into which its boxes
+//     travel two boxes ahead. Each warp reports to the leader's accumulator_empty when it has read its part.
 //
 // Every wait is bounded: on a timeout the CTA records kStatusWaitTimeout, gives outstanding copies time to land, joins the cluster
 // barrier, frees its tensor memory and returns.
@@ -59,10 +59,11 @@ constexpr int kThreads = 320;     // producer warp, MMA warp, 8 epilogue warps (
 constexpr uint32_t kHalfBytes = 128 * BK * 2;                   // 16 KB: one operand half of one stage
 constexpr uint32_t kStageBytes = 2 * kHalfBytes;                // this CTA's A half + B half
 constexpr int kGroup = 8;                                       // column tiles per group of the walk
-// Shared memory per CTA: a ring of operand stages and, for each of the eight epilogue warps, a ring of 4 KB staging slots. A second input
-// of the epilogue needs a third slot, so that its boxes can travel two boxes ahead; then a stage less fits.
+// Shared memory per CTA: a ring of operand stages and, for each of the eight epilogue warps, 4 KB staging slots. A second input of the
+// epilogue needs three slots, so that its boxes can travel two boxes ahead; then two stages less fit. (Without one, two slots and five
+// stages: 54.3 instead of 47.1 us at 8192 x 1024 x 3200, and nothing gained where the epilogue is what takes the time.)
 template <bool kSrc> struct Ring {
-  static constexpr int kStages = kSrc ? 4 : 5, kSlots = kSrc ? 3 : 2;
+  static constexpr int kStages = kSrc ? 4 : 6, kSlots = kSrc ? 3 : 1;
   static constexpr uint32_t kBytes = kStages * kStageBytes + 8 * kSlots * 4096 + 1024;
 };
 constexpr uint32_t kPeerMask = 0xFEFFFFFFu;                     // clears the CTA-rank bit of a shared::cluster address: rank 0's copy
@@ -178,11 +179,22 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const _
         if (++s == (uint32_t)kStages) { s = 0; ph ^= 1u; }
       }
     }
-  } else if (warp == 1 && lane == 0 && rank == 0) {
-    // ------------------------------------------------------------------ MMA issuer (leader only)
+  } else if (warp == 1 && rank == 0) {
+    // ------------------------------------------------------------------ MMA issuer (leader only; the whole warp, one lane issues)
+    // One issuer serves the SM pair, so a stage's four MMAs and commit must take less to issue than the 512 cycles they run: elect_one, and
+    // descriptors that advance by adding to the 16-byte address field. (Issued from a branch of lane 0, with descriptors built for each:
+    // 723 instead of 672 us at 8192^3, 143 instead of 130 at 16384 x 2048 x 3200.)
     // instruction descriptor: D = f32, A = B = bf16, majors, N >> 3, M >> 4 with M = 256 (both CTAs' rows)
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((A_MN ? 1u : 0u) << 15) | ((B_MN ? 1u : 0u) << 16) |
                            ((uint32_t)(TN >> 3) << 17) | ((uint32_t)((2 * TM) >> 4) << 24);
+    const uint32_t base = smem_u32(smem);
+    const uint64_t d_a = A_MN ? make_desc(base, BK * 128, 1024) : make_desc(base, 16, 1024);
+    const uint64_t d_b = B_MN ? make_desc(base + kHalfBytes, BK * 128, 1024) : make_desc(base + kHalfBytes, 16, 1024);
+    constexpr uint64_t kStepA = (A_MN ? 2048 : 32) >> 4, kStepB = (B_MN ? 2048 : 32) >> 4;        // 16 reduction elements further
+    const bool leader = elect_one();
+    auto wait_all = [&](uint64_t* bar, uint32_t parity) -> bool {               // one outcome for the whole warp
+      return __all_sync(0xffffffffu, mbar_wait(bar, parity, &abort_flag) ? 1 : 0) != 0;
+    };
     bool ok = true;
     uint32_t s = 0, ph = 0;
     int ti = 0;                                                // tiles since the start
@@ -190,25 +202,25 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const _
       const PairTile tile(t, mt, nt, splits, total_kb, rank);
       if (tile.num_kb == 0) continue;
       const int buf = ti & 1;
-      ok = mbar_wait(&acc_empty[buf], (uint32_t)((ti >> 1) & 1) ^ 1u, &abort_flag);      // the epilogues of tile ti - 2 have read it
+      ok = wait_all(&acc_empty[buf], (uint32_t)((ti >> 1) & 1) ^ 1u);      // the epilogues of tile ti - 2 have read it
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t acc = tmem_base + (uint32_t)(buf * TN);
       for (int kb = 0; kb < tile.num_kb; ++kb) {
-        ok = mbar_wait(&full_bar[s], ph, &abort_flag);
+        ok = wait_all(&full_bar[s], ph);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t sa = smem_u32(smem + s * kStageBytes), sb = sa + kHalfBytes;
+        const uint64_t da = d_a + (uint64_t)(s * (kStageBytes >> 4)), db = d_b + (uint64_t)(s * (kStageBytes >> 4));
+        if (leader) {
 #pragma unroll
-        for (int k = 0; k < BK / UK; ++k) {
-          const uint64_t da = A_MN ? make_desc(sa + k * 2048, BK * 128, 1024) : make_desc(sa + k * 32, 16, 1024);
-          const uint64_t db = B_MN ? make_desc(sb + k * 2048, BK * 128, 1024) : make_desc(sb + k * 32, 16, 1024);
-          umma_bf16_pair(acc, da, db, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          for (int k = 0; k < BK / UK; ++k) umma_bf16_pair(acc, da + k * kStepA, db + k * kStepB, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          umma_commit_pair(&empty_bar[s]);
         }
-        umma_commit_pair(&empty_bar[s]);
+        __syncwarp();
         if (++s == (uint32_t)kStages) { s = 0; ph ^= 1u; }
       }
-      if (ok) umma_commit_pair(&acc_full[buf]);
+      if (ok && leader) umma_commit_pair(&acc_full[buf]);
+      __syncwarp();
       ++ti;
     }
   } else if (warp >= 2) {
@@ -288,7 +300,7 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const _
             fetch_next();
           }
         } else {
-          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");      // the box before the last has left this slot
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");      // the box before this one has left the slot
           __syncwarp();
         }
         const float* bias_at = bias != nullptr && tile.first_split ? bias + col : nullptr;
