@@ -437,3 +437,46 @@ def test_click_loss_leaves_other_losses_and_hooks_alone():
         assert torch.equal(got, fn(logit, label))
     with pytest.raises(ValueError):
         click_loss(mlp, x, torch.ones(5, device=DEV), torch.nn.BCEWithLogitsLoss())
+
+
+@pytest.mark.parametrize("dims", [(24, 35, 100, 5), (16, 1), (7, 300, 201, 3), (64, 188, 191, 12), (480, 1024, 256, 1)])
+@pytest.mark.parametrize("M", [1, 333])
+def test_mlp_with_biases_of_any_width(dims, M):
+    """Biases as large as the sums, in layers of 8 n and of other widths on both sides of 192, against plain torch on the same bf16 values, column by
+    column: a bias that is left out, shifted, or read past its end is off by the size of the output. Each layer rounds to bf16 (2^-9 of an entry),
+    a hidden entry may round the other way (2^-8) and three layers add up: 1e-2. The columns of the padding are zeros."""
+    torch.manual_seed(sum(dims) + M)
+    mlp = D.MLP(list(dims), final_act=False).to(DEV)
+    for layer in mlp.layers:
+        torch.nn.init.normal_(layer.bias)
+    x = torch.randn(M, dims[0], device=DEV)
+    h = x.bfloat16().double()
+    for layer in mlp.layers:
+        h = h @ layer.weight.detach().bfloat16().double().t() + layer.bias.detach().double()
+        h = (torch.relu(h) if layer.act else h).bfloat16().double()
+    y = mlp.forward_padded(x)
+    assert y.shape == (M, D._pad8(dims[-1])) and torch.count_nonzero(y[:, dims[-1]:]) == 0
+    err = (y[:, :dims[-1]].double() - h).norm(dim=0) / h.norm(dim=0).clamp_min(0.1 * M ** 0.5)
+    assert float(err.max()) < 1e-2, err
+    y.backward(torch.ones_like(y))
+    last = mlp.layers[-1].bias.grad
+    assert torch.equal(last, torch.full_like(last, M)) and recis_b200.native().dense_status(DEV) == 0
+
+
+@pytest.mark.parametrize("B", [1, 1000])
+def test_click_logit_matches_plain_torch(B):
+    """Logit and loss of a tower with biases against plain torch from its weights; the last layer's output is rounded to bf16: 2^-8 of it."""
+    torch.manual_seed(B)
+    mlp = D.MLP([24, 16, 1], final_act=False).to(DEV)
+    for layer in mlp.layers:
+        torch.nn.init.normal_(layer.bias, std=3.0)
+    x, extra = torch.randn(B, 24, device=DEV), torch.randn(B, 1, device=DEV)
+    label = (torch.rand(B, 1, device=DEV) < 0.3).float()
+    h = x.bfloat16().double()
+    for layer in mlp.layers:
+        h = h @ layer.weight.detach().bfloat16().double().t() + layer.bias.detach().double()
+        h = torch.relu(h).bfloat16().double() if layer.act else h
+    loss, logit = D.click_loss(mlp, x, label, torch.nn.BCEWithLogitsLoss(), extra)
+    assert float((logit.double() - extra.double() - h).abs().max()) <= 2 ** -7 * float(h.abs().max())
+    want = torch.nn.functional.binary_cross_entropy_with_logits(logit.detach().double(), label.double())
+    assert abs(float(loss.detach()) - float(want)) <= 1e-5 * float(want)
