@@ -385,9 +385,6 @@ ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const _
             st_shared16((prow ^ (uint32_t)(((c >> 3) & 7) << 4)) + (uint32_t)((c >> 6) * kBlk), pk[0], pk[1], pk[2], pk[3]);
           }
           l = fmaf(l, alpha, (sum[0] + sum[2]) + (sum[1] + sum[3]));
-        } else if (g > 0) {                                                   // every warp follows every phase of o_full: the wait behind the last step
-          ok = wait_all(&o_full, (uint32_t)((g - 1) & 1));                    // is for that step's product, not for an older one of the same parity
-          if (!ok) break;
         }
         if (valid & 15) {
           // V rows between the last key and the end of the last 16-key step become zeros, so that the zeros of P never meet a non-finite value
@@ -404,7 +401,11 @@ ragged_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const _
         if (lane == 0) mbar_arrive(&p_full);
       }
       if (!ok) break;
-      // ---- the item's O
+      // ---- the item's O. A warp without rows has not waited for the products before the last one, and where the last but one still runs, this wait
+      // passes on the phase before that, which has the same parity. Such a warp reads nothing of O, and what it then arrives on, o_empty, is the
+      // phase of this item all the same: the second S of an item is multiplied only after the o_empty of the item before is complete, and
+      // the first S of the next item only after this item's last product is issued. The hand-back itself waits for warp 0, which always has
+      // rows. (Following every phase cost 17.0 -> 18.2 us at 590 sequences of 1..40 tokens, 2 heads.)
       ok = wait_all(&o_full, (uint32_t)((g - 1) & 1));
       if (!ok) break;
       fence_after_sync();
