@@ -105,6 +105,224 @@ __device__ __forceinline__ void st_shared16(uint32_t addr, uint32_t a, uint32_t 
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
+// One thread's row of a 128-key tile of S (tensor memory at `trow`): new running maximum and sum, P = 2^(S * scale_log2 - m)
+// written as bf16 into the two K-major blocks of `ptile`. Returns the factor by which what was accumulated under the old
+// maximum shrinks. kMask selects whether key columns >= valid are masked: a full tile pays for no compare or select.
+// The row is read from tensor memory once (four 32-column reads in flight) and stays in registers for both passes; the
+// maximum and the sum run as four independent chains each, since one warp per scheduler hides no dependent latency.
+template <bool kMask>
+__device__ __forceinline__ float softmax_row(uint32_t trow, int valid, float scale_log2, int t, uint8_t* ptile, float& m, float& l) {
+  uint32_t s0[32], s1[32], s2[32], s3[32];
+  __syncwarp();
+  tmem_ld32(trow, s0);
+  tmem_ld32(trow + 32u, s1);
+  tmem_ld32(trow + 64u, s2);
+  tmem_ld32(trow + 96u, s3);
+  tmem_ld_wait();
+  // masking is a select on the value (no branch per element): a masked key becomes -inf here and an exact zero after the
+  // exponential; scale_log2 > 0, so the maximum can be taken before scaling
+  if (kMask) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      if (i >= valid) s0[i] = 0xff800000u;
+      if (32 + i >= valid) s1[i] = 0xff800000u;
+      if (64 + i >= valid) s2[i] = 0xff800000u;
+      if (96 + i >= valid) s3[i] = 0xff800000u;
+    }
+  }
+  float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    mx0 = fmaxf(mx0, __uint_as_float(s0[i]));
+    mx1 = fmaxf(mx1, __uint_as_float(s1[i]));
+    mx2 = fmaxf(mx2, __uint_as_float(s2[i]));
+    mx3 = fmaxf(mx3, __uint_as_float(s3[i]));
+  }
+  const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
+  const float m_new = fmaxf(m, mx * scale_log2);
+  const float alpha = (m == -INFINITY) ? 0.f : fast_exp2(m - m_new);
+  float sum0 = 0.f, sum1 = 0.f, sum2 = 0.f, sum3 = 0.f;
+#pragma unroll
+  for (int q4 = 0; q4 < 4; ++q4) {                 // 32 key columns per quarter; two quarters per 64-wide K-major block
+    uint8_t* blk = ptile + (q4 >> 1) * kBlk;
+    uint32_t pk[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const uint32_t ua = q4 == 0 ? s0[2 * i] : q4 == 1 ? s1[2 * i] : q4 == 2 ? s2[2 * i] : s3[2 * i];
+      const uint32_t ub = q4 == 0 ? s0[2 * i + 1] : q4 == 1 ? s1[2 * i + 1] : q4 == 2 ? s2[2 * i + 1] : s3[2 * i + 1];
+      // -inf * scale_log2 - m_new = -inf (m_new is finite whenever the tile has one existing key): 2^-inf = 0
+      const float p0 = fast_exp2(fmaf(__uint_as_float(ua), scale_log2, -m_new));
+      const float p1 = fast_exp2(fmaf(__uint_as_float(ub), scale_log2, -m_new));
+      if (i & 1) { sum1 += p0; sum3 += p1; } else { sum0 += p0; sum2 += p1; }
+      pk[i] = pack_bf16x2(p0, p1);
+    }
+#pragma unroll
+    for (int cq = 0; cq < 4; ++cq)
+      *reinterpret_cast<uint4*>(blk + swizzle128_offset(t, (q4 & 1) * 32 + cq * 8)) =
+          make_uint4(pk[cq * 4], pk[cq * 4 + 1], pk[cq * 4 + 2], pk[cq * 4 + 3]);
+  }
+  l = l * alpha + ((sum0 + sum1) + (sum2 + sum3));
+  m = m_new;
+  return alpha;
+}
+
+// Small batches: one CTA of 128 threads per work item (blockIdx: query tile, sequence, head), its loads, MMAs and exponentials one after the other,
+// and two to an SM. There is no counter to clear, no work to fetch and one role to wake, which is what a few hundred short items take longest
+// for; with the same steps, sums and roundings as in the persistent kernel below, every output is the same to the bit.
+__global__ void __launch_bounds__(128, 2)
+ragged_attention_fwd_item_kernel(const __grid_constant__ CUtensorMap map_qkv, const int32_t* __restrict__ offsets, int64_t T, int H, float scale_log2,
+                            __nv_bfloat16* __restrict__ out, float* __restrict__ lse2, int64_t* __restrict__ status) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t bar_q, bar_k, bar_v, bar_s, bar_o;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_flag;
+  const int b = blockIdx.y, h = blockIdx.z, qt = blockIdx.x;
+  const int s0 = offsets[b], L = offsets[b + 1] - s0;
+  // Rows that no tile computes read as zeros: tokens in front of and behind the sequences, and those of a sequence that is longer than the
+  // bound the grid was sized with.
+  const bool edge0 = qt == 0 && b == 0 && s0 > 0, edge1 = qt == 0 && b == (int)gridDim.y - 1 && s0 + L < T;
+  const bool edge2 = qt == (int)gridDim.x - 1 && L > (qt + 1) * kTile;
+  if (edge0 || edge1 || edge2) {
+#pragma unroll 1
+    for (int e = 0; e < 3; ++e) {
+      if (!(e == 0 ? edge0 : e == 1 ? edge1 : edge2)) continue;
+      const int64_t from = e == 0 ? 0 : e == 1 ? s0 + L : s0 + (qt + 1) * kTile, to = e == 0 ? (int64_t)s0 : e == 1 ? T : (int64_t)s0 + L;
+#pragma unroll 1
+      for (int64_t row = from + (threadIdx.x >> 3); row < to; row += 16) {
+        reinterpret_cast<uint4*>(out + (row * H + h) * kHead)[threadIdx.x & 7] = make_uint4(0u, 0u, 0u, 0u);
+        if (lse2 && (threadIdx.x & 7) == 0) lse2[row * H + h] = 0.f;
+      }
+    }
+  }
+  if (qt * kTile >= L) return;                                   // uniform for the CTA, before any barrier or allocation
+
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* qtile = smem;                  // [128 q][64 d]      K-major A of S = Q K^T
+  uint8_t* ktile = smem + kBlk;           // [128 keys][64 d]   K-major B of S
+  uint8_t* vtile = smem + 2 * kBlk;       // [128 keys][64 d]   MN-major B of PV (N = d, K = key)
+  uint8_t* ptile = smem + 3 * kBlk;       // 2 x [128 q][64 keys] K-major A of PV
+  const int t = threadIdx.x, warp = t >> 5;
+  // Q, K and V tiles arrive by TMA straight from the packed [T, 3 * H * 64] matrix (box of 128 rows x 64 columns, 128-byte
+  // swizzle). Rows past the end of the sequence belong to the next sequence (or read as zeros past the end of the matrix):
+  // surplus query rows are computed and never stored, surplus keys are masked in the softmax, and the surplus rows of the V
+  // tile are zeroed in shared memory, so that a zero probability never meets a non-finite value.
+  const int xq = h * kHead, xk = (H + h) * kHead, xv = (2 * H + h) * kHead;
+  if (t == 0) {
+    abort_flag = 0;
+    mbar_init(&bar_q, 1); mbar_init(&bar_k, 1); mbar_init(&bar_v, 1); mbar_init(&bar_s, 1); mbar_init(&bar_o, 1);
+    mbar_fence_init();
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_qkv) : "memory");
+    mbar_expect_tx(&bar_q, kBlk); tma_load_2d(qtile, &map_qkv, xq, s0 + qt * kTile, &bar_q);
+    mbar_expect_tx(&bar_k, kBlk); tma_load_2d(ktile, &map_qkv, xk, s0, &bar_k);
+    mbar_expect_tx(&bar_v, kBlk); tma_load_2d(vtile, &map_qkv, xv, s0, &bar_v);
+  }
+  if (warp == 0) tmem_alloc(&tmem_slot, kFwdTmemCols);
+
+  const int q = qt * kTile + t;
+  const bool q_ok = q < L;
+  float o[kHead];
+#pragma unroll
+  for (int d = 0; d < kHead; ++d) o[d] = 0.f;
+  float m = -INFINITY, l = 0.f;
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  const uint32_t tmem = tmem_slot;
+  const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
+  const uint32_t idesc_s = make_idesc_bf16(kTile, kTile, false, false);
+  const uint32_t idesc_o = make_idesc_bf16(kTile, kHead, false, true);
+  bool ok = true;
+
+  const int n_kv = (L + kTile - 1) / kTile;
+  for (int j = 0; j < n_kv && ok; ++j) {
+    const uint32_t ph = (uint32_t)(j & 1);
+    if (t == 0) {
+      bool got = (j > 0 || mbar_wait(&bar_q, 0, &abort_flag)) && mbar_wait(&bar_k, ph, &abort_flag);
+      if (got) {
+        fence_after_sync();
+        const uint32_t sq = smem_u32(qtile), sk = smem_u32(ktile);
+#pragma unroll
+        for (int k = 0; k < kHead / 16; ++k)
+          umma_bf16(tmem, make_desc(sq + k * 32, 16, 1024), make_desc(sk + k * 32, 16, 1024), idesc_s, k > 0 ? 1u : 0u);
+        umma_commit(&bar_s);
+      }
+    }
+    // the outcome of a bounded wait is made uniform for the CTA: every thread takes the same path through the barriers below
+    ok = __syncthreads_and(mbar_wait(&bar_s, ph, &abort_flag) ? 1 : 0) != 0;
+    fence_after_sync();
+    if (!ok) break;
+    // S is complete, so the K tile is free: the next one travels while this tile's softmax and P V run
+    if (t == 0 && j + 1 < n_kv) { mbar_expect_tx(&bar_k, kBlk); tma_load_2d(ktile, &map_qkv, xk, s0 + (j + 1) * kTile, &bar_k); }
+
+    // ---- online softmax on this thread's row of S; only the sequence's last key tile can hold keys that do not exist
+    const int valid = min(kTile, L - j * kTile);                 // key columns of this tile that exist
+    const int steps = (valid + 15) >> 4;                         // 16-key steps of the product with V
+    float alpha = 1.f;
+    if (qt * kTile + warp * 32 >= L) { /* none of this warp's rows exist: what their P holds only reaches rows that are not stored */ }
+    else if (valid == kTile) alpha = softmax_row<false>(tmem + lane_base, kTile, scale_log2, t, ptile, m, l);
+    else alpha = softmax_row<true>(tmem + lane_base, valid, scale_log2, t, ptile, m, l);
+
+    if (valid < kTile) {
+      // last, partial tile: the V rows past the end of the sequence become zeros (this thread's row, once V has landed)
+      ok = mbar_wait(&bar_v, ph, &abort_flag);
+      if (ok && t >= valid && t < steps * 16) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(vtile + swizzle128_offset(t, c * 8)) = make_uint4(0u, 0u, 0u, 0u);
+      }
+    }
+    fence_smem_to_async();
+    fence_before_sync();
+    ok = __syncthreads_and(ok ? 1 : 0) != 0;
+    fence_after_sync();
+    if (!ok) break;
+    if (t == 0) {
+      if (mbar_wait(&bar_v, ph, &abort_flag)) {
+        fence_after_sync();
+        const uint32_t sp = smem_u32(ptile), sv = smem_u32(vtile);
+        for (int k = 0; k < steps; ++k)
+          umma_bf16(tmem + kFwdO, make_desc(sp + (k >> 2) * kBlk + (k & 3) * 32, 16, 1024), make_desc(sv + k * 2048, kBlk, 1024), idesc_o,
+                    k > 0 ? 1u : 0u);
+        umma_commit(&bar_o);
+      }
+    }
+    ok = __syncthreads_and(mbar_wait(&bar_o, ph, &abort_flag) ? 1 : 0) != 0;
+    fence_after_sync();
+    if (!ok) break;
+    // P V is complete, so the V tile is free
+    if (t == 0 && j + 1 < n_kv) { mbar_expect_tx(&bar_v, kBlk); tma_load_2d(vtile, &map_qkv, xv, s0 + (j + 1) * kTile, &bar_v); }
+    {
+      uint32_t r0[32], r1[32];
+      __syncwarp();
+      tmem_ld32(tmem + lane_base + kFwdO, r0);
+      tmem_ld32(tmem + lane_base + kFwdO + 32u, r1);
+      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {           // O = O * alpha + P V, one multiply-add per element
+        o[i] = fmaf(o[i], alpha, __uint_as_float(r0[i]));
+        o[32 + i] = fmaf(o[32 + i], alpha, __uint_as_float(r1[i]));
+      }
+    }
+  }
+
+  if (ok && q_ok) {
+    const float inv = l > 0.f ? 1.f / l : 0.f;
+    __nv_bfloat16* dst = out + (int64_t)(s0 + q) * H * kHead + h * kHead;
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      reinterpret_cast<uint4*>(dst)[c] = make_uint4(pack_bf16x2(o[c * 8] * inv, o[c * 8 + 1] * inv), pack_bf16x2(o[c * 8 + 2] * inv, o[c * 8 + 3] * inv),
+                                                    pack_bf16x2(o[c * 8 + 4] * inv, o[c * 8 + 5] * inv), pack_bf16x2(o[c * 8 + 6] * inv, o[c * 8 + 7] * inv));
+    if (lse2) lse2[(int64_t)(s0 + q) * H + h] = m + log2f(l);
+  }
+  if (abort_flag) {
+    // a wait ran out: a copy may still be on its way into shared memory; give it time before the memory goes away
+    for (int i = 0; i < 64; ++i) __nanosleep(1000);
+  }
+  fence_before_sync();
+  __syncthreads();
+  if (warp == 0) { __syncwarp(); fence_after_sync(); tmem_dealloc(tmem, kFwdTmemCols); }
+  if (t == 0 && abort_flag) rb::set_status(status, rb::kStatusWaitTimeout);
+}
+
 // Rows [from, to) of out and lse become zeros; `threads` threads, this one is `t`.
 __device__ __forceinline__ void clear_rows(int64_t from, int64_t to, int H, __nv_bfloat16* out, float* lse2, int64_t t, int64_t threads) {
   for (int64_t i = from * H * 8 + t; i < to * H * 8; i += threads) {
@@ -1002,32 +1220,42 @@ extern "C" int rb_ragged_attention_fwd(const void* qkv, const int32_t* offsets, 
   const int tiles = (int)(((int64_t)max_len + kTile - 1) / kTile);
   const int64_t items = (int64_t)tiles * B * H;
   if (items > (int64_t)1 << 31) return 1;
-  // Items are dealt out one per CTA, which saves the counter and its clearing, where that is one round of them (a sequence of 100 tokens, 4 heads:
-  // 10.3 us, fetched 12.3; 64 of 1..128 tokens: 14.3, fetched 15.7), and up to three rounds of items of sequences of several tiles (15
-  // sequences of 1..1000 tokens, 4 heads: 28.6 us, fetched 34.4) or of few tokens (64 of 1..128 tokens under a bound of 256: 16.4, fetched
-  // 18.4). 37 sequences of 1..1000 tokens, 1184 items: 59 dealt out, 56 fetched. Under a loose bound most items are empty and cost a fetched
-  // batch less; where the tokens make about one round of items and are long ones, dealing stays ahead up to eight rounds (15 sequences under
-  // four times their length, 1800 items: 36.9, fetched 43.2; under eight times, 3600 items: 47.1, fetched 45.0).
-  const int slots = kFwdCtas * 148;
-  const int64_t most = (T / kTile + B) * H;          // items that hold a token, at most
-  const bool few = most <= slots * 4 / 3;
-  const bool dealt = items <= slots || (items <= 3 * slots && (tiles > 2 || few)) || (few && T >= (int64_t)2 * kTile * B && items <= 8 * slots);
   CUtensorMap map_qkv, map_rows;
   if (rb_tensor_map_2d(&map_qkv, qkv, T, (int64_t)3 * H * kHead, (int64_t)3 * H * kHead, kHead, kTile, 0) != 0 ||
       rb_tensor_map_2d(&map_rows, qkv, T, (int64_t)3 * H * kHead, (int64_t)3 * H * kHead, kHead, 32, 0) != 0)
     return 1;
   static bool attr = false;
   if (!attr) {
-    if (cudaFuncSetAttribute(ragged_attention_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem) != cudaSuccess) return 3;
+    if (cudaFuncSetAttribute(ragged_attention_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem) != cudaSuccess ||
+        cudaFuncSetAttribute(ragged_attention_fwd_item_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem) != cudaSuccess)
+      return 3;
     attr = true;
   }
+  const float scale_log2 = scale * 1.4426950408889634f;
+  const int slots = kFwdCtas * 148;
+  const int64_t most = (T / kTile + B) * H;          // items that hold a token, at most
+  // Sequences of one tile and a half on average or less run on a CTA per item up to three rounds of items with a token and eight rounds of them in
+  // all (100 sequences of 128 tokens, 4 heads: 11.4 us, persistent 14.4; 64 of 1..128 tokens under four times that: 12.6 and 16.5; 590 of
+  // 1..90, one head: 12.9 and 14.5; the other way round 590 of 1..40, 2 heads, 1180 items: 21.3 and 16.8; 200 of 1..100, 2 heads, under eight
+  // times that, 2800 items: 22.5 and 20.5; longer ones: 100 of 1..500, one head: 17.0 and 16.3).
+  if (T <= (int64_t)(kTile * 3 / 2) * B && most <= 3 * slots && items <= 8 * slots) {
+    ragged_attention_fwd_item_kernel<<<dim3(tiles, B, H), 128, kFwdSmem, st>>>(map_qkv, offsets, T, H, scale_log2, reinterpret_cast<__nv_bfloat16*>(out),
+                                                                             lse2, status);
+    rb::note_launch();
+    return cudaGetLastError() == cudaSuccess ? 0 : 4;
+  }
+  // Items are dealt out one per CTA, which saves the counter and its clearing, up to one round of them, three rounds of items of long sequences
+  // (15 sequences of 1..1000 tokens, 4 heads: 28.6 us, fetched 34.4; 37 of them, 1184 items: 59 and 56), and eight rounds where the tokens make
+  // about one: under a loose bound most items are empty, and a fetched batch of them costs less only from there on (15 sequences under four
+  // times their length, 1800 items: 36.9, fetched 43.2; under eight times, 3600 items: 47.1 and 45.0).
+  const bool dealt = items <= slots || (items <= 3 * slots && tiles > 2) || (most <= slots * 4 / 3 && T >= (int64_t)2 * kTile * B && items <= 8 * slots);
   if (dealt) counter = nullptr;
   else if (cudaMemsetAsync(counter, 0, sizeof(unsigned), st) != cudaSuccess) return 4;
   // Items fetched at a time: one where that is about 32 fetches per CTA, more under a loose bound, where most items are empty.
   const int grid = (int)(dealt ? items : std::min<int64_t>(items, slots));
   const int chunk = (int)std::min<int64_t>(32, std::max<int64_t>(1, items / (32 * slots)));
-  ragged_attention_fwd_kernel<<<grid, kFwdThreads, kFwdSmem, st>>>(map_qkv, map_rows, offsets, T, B, H, tiles, chunk, scale * 1.4426950408889634f,
-                                        reinterpret_cast<__nv_bfloat16*>(out), lse2, counter, status);
+  ragged_attention_fwd_kernel<<<grid, kFwdThreads, kFwdSmem, st>>>(map_qkv, map_rows, offsets, T, B, H, tiles, chunk, scale_log2,
+                                                                  reinterpret_cast<__nv_bfloat16*>(out), lse2, counter, status);
   rb::note_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }

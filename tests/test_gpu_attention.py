@@ -304,7 +304,8 @@ def test_outputs_of_a_sequence_do_not_depend_on_its_batch(repeat, H, bound, spre
 
 @pytest.mark.parametrize("lens,H", [([5], 1), ([100], 4), ([64, 1, 128] * 20, 4), ([300, 17], 8), ([1000, 400, 30, 999], 4), ([129, 0, 256] * 40, 2)])
 def test_forward_does_not_depend_on_the_bound(lens, H):
-    """The bound decides how work items are dealt out or fetched, on both sides of one, three and eight rounds of them, and nothing else."""
+    """The bound and the lengths decide which kernel runs and how work items are dealt out or fetched, on both sides of one, three and eight rounds
+    of them, and nothing else."""
     import recis_b200
     C = recis_b200.native()
     qkv, offs, _ = _case(lens, H, seed=11)
@@ -315,3 +316,20 @@ def test_forward_does_not_depend_on_the_bound(lens, H):
     assert C.dense_status("cuda:0") == 0
     ref, _ = _oracle(qkv, [n for n in lens if n], H)
     assert (a[0].float().cpu() - ref).norm() / ref.norm() < 1e-2
+
+
+@pytest.mark.parametrize("lens,H", [([191, 193], 1), ([193, 193], 1), ([128] * 111, 4), ([128] * 112, 4), ([1] * 888, 1), ([1] * 889, 1), ([0, 0, 90, 0], 3)])
+def test_forward_on_both_sides_of_a_cta_per_item(lens, H):
+    """Batches on both sides of the rule for small ones, with tokens in front of and behind the sequences: rows of every sequence against the
+    fp32 computation, rows of none as zeros. Bounds as above."""
+    import recis_b200
+    C = recis_b200.native()
+    qkv, offs, _ = _case(lens, H, seed=12)
+    pad = torch.full((3, 3 * H * 64), float("nan")).to(torch.bfloat16)
+    out, lse = C.ragged_attention_fwd(torch.cat([pad, qkv, pad]).to(DEV), (offs + 3).to(DEV), H, max(lens), 0.125)
+    assert C.dense_status("cuda:0") == 0
+    got = out.float().cpu()
+    for rows in (slice(0, 3), slice(3 + len(qkv), None)):
+        assert torch.count_nonzero(got[rows]) == 0 and torch.count_nonzero(lse[rows]) == 0
+    ref, _ = _oracle(qkv, [n for n in lens if n], H)
+    assert (got[3:3 + len(qkv)] - ref).norm() / ref.norm() < 1e-2
