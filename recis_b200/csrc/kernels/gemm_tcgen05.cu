@@ -552,6 +552,20 @@ int tile_width(int MM, int NN, int splits) {
   return 2 * wide <= 148 && NN > 64 ? 64 : 128;
 }
 
+// Parts of a split reduction on `pairs` tiles of 256 x 256: at least `parts`, and so many that the last round of the 74 pairs of SMs is full.
+// A part costs its reduction steps and about 16 more (filling the ring, the last epilogue). dW 1024 x 2048 of 65536 rows in 4 parts, 128 in
+// all: 204 us, in 9: 194; 1280 x 1280 of 16384 rows in 6 and 8: 66.6 and 58.4. Two parts stay two: their sum does not depend on which comes
+// first, that of more does.
+int64_t whole_rounds(int64_t pairs, int64_t parts, int64_t steps) {
+  int64_t best = parts, best_cost = 0;
+  for (int64_t p = parts; parts > 2 && p <= 4 * parts; ++p) {
+    const int64_t each = (steps + p - 1) / p, in_use = (steps + each - 1) / each;          // (the last parts may be empty)
+    const int64_t cost = (pairs * in_use + 73) / 74 * (each + 16);
+    if (best_cost == 0 || cost < best_cost) { best_cost = cost; best = p; }
+  }
+  return best;
+}
+
 template <bool A_MN, bool B_MN, typename OutT>
 int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const CUtensorMap& ms, int has_src, int tma_out, int BN, void* out,
            const float* bias, const float* beta_src, const RbGemmEpilogue& epi, int MM, int NN, int KK, int ldo, int relu, int splits,
@@ -628,15 +642,17 @@ extern "C" int rb_gemm_bf16_ex(const void* a, int64_t lda, int a_mn, const void*
   if ((reinterpret_cast<uintptr_t>(a) & 15) || (reinterpret_cast<uintptr_t>(b) & 15) || (lda % 8) || (ldb % 8)) return 1;
   // Pairs of SMs on 256 x 256 tiles from more than one round of the 74 pairs on; below that the one-CTA kernel starts and ends faster
   // (8192 x 256 x 512: 13.3 against 15.4 us, equal at 64 tiles, 17.4 against 15.4 at 16384 x 512 x 256). Column sums, which a pair adds up
-  // over its tiles: from half a round on (18500 x 256 x 256: 26.6 against 16.4 us). A split reduction is cut into about 128 parts in all
-  // (two rounds), pairs take it when there is work for 96 of them (dW 512 x 1024 of 8192 rows: 23.6 against 18.4 us; dW 256 x 512 of 8192
-  // rows, 64 parts: 13.3 against 15.3).
+  // over its tiles: from half a round on (18500 x 256 x 256: 26.6 against 16.4 us), and where 32 row tiles add to one column tile
+  // (8192 x 256 x 256: 10.6 against 8.9; 2048 x 1024 x 256: 12.3 against 14.3). A split reduction is cut into about 128 parts in all, pairs take
+  // it when there is work for 96 of them (dW 512 x 1024 of 8192 rows: 23.6 against 18.4 us; dW 256 x 512 of 8192 rows, 64 parts: 13.3
+  // against 15.3).
   const int pmode = pair_mode();
   if (pmode != 0 && MM >= 192 && NN >= 192 && !short_bias) {
     const int64_t pairs = (int64_t)((MM + 255) / 256) * ((NN + 255) / 256), total_kb = (KK + BK - 1) / BK;
     const int64_t psplits = splits > 1 ? std::max<int64_t>(1, std::min((128 + pairs - 1) / pairs, total_kb / 4)) : 1;
-    if (pmode == 1 || (splits > 1 ? pairs * psplits >= 96 : pairs > (epi.colsum != nullptr ? 37 : 74))) {
-      const int rc = rb_gemm_bf16_pair(a, lda, a_mn, b, ldb, b_mn, out, ldo, out_fp32, bias, beta_src, &epi, MM, NN, KK, relu, (int)psplits,
+    const bool narrow = epi.colsum != nullptr && MM >= 32 * 256;
+    if (pmode == 1 || (splits > 1 ? pairs * psplits >= 96 : pairs > (epi.colsum != nullptr ? 37 : 74) || narrow)) {
+      const int rc = rb_gemm_bf16_pair(a, lda, a_mn, b, ldb, b_mn, out, ldo, out_fp32, bias, beta_src, &epi, MM, NN, KK, relu, (int)whole_rounds(pairs, psplits, total_kb),
                                        splits > 1, status, st);
       if (rc != 7) return rc;
     }

@@ -94,3 +94,29 @@ def test_gemm_epilogues_over_several_rounds_of_tiles(M, N, K, odd):
     assert rel(dx, ref * keep) < 4e-3 and float(dx[keep == 0].float().abs().max()) == 0.0
     assert rel(db, (ref * keep).sum(0)) < 1e-4
     assert C.dense_status(DEV) == 0
+
+
+@pytest.mark.parametrize("N,K,M", [(1280, 1280, 16392), (1024, 1024, 8200), (2304, 768, 20000), (256, 512, 40008), (2048, 3200, 4104), (200, 264, 65544)])
+def test_split_reductions_in_parts_of_any_length(N, K, M):
+    """dW = dy^T x over many rows, cut into parts that fill whole rounds of SMs, with a last part that is shorter or empty, added to the output:
+    against fp64 on the same bf16 values; sums of M products in fp32 in any order: 1e-5 by norm."""
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    dy, x = (torch.randn(M, n, generator=g, device=DEV).bfloat16() for n in (N, K))
+    out = C.gemm_bf16(dy, x, None, False, True, True, True, None)
+    ref = sum(a.double().t() @ b.double() for a, b in zip(dy.split(8192), x.split(8192)))
+    assert float((out.double() - ref).norm() / ref.norm()) < 1e-5
+    C.gemm_bf16(dy, x, None, False, True, True, True, out)                 # on top of itself
+    assert float((out.double() - 2 * ref).norm() / (2 * ref).norm()) < 1e-5
+    assert C.dense_status(DEV) == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(8191, 256, 256), (8192, 192, 64), (8200, 256, 72), (9001, 200, 264)])
+def test_column_sums_of_one_column_tile(M, N, K):
+    """Column sums on both sides of the rows from which a pair of SMs adds them up over its tiles; bounds as for the masked shapes above."""
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    dy, w = torch.randn(M, K, generator=g, device=DEV).bfloat16(), (torch.randn(K, N, generator=g, device=DEV) * 0.1).bfloat16()
+    y = torch.randn(M, N, generator=g, device=DEV).bfloat16()
+    dx, db = C.gemm_dgrad_fused(dy, w, y)
+    ref = (dy.double() @ w.double()) * (y > 0)
+    assert float((dx.double() - ref).norm() / ref.norm()) < 4e-3 and float((db.double() - ref.sum(0)).norm() / ref.sum(0).norm()) < 1e-4
+    assert C.dense_status(DEV) == 0
