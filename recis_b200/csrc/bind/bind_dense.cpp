@@ -288,11 +288,14 @@ std::tuple<Tensor, Tensor> gemm_dgrad_fused(const Tensor& dy, const Tensor& w, O
   auto db = db_out.has_value() && db_out->defined() ? *db_out : torch::zeros({NN}, dy.options().dtype(torch::kFloat32));
   TORCH_CHECK(db.scalar_type() == torch::kFloat32 && db.is_contiguous() && db.numel() == NN, "db_out: contiguous fp32 [K]");
   RbGemmEpilogue epi{nullptr, 0, db.data_ptr<float>(), 0};
+  Tensor m;
   if (mask.has_value() && mask->defined()) {
     TORCH_CHECK(mask->scalar_type() == torch::kBFloat16 && mask->dim() == 2 && mask->stride(1) == 1 && mask->size(0) == MM && mask->size(1) == NN,
                 "mask: bf16 [M, K]");
-    epi.mask_src = mask->data_ptr();
-    epi.mask_ld = mask->stride(0);
+    // off a 16-byte line, rows or the whole, the kernel would read it element by element instead of as boxes (as for a residual below)
+    m = NN % 8 == 0 ? aligned16(mask->stride(0) % 8 ? mask->contiguous() : *mask) : *mask;
+    epi.mask_src = m.data_ptr();
+    epi.mask_ld = m.stride(0);
   }
   Tensor& st = status_word(dy.device());
   const int rc = rb_gemm_bf16_ex(dy.data_ptr(), dy.stride(0), 0, w.data_ptr(), w.stride(0), 1, out.data_ptr(), out.stride(0), 0, nullptr, nullptr,
@@ -357,6 +360,9 @@ Tensor gemm_bf16_residual(const Tensor& a, const Tensor& b, OptT bias, const Ten
               residual.size(1) == NN, "residual: contiguous fp32 [M, N]");
   c10::cuda::CUDAGuard g(a.device());
   auto out = torch::empty({MM, NN}, a.options().dtype(torch::kFloat32));
+  // A residual off a 16-byte line is copied: only as boxes does it travel beside the main loop, and the copy is less than what reading it row by
+  // row costs (65536 x 1024 x 256: 416 -> 191 us, aligned 107; 64 x 256 x 256: 18.5 -> 15.4, aligned 10.2).
+  const Tensor res = NN % 4 == 0 ? aligned16(residual) : residual;
   const float* bp = nullptr;
   Tensor bias_f;
   if (bias.has_value() && bias->defined()) {
@@ -366,7 +372,7 @@ Tensor gemm_bf16_residual(const Tensor& a, const Tensor& b, OptT bias, const Ten
   }
   Tensor& st = status_word(a.device());
   const int rc = rb_gemm_bf16(a.data_ptr(), a.stride(0), 0, b.data_ptr(), b.stride(0), 0, out.data_ptr(), out.stride(0), 1, bp,
-                              residual.data_ptr<float>(), (int)MM, (int)NN, (int)KK, 0, 1, st.data_ptr<int64_t>(),
+                              res.data_ptr<float>(), (int)MM, (int)NN, (int)KK, 0, 1, st.data_ptr<int64_t>(),
                               at::cuda::getCurrentCUDAStream());
   TORCH_CHECK(rc == 0, "rb_gemm_bf16 failed with code ", rc);
   return out;

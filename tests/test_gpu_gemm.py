@@ -120,3 +120,20 @@ def test_column_sums_of_one_column_tile(M, N, K):
     ref = (dy.double() @ w.double()) * (y > 0)
     assert float((dx.double() - ref).norm() / ref.norm()) < 4e-3 and float((db.double() - ref.sum(0)).norm() / ref.sum(0).norm()) < 1e-4
     assert C.dense_status(DEV) == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(333, 201, 72), (20001, 203, 264), (1000, 1030, 128)])
+def test_epilogues_of_outputs_that_no_map_takes(M, N, K):
+    """Residual, mask and column sums of outputs whose rows start off a 16-byte line: read and written row by row. Bounds as above."""
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    rn = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    x, w, bias, res, mask = rn(M, K).bfloat16(), (rn(N, K) * 0.1).bfloat16(), rn(N), rn(M, N), rn(M, N).bfloat16()
+    wt = torch.zeros(K, (N + 7) // 8 * 8, device=DEV).bfloat16()
+    wt[:, :N] = w.t()
+    ref = x.double() @ w.double().t()
+    rel = lambda a, b: float((a.double() - b).norm() / b.norm())
+    assert rel(C.gemm_bf16_residual(x, w, bias, res), ref + bias + res) < 1e-4
+    dx, db = C.gemm_dgrad_fused(x, wt[:, :N], mask)
+    ref = ref * (mask > 0)
+    assert rel(dx, ref) < 4e-3 and rel(db, ref.sum(0)) < 1e-4 and torch.count_nonzero(dx[mask <= 0]) == 0
+    assert C.dense_status(DEV) == 0
