@@ -534,7 +534,7 @@ void init_dense(py::module& m) {
     auto out = torch::empty({T, H * 64}, qkv.options());                         // the kernel writes every row
     auto lse_buf = torch::empty({T * H + 1}, qkv.options().dtype(torch::kFloat32));     // and the kernel's work counter behind it
     auto lse = lse_buf.narrow(0, 0, T * H).view({T, H});
-    const int rc = rb_ragged_attention_fwd(qkv.data_ptr(), offsets.data_ptr<int32_t>(), T, (int)B, (int)H, (int)max_len, (float)scale,
+    const int rc = rb_ragged_attention_fwd(qkv.data_ptr(), offsets.data_ptr<int32_t>(), T, (int)B, (int)H, (int)std::min<int64_t>(max_len, INT32_MAX), (float)scale,
                                            out.data_ptr(), lse.data_ptr<float>(), reinterpret_cast<unsigned*>(lse_buf.data_ptr<float>() + T * H),
                                            status_word(qkv.device()).data_ptr<int64_t>(),
                                            at::cuda::getCurrentCUDAStream());
@@ -557,7 +557,7 @@ void init_dense(py::module& m) {
     Tensor dq_acc;
     if (max_len > 128) dq_acc = torch::zeros({T, H * 64}, f32);
     const int rc = rb_ragged_attention_bwd(qkv.data_ptr(), out.data_ptr(), d_out.data_ptr(), lse.data_ptr<float>(), scratch.data_ptr<float>(),
-                                           offsets.data_ptr<int32_t>(), T, (int)B, (int)H, (int)max_len, (float)scale,
+                                           offsets.data_ptr<int32_t>(), T, (int)B, (int)H, (int)std::min<int64_t>(max_len, INT32_MAX), (float)scale,
                                            dq_acc.defined() ? dq_acc.data_ptr<float>() : nullptr, dqkv.data_ptr(),
                                            status_word(qkv.device()).data_ptr<int64_t>(), at::cuda::getCurrentCUDAStream());
     TORCH_CHECK(rc == 0, "ragged_attention_bwd failed (code ", rc, ")");

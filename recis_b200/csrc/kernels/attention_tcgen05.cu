@@ -1217,9 +1217,10 @@ extern "C" int rb_ragged_attention_fwd(const void* qkv, const int32_t* offsets, 
                                        float* lse2, unsigned* counter, int64_t* status, cudaStream_t st) {
   if (B <= 0 || H <= 0 || max_len <= 0 || T <= 0) return 0;
   if ((reinterpret_cast<uintptr_t>(qkv) & 15) || (reinterpret_cast<uintptr_t>(out) & 15)) return 1;
-  const int tiles = (int)(((int64_t)max_len + kTile - 1) / kTile);
+  int tiles = (int)(((int64_t)max_len + kTile - 1) / kTile);
+  if ((int64_t)tiles * B * H > (int64_t)1 << 31) return 1;
+  tiles = (int)std::min<int64_t>(tiles, (T + kTile - 1) / kTile);      // no sequence is longer: row numbers of the last tile stay in 32 bits
   const int64_t items = (int64_t)tiles * B * H;
-  if (items > (int64_t)1 << 31) return 1;
   CUtensorMap map_qkv, map_rows;
   if (rb_tensor_map_2d(&map_qkv, qkv, T, (int64_t)3 * H * kHead, (int64_t)3 * H * kHead, kHead, kTile, 0) != 0 ||
       rb_tensor_map_2d(&map_rows, qkv, T, (int64_t)3 * H * kHead, (int64_t)3 * H * kHead, kHead, 32, 0) != 0)
@@ -1271,9 +1272,10 @@ extern "C" int rb_ragged_attention_bwd(const void* qkv, const void* out, const v
   if ((reinterpret_cast<uintptr_t>(qkv) & 15) || (reinterpret_cast<uintptr_t>(d_out) & 15) || (reinterpret_cast<uintptr_t>(dqkv) & 15) ||
       (reinterpret_cast<uintptr_t>(out) & 15) || (!single && (dq_acc == nullptr || (reinterpret_cast<uintptr_t>(dq_acc) & 15))))
     return 1;
-  const int tiles = (max_len + kTile - 1) / kTile;
+  int tiles = (int)(((int64_t)max_len + kTile - 1) / kTile);
+  if ((int64_t)tiles * B * H > (int64_t)1 << 30) return 1;
+  tiles = (int)std::min<int64_t>(tiles, (T + kTile - 1) / kTile);      // as in the forward
   const int64_t items = (int64_t)tiles * B * H;
-  if (items > (int64_t)1 << 30) return 1;
   const size_t smem = 1024 + 14 * (size_t)kBlk;
   CUtensorMap map_qkv, map_do, map_dq;
   if (rb_tensor_map_2d(&map_qkv, qkv, T, (int64_t)3 * H * kHead, (int64_t)3 * H * kHead, kHead, kTile, 0) != 0 ||

@@ -333,3 +333,17 @@ def test_forward_on_both_sides_of_a_cta_per_item(lens, H):
         assert torch.count_nonzero(got[rows]) == 0 and torch.count_nonzero(lse[rows]) == 0
     ref, _ = _oracle(qkv, [n for n in lens if n], H)
     assert (got[3:3 + len(qkv)] - ref).norm() / ref.norm() < 1e-2
+
+
+@pytest.mark.parametrize("bound", [2**31 - 128, 2**31 - 1, 2**33])
+def test_bounds_at_the_end_of_32_bits(bound):
+    """A bound that says "any length": the row numbers behind its last tile do not fit in 32 bits. Outputs and gradients are those of the tight one."""
+    import recis_b200
+    C = recis_b200.native()
+    lens, H = [200, 3, 128], 2
+    qkv, offs, d_out = (t.to(DEV) for t in _case(lens, H, seed=13))
+    want = C.ragged_attention_fwd(qkv, offs, H, 256, 0.125)
+    got = C.ragged_attention_fwd(qkv, offs, H, bound, 0.125)
+    assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])
+    a, b = (C.ragged_attention_bwd(qkv, got[0], d_out, got[1], offs, H, n, 0.125) for n in (256, bound))
+    assert (a.float() - b.float()).norm() <= 1e-2 * a.float().norm() and C.dense_status("cuda:0") == 0
