@@ -17,12 +17,12 @@
 // under P V. Keys past the end of a sequence are masked in the softmax; query rows past the end are computed on whatever is there and not
 // stored; of a partial tile only the 32-row boxes that hold a row are loaded.
 //
-// What bounds it is the latency of a step - score, exponentials, product, in sequence for a query tile - with two query
-// tiles to an SM (tensor memory holds no more); the exponentials take two fifths of the special-function units' cycles. Measured on a B200
-// (before: one CTA of 128 threads per item, loads, MMAs and exponentials one after the other, P through shared memory, O in registers):
-//   256 sequences of 50..1000 tokens, 4 heads:  290 -> 225 us (83 GFLOP in existing elements: 367 TFLOP/s)
-//   3000 sequences of 1..90 tokens, 8 heads:    423 -> 235 us; under a bound of 360 instead of 90: 623 -> 240 us
-//   37 sequences of 1..1000 tokens, 4 heads:     55 -> 51 us;  one sequence of 1000 tokens, 8 heads: 27 -> 24.6 us
+// What bounds it is the latency of a step - score, exponentials, product, in sequence for a query tile - with two query tiles to an SM (tensor
+// memory holds no more): no unit is near its limit (first case below: tensor pipe 21 %, special-function units 40 %, issue slots 38 %).
+// Measured on a B200 with cold L2 (before: the kernel with a CTA per item below, which small batches still use):
+//   256 sequences of 50..1000 tokens, 4 heads:  311 -> 235 us (93 GFLOP in existing elements: 395 TFLOP/s)
+//   3000 sequences of 1..90 tokens, 8 heads:    425 -> 230 us; under a bound of 1000 instead of 90: 1319 -> 235 us
+//   37 sequences of 1..1000 tokens, 4 heads:     58 -> 57 us;  one sequence of 1000 tokens, 8 heads: 27 -> 24.6 us
 //
 // The reference has no attention kernel; its sequence example pads to the longest sequence and calls the library SDPA
 // (examples/seq2seq/transformer.py:36-38). Waits are bounded; a timeout sets the status word and the CTA frees its tensor
@@ -735,8 +735,9 @@ attention_dq_store_kernel(const float* __restrict__ dq_acc, int64_t T, int cols,
 // One persistent CTA per SM with separate roles: warps 0..7 compute (two threads per query row, each with two of the four chunks of 32
 // key columns), warp 8 fetches work and issues the TMA loads, warp 9 issues the MMAs. Work items come from a counter, so that sequences of very different length balance; K / V and Q / dO are double buffered across items, so the loads of the
 // next item run under this one. The S and dP of step g + 1 are multiplied as soon as step g has them in registers, and the three
-// products of step g - 1 run while step g computes its exponentials. What shared memory has to move per step bounds it: 208 KB of
-// operand reads for the MMAs, 64 KB of P and dS, 32 KB of arriving tiles, 64 KB for dQ on its way out.
+// products of step g - 1 run while step g computes its exponentials. No unit is near its limit (256 sequences of 50..1000 tokens, 4 heads:
+// tensor pipe 26 %, L1 and shared memory 33 %, special-function units 19 %, issue slots 36 %): what bounds it is the chain load -> S, dP ->
+// exponentials -> products -> results of a step, with eight compute warps on an SM to cover it.
 // Parts of a tile that lie outside the sequence cost nothing: chunks of columns and warps of rows without an existing element are
 // neither computed nor written, and the reductions stop at the last 16 rows that hold one. (Left-over values in unwritten parts only
 // reach rows of the results that are not stored.)
@@ -750,17 +751,18 @@ attention_dq_store_kernel(const float* __restrict__ dq_acc, int64_t T, int cols,
 // `tiles` below); the others get a zero dQ. With kSingle that is query tile 0 with one key tile after the other, whose dQ add up in
 // tensor memory until the last of them.
 //
-// Measured on a B200 (this kernel alone; before: one CTA of 128 threads per item, loads / MMAs / exponentials one after the other):
-//   256 sequences of 50..1000 tokens, 4 heads:  807 -> 523 us (231 GFLOP in existing elements: 440 TFLOP/s)
-//   3000 sequences of 1..90 tokens, 8 heads:   1288 -> 407 us (2.2 GFLOP, 0.84 GB read and written: 2.1 TB/s; fixed cost per item)
+// Measured on a B200 with cold L2 (this kernel alone; before: one CTA of 128 threads per item, loads / MMAs / exponentials one after the other; in
+// brackets with the MMAs issued from a branch of one lane):
+//   256 sequences of 50..1000 tokens, 4 heads:  807 -> 489 us (528; 232 GFLOP in existing elements: 475 TFLOP/s)
+//   3000 sequences of 1..90 tokens, 8 heads:   1288 -> 385 us (405; 0.84 GB read and written: 2.2 TB/s; fixed cost per item)
 // and no zeroed fp32 gradient of q, k and v (413 MB resp. 826 MB of it) nor its conversion to bf16 around it any more.
 constexpr uint32_t kColS = 0, kColDP = 128, kColDV = 256, kColDK = 320, kColDQ = 384;
 constexpr int kBwdCompute = 8;                       // compute warps
 constexpr int kBwdThreads = (kBwdCompute + 4) * 32;  // and one warpgroup of control warps, two of them idle (register split below)
 // Work items fetched at a time: four where an item is one step and a fetch would not hide behind it, one where items are up to many steps
-// long and a group of four made some SMs finish a sixth later than the rest (256 sequences of 50..1000 tokens: 585 -> 523 us). Which of the
-// two is chosen by the caller's bound, the only thing the host knows. Under a loose bound most items are empty and a single fetch costs more
-// (3000 sequences of 1..90 tokens, 8 heads: 0.46 ms under a bound of 90, 1.39 ms under 1000).
+// long and a group of four made some SMs finish a sixth later than the rest (256 sequences of 50..1000 tokens, before the MMA warp ran converged:
+// 585 -> 523 us). Which of the two is chosen by the caller's bound. Under a loose bound most items are empty and a single fetch costs more
+// (3000 sequences of 1..90 tokens, 8 heads: 385 us under a bound of 90, 1191 under 1000).
 constexpr int kBwdChunkShort = 4, kBwdChunkLong = 1;
 
 // N key columns of one query row: pk = bf16 pairs of P, dk = bf16 pairs of dS. kMask: columns >= valid give exact zeros (S and dP
@@ -1070,7 +1072,7 @@ ragged_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_qkv, const _
     };
     // One flat loop over the steps of all items, so that every part of the body exists once: with one step per item each part runs
     // once per item on eight warps, and fetching instructions was what bounded the kernel while the body was spelt out (the largest
-    // stall reason by far; 610 us against 407 us at 3000 sequences of up to 90 tokens x 8 heads).
+    // stall reason by far; 610 us against the 407 of then at 3000 sequences of up to 90 tokens x 8 heads).
     AttnItem item{0, 0, 0, 0};
     int it = 0, g = 0, i = 0, n_q = 0, valid_k = 0;
     float lse_next = 0.f, delta_next = 0.f;                                   // this row's lse and delta, fetched one step ahead

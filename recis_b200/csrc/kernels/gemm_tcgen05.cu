@@ -546,7 +546,9 @@ int launch_one(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& 
   return cudaGetLastError() == cudaSuccess ? 0 : 4;
 }
 
-// Width of the column tiles: 64 where 128-wide ones would leave half of the SMs without work.
+// Width of the column tiles: 64 where 128-wide ones would leave half of the SMs without work: a tile's MMAs and its epilogue take less
+// (64 x 256 x 256, bias + ReLU: 4.9 against 5.6 us; 512 x 256 x 1024: 8.8 and 9.6; 4096 x 256 x 3200, 64 wide tiles: 21.1 and 21.1; with a
+// residual 5.8 and 7.1, 9.9 and 11.4, 22.0 and 22.9).
 int tile_width(int MM, int NN, int splits) {
   const int64_t wide = (int64_t)((NN + 127) / 128) * ((MM + BM - 1) / BM) * splits;
   return 2 * wide <= 148 && NN > 64 ? 64 : 128;
@@ -570,6 +572,8 @@ template <bool A_MN, bool B_MN, typename OutT>
 int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const CUtensorMap& ms, int has_src, int tma_out, int BN, void* out,
            const float* bias, const float* beta_src, const RbGemmEpilogue& epi, int MM, int NN, int KK, int ldo, int relu, int splits,
            int64_t* status, cudaStream_t st) {
+  // six stages as long as every CTA has an SM to itself (4096 x 128 x 3200: 20.8 us, with three 22.5; 8192 x 256 x 3200: 22.5 and 23.9; no
+  // difference up to 256 reduction elements)
   const int64_t ctas = (int64_t)((NN + BN - 1) / BN) * ((MM + BM - 1) / BM) * splits;
   auto go = !tma_out     ? launch_one<A_MN, B_MN, OutT, false, 128, 3>
             : ctas > 148 ? launch_one<A_MN, B_MN, OutT, true, 128, 3>
@@ -641,7 +645,8 @@ extern "C" int rb_gemm_bf16_ex(const void* a, int64_t lda, int a_mn, const void*
   // TMA constraints: 16-byte aligned base, row pitch a multiple of 16 bytes
   if ((reinterpret_cast<uintptr_t>(a) & 15) || (reinterpret_cast<uintptr_t>(b) & 15) || (lda % 8) || (ldb % 8)) return 1;
   // Pairs of SMs on 256 x 256 tiles from more than one round of the 74 pairs on; below that the one-CTA kernel starts and ends faster
-  // (8192 x 256 x 512: 13.3 against 15.4 us, equal at 64 tiles, 17.4 against 15.4 at 16384 x 512 x 256). Column sums, which a pair adds up
+  // (bias + ReLU, 256, 1024 and 3200 reduction elements, us: 32 tiles 6.1, 10.6, 21.9 against 7.5, 11.8, 21.5 on pairs; 64 tiles 7.3, 13.4, 29.7
+  // and 7.8, 13.2, 25.9; 75 tiles 10.8, 21.2, 49.8 and 9.6, 17.1, 37.3; 96 tiles 11.5, 22.4, 50.9 and 9.8, 18.0, 40.1). Column sums, which a pair adds up
   // over its tiles: from half a round on (18500 x 256 x 256: 26.6 against 16.4 us), and where 32 row tiles add to one column tile
   // (8192 x 256 x 256: 10.6 against 8.9; 2048 x 1024 x 256: 12.3 against 14.3). A split reduction is cut into about 128 parts in all, pairs take
   // it when there is work for 96 of them (dW 512 x 1024 of 8192 rows: 23.6 against 18.4 us; dW 256 x 512 of 8192 rows, 64 parts: 13.3

@@ -27,10 +27,13 @@
 // Operands may be K-major or MN-major as in the one-CTA kernel.
 //
 // Measured on a B200 (L2 cold; before: one tile per CTA, two CTAs to an SM, a row per lane and conditions per element in the epilogue):
-//   269000 x 1024 x 256, bias + ReLU, bf16 out:   321 -> 141 us (its 551 MB of output alone take 145 us to fill)
-//   the same with mask and column sums:           497 -> 249 us (1.24 GB: 5.0 TB/s)
-//   269000 x 256 x 1024, fp32 residual in / out:  332 -> 180 us (1.1 GB: 6.1 TB/s)
-//   16384 x 2048 x 3200, bias + ReLU:             172 -> 143 us (1.50 PFLOP/s)
+//   269000 x 1024 x 256, bias + ReLU, bf16 out:   325 -> 141 us (its 551 MB of output alone take 145 us to fill)
+//   the same with mask and column sums:           510 -> 246 us (1.24 GB: 5.0 TB/s)
+//   269000 x 256 x 1024, fp32 residual in / out:  343 -> 186 us (1.1 GB: 5.9 TB/s)
+//   16384 x 2048 x 3200, bias + ReLU:             174 -> 131 us (1.64 PFLOP/s; the tensor pipe is busy 95 % of the cycles)
+//   dW 2048 x 3200 of 16384 rows:                 178 -> 186 us (104 tiles of the whole reduction are two rounds however they are dealt)
+// Tiles are dealt out before the start. Where a kernel of another stream holds SMs, as the exchange of a step on several GPUs may, a pair that
+// starts late still has its whole share; what that costs has not been measured.
 // What bounded the short reductions was the epilogue: first its instructions (finish_box), then the arrival on the leader's
 // accumulator_empty, which with release semantics at cluster scope waited for the warp's stores (206 -> 141 us in the first case).
 //

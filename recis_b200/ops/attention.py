@@ -4,8 +4,9 @@
 (q | k | v) of a batch of sequences stored back to back and returns ``[total_tokens, hidden]``.
 
 Two implementations:
-* the tensor-core kernels (``csrc/kernels/attention_tcgen05.cu``): no padding, head width 64; forward with one CTA per (sequence, head,
-  128-row tile), backward with one persistent CTA per SM: what CUDA training uses;
+* the tensor-core kernels (``csrc/kernels/attention_tcgen05.cu``): no padding, head width 64; forward with two persistent CTAs per SM, small
+  batches with one CTA per (sequence, head, 128-row tile) and the same outputs to the bit, backward with one persistent CTA per SM: what
+  CUDA training uses;
 * the padded path: scatter into ``[batch, max_len, heads, head_dim]``, ``F.scaled_dot_product_attention`` with a key-padding
   mask, gather the valid positions back. Differentiable; other head widths, CPU tensors, ``RECIS_ATTENTION=padded``.
 """

@@ -76,8 +76,8 @@ def test_dgrad_with_relu_mask_and_bias_gradient_in_the_epilogue(M, N, K, masked)
 @pytest.mark.parametrize("odd", [False, True])
 def test_gemm_epilogues_over_several_rounds_of_tiles(M, N, K, odd):
     """Bias + ReLU, residual and mask + column sums where a pair of SMs walks several tiles (ten column tiles included) and where one
-    CTA has one tile, with rows and columns that end inside a box. ``odd``: a bias off its 8-byte line, a residual and a mask that no TMA
-    map takes. Bounds: bf16 rounding 2^-9 per entry of bf16 outputs, accumulation order in fp32 ones (as above)."""
+    CTA has one tile, with rows and columns that end inside a box. ``odd``: a bias off its 8-byte line, a residual and a mask off their
+    16-byte lines, which the bindings copy to one. Bounds: bf16 rounding 2^-9 per entry of bf16 outputs, accumulation order in fp32 ones (as above)."""
     g = torch.Generator(device=DEV).manual_seed(M + N + K)
     rn = lambda *s: torch.randn(*s, generator=g, device=DEV)
     x, w = rn(M, K).bfloat16(), (rn(N, K) * 0.1).bfloat16()
